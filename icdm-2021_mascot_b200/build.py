@@ -19,7 +19,7 @@ BIN = os.path.join(HERE, "bin")
 NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 
-LIB_SOURCES = ["mascot_api.cu", "setup.cu", "shard.cu", "train_kernels.cu", "eval_kernels.cu", "prep_kernels.cu", "probe.cu"]
+LIB_SOURCES = ["mascot_api.cu", "setup.cu", "shard.cu", "train_kernels.cu", "eval_kernels.cu", "prep_kernels.cu", "host_copy.cu", "device_pool.cu", "probe.cu"]
 CLI_SOURCES = {"quantized_mf": "quantized_mf.cpp", "test_mf": "test_mf.cpp", "convert_ratings": "convert_ratings.cpp"}
 
 
@@ -49,7 +49,7 @@ def build_library(force=False, verbose=True, ptxas_verbose=False):
             cmd = ["nvcc"] + NVCC_FLAGS + (["-Xptxas", "-v"] if ptxas_verbose else []) + ["-c", s, "-o", o]
             _run(cmd, verbose)
         objs.append(o)
-    _run(["nvcc", "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB] + objs + ["-lcudart", "-ldl"], verbose)
+    _run(["nvcc", "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB] + objs + ["-lcudart", "-ldl", "-lpthread"], verbose)
     return LIB
 
 

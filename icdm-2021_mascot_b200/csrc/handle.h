@@ -3,6 +3,7 @@
 #pragma once
 #include <cstdio>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -83,6 +84,7 @@ struct mascot_handle {
     mascot_timings timings = {};         // accumulated phase times (mascot_get_timings)
     bool l2_window_set = false;          // a persisting access-policy window is installed on `stream`
     size_t l2_limit_before = 0;          // the process's persisting-L2 limit before this engine changed it
+    std::unordered_map<const void*, size_t> reserved;   // bytes behind each buffer of reserve()
 };
 
 namespace mascot {
@@ -105,13 +107,32 @@ int fail(mascot_handle* h, int code, const std::string& msg);
 // Host clock in microseconds (phases that end with a synchronisation are timed with it).
 double now_us();
 
+// ---- device_pool.cu: device memory of engines and of handle-free calls, in the order of a stream ----
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);    // from the current device's pool
+void pool_free(void* p, cudaStream_t st);
+void pool_trim();                                                  // gives the current device's idle pool memory back
+
 template <typename T>
-cudaError_t dev_alloc(T** p, size_t count) {
-    return cudaMalloc(reinterpret_cast<void**>(p), sizeof(T) * (count ? count : 1));
+cudaError_t dev_alloc(T** p, size_t count, cudaStream_t st) {
+    return pool_alloc(reinterpret_cast<void**>(p), sizeof(T) * (count ? count : 1), st);
 }
 
 template <typename T>
-void dev_free(T*& p) { if (p) { cudaFree(p); p = nullptr; } }
+void dev_free(T*& p, cudaStream_t st) { if (p) { pool_free(p, st); p = nullptr; } }
+
+// Room for `count` elements behind a buffer of the engine, contents undefined.  A buffer that is large enough stays:
+// an engine that is given new ratings of about the same size maps no memory at all.  One that is far too large goes.
+template <typename T>
+cudaError_t reserve(mascot_handle* h, T** p, size_t count) {
+    const size_t bytes = sizeof(T) * (count ? count : 1);
+    size_t& have = h->reserved[p];
+    if (*p && have >= bytes && (have <= 4 * bytes || have < (256u << 20))) return cudaSuccess;
+    dev_free(*p, h->stream);
+    have = 0;
+    const cudaError_t e = pool_alloc(reinterpret_cast<void**>(p), bytes, h->stream);
+    if (e == cudaSuccess) have = bytes;
+    return e;
+}
 
 // ---- mascot_api.cu ----
 void free_ratings(mascot_handle* h);

@@ -18,6 +18,7 @@
 
 #include "../../include/mascot.h"
 #include "handle.h"
+#include "host_copy.h"
 
 using namespace mascot;
 
@@ -82,11 +83,11 @@ int mascot::fail(mascot_handle* h, int code, const std::string& msg) {
 namespace mascot {
 
 void free_ratings(mascot_handle* h) {
-    dev_free(h->tr_r); dev_free(h->tr_u); dev_free(h->tr_i); dev_free(h->tr_src);
-    dev_free(h->te_r); dev_free(h->te_u); dev_free(h->te_i);
-    dev_free(h->P.f16); dev_free(h->P.f32); dev_free(h->Q.f16); dev_free(h->Q.f32);
-    dev_free(h->d_uprec_row); dev_free(h->d_iprec_row); dev_free(h->d_ugroup); dev_free(h->d_igroup);
-    dev_free(h->d_umap); dev_free(h->d_imap); dev_free(h->d_stats); dev_free(h->d_block_err);
+    dev_free(h->tr_r, h->stream); dev_free(h->tr_u, h->stream); dev_free(h->tr_i, h->stream); dev_free(h->tr_src, h->stream);
+    dev_free(h->te_r, h->stream); dev_free(h->te_u, h->stream); dev_free(h->te_i, h->stream);
+    dev_free(h->P.f16, h->stream); dev_free(h->P.f32, h->stream); dev_free(h->Q.f16, h->stream); dev_free(h->Q.f32, h->stream);
+    dev_free(h->d_uprec_row, h->stream); dev_free(h->d_iprec_row, h->stream); dev_free(h->d_ugroup, h->stream); dev_free(h->d_igroup, h->stream);
+    dev_free(h->d_umap, h->stream); dev_free(h->d_imap, h->stream); dev_free(h->d_stats, h->stream); dev_free(h->d_block_err, h->stream);
     h->have_ratings = h->have_factors = false;
 }
 
@@ -189,8 +190,8 @@ int recode_side(mascot_handle* h, bool users) {
 
 int need_scratch(mascot_handle* h, size_t bytes) {
     if (h->scratch_bytes >= bytes) return MASCOT_OK;
-    dev_free(h->d_scratch); h->scratch_bytes = 0;
-    CU(h, cudaMalloc(&h->d_scratch, bytes));
+    dev_free(h->d_scratch, h->stream); h->scratch_bytes = 0;
+    CU(h, pool_alloc(&h->d_scratch, bytes, h->stream));
     h->scratch_bytes = bytes;
     return MASCOT_OK;
 }
@@ -408,8 +409,8 @@ int mascot_create(const mascot_config* cfg, mascot_handle** out) {
     cudaError_t e = cudaSetDevice(cfg->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     for (int j = 0; j < 4 && e == cudaSuccess; j++) e = cudaEventCreate(&h->ev[j]);
-    if (e == cudaSuccess) e = dev_alloc(&h->counters.d_slots, 4);
-    if (e == cudaSuccess) e = cudaMemset(h->counters.d_slots, 0, 4 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = dev_alloc(&h->counters.d_slots, 4, h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->counters.d_slots, 0, 4 * sizeof(unsigned long long), h->stream);
     if (e != cudaSuccess) {
         std::string msg = std::string("CUDA set-up failed: ") + cudaGetErrorString(e);
         mascot_destroy(h);
@@ -425,12 +426,13 @@ int mascot_destroy(mascot_handle* h) {
     l2_window_remove(h);
     free_ratings(h);
     shard_destroy(h);
-    dev_free(h->d_scratch); dev_free(h->counters.d_slots); dev_free(h->d_err_flag);
+    if (h->stream) cudaStreamSynchronize(h->stream);       // the staging buffers below are freed on the other stream
+    dev_free(h->d_scratch, h->stream); dev_free(h->counters.d_slots, h->stream); dev_free(h->d_err_flag, h->stream);
     for (auto& ev : h->ev) if (ev) cudaEventDestroy(ev);
     for (int b = 0; b < 2; b++) {
         if (h->ev_copied[b]) cudaEventDestroy(h->ev_copied[b]);
         if (h->ev_free[b]) cudaEventDestroy(h->ev_free[b]);
-        if (h->d_stage[b]) cudaFree(h->d_stage[b]);
+        dev_free(h->d_stage[b], h->copy_stream);
     }
     if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -463,9 +465,8 @@ int mascot_reload_train(mascot_handle* h, const mascot_rating* train, uint64_t n
     if (n_train >= (1ull << 32)) return fail(h, MASCOT_ERR_BAD_ARG, "too many ratings (limit 2^32 - 1 per engine)");
     CU(h, cudaSetDevice(h->cfg.device));
     if (n_train != h->n_train) {
-        dev_free(h->tr_r); dev_free(h->tr_u); dev_free(h->tr_i); dev_free(h->tr_src);
-        CU(h, dev_alloc(&h->tr_r, n_train)); CU(h, dev_alloc(&h->tr_u, n_train)); CU(h, dev_alloc(&h->tr_i, n_train));
-        CU(h, dev_alloc(&h->tr_src, n_train));
+        CU(h, reserve(h, &h->tr_r, n_train)); CU(h, reserve(h, &h->tr_u, n_train)); CU(h, reserve(h, &h->tr_i, n_train));
+        CU(h, reserve(h, &h->tr_src, n_train));
         h->n_train = n_train;
         h->seg_off.assign({0, n_train});           // a stream of another length is one segment
         h->cls_off.clear(); h->partitioned = false;
@@ -475,7 +476,7 @@ int mascot_reload_train(mascot_handle* h, const mascot_rating* train, uint64_t n
     int rc = need_scratch(h, bytes);
     if (rc != MASCOT_OK) return rc;
     CU(h, cudaMemsetAsync(h->d_err_flag, 0, sizeof(uint32_t), h->stream));
-    CU(h, cudaMemcpyAsync(h->d_scratch, train, bytes, cudaMemcpyHostToDevice, h->stream));
+    CU(h, copy_to_device(h->d_scratch, train, bytes, h->stream));
     CU(h, encode_segments(h, static_cast<const mascot_rating*>(h->d_scratch), h->seg_off, h->cfg.shuffle != 0,
                           h->tr_r, h->tr_u, h->tr_i, h->tr_src));
     uint32_t bad = 0;
@@ -499,39 +500,40 @@ static int scatter_from_device(mascot_handle* h, const float* dP, const float* d
     return l2_window_install(h);
 }
 
+// Both factor matrices as fp32 rows in the scratch buffer: what set_factors uploads, init_factors fills and
+// get_factors collects.
+static int factor_scratch(mascot_handle* h, float** dP, float** dQ) {
+    const size_t pu = ((size_t)h->n_users * h->K + 63) / 64 * 64, qi = (size_t)h->n_items * h->K;
+    const int rc = need_scratch(h, sizeof(float) * (pu + qi));
+    if (rc != MASCOT_OK) return rc;
+    *dP = static_cast<float*>(h->d_scratch);
+    *dQ = *dP + pu;
+    return MASCOT_OK;
+}
+
 int mascot_set_factors(mascot_handle* h, const float* P, const float* Q) {
     if (!h) return MASCOT_ERR_BAD_ARG;
     if (!P || !Q) return fail(h, MASCOT_ERR_BAD_ARG, "null factor matrix");
     if (!h->have_ratings) return fail(h, MASCOT_ERR_STATE, "mascot_set_ratings must come first");
     CU(h, cudaSetDevice(h->cfg.device));
-    const size_t pu = (size_t)h->n_users * h->K, qi = (size_t)h->n_items * h->K;
     float *dP = nullptr, *dQ = nullptr;
-    CU(h, dev_alloc(&dP, pu));
-    cudaError_t e = dev_alloc(&dQ, qi);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dP, P, sizeof(float) * pu, cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dQ, Q, sizeof(float) * qi, cudaMemcpyHostToDevice, h->stream);
-    int rc = MASCOT_OK;
-    if (e == cudaSuccess) rc = scatter_from_device(h, dP, dQ);
-    cudaFree(dP); cudaFree(dQ);
-    CU(h, e);
-    return rc;
+    const int rc = factor_scratch(h, &dP, &dQ);
+    if (rc != MASCOT_OK) return rc;
+    CU(h, copy_to_device(dP, P, sizeof(float) * (size_t)h->n_users * h->K, h->stream));
+    CU(h, copy_to_device(dQ, Q, sizeof(float) * (size_t)h->n_items * h->K, h->stream));
+    return scatter_from_device(h, dP, dQ);
 }
 
 int mascot_init_factors(mascot_handle* h) {
     if (!h) return MASCOT_ERR_BAD_ARG;
     if (!h->have_ratings) return fail(h, MASCOT_ERR_STATE, "mascot_set_ratings must come first");
     CU(h, cudaSetDevice(h->cfg.device));
-    const size_t pu = (size_t)h->n_users * h->K, qi = (size_t)h->n_items * h->K;
     float *dP = nullptr, *dQ = nullptr;
-    CU(h, dev_alloc(&dP, pu));
-    cudaError_t e = dev_alloc(&dQ, qi);
-    if (e == cudaSuccess) e = launch_init_normal(dP, pu, h->cfg.seed, 1, h->stream);
-    if (e == cudaSuccess) e = launch_init_normal(dQ, qi, h->cfg.seed, 2, h->stream);
-    int rc = MASCOT_OK;
-    if (e == cudaSuccess) rc = scatter_from_device(h, dP, dQ);
-    cudaFree(dP); cudaFree(dQ);
-    CU(h, e);
-    return rc;
+    const int rc = factor_scratch(h, &dP, &dQ);
+    if (rc != MASCOT_OK) return rc;
+    CU(h, launch_init_normal(dP, (size_t)h->n_users * h->K, h->cfg.seed, 1, h->stream));
+    CU(h, launch_init_normal(dQ, (size_t)h->n_items * h->K, h->cfg.seed, 2, h->stream));
+    return scatter_from_device(h, dP, dQ);
 }
 
 }  // extern "C"
@@ -879,15 +881,14 @@ int mascot_train_epoch_streamed(mascot_handle* h, uint32_t epoch, const mascot_r
     }
     const uint64_t piece = std::min<uint64_t>(kPiece, std::max<uint64_t>(n_train, 1));
     if (h->stage_ratings < piece) {
-        for (int b = 0; b < 2; b++) { if (h->d_stage[b]) cudaFree(h->d_stage[b]); h->d_stage[b] = nullptr; }
+        for (int b = 0; b < 2; b++) dev_free(h->d_stage[b], h->copy_stream);
         h->stage_ratings = 0;
-        for (int b = 0; b < 2; b++) CU(h, cudaMalloc(&h->d_stage[b], sizeof(mascot_rating) * piece));
+        for (int b = 0; b < 2; b++) CU(h, dev_alloc(&h->d_stage[b], piece, h->copy_stream));
         h->stage_ratings = piece;
     }
     if (n_train != h->n_train) {
-        dev_free(h->tr_r); dev_free(h->tr_u); dev_free(h->tr_i); dev_free(h->tr_src);
-        CU(h, dev_alloc(&h->tr_r, n_train)); CU(h, dev_alloc(&h->tr_u, n_train)); CU(h, dev_alloc(&h->tr_i, n_train));
-        CU(h, dev_alloc(&h->tr_src, n_train));
+        CU(h, reserve(h, &h->tr_r, n_train)); CU(h, reserve(h, &h->tr_u, n_train)); CU(h, reserve(h, &h->tr_i, n_train));
+        CU(h, reserve(h, &h->tr_src, n_train));
         h->n_train = n_train;
     }
     CU(h, cudaMemsetAsync(h->d_err_flag, 0, sizeof(uint32_t), h->stream));
@@ -917,7 +918,7 @@ int mascot_train_epoch_streamed(mascot_handle* h, uint32_t epoch, const mascot_r
         const int b = (int)(c & 1);
         const uint64_t off = h->seg_off[c], len = h->seg_off[c + 1] - off;
         if (c >= 2) CU(h, cudaStreamWaitEvent(h->copy_stream, h->ev_free[b], 0));
-        CU(h, cudaMemcpyAsync(h->d_stage[b], train + off, sizeof(mascot_rating) * len, cudaMemcpyHostToDevice, h->copy_stream));
+        CU(h, copy_to_device(h->d_stage[b], train + off, sizeof(mascot_rating) * len, h->copy_stream));
         CU(h, cudaEventRecord(h->ev_copied[b], h->copy_stream));
         CU(h, cudaStreamWaitEvent(h->stream, h->ev_copied[b], 0));
         CU(h, launch_encode_stream(h->d_stage[b], len, h->cfg.shuffle != 0, h->cfg.seed + 0x9e3779b97f4a7c15ull * c, h->d_umap, h->d_imap,
@@ -991,7 +992,10 @@ int mascot_release_scratch(mascot_handle* h) {
     if (!h) return MASCOT_ERR_BAD_ARG;
     CU(h, cudaSetDevice(h->cfg.device));
     CU(h, cudaStreamSynchronize(h->stream));
-    dev_free(h->d_scratch); h->scratch_bytes = 0;
+    dev_free(h->d_scratch, h->stream); h->scratch_bytes = 0;
+    CU(h, cudaStreamSynchronize(h->stream));
+    pool_trim();
+    release_copy_rings();
     return MASCOT_OK;
 }
 
@@ -1042,20 +1046,21 @@ int mascot_get_factors(mascot_handle* h, float* P, float* Q, int order) {
     if (!h->have_factors) return fail(h, MASCOT_ERR_STATE, "no factors yet");
     if (order != 0 && order != 1) return fail(h, MASCOT_ERR_BAD_ARG, "order must be 0 or 1");
     CU(h, cudaSetDevice(h->cfg.device));
-    auto one = [&](float* dst, Arena a, const uint8_t* prow, uint32_t rows, const uint32_t* map, const RowLayout& lay) -> int {
-        if (!dst) return MASCOT_OK;
-        float* d = nullptr;
-        CU(h, dev_alloc(&d, (size_t)rows * h->K));
-        cudaError_t e = launch_gather_factors(h->K, a, prow, rows, order == 0 ? map : nullptr, lay, d, h->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(dst, d, sizeof(float) * (size_t)rows * h->K, cudaMemcpyDeviceToHost, h->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-        cudaFree(d);
-        CU(h, e);
-        return MASCOT_OK;
-    };
-    int rc = one(P, h->P, h->d_uprec_row, h->n_users, h->d_umap, h->ulay);
+    float *dP = nullptr, *dQ = nullptr;
+    const int rc = factor_scratch(h, &dP, &dQ);
     if (rc != MASCOT_OK) return rc;
-    return one(Q, h->Q, h->d_iprec_row, h->n_items, h->d_imap, h->ilay);
+    CopySpan spans[2];
+    int n = 0;
+    if (P) {
+        CU(h, launch_gather_factors(h->K, h->P, h->d_uprec_row, h->n_users, order == 0 ? h->d_umap : nullptr, h->ulay, dP, h->stream));
+        spans[n++] = CopySpan{P, dP, sizeof(float) * (size_t)h->n_users * h->K};
+    }
+    if (Q) {
+        CU(h, launch_gather_factors(h->K, h->Q, h->d_iprec_row, h->n_items, order == 0 ? h->d_imap : nullptr, h->ilay, dQ, h->stream));
+        spans[n++] = CopySpan{Q, dQ, sizeof(float) * (size_t)h->n_items * h->K};
+    }
+    CU(h, copy_to_host(spans, n, h->stream));
+    return MASCOT_OK;
 }
 
 int mascot_get_group_info(mascot_handle* h, int side, uint32_t* n_groups, uint32_t* end_idx, uint8_t* precision, float* error) {
@@ -1121,9 +1126,8 @@ int mascot_get_test_ratings(mascot_handle* h, mascot_rating* out, int order) {
     CU(h, cudaSetDevice(h->cfg.device));
     const uint64_t n = h->n_test;
     std::vector<float> r(n); std::vector<uint32_t> u(n), i(n);
-    CU(h, cudaMemcpy(r.data(), h->te_r, sizeof(float) * n, cudaMemcpyDeviceToHost));
-    CU(h, cudaMemcpy(u.data(), h->te_u, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost));
-    CU(h, cudaMemcpy(i.data(), h->te_i, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost));
+    const CopySpan spans[3] = {{r.data(), h->te_r, sizeof(float) * n}, {u.data(), h->te_u, sizeof(uint32_t) * n}, {i.data(), h->te_i, sizeof(uint32_t) * n}};
+    CU(h, copy_to_host(spans, 3, h->stream));
     std::vector<uint32_t> s2u, s2i;
     if (order == 0 && h->sorted_space) {
         s2u.resize(h->n_users); s2i.resize(h->n_items);
@@ -1156,7 +1160,8 @@ int mascot_get_stream_order(mascot_handle* h, uint32_t* src_out) {
     if (!h->have_ratings) return fail(h, MASCOT_ERR_STATE, "mascot_set_ratings must come first");
     if (!h->tr_src) return fail(h, MASCOT_ERR_UNSUPPORTED, "streams of 2^32 ratings or more keep no order map");
     CU(h, cudaSetDevice(h->cfg.device));
-    CU(h, cudaMemcpy(src_out, h->tr_src, sizeof(uint32_t) * h->n_train, cudaMemcpyDeviceToHost));
+    const CopySpan span{src_out, h->tr_src, sizeof(uint32_t) * h->n_train};
+    CU(h, copy_to_host(&span, 1, h->stream));
     return MASCOT_OK;
 }
 
@@ -1165,11 +1170,11 @@ int mascot_rmse_device(const float* d_P, const float* d_Q, uint32_t k, const mas
     if (k != 64 && k != 128) return fail(nullptr, MASCOT_ERR_BAD_ARG, "k must be 64 or 128");
     const size_t blocks = (size_t)((n_test + 511) / 512);
     float* d_err = nullptr;
-    CU(nullptr, dev_alloc(&d_err, blocks));
+    CU(nullptr, dev_alloc(&d_err, blocks, nullptr));
     std::vector<float> part(blocks);
     cudaError_t e = launch_rmse_plain((int)k, d_test, n_test, d_P, d_Q, d_err, nullptr);
     if (e == cudaSuccess) e = cudaMemcpy(part.data(), d_err, sizeof(float) * blocks, cudaMemcpyDeviceToHost);
-    cudaFree(d_err);
+    dev_free(d_err, nullptr);
     CU(nullptr, e);
     *rmse = (double)reference_rmse_from_partials(part, n_test);
     return MASCOT_OK;
@@ -1188,15 +1193,15 @@ int mascot_rmse_host(const float* P, uint32_t n_users, const float* Q, uint32_t 
     }
     CU(nullptr, cudaSetDevice(device));
     float *dP = nullptr, *dQ = nullptr; mascot_rating* dT = nullptr;
-    cudaError_t e = dev_alloc(&dP, (size_t)n_users * k);
-    if (e == cudaSuccess) e = dev_alloc(&dQ, (size_t)n_items * k);
-    if (e == cudaSuccess) e = dev_alloc(&dT, n_test);
-    if (e == cudaSuccess) e = cudaMemcpy(dP, P, sizeof(float) * (size_t)n_users * k, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(dQ, Q, sizeof(float) * (size_t)n_items * k, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(dT, test, sizeof(mascot_rating) * n_test, cudaMemcpyHostToDevice);
+    cudaError_t e = dev_alloc(&dP, (size_t)n_users * k, nullptr);
+    if (e == cudaSuccess) e = dev_alloc(&dQ, (size_t)n_items * k, nullptr);
+    if (e == cudaSuccess) e = dev_alloc(&dT, n_test, nullptr);
+    if (e == cudaSuccess) e = copy_to_device(dP, P, sizeof(float) * (size_t)n_users * k, nullptr);
+    if (e == cudaSuccess) e = copy_to_device(dQ, Q, sizeof(float) * (size_t)n_items * k, nullptr);
+    if (e == cudaSuccess) e = copy_to_device(dT, test, sizeof(mascot_rating) * n_test, nullptr);
     int rc = MASCOT_OK;
     if (e == cudaSuccess) rc = mascot_rmse_device(dP, dQ, k, dT, n_test, rmse);
-    cudaFree(dP); cudaFree(dQ); cudaFree(dT);
+    dev_free(dP, nullptr); dev_free(dQ, nullptr); dev_free(dT, nullptr);
     CU(nullptr, e);
     return rc;
 }

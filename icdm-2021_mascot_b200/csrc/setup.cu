@@ -22,6 +22,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include "handle.h"
+#include "host_copy.h"
 
 namespace mascot {
 
@@ -177,11 +178,11 @@ int build_side(mascot_handle* h, bool users, const std::vector<uint32_t>& s2o, c
     uint16_t** dg = users ? &h->d_ugroup : &h->d_igroup;
     uint8_t** dp = users ? &h->d_uprec_row : &h->d_iprec_row;
     uint32_t** dm = users ? &h->d_umap : &h->d_imap;
-    CU(h, dev_alloc(dg, rows)); CU(h, dev_alloc(dp, rows));
+    CU(h, reserve(h, dg, rows)); CU(h, reserve(h, dp, rows));
     CU(h, cudaMemcpyAsync(*dg, group.data(), sizeof(uint16_t) * rows, cudaMemcpyHostToDevice, h->stream));
     CU(h, cudaMemcpyAsync(*dp, flags.data(), sizeof(uint8_t) * rows, cudaMemcpyHostToDevice, h->stream));
     if (h->sorted_space) {
-        CU(h, dev_alloc(dm, n));
+        CU(h, reserve(h, dm, n));
         CU(h, cudaMemcpyAsync(*dm, row_of_id.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, h->stream));
     }
     CU(h, cudaStreamSynchronize(h->stream));       // the host vectors above end with this call
@@ -210,16 +211,17 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     NvtxRange range("mascot: rating set-up");
     CU(h, cudaSetDevice(h->cfg.device));
     l2_window_remove(h);
-    free_ratings(h);
+    h->have_ratings = h->have_factors = false;       // the buffers stay and are used again where they are large enough
     h->n_users = n_users; h->n_items = n_items; h->n_test = 0; h->n_train = 0;
     h->cls_off.clear(); h->partitioned = false;
     h->sorted_space = h->grouped || sharded;
+    if (!h->sorted_space) { dev_free(h->d_umap, h->stream); dev_free(h->d_imap, h->stream); }      // identity
     h->ulay = RowLayout(); h->ilay = RowLayout();
     h->ulay.n = n_users; h->ilay.n = n_items;
     if (sharded && rq.world > 1) { h->ulay.parts = (uint32_t)rq.world; h->ulay.rows_per_part = (n_users + rq.world - 1) / rq.world; h->ulay.snake = 1; }
     if (sharded && rq.blocks > 1) { h->ilay.parts = rq.blocks; h->ilay.rows_per_part = (n_items + rq.blocks - 1) / rq.blocks; }
     h->urows = layout_rows(h->ulay); h->irows = layout_rows(h->ilay);
-    if (!h->d_err_flag) CU(h, dev_alloc(&h->d_err_flag, 1));
+    if (!h->d_err_flag) CU(h, reserve(h, &h->d_err_flag, 1));
     CU(h, cudaMemsetAsync(h->d_err_flag, 0, sizeof(uint32_t), h->stream));
 
     // ---- scratch: the uploaded arrays and the sort buffers ----
@@ -256,7 +258,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
 
     double t_phase = now_us();
     // ---- 1. training ratings: upload, check, degrees ----
-    if (n_all) CU(h, cudaMemcpyAsync(aos, rq.train, sizeof(NodeAos) * n_all, cudaMemcpyHostToDevice, h->stream));
+    if (n_all) CU(h, copy_to_device(aos, rq.train, sizeof(NodeAos) * n_all, h->stream));
     CU(h, cudaMemsetAsync(d_udeg, 0, sizeof(uint32_t) * n_users, h->stream));
     CU(h, cudaMemsetAsync(d_ideg, 0, sizeof(uint32_t) * n_items, h->stream));
     if (n_all) {
@@ -339,7 +341,6 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
         }
         CU(h, cudaMemcpyAsync(ideg_local.data(), d_ldeg, sizeof(uint32_t) * n_items, cudaMemcpyDeviceToHost, h->stream));
         CU(h, cudaStreamSynchronize(h->stream));
-        dev_free(h->d_igroup); dev_free(h->d_iprec_row); dev_free(h->d_imap);
     }
     { const double t_g = now_us();
       if ((rc = build_side(h, false, is2o, icnt, ideg_local, std::max<uint64_t>(n_local, 1))) != MASCOT_OK) return rc;
@@ -350,8 +351,8 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     h->init_uerr.assign(h->uend.size(), 1.f); h->init_ierr.assign(h->iend.size(), 1.f);   // mf_methods.cu:150-151
 
     // ---- 6. the coded training stream ----
-    CU(h, dev_alloc(&h->tr_r, n_local)); CU(h, dev_alloc(&h->tr_u, n_local)); CU(h, dev_alloc(&h->tr_i, n_local));
-    CU(h, dev_alloc(&h->tr_src, n_local));
+    CU(h, reserve(h, &h->tr_r, n_local)); CU(h, reserve(h, &h->tr_u, n_local)); CU(h, reserve(h, &h->tr_i, n_local));
+    CU(h, reserve(h, &h->tr_src, n_local));
     if (n_local) {
         CU(h, encode_segments(h, reinterpret_cast<const mascot_rating*>(enc_src), seg, h->cfg.shuffle != 0, h->tr_r, h->tr_u, h->tr_i, h->tr_src));
         if (src_through) {          // positions in the caller's array, not in the selected copy
@@ -364,7 +365,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     uint64_t n_test = rq.n_test;
     if (rq.n_test) {
         CU(h, cudaStreamSynchronize(h->stream));          // aos / aos2 are reused
-        CU(h, cudaMemcpyAsync(aos, rq.test, sizeof(NodeAos) * rq.n_test, cudaMemcpyHostToDevice, h->stream));
+        CU(h, copy_to_device(aos, rq.test, sizeof(NodeAos) * rq.n_test, h->stream));
         check_hist_kernel<<<grid_for(rq.n_test, 256), 256, 0, h->stream>>>(aos, rq.n_test, n_users, n_items, nullptr, nullptr, h->d_err_flag);
         CU(h, cudaGetLastError());
         CU(h, cudaMemcpyAsync(&bad, h->d_err_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
@@ -395,13 +396,13 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
             CU(h, cudaGetLastError());
             std::swap(cur, other);
         }
-        CU(h, dev_alloc(&h->te_r, n_test)); CU(h, dev_alloc(&h->te_u, n_test)); CU(h, dev_alloc(&h->te_i, n_test));
+        CU(h, reserve(h, &h->te_r, n_test)); CU(h, reserve(h, &h->te_u, n_test)); CU(h, reserve(h, &h->te_i, n_test));
         if (n_test) {
             const std::vector<uint64_t> whole = {0, n_test};
             CU(h, encode_segments(h, reinterpret_cast<const mascot_rating*>(cur), whole, false, h->te_r, h->te_u, h->te_i, nullptr));
         }
     } else {
-        CU(h, dev_alloc(&h->te_r, 0)); CU(h, dev_alloc(&h->te_u, 0)); CU(h, dev_alloc(&h->te_i, 0));
+        CU(h, reserve(h, &h->te_r, 0)); CU(h, reserve(h, &h->te_u, 0)); CU(h, reserve(h, &h->te_i, 0));
     }
     h->n_test = n_test;
     CU(h, cudaStreamSynchronize(h->stream));
@@ -410,20 +411,20 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     // ---- factor arenas and statistics ----
     const size_t pu = (size_t)h->urows * h->K, qi = (size_t)h->irows * h->K;
     if (h->kind == KIND_MIXED || h->kind == KIND_MEMQUANT || h->kind == KIND_SWITCH) {
-        CU(h, dev_alloc(&h->P.f16, pu)); CU(h, dev_alloc(&h->Q.f16, qi));
+        CU(h, reserve(h, &h->P.f16, pu)); CU(h, reserve(h, &h->Q.f16, qi));
         CU(h, cudaMemsetAsync(h->P.f16, 0, sizeof(__half) * pu, h->stream)); CU(h, cudaMemsetAsync(h->Q.f16, 0, sizeof(__half) * qi, h->stream));
     }
     if (h->kind != KIND_MEMQUANT) {
-        CU(h, dev_alloc(&h->P.f32, pu)); CU(h, dev_alloc(&h->Q.f32, qi));
+        CU(h, reserve(h, &h->P.f32, pu)); CU(h, reserve(h, &h->Q.f32, qi));
         CU(h, cudaMemsetAsync(h->P.f32, 0, sizeof(float) * pu, h->stream)); CU(h, cudaMemsetAsync(h->Q.f32, 0, sizeof(float) * qi, h->stream));
     }
     h->stats_copies = h->cfg.deterministic ? 1 : kStatCopies;
     h->stats_stride = (stats_floats(h) + 63) / 64 * 64;
-    CU(h, dev_alloc(&h->d_stats, h->stats_stride * h->stats_copies));
+    CU(h, reserve(h, &h->d_stats, h->stats_stride * h->stats_copies));
     CU(h, cudaMemsetAsync(h->d_stats, 0, sizeof(float) * h->stats_stride * h->stats_copies, h->stream));
     h->h_stats.assign(stats_floats(h), 0.f);
     const size_t blocks = (size_t)((n_test + 511) / 512);
-    CU(h, dev_alloc(&h->d_block_err, blocks));
+    CU(h, reserve(h, &h->d_block_err, blocks));
     h->h_block_err.assign(blocks, 0.f);
     CU(h, cudaStreamSynchronize(h->stream));
     // the set-up's own use of the scratch buffer is over: the sort below may re-carve it

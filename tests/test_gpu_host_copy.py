@@ -1,0 +1,47 @@
+"""Factor matrices of every size class of the staged host copies: below the direct limit, pieces of one thread, ragged
+last pieces, several blocks of whole slots, host addresses off every boundary; and buffers kept from one set of
+ratings for the next, larger or smaller."""
+import numpy as np
+import pytest
+
+from helpers import assert_bit_equal, random_problem
+
+pytestmark = pytest.mark.gpu
+
+
+def unaligned(a, off):
+    """The same values at an address `off` floats past an allocation."""
+    raw = np.empty(a.size + off, np.float32)
+    raw[off:] = a.reshape(-1)
+    return raw[off:].reshape(a.shape)
+
+
+@pytest.mark.parametrize("n_users,n_items,off", [(3, 2, 0), (511, 257, 1), (769, 1, 3), (4099, 1023, 5), (20011, 333, 7), (131072, 65537, 1), (150001, 70001, 9)])
+def test_factors_go_in_and_come_out_unchanged(mascot, n_users, n_items, off):
+    k = 64
+    rng = np.random.default_rng(n_users)
+    R, P, Q = random_problem(rng, n_users, n_items, 50, k)
+    eng = mascot.Engine(mascot.default_config(version=mascot.V_SGD, k=k, deterministic=1, shuffle=0))
+    eng.set_ratings(R, R, n_users, n_items)
+    for _ in range(2):
+        eng.set_factors(unaligned(P, off), unaligned(Q, off + 2))
+        Pg, Qg = eng.get_factors(0)
+        assert_bit_equal(Pg, P, "P")
+        assert_bit_equal(Qg, Q, "Q")
+        eng.release_scratch()
+    eng.close()
+
+
+def test_an_engine_takes_larger_and_smaller_ratings(mascot, oracle):
+    k = 128
+    eng = mascot.Engine(mascot.default_config(version=mascot.V_SGD, k=k, deterministic=1, shuffle=0, lam=0.05))
+    for n_users, n_items, n in ((50, 40, 900), (3000, 2000, 20011), (60, 1, 33), (3000, 1999, 20001)):
+        R, P, Q = random_problem(np.random.default_rng(n), n_users, n_items, n, k)
+        eng.set_ratings(R, R[:17], n_users, n_items)
+        eng.set_factors(P, Q)
+        eng.train_epoch(0)
+        oracle.sgd_run(k, R, None, P, Q, 0.01, 0.05, oracle.rules_reference())
+        Pg, Qg = eng.get_factors(0)
+        assert_bit_equal(Pg, P, "P")
+        assert_bit_equal(Qg, Q, "Q")
+    eng.close()
