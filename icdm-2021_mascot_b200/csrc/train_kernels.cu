@@ -8,11 +8,17 @@
 // workers:
 //   * every lane holds eight consecutive physical elements of a row (one 128-bit access for
 //     binary16 storage, two for fp32);
+//   * the workers of a warp go through their ratings in step, with whole-warp shuffles, and the loop has no branch
+//     that they could take differently: what only some of them do (a new item row, a dropped write-back) is
+//     predicated, chunks are fetched and tickets drawn without branches, and a worker that has run out of ratings goes
+//     on with empty records.  Per-worker branches cost a warp barrier in front of every shuffle and split the update
+//     into pieces that cannot be scheduled into each other: 131 warp instructions per step of all workers of a warp
+//     before, 90 now.
 //   * the rating records of a chunk (one rating per lane) are loaded one chunk ahead, tagged
-//     (repeated user, start of an item run, repeated item) and put into shared memory, from where
+//     (repeated user, start of an item run, repeated item, dropped write-back) and put into shared memory, from where
 //     the worker reads one rating with a single 128-bit broadcast load;
-//   * rows travel global -> shared memory by cp.async into small per-worker rings, user rows a few
-//     ratings ahead, item rows one rating ahead; copy groups complete in order, so the wait for the
+//   * rows travel global -> shared memory by cp.async into small per-worker rings, user rows five
+//     ratings ahead, item rows three; copy groups complete in order, so the wait for the
 //     row of rating j leaves the younger copies in flight (register loads cannot do that: the wait
 //     for an old load also waits for every younger load on the same scoreboard);
 //   * the row of an item that repeats (the stream is item-sorted inside shuffle windows) stays in
@@ -23,8 +29,17 @@
 //     so racing updates of one user add up instead of overwriting each other (add_row_delta).
 // The item lead is short on purpose.  Between the request of an item row and its write-back (a plain
 // store, once per run) every update another worker makes to that row is lost, so the loss grows with
-// (workers x lead); measured on the 100M-rating configuration with plain stores on both sides, a lead
-// of seven ratings costs 1.5 % of final RMSE where three (users) and one (items) cost nothing.
+// (workers x lead time).  The leads are counted in ratings, and a rating takes 0.2 us where it took 0.35 when the leads
+// were three and one: the same time, and the same RMSE (0.5169 after one epoch, 0.5180 after six on the k=64
+// configuration either way).  With leads of three and two the 8M-rating configuration took 1.65 ms per epoch instead
+// of 1.39, the k=64 one 1.97 instead of 1.65; user leads of six and seven gave nothing more.
+//
+// WHAT BOUNDS IT (one B200, k=128, binary16 rows).  Sets with few workers per SM (8M ratings: one warp per scheduler):
+// the chain of one update - dot product, four shuffle steps, update - and the 90 instructions around it, 2.42 -> 1.39
+// ms per epoch.  Full SMs (100M ratings, 7.17 -> 5.50 ms): the L2 and its reductions.  18.3e9 updates/s write 4.7 TB/s of
+// reductions and read as much again; a kernel that does nothing but read random rows and reduce into them reaches
+// 17.6e9 rows/s on this GPU with evenly spread rows and 10.9e9 with Zipf ones (8.6e9 and 7.1e9 with fp32 rows, which is
+// what bounds the classes with fp32 user rows).
 //
 // ELEMENT ORDER.  layout.cuh stores rows permuted so that lane m of a worker holds the elements of
 // reference lanes m and m+16 (k=128) or m, m+16, m+8, m+24 (k=64).  With pair products
@@ -116,54 +131,83 @@ template <int MODE> __device__ __forceinline__ bool is_f32(uint32_t code) {
     return MODE == ROWS_F32 || (MODE == ROWS_DYN && (code & kPrecBit));
 }
 
-// Row slice of lane m: L2-only loads/stores (rows are shared between SMs and never reused from L1).
-template <int K, int MODE>
-__device__ __forceinline__ Raw<MODE> ld_row(const Arena& A, uint32_t code, int m) {
-    const uint32_t row = code & kIdMask;
-    Raw<MODE> r;
-    if (is_f32<MODE>(code)) {
-        const uint4* p = reinterpret_cast<const uint4*>(A.f32 + (size_t)row * K) + m;     // first half; second half K/8 uint4 on
-        r.a = __ldcg(p);
-        if constexpr (MODE != ROWS_HALF) r.b = __ldcg(p + K / 8);
-    } else {
-        r.a = __ldcg(reinterpret_cast<const uint4*>(A.f16 + (size_t)row * K) + m);
+// The rows of one side as a lane sees them: addresses of its slice of row 0 in the two arenas.  (One multiply-add
+// makes the address of a row; the second half of an fp32 row is 2 K bytes further on.)
+template <int K, int MODE> struct Rows {
+    const unsigned char* b16;
+    const unsigned char* b32;
+    __device__ __forceinline__ Rows(const Arena& A, int m)
+        : b16(reinterpret_cast<const unsigned char*>(A.f16) + 16 * m), b32(reinterpret_cast<const unsigned char*>(A.f32) + 16 * m) {}
+    __device__ __forceinline__ const unsigned char* at(uint32_t code) const {
+        if constexpr (MODE == ROWS_HALF) return b16 + (uint64_t)code * (2u * K);
+        else if constexpr (MODE == ROWS_F32) return b32 + (uint64_t)code * (4u * K);
+        else return (code & kPrecBit) ? b32 + (uint64_t)(code & kIdMask) * (4u * K) : b16 + (uint64_t)(code & kIdMask) * (2u * K);
     }
-    return r;
-}
-template <int K, int MODE>
-__device__ __forceinline__ void st_row(const Arena& A, uint32_t code, int m, const Raw<MODE>& r) {
-    const uint32_t row = code & kIdMask;
-    if (is_f32<MODE>(code)) {
-        uint4* p = reinterpret_cast<uint4*>(A.f32 + (size_t)row * K) + m;
-        __stcg(p, r.a);
-        if constexpr (MODE != ROWS_HALF) __stcg(p + K / 8, r.b);
-    } else {
-        __stcg(reinterpret_cast<uint4*>(A.f16 + (size_t)row * K) + m, r.a);
-    }
+};
+
+// `go` for the second half of a row: fp32 rows only
+template <int MODE> __device__ __forceinline__ unsigned second_half(unsigned go, uint32_t code) {
+    return MODE == ROWS_DYN ? ((code & kPrecBit) ? go : 0u) : go;
 }
 
-// Adds (now - before) to a row instead of storing `now`: with several workers on the same row at the
-// same time a plain store erases what the others wrote since this worker read the row, a reduction
-// keeps it.  (Not used for rows flagged kHotBit: summing the changes of very many concurrent updates
-// that all started from the same stale value multiplies the step; there the plain store stays.)  When nobody else touched the row the result equals `now` (the difference of two nearby
-// values is exact).  128-bit vector reductions, fire and forget.
+// Predicated accesses to a lane's 16 bytes: the code around them stays free of branches, which two or four workers of
+// a warp would take one after the other.
+template <int OFF> __device__ __forceinline__ void ldg_if(unsigned go, uint4& v, const unsigned char* p) {
+    asm volatile("{ .reg .pred g; setp.ne.u32 g, %4, 0; @g ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%5 + %6]; }" : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+                 : "r"(go), "l"(p), "n"(OFF) : "memory");
+}
+template <int OFF> __device__ __forceinline__ void stg_if(unsigned go, const unsigned char* p, const uint4& v) {
+    asm volatile("{ .reg .pred g; setp.ne.u32 g, %4, 0; @g st.global.cg.v4.u32 [%5 + %6], {%0, %1, %2, %3}; }" ::"r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w),
+                 "r"(go), "l"(p), "n"(OFF) : "memory");
+}
+template <int OFF> __device__ __forceinline__ void lds_if(unsigned go, uint4& v, unsigned addr) {
+    asm volatile("{ .reg .pred g; setp.ne.u32 g, %4, 0; @g ld.shared.v4.u32 {%0, %1, %2, %3}, [%5 + %6]; }" : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+                 : "r"(go), "r"(addr), "n"(OFF) : "memory");
+}
+
+// Row slice of a lane, L2 only (rows are shared between SMs and never reused from L1).
 template <int K, int MODE>
-__device__ __forceinline__ void add_row_delta(const Arena& A, uint32_t code, int m, const Raw<MODE>& now, const Raw<MODE>& before) {
-    const uint32_t row = code & kIdMask;
+__device__ __forceinline__ void ld_row_if(unsigned go, Raw<MODE>& r, const Rows<K, MODE>& A, uint32_t code) {
+    const unsigned char* p = A.at(code);
+    ldg_if<0>(go, r.a, p);
+    if constexpr (MODE != ROWS_HALF) ldg_if<2 * K>(second_half<MODE>(go, code), r.b, p);
+}
+template <int K, int MODE>
+__device__ __forceinline__ void st_row_if(unsigned go, const Rows<K, MODE>& A, uint32_t code, const Raw<MODE>& r) {
+    const unsigned char* p = A.at(code);
+    stg_if<0>(go, p, r.a);
+    if constexpr (MODE != ROWS_HALF) stg_if<2 * K>(second_half<MODE>(go, code), p, r.b);
+}
+
+// Adds (now - before) to a row, unless `skip`, instead of storing `now`: with several workers on the same row at the
+// same time a plain store erases what the others wrote since this worker read the row, a reduction keeps it.  When
+// nobody else touched the row the result equals `now` (the difference of two nearby values is exact).  128-bit
+// vector reductions, fire and forget, predicated rather than branched around: the update stays one straight piece
+// of code, in which the scheduler can fill the latency of the dot product.
+template <int OFF> __device__ __forceinline__ void red_f32x4(const unsigned char* p, unsigned skip, float x, float y, float z, float w) {
+    asm volatile("{ .reg .pred s; setp.ne.u32 s, %5, 0; @!s red.global.add.v4.f32 [%0 + %6], {%1, %2, %3, %4}; }" ::"l"(p), "f"(x), "f"(y), "f"(z),
+                 "f"(w), "r"(skip), "n"(OFF) : "memory");
+}
+template <int K, int MODE>
+__device__ __forceinline__ void add_row_delta(const Rows<K, MODE>& A, uint32_t code, unsigned skip, const Raw<MODE>& now, const Raw<MODE>& before) {
+    const unsigned char* p = A.at(code);
     if (is_f32<MODE>(code)) {
         if constexpr (MODE != ROWS_HALF) {
-            float4* p = reinterpret_cast<float4*>(A.f32 + (size_t)row * K) + m;
             const V8f n = v8f_of(now.a, now.b), o = v8f_of(before.a, before.b);
-            atomicAdd(p, make_float4(__fsub_rn(n.x[0], o.x[0]), __fsub_rn(n.x[1], o.x[1]), __fsub_rn(n.x[2], o.x[2]), __fsub_rn(n.x[3], o.x[3])));
-            atomicAdd(p + K / 8, make_float4(__fsub_rn(n.x[4], o.x[4]), __fsub_rn(n.x[5], o.x[5]), __fsub_rn(n.x[6], o.x[6]), __fsub_rn(n.x[7], o.x[7])));
+            const float2 minus = make_float2(-1.f, -1.f);      // n - o as fma(-1, o, n): the same single rounding, two lanes at once
+            float2 d[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) d[j] = __ffma2_rn(minus, make_float2(o.x[2 * j], o.x[2 * j + 1]), make_float2(n.x[2 * j], n.x[2 * j + 1]));
+            red_f32x4<0>(p, skip, d[0].x, d[0].y, d[1].x, d[1].y);
+            red_f32x4<2 * K>(p, skip, d[2].x, d[2].y, d[3].x, d[3].y);
         }
     } else {
         const V8h n = v8h_of(now.a), o = v8h_of(before.a);
         unsigned d[4];
 #pragma unroll
         for (int t = 0; t < 4; t++) { const __half2 x = __hsub2(n.v[t], o.v[t]); d[t] = *reinterpret_cast<const unsigned*>(&x); }
-        uint4* p = reinterpret_cast<uint4*>(A.f16 + (size_t)row * K) + m;
-        asm volatile("red.global.add.noftz.v4.f16x2 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(d[0]), "r"(d[1]), "r"(d[2]), "r"(d[3]) : "memory");
+        asm volatile("{ .reg .pred s; setp.ne.u32 s, %5, 0; @!s red.global.add.noftz.v4.f16x2 [%0], {%1, %2, %3, %4}; }" ::"l"(p), "r"(d[0]), "r"(d[1]),
+                     "r"(d[2]), "r"(d[3]), "r"(skip) : "memory");
     }
 }
 
@@ -184,11 +228,12 @@ __device__ __forceinline__ float pair_partial(const V8f& a, const V8f& b) {
     const float2 t = __fadd2_rn(f02, f13);                                     // (f0+f1, f2+f3)
     return __fadd_rn(t.x, t.y);
 }
-__device__ __forceinline__ __half pair_partial(const V8h& p, const V8h& q) {
+// binary16: both halves of the result hold the lane partial, so the butterfly below and the error need no unpacking.
+__device__ __forceinline__ __half2 pair_partial(const V8h& p, const V8h& q) {
     const __half2 f02 = __hfma2(p.v[0], q.v[0], __hmul2_rn(p.v[1], q.v[1]));   // (f_0, f_2)
     const __half2 f13 = __hfma2(p.v[2], q.v[2], __hmul2_rn(p.v[3], q.v[3]));   // (f_1, f_3)
     const __half2 t = __hadd2_rn(f02, f13);                                     // (f_0+f_1, f_2+f_3)
-    return __hadd_rn(__low2half(t), __high2half(t));
+    return __hadd2_rn(__low2half2(t), __high2half2(t));
 }
 // k=128 only: the left-to-right product chain of a reference lane over its four elements,
 // fma(a3,b3, fma(a2,b2, fma(a0,b0, a1*b1))), for the two reference lanes this lane holds
@@ -211,9 +256,12 @@ __device__ __forceinline__ float worker_sum(float x, unsigned wmask) {
     return x;
 }
 template <int TS>
-__device__ __forceinline__ __half worker_sum(__half x, unsigned wmask) {
+__device__ __forceinline__ __half2 worker_sum(__half2 x, unsigned wmask) {
 #pragma unroll
-    for (int d = TS / 2; d >= 1; d >>= 1) x = __hadd_rn(x, __shfl_xor_sync(wmask, x, d));
+    for (int d = TS / 2; d >= 1; d >>= 1) {
+        const unsigned o = __shfl_xor_sync(wmask, *reinterpret_cast<const unsigned*>(&x), d);
+        x = __hadd2_rn(x, *reinterpret_cast<const __half2*>(&o));
+    }
     return x;
 }
 
@@ -225,10 +273,10 @@ __device__ __forceinline__ V8f grad(float e, const V8f& y, float lam, const V8f&
     for (int j = 0; j < 4; j++) set_pr(g, j, __ffma2_rn(e2, pr(y, j), __fmul2_rn(nlam2, pr(x, j))));
     return g;
 }
-__device__ __forceinline__ V8h grad(__half2 e, const V8h& y, __half2 lam, const V8h& x) {
+__device__ __forceinline__ V8h grad(__half2 e, const V8h& y, __half2 nlam, const V8h& x) {
     V8h g;
 #pragma unroll
-    for (int s = 0; s < 4; s++) g.v[s] = __hfma2(e, y.v[s], __hneg2(__hmul2_rn(lam, x.v[s])));
+    for (int s = 0; s < 4; s++) g.v[s] = __hfma2(e, y.v[s], __hmul2_rn(nlam, x.v[s]));     // (-lam) * x == -(lam * x), bit for bit
     return g;
 }
 __device__ __forceinline__ V8f step(float lr, const V8f& g, const V8f& x) {
@@ -247,9 +295,9 @@ __device__ __forceinline__ V8h step(__half2 lr, const V8h& g, const V8h& x) {
 
 struct Consts {
     float lr, lam;
-    __half2 lr_h, lam_h;          // mascot_sgd_kernel.h:79-80
-    __half mpt_scale;             // mpt_sgd_kernel.h:15-16
-    __half2 mpt_lam;              // mf_methods.cu:764-765
+    __half2 lr_h, nlam_h;         // mascot_sgd_kernel.h:79-80 (lambda negated)
+    __half2 mpt_scale;            // mpt_sgd_kernel.h:15-16
+    __half2 mpt_nlam;             // mf_methods.cu:764-765 (negated)
     float mpt_rev;
     int bits;                     // MuPPET: width of the forward and the backward pass
     int afp_epoch, afp_init_threshold;   // AFP: epoch index; ratings per worker / 10 (afp_sgd_kernel.h:143)
@@ -591,19 +639,25 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
     st.cur = cur + 1;
 }
 
-// One update.  p_raw / q_raw are the row slices in their storage precision; both are replaced by the
-// updated values.  Statistics go to `acc` when the rating is sampled.
+// Does a launch work with binary16 ratings?  Its records then hold the converted value in both halves of a word.
+template <int KIND, int UM, int IM> constexpr bool kHalfRating =
+    KIND == KIND_MPT || ((KIND == KIND_MIXED || KIND == KIND_SWITCH) && UM == ROWS_HALF && IM == ROWS_HALF);
+__device__ __forceinline__ __half2 half2_of(uint32_t w) { return *reinterpret_cast<const __half2*>(&w); }
+
+// One update.  rw is the rating as its record holds it; p_raw / q_raw are the row slices in their storage precision,
+// both replaced by the updated values.  The workers of a warp come here together, with `wmask` the whole warp - or,
+// where they may take different branches (ROWS_DYN), each with the mask of its own lanes.
 template <int K, int KIND, int UM, int IM, bool STATS>
-__device__ __forceinline__ void update_one(const Consts& c, float r, uint32_t uc, uint32_t ic, Raw<UM>& p_raw, Raw<IM>& q_raw,
-                                           bool sampled, Sample& smp, AfpState& afp, unsigned wmask) {
+__device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_t uc, uint32_t ic, Raw<UM>& p_raw, Raw<IM>& q_raw,
+                                           Sample& smp, AfpState& afp, unsigned wmask, unsigned gmask) {
     constexpr int TS = K / 8;
     if (STATS) { smp.user = false; smp.item = false; }
     if constexpr (KIND == KIND_MPT) {
         const V8f p = as_v8f(p_raw), q = as_v8f(q_raw);
         const V8h ph = narrow(p), qh = narrow(q);
-        const __half dot = worker_sum<TS>(pair_partial(ph, qh), wmask);
-        const __half2 e = __half2half2(__hmul_rn(c.mpt_scale, __hsub_rn(__float2half_rn(r), dot)));
-        const V8f gp = widen(grad(e, qh, c.mpt_lam, ph)), gq = widen(grad(e, ph, c.mpt_lam, qh));
+        const __half2 dot = worker_sum<TS>(pair_partial(ph, qh), wmask);
+        const __half2 e = __hmul2_rn(c.mpt_scale, __hsub2_rn(half2_of(rw), dot));
+        const V8f gp = widen(grad(e, qh, c.mpt_nlam, ph)), gq = widen(grad(e, ph, c.mpt_nlam, qh));
         V8f po, qo;
         const float2 lr2 = make_float2(c.lr, c.lr), rev2 = make_float2(c.mpt_rev, c.mpt_rev);
 #pragma unroll
@@ -614,39 +668,39 @@ __device__ __forceinline__ void update_one(const Consts& c, float r, uint32_t uc
         put(p_raw, po); put(q_raw, qo);
     } else if constexpr (KIND == KIND_MUPPET) {
         V8f p = as_v8f(p_raw), q = as_v8f(q_raw);
-        muppet_update<K>(c, r, p, q, smp.gp, smp.gq, wmask);
+        muppet_update<K>(c, __uint_as_float(rw), p, q, smp.gp, smp.gq, wmask);
         put(p_raw, p); put(q_raw, q);
-        if (STATS && sampled && c.bits != 32) smp.user = true;
+        if (STATS && c.bits != 32) smp.user = true;
     } else if constexpr (KIND == KIND_AFP) {
         V8f p = as_v8f(p_raw), q = as_v8f(q_raw);
-        afp_update<K>(c, afp, r, p, q, wmask);
+        afp_update<K>(c, afp, __uint_as_float(rw), p, q, gmask);
         put(p_raw, p); put(q_raw, q);
     } else if constexpr (KIND == KIND_MEMQUANT) {
         const V8f p = widen(as_v8h(p_raw)), q = widen(as_v8h(q_raw));
         const float part = (K == 128) ? chain_partial_k128(p, q) : pair_partial(p, q);
-        const float e = __fsub_rn(r, worker_sum<TS>(part, wmask));
+        const float e = __fsub_rn(__uint_as_float(rw), worker_sum<TS>(part, wmask));
         put(p_raw, narrow(step(c.lr, grad(e, q, c.lam, p), p)));
         put(q_raw, narrow(step(c.lr, grad(e, p, c.lam, q), q)));
     } else {
         const bool uf = is_f32<UM>(uc), itf = is_f32<IM>(ic);
         auto both_half = [&]() {
             const V8h p = as_v8h(p_raw), q = as_v8h(q_raw);
-            const __half dot = worker_sum<TS>(pair_partial(p, q), wmask);
-            const __half2 e = __half2half2(__hsub_rn(__float2half_rn(r), dot));
-            const V8h gp = grad(e, q, c.lam_h, p), gq = grad(e, p, c.lam_h, q);
+            const __half2 dot = worker_sum<TS>(pair_partial(p, q), wmask);
+            const __half2 e = __hsub2_rn(kHalfRating<KIND, UM, IM> ? half2_of(rw) : __float2half2_rn(__uint_as_float(rw)), dot);
+            const V8h gp = grad(e, q, c.nlam_h, p), gq = grad(e, p, c.nlam_h, q);
             put(p_raw, step(c.lr_h, gp, p));
             put(q_raw, step(c.lr_h, gq, q));
-            if (STATS && sampled) { smp.gp = widen(gp); smp.gq = widen(gq); smp.user = true; smp.item = true; }
+            if (STATS) { smp.gp = widen(gp); smp.gq = widen(gq); smp.user = true; smp.item = true; }
         };
         auto some_f32 = [&]() {
             const V8f p = uf ? as_v8f(p_raw) : widen(as_v8h(p_raw));
             const V8f q = itf ? as_v8f(q_raw) : widen(as_v8h(q_raw));
-            const float e = __fsub_rn(r, worker_sum<TS>(pair_partial(p, q), wmask));
+            const float e = __fsub_rn(__uint_as_float(rw), worker_sum<TS>(pair_partial(p, q), wmask));
             const V8f gp = grad(e, q, c.lam, p), gq = grad(e, p, c.lam, q);
             const V8f po = step(c.lr, gp, p), qo = step(c.lr, gq, q);
             if (uf) put(p_raw, po); else put(p_raw, narrow(po));
             if (itf) put(q_raw, qo); else put(q_raw, narrow(qo));
-            if (STATS && sampled) { smp.gp = gp; smp.gq = gq; smp.user = !uf; smp.item = !itf; }
+            if (STATS) { smp.gp = gp; smp.gq = gq; smp.user = !uf; smp.item = !itf; }
         };
         if constexpr (UM == ROWS_HALF && IM == ROWS_HALF) both_half();
         else if constexpr (UM != ROWS_DYN && IM != ROWS_DYN) some_f32();
@@ -659,175 +713,226 @@ __device__ __forceinline__ void update_one(const Consts& c, float r, uint32_t uc
 // an old row to every younger load that shares its scoreboard, which exposes one full memory
 // latency per rating; copy groups complete in order, so waiting for the group of rating j leaves
 // the copies of ratings j+1 .. j+D in flight.
-__device__ __forceinline__ void cp16(void* smem_dst, const void* gsrc) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gsrc) : "memory");
+// Shared memory is addressed by its 32-bit address.
+template <int OFF> __device__ __forceinline__ void cp16(unsigned dst, const unsigned char* src) {
+    asm volatile("cp.async.cg.shared.global [%0 + %2], [%1 + %2], 16;" ::"r"(dst), "l"(src), "n"(OFF) : "memory");
+}
+template <int OFF> __device__ __forceinline__ void cp16_if_row(uint32_t row, unsigned dst, const unsigned char* src) {
+    asm volatile("{ .reg .pred g; setp.ne.u32 g, %2, 0xffffffff; @g cp.async.cg.shared.global [%0 + %3], [%1 + %3], 16; }" ::"r"(dst), "l"(src), "r"(row), "n"(OFF) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ uint4 lds128(unsigned addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
 
 // Slot layout = row layout: the first 16 bytes of every lane, then (fp32 rows) the second 16 bytes of
 // every lane (layout.cuh), so that neither the 128-bit shared-memory accesses of neighbouring lanes collide
-// on a bank nor the global accesses of a worker touch partial sectors.
+// on a bank nor the global accesses of a worker touch partial sectors.  `slot` includes the lane's 16 m.
 template <int K, int MODE>
-__device__ __forceinline__ void cp_row(unsigned char* slot, const Arena& A, uint32_t code, int m) {
-    const uint32_t row = code & kIdMask;
-    if (is_f32<MODE>(code)) {
-        const unsigned char* g = reinterpret_cast<const unsigned char*>(A.f32 + (size_t)row * K) + 16 * m;
-        cp16(slot + 16 * m, g);
-        if constexpr (MODE != ROWS_HALF) cp16(slot + 2 * K + 16 * m, g + 2 * K);       // second half of the row
-    } else {
-        cp16(slot + 16 * m, reinterpret_cast<const unsigned char*>(A.f16 + (size_t)row * K) + 16 * m);
-    }
+__device__ __forceinline__ void cp_row(unsigned slot, const Rows<K, MODE>& A, uint32_t code) {
+    const unsigned char* g = A.at(code);
+    cp16<0>(slot, g);
+    if constexpr (MODE == ROWS_F32) cp16<2 * K>(slot, g);                                   // second half of the row
+    if constexpr (MODE == ROWS_DYN) cp16_if_row<2 * K>((code & kPrecBit) ? 0u : kNoRow, slot, g);
 }
 template <int K, int MODE>
-__device__ __forceinline__ Raw<MODE> lds_row(const unsigned char* slot, uint32_t code, int m) {
+__device__ __forceinline__ void cp_row_if(unsigned slot, const Rows<K, MODE>& A, uint32_t code) {      // kNoRow: nothing
+    const unsigned char* g = A.at(code);
+    cp16_if_row<0>(code, slot, g);
+    if constexpr (MODE == ROWS_F32) cp16_if_row<2 * K>(code, slot, g);
+    if constexpr (MODE == ROWS_DYN) cp16_if_row<2 * K>((code & kPrecBit) ? code : kNoRow, slot, g);
+}
+template <int K, int MODE>
+__device__ __forceinline__ Raw<MODE> lds_row(unsigned slot, uint32_t code) {
     Raw<MODE> r;
-    r.a = *reinterpret_cast<const uint4*>(slot + 16 * m);
-    if constexpr (MODE != ROWS_HALF) {
-        if (is_f32<MODE>(code)) r.b = *reinterpret_cast<const uint4*>(slot + 2 * K + 16 * m);
-    }
+    r.a = lds128(slot);
+    if constexpr (MODE == ROWS_F32) r.b = lds128(slot + 2 * K);
+    if constexpr (MODE == ROWS_DYN) { if (is_f32<MODE>(code)) r.b = lds128(slot + 2 * K); }
     return r;
 }
 
-// One rating as the worker's lanes read it from shared memory (one 128-bit broadcast load).
-constexpr uint32_t F_VALID = 1u;    // there is a rating at this position
-constexpr uint32_t F_UDUP = 2u;     // its user also occurs among the NS ratings before it: read the row at use
-constexpr uint32_t F_RS = 4u;       // its item differs from the item of the rating before it (a run starts)
-constexpr uint32_t F_IDUP = 8u;     // run start whose item also occurs among the NS ratings before it
+// One rating as the worker's lanes read it from shared memory (one 128-bit broadcast load): flags, item id, user id
+// (both without the marks nobody reads any more), rating.
+constexpr uint32_t F_UDUP = 1u;     // its user also occurs among the ratings whose update may not be in the copied row: read the row at use
+constexpr uint32_t F_RS = 2u;       // its item differs from the item of the rating before it (a run starts)
+constexpr uint32_t F_IDUP = 4u;     // run start whose item also occurs shortly before
+constexpr uint32_t F_DROP = 8u;     // the user row is not written back (an update of a very popular user, or no rating at all)
+constexpr uint32_t F_NONE = 16u;    // there is no rating at this position
 
 constexpr int kSpan = 8;            // consecutive chunks handed out together (the longest run of one ticket)
 
-// Shared memory of one worker: two chunks of records, then the user ring, then the item ring.  A ring
+// Shared memory of one worker: two chunks of records, what to request while each of them is processed (8 bytes: the
+// user row of the rating D further on, the item row of the rating DI further on if a run starts there), then the user
+// ring, then the item ring.  A ring
 // slot is as large as the widest row its side can hold in this launch.
 template <int K, int UM, int IM, int NS, int NSI> struct WorkerSmem {
     static constexpr int TS = K / 8;
     static constexpr int kURowBytes = K * (UM == ROWS_HALF ? 2 : 4);
     static constexpr int kIRowBytes = K * (IM == ROWS_HALF ? 2 : 4);
-    static constexpr int kRecBytes = 2 * TS * 16;
-    static constexpr int kBytes = kRecBytes + NS * kURowBytes + NSI * kIRowBytes;
+    static constexpr int kRecBytes = 2 * TS * 16 + 2 * TS * 8;
+    // The records of the workers of a warp are shifted by 16 bytes from worker to worker: those read at the same time
+    // then lie in different banks.  The rings stay at multiples of 128 bytes (off them, copies and loads of rows touch
+    // a line more each: 5.9 instead of 5.5 ms per epoch of the 100M-rating set).
+    static constexpr int kShift = 128;
+    static constexpr int kBytes = kRecBytes + kShift + NS * kURowBytes + NSI * kIRowBytes;
 };
 
-// NS / NSI: slots of the user / item ring.  User rows are requested D ratings ahead, item rows DI
-// ratings ahead (DI <= D <= NS-1, DI <= NSI-1).  The lead is kept as short as the memory latency allows: a row that another
-// worker updates between the request and the write-back loses that update, and the chance of that
-// grows with the lead.
+// NS / NSI: slots of the user / item ring.  User rows are requested D ratings ahead, item rows DI ratings ahead; a
+// user row is read from its slot one rating before its own, so a slot is free for the request of a rating D < NS ahead.
+// The lead is kept as short as the memory latency allows: an item row that another worker updates between the
+// request and the write-back loses that update, and the chance of that grows with the lead.
 template <int K, int KIND, int UM, int IM, bool STATS, int NS, int NSI, int D, int DI>
 __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !STATS) ? 4 : ((UM == ROWS_DYN || STATS || KIND == KIND_AFP) ? 2 : 3)) train_kernel(const KernelArgs a) {
     using SM = WorkerSmem<K, UM, IM, NS, NSI>;
     constexpr int TS = SM::TS;                     // lanes per worker = ratings per chunk
-    static_assert(TS % NS == 0, "the ring must divide the chunk");
-    static_assert(DI >= 1 && DI <= D && D == NS - 1 && DI <= NSI - 1 && NS % NSI == 0, "leads must fit the rings");
+    constexpr unsigned kAll = 0xffffffffu;
+    static_assert(TS % NS == 0 && (NS & (NS - 1)) == 0 && (NSI & (NSI - 1)) == 0, "the rings must divide the chunk");
+    static_assert(DI >= 1 && D >= 2 && DI <= D && D < NS && DI < NSI && NSI <= NS, "leads must fit the rings");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int m = lane % TS;
-    const unsigned wmask = (TS == 32) ? 0xffffffffu : (((1u << TS) - 1u) << (lane - m));
-    const uint64_t worker = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / TS;
-    const uint64_t W = a.workers;
-    const uint64_t nchunks = (a.s.n + TS - 1) / TS;
+    const unsigned gmask = ((1u << TS) - 1u) << (lane - m);      // the lanes of this worker
+    const unsigned worker = (blockIdx.x * blockDim.x + threadIdx.x) / TS;
+    const unsigned W = a.workers;
+    // fewer than 2^32 ratings, so chunks are counted in 32 bits
+    const unsigned nchunks = (unsigned)((a.s.n + TS - 1) / TS);
 
     unsigned char* const mine = smem_raw + (size_t)(threadIdx.x / TS) * SM::kBytes;
-    uint4* const recs = reinterpret_cast<uint4*>(mine);                  // [2][TS]
-    unsigned char* const uring = mine + SM::kRecBytes;                    // [NS][kURowBytes]
-    unsigned char* const iring = uring + NS * SM::kURowBytes;             // [NSI][kIRowBytes]
+    uint4* const recs = reinterpret_cast<uint4*>(mine + 16 * (lane / TS));      // [2][TS]
+    uint32_t* const reqs = reinterpret_cast<uint32_t*>(recs + 2 * TS);          // [2][TS][user, item]
+    const unsigned s_rec = (unsigned)__cvta_generic_to_shared(recs);
+    const unsigned s_req = s_rec + 2 * TS * 16;
+    const unsigned uring = (unsigned)__cvta_generic_to_shared(mine) + SM::kRecBytes + SM::kShift + 16 * m;      // [NS][kURowBytes]
+    const unsigned iring = uring + NS * SM::kURowBytes;                   // [NSI][kIRowBytes]
+    const Rows<K, UM> P(a.P, m);
+    const Rows<K, IM> Q(a.Q, m);
 
     Consts c;
     c.lr = a.lr; c.lam = a.lam;
     c.lr_h = __half2half2(__float2half_rn(a.lr));
-    c.lam_h = __half2half2(__float2half_rn(a.lam));
-    c.mpt_scale = __float2half_rn(1000.0f);
-    c.mpt_lam = __half2half2(__float2half_rn(__fmul_rn(a.lam, 1000.0f)));
+    c.nlam_h = __half2half2(__float2half_rn(-a.lam));
+    c.mpt_scale = __float2half2_rn(1000.0f);
+    c.mpt_nlam = __half2half2(__float2half_rn(-__fmul_rn(a.lam, 1000.0f)));
     c.mpt_rev = __fdiv_rn(1.0f, 1000.0f);
     c.bits = a.bits;
     c.afp_epoch = a.epoch;
     c.afp_init_threshold = (int)((float)((a.s.n + W - 1) / W) / 10.0f);
     // only the mixed-precision mode reads the precision bit of an id
-    constexpr uint32_t kKeep = (UM == ROWS_DYN || IM == ROWS_DYN) ? 0xffffffffu : (kIdMask | kHotBit);
-
-    if (worker >= W) return;
+    constexpr uint32_t kKeep = (UM == ROWS_DYN || IM == ROWS_DYN) ? (kPrecBit | kIdMask) : kIdMask;
 
     // ---- which chunks this worker processes ----
     // Runs of consecutive chunks: first the static runs [worker*kSpan, +kSpan) and [(worker+W)*kSpan,
     // +kSpan), then runs handed out by the shared counter, which counts chunks beyond the static part.
     // A dynamic run is kSpan chunks long while plenty of work is left and shrinks to a single chunk as
     // the counter nears the end (its length is what is left, as seen at the previous ticket, divided by
-    // twice the number of workers), so that the workers finish within about one chunk of each other.  A
+    // about twice the number of workers), so that the workers finish within about one chunk of each other.  A
     // ticket is requested one run before it is needed and stays in lane 0 until then, so the launch
-    // neither waits for the counter nor depends on all blocks being resident.
-    const uint64_t static_chunks = 2 * W * kSpan;
-    const uint64_t dyn_chunks = nchunks > static_chunks ? nchunks - static_chunks : 0;
-    auto run_length = [&](unsigned long long seen) -> unsigned {
-        const uint64_t left = dyn_chunks > seen ? dyn_chunks - seen : 0;
-        const uint64_t g = left / (2 * W);
-        return g >= (uint64_t)kSpan ? (unsigned)kSpan : (g < 1 ? 1u : (unsigned)g);
+    // neither waits for the counter nor depends on all blocks being resident.  Lanes beyond the last worker keep
+    // their warp company without chunks of their own.
+    // The code from here to the end of the loop has no branch that the workers of a warp could take differently: what
+    // only some lanes do is predicated.  (With divergent branches around, the compiler puts a warp barrier in front
+    // of every shuffle and vote of the loop.)
+    const unsigned static_chunks = 2 * W * kSpan;
+    const unsigned dyn_chunks = nchunks > static_chunks ? nchunks - static_chunks : 0;
+    const unsigned share_log2 = 32 - __clz(2 * W - 1);              // 2 W rounded up to a power of two
+    auto run_length = [&](unsigned seen) -> unsigned {
+        const unsigned g = (dyn_chunks > seen ? dyn_chunks - seen : 0) >> share_log2;
+        return min(max(g, 1u), (unsigned)kSpan);
     };
-    uint64_t run_cur = worker * kSpan, run_next = (worker + W) * kSpan;
+    // lane 0 of a worker takes `len` chunks off the shared counter
+    auto draw_ticket = [&](bool go, unsigned len) -> unsigned {
+        unsigned long long t = 0;
+        asm volatile("{ .reg .pred g; setp.ne.u32 g, %1, 0; @g atom.global.add.u64 %0, [%2], %3; }" : "+l"(t) : "r"((unsigned)(go && m == 0)), "l"(a.next_chunk),
+                     "l"((unsigned long long)len) : "memory");
+        return (unsigned)t;
+    };
+    const bool works = worker < W;
+    unsigned run_cur = works ? worker * kSpan : nchunks, run_next = (worker + W) * kSpan;
     unsigned len_cur = kSpan, len_next = kSpan, kin = 0;
-    unsigned tlen = run_length(0);
-    unsigned long long ticket = (m == 0) ? atomicAdd(a.next_chunk, (unsigned long long)tlen) : 0ull;
+    unsigned tlen = run_length(0), ticket = draw_ticket(works, tlen);
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.zero_counter = 0ull;      // the counter of the launch after next
-    auto next_chunk_id = [&]() -> uint64_t {
-        if (run_cur >= nchunks) return ~0ull;
-        const uint64_t ci = run_cur + kin;
-        if (++kin == len_cur) {
+    auto next_chunk_id = [&]() -> unsigned {
+        const bool left = run_cur < nchunks;
+        const unsigned ci = left ? run_cur + kin : nchunks;
+        const bool turn = left && ++kin == len_cur;
+        const unsigned drawn = __shfl_sync(kAll, ticket, 0, TS), drawn_len = __shfl_sync(kAll, tlen, 0, TS);
+        if (turn) {
             kin = 0;
             run_cur = run_next; len_cur = len_next;
-            const unsigned lo = __shfl_sync(wmask, (unsigned)ticket, 0, TS), hi = __shfl_sync(wmask, (unsigned)(ticket >> 32), 0, TS);
-            len_next = __shfl_sync(wmask, tlen, 0, TS);
-            run_next = static_chunks + (((uint64_t)hi << 32) | lo);
-            if (m == 0) { tlen = run_length(ticket); ticket = atomicAdd(a.next_chunk, (unsigned long long)tlen); }
+            len_next = drawn_len;
+            run_next = static_chunks + drawn;
+            tlen = run_length(drawn);
         }
-        return ci < nchunks ? ci : ~0ull;
+        const unsigned t = draw_ticket(turn, tlen);
+        if (turn) ticket = t;
+        return ci;
     };
 
     // ---- chunk pipeline: global loads (registers) -> flags -> records in shared memory -> use ----
-    struct Loaded { float r; uint32_t u, i; int cnt; uint64_t base; };
-    auto fetch_chunk = [&](uint64_t ci) {
-        Loaded k; k.r = 0.f; k.u = kNoRow; k.i = kNoRow; k.cnt = 0; k.base = 0;
-        if (ci < nchunks) {
-            k.base = ci * TS;
-            const uint64_t left = a.s.n - k.base;
-            k.cnt = left < (uint64_t)TS ? (int)left : TS;
-            if (m < k.cnt) {
-                k.r = __ldg(a.s.r + k.base + m);
-                k.u = __ldg(a.s.u + k.base + m) & kKeep;
-                k.i = __ldg(a.s.i + k.base + m) & kKeep;
-            }
-        }
+    struct Loaded { float r; uint32_t u, i; int cnt; };
+    auto fetch_chunk = [&](unsigned ci) {
+        Loaded k;
+        const uint64_t base = (uint64_t)ci * TS;
+        k.cnt = ci < nchunks ? (int)min((uint64_t)TS, a.s.n - base) : 0;
+        const bool in = m < k.cnt;
+        const uint64_t at = in ? base + m : 0;         // any rating there is
+        k.r = __ldg(a.s.r + at);
+        k.u = __ldg(a.s.u + at);
+        k.i = __ldg(a.s.i + at) & kKeep;
+        if (!in) { k.u = kNoRow; k.i = kNoRow; }
         return k;
     };
+    unsigned hot_seen = worker;             // counts the ratings of marked users this worker has met
+    const unsigned hot_mask = (1u << a.hot_user_shift) - 1u;
     uint32_t prev_u = kNoRow, prev_i = kNoRow;        // lane m: rating m of the chunk before `inflight`
     Loaded inflight = fetch_chunk(next_chunk_id());
-    uint64_t base0 = 0, base1 = 0;              // stream position of the first rating of each buffer
-    // Turns `inflight` into records in buffer `b` and starts loading the chunk after it.
-    auto publish = [&](int b) {
+    // Turns `inflight` into records in buffer `b` and starts loading the chunk after it; returns its rating count.
+    auto publish = [&](int b) -> int {
+        __syncwarp();
+        const bool valid = m < inflight.cnt;
+        // A marked user (see the set-up): every 2^shift-th update of marked rows that this worker meets is written
+        // back; the others are dropped.
+        const bool hot = valid && (inflight.u & kHotBit) && a.add_user_delta;
+        const unsigned hot_set = (__ballot_sync(kAll, hot) & gmask) >> (lane - m);
+        const bool drop = hot && ((hot_seen + __popc(hot_set & ((2u << m) - 1u))) & hot_mask) != 0u;
+        hot_seen += __popc(hot_set);
+        const uint32_t u = valid ? inflight.u & kKeep : kNoRow, i = inflight.i;
         bool udup = false, idup = false, rs = false;
 #pragma unroll
-        for (int d = 1; d <= NS; d++) {
+        for (int d = 1; d <= (D > DI + 2 ? D + 1 : DI + 3); d++) {
             // the rating d places earlier: lane m-d of this chunk, or lane m-d+TS of the previous one;
             // the SOURCE lane knows which of its two values a reader d lanes further on wants
             const bool from_this = m < TS - d;
-            const uint32_t su = __shfl_sync(wmask, from_this ? inflight.u : prev_u, (m - d) & (TS - 1), TS);
-            const uint32_t si = __shfl_sync(wmask, from_this ? inflight.i : prev_i, (m - d) & (TS - 1), TS);
-            udup |= su == inflight.u;
-            if (d == 1) rs = si != inflight.i; else idup |= si == inflight.i;
+            if (d <= D + 1) udup |= __shfl_sync(kAll, from_this ? u : prev_u, (m - d) & (TS - 1), TS) == u;
+            if (d <= DI + 3) {
+                const bool same = __shfl_sync(kAll, from_this ? i : prev_i, (m - d) & (TS - 1), TS) == i;
+                if (d == 1) rs = !same; else idup |= same;
+            }
         }
-        uint32_t f = 0;
-        if (m < inflight.cnt) f = F_VALID | (udup ? F_UDUP : 0u) | (rs ? F_RS : 0u) | ((rs && idup) ? F_IDUP : 0u);
-        recs[b * TS + m] = make_uint4(f, inflight.i, inflight.u, __float_as_uint(inflight.r));
-        if (b) base1 = inflight.base; else base0 = inflight.base;
-        prev_u = inflight.u; prev_i = inflight.i;
-        inflight = (inflight.cnt > 0) ? fetch_chunk(next_chunk_id()) : inflight;
-        __syncwarp(wmask);
+        // The position after a worker's last rating starts a run of nothing, which writes the last item row back.
+        const uint32_t f = valid ? (udup ? F_UDUP : 0u) | (rs ? F_RS : 0u) | ((rs && idup) ? F_IDUP : 0u) | (drop ? F_DROP : 0u)
+                                 : F_NONE | F_DROP | (m == inflight.cnt ? F_RS : 0u);
+        uint32_t rw = __float_as_uint(inflight.r);
+        if constexpr (kHalfRating<KIND, UM, IM>) { const __half2 h = __float2half2_rn(inflight.r); rw = *reinterpret_cast<const uint32_t*>(&h); }
+        recs[b * TS + m] = make_uint4(f, valid ? i : 0u, valid ? u : 0u, rw);
+        const int pos = b * TS + m;
+        reqs[2 * ((pos - D) & (2 * TS - 1))] = valid ? u : 0u;
+        reqs[2 * ((pos - DI) & (2 * TS - 1)) + 1] = (f & F_RS) ? (valid ? i : 0u) : kNoRow;
+        prev_u = u; prev_i = i;
+        const int cnt = inflight.cnt;
+        inflight = fetch_chunk(next_chunk_id());
+        __syncwarp();
+        return cnt;
     };
-    publish(0);
-    publish(1);
+    int cnt_cur = publish(0), cnt_next = publish(1);
 
-    unsigned hot_seen = worker;                       // counts the ratings of marked users this worker has met
-    const unsigned hot_mask = (1u << a.hot_user_shift) - 1u;
     // item row of the current run
-    uint32_t cur_ic = kNoRow;
-    Raw<IM> q;
+    uint32_t cur_ic = 0;
+    unsigned have_item = 0;                          // F_RS while there is one
+    Raw<IM> q = Raw<IM>();
 
     // item-side statistics of the current run of equal item groups
     V8f gq_acc; float nq_acc = 0.f; uint32_t acc_group = kNoRow;
@@ -848,7 +953,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
             // muppet_sgd_kernel.h:266-285, sgd_kernel.h:266-285: the squared norm of both gradients goes to the
             // worker's running sum, the element-wise sum of both gradients to k shared accumulators
             if (smp.user) {
-                const float n = worker_sum<TS>(muppet_norm_partial<K>(smp.gp, smp.gq), wmask);
+                const float n = worker_sum<TS>(muppet_norm_partial<K>(smp.gp, smp.gq), gmask);
                 V8f both;
 #pragma unroll
                 for (int t = 0; t < 8; t++) both.x[t] = __fadd_rn(smp.gp.x[t], smp.gq.x[t]);
@@ -859,13 +964,13 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
         }
         if (smp.user) {
             const uint32_t g = a.st.ugroup[uc & kIdMask];
-            const float n = worker_sum<TS>(pair_partial(smp.gp, smp.gp), wmask);
+            const float n = worker_sum<TS>(pair_partial(smp.gp, smp.gp), gmask);
             red_add8(gsum_p + (size_t)g * K + 8 * m, smp.gp);
             if (m == 0) atomicAdd(nsum_p + g, n);
         }
         if (smp.item) {
             const uint32_t g = a.st.igroup[ic & kIdMask];
-            const float n = worker_sum<TS>(pair_partial(smp.gq, smp.gq), wmask);
+            const float n = worker_sum<TS>(pair_partial(smp.gq, smp.gq), gmask);
             if (g != acc_group) {
                 flush_item_stats();
                 acc_group = g; nq_acc = 0.f;
@@ -881,95 +986,72 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     AfpState afp;
     afp.user = AfpSide{8, 1.f, 0.f, 0}; afp.item = afp.user; afp.back = afp.user; afp.cur = 0;
 
-    // requests the user row of the rating with record `rx` / the item row of the rating whose first
-    // two record words are `ri`, into ring slot `slot`
-    auto request_user = [&](const uint4& rx, int slot) {
-        if ((rx.x & (F_VALID | F_UDUP)) == F_VALID) cp_row<K, UM>(uring + slot * SM::kURowBytes, a.P, rx.z, m);
-    };
-    auto request_item = [&](const uint2& ri, int slot) {
-        if ((ri.x & (F_VALID | F_RS | F_IDUP)) == (F_VALID | F_RS)) cp_row<K, IM>(iring + slot * SM::kIRowBytes, a.Q, ri.y, m);
-    };
-    // Copy groups complete in order.  Every iteration commits two: first the item row of the rating
-    // DI ahead, then the user row of the rating D ahead.  When rating j is used, the groups younger
-    // than its item row's are 2*DI-1 and those younger than its user row's are 2*(D-1); waiting for
-    // exactly that many to remain pending leaves every younger copy in flight.
-    constexpr int kPendUser = 2 * (D - 1);
-    constexpr int kPendItem = (2 * DI - 1 < kPendUser) ? 2 * DI - 1 : kPendUser;
-    // The records of the ratings j .. j+D live in a register queue indexed like the user ring (the
-    // record of rating x in slot x mod NS): each record is read from shared memory once, D ratings
-    // before its rating is processed, and serves the user request, the item request and the update.
-    uint4 rq[NS];
-    // prologue: the groups of the iterations -D .. -1
+    // requests the user row / the item row of a rating into ring slot `slot`
+    auto request_user = [&](uint32_t uc, int slot) { cp_row<K, UM>(uring + slot * SM::kURowBytes, P, uc); };
+    auto request_item = [&](uint32_t ic, int slot) { cp_row_if<K, IM>(iring + slot * SM::kIRowBytes, Q, ic); };
+    // Copy groups complete in order, and every rating commits one: the item row of the rating DI ahead and the user
+    // row of the rating D ahead.  Before rating j commits, the groups younger than the user row of rating j+1 are
+    // D - 2, those younger than the item row of rating j are DI - 1: waiting for exactly that many to remain
+    // pending leaves every younger copy in flight.
 #pragma unroll
     for (int t = 0; t < D; t++) {
-        rq[t] = recs[t];
-        if (t - (D - DI) >= 0) request_item(make_uint2(rq[t - (D - DI)].x, rq[t - (D - DI)].y), (t - (D - DI)) & (NSI - 1));
-        cp_commit();
-        request_user(rq[t], t);
+        if (t >= D - DI) request_item((recs[t - (D - DI)].x & F_RS) ? recs[t - (D - DI)].y : kNoRow, (t - (D - DI)) & (NSI - 1));
+        request_user(recs[t].z, t);
         cp_commit();
     }
+    uint4 rec = recs[0];
+    cp_wait<D - 1>();
+    Raw<UM> p = lds_row<K, UM>(uring, rec.z);
 
     int cb = 0;                                     // buffer of the chunk in use
-    for (;;) {
-        const uint4* const rc = recs + cb * TS;
-        const uint4* const rn = recs + (cb ^ 1) * TS;
-        bool more = true;
+    while (__any_sync(kAll, cnt_cur > 0)) {
 #pragma unroll 1
-        for (int jb = 0; jb < TS && more; jb += NS) {
+        for (int jb = 0; jb < TS; jb += NS) {
+            // this group of NS records and the next one (in the other buffer at the end of a chunk)
+            const unsigned r0 = s_rec + 16 * (cb * TS + jb), r1 = s_rec + 16 * ((cb * TS + jb + NS) & (2 * TS - 1));
+            const unsigned q0 = s_req + 8 * (cb * TS + jb);
 #pragma unroll
             for (int t = 0; t < NS; t++) {
-                const int j = jb + t;
-                {   // the record of the rating D ahead takes the slot of the rating processed last
-                    const int x = j + D;
-                    rq[(t + D) & (NS - 1)] = (x < TS) ? rc[x] : rn[x - TS];
+                const uint32_t uc = rec.z, ic = rec.y, f = rec.x, rw = rec.w;
+                if (__any_sync(kAll, f & (F_RS | F_UDUP))) {
+                    // a run of equal items ends for at least one of the warp's workers (or a row has to be read again)
+                    cp_wait<DI - 1>();
+                    const unsigned start = f & F_RS;
+                    st_row_if<K, IM>(start & have_item, Q, cur_ic, q);
+                    const unsigned slot = iring + (t & (NSI - 1)) * SM::kIRowBytes;
+                    lds_if<0>(start, q.a, slot);
+                    if constexpr (IM != ROWS_HALF) lds_if<2 * K>(second_half<IM>(start, ic), q.b, slot);
+                    if (__any_sync(kAll, f & (F_IDUP | F_UDUP))) {
+                        ld_row_if<K, IM>(f & F_IDUP, q, Q, ic);
+                        ld_row_if<K, UM>(f & F_UDUP, p, P, uc);
+                    }
+                    if (start) { cur_ic = ic; have_item = (f & F_NONE) ? 0u : F_RS; }
                 }
-                const uint4 rec = rq[t];
-                if (!(rec.x & F_VALID)) { more = false; break; }
-                const uint32_t uc = rec.z, ic = rec.y;
-                const float r = __uint_as_float(rec.w);
-                const bool sampled = STATS && ((cb ? base1 : base0) + j >= a.st.first_sample_pos);
-                if (rec.x & F_RS) {
-                    cp_wait<kPendItem>();
-                    if (cur_ic != kNoRow) st_row<K, IM>(a.Q, cur_ic, m, q);
-                    if (rec.x & F_IDUP) q = ld_row<K, IM>(a.Q, ic, m);
-                    else q = lds_row<K, IM>(iring + (t & (NSI - 1)) * SM::kIRowBytes, ic, m);
-                    cur_ic = ic;
-                } else {
-                    cp_wait<kPendUser>();
-                }
-                Raw<UM> p;
-                if (rec.x & F_UDUP) p = ld_row<K, UM>(a.P, uc, m);
-                else p = lds_row<K, UM>(uring + t * SM::kURowBytes, uc, m);
-                // request the user row of the rating D ahead and the item row of the rating DI ahead,
-                // into slots whose previous contents have been consumed
-                {
-                    const uint4& ri = rq[(t + DI) & (NS - 1)];
-                    request_item(make_uint2(ri.x, ri.y), (t + DI) & (NSI - 1));
-                    cp_commit();
-                    request_user(rq[(t + D) & (NS - 1)], (t + D) & (NS - 1));
-                    cp_commit();
-                }
+                // the next rating's record and user row
+                rec = lds128(t + 1 < NS ? r0 + 16 * (t + 1) : r1);
+                cp_wait<D - 2>();
+                const Raw<UM> p_next = lds_row<K, UM>(uring + ((t + 1) & (NS - 1)) * SM::kURowBytes, rec.z);
+                // requests into slots whose contents have been consumed
+                uint32_t req_u, req_i;
+                asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(req_u), "=r"(req_i) : "r"(q0 + 8 * t) : "memory");
+                request_item(req_i, (t + DI) & (NSI - 1));
+                request_user(req_u, (t + D) & (NS - 1));
+                cp_commit();
                 const Raw<UM> p_before = p;
-                update_one<K, KIND, UM, IM, STATS>(c, r, uc, ic, p, q, sampled, smp, afp, wmask);
-                if (a.add_user_delta) {
-                    // A marked user (see the set-up): every 2^shift-th update of a marked row that this worker meets
-                    // is written back; the others are dropped.
-                    bool keep = true;
-                    if (uc & kHotBit) keep = ((++hot_seen) & hot_mask) == 0u;
-                    if (keep) add_row_delta<K, UM>(a.P, uc, m, p, p_before);
-                } else {
-                    st_row<K, UM>(a.P, uc, m, p);
-                }
-                if (STATS && sampled) record(smp, uc, ic);
+                constexpr bool kDyn = UM == ROWS_DYN || IM == ROWS_DYN;
+                update_one<K, KIND, UM, IM, STATS>(c, rw, uc, ic, p, q, smp, afp, kDyn ? gmask : kAll, gmask);
+                if (a.add_user_delta) add_row_delta<K, UM>(P, uc, f & F_DROP, p, p_before);
+                else st_row_if<K, UM>(~f & F_DROP, P, uc, p);
+                if (STATS) { if (!(f & F_NONE)) record(smp, uc, ic); }
+                p = p_next;
             }
         }
-        if (!more) break;
-        __syncwarp(wmask);           // every lane has read this buffer's records
-        publish(cb);                 // the chunk after next takes the buffer of the finished one
+        cnt_cur = cnt_next;
+        cnt_next = publish(cb);      // the chunk after next takes the buffer of the finished one
         cb ^= 1;
     }
     cp_wait<0>();
-    if (cur_ic != kNoRow) st_row<K, IM>(a.Q, cur_ic, m, q);
+    st_row_if<K, IM>(have_item, Q, cur_ic, q);
     if (STATS) {
         if constexpr (KIND == KIND_MUPPET || KIND == KIND_SWITCH) { if (m == 0) atomicAdd(nsum_p, nq_acc); }
         else flush_item_stats();
@@ -1063,7 +1145,9 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
     // and the occupancy query trims the number of blocks per SM accordingly.
     // (Requesting fp32 item rows two ratings ahead, into an item ring of four slots, was measured as well and
     // changed nothing either - 13.99 against 14.06 ms per promoted epoch on the 100M-rating configuration.)
-    return launch_ns<K, KIND, UM, IM, STATS, 4, 2, 3, 1>(args, per_sm, workers, st, shape, dry);
+    constexpr bool kFixedPoint = KIND == KIND_AFP || KIND == KIND_MUPPET;
+    constexpr int NS = kFixedPoint ? 4 : 8, D = kFixedPoint ? 3 : 5, DI = kFixedPoint ? 2 : 3;
+    return launch_ns<K, KIND, UM, IM, STATS, NS, 4, D, DI>(args, per_sm, workers, st, shape, dry);
 }
 
 template <int K, int KIND, int UM, int IM>
