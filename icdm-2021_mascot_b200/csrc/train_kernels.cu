@@ -339,21 +339,30 @@ struct KernelArgs {
 // Power-of-two scale for a `bits`-wide fixed-point grid that covers [lo, hi]: the reference takes
 // floor(log2(min(|qmax/hi|, |qmin/lo|))) with qmax = 2^(bits-1)-0.5, qmin = -2^(bits-1)-0.5, stores
 // it in an unsigned index (negative -> 0) and scales by 2^index.
-__device__ __forceinline__ float muppet_scale(int bits, float hi, float lo) {
-    if (hi == 0.f && lo == 0.f) return 1.f;
-    const float val = (float)(1 << (bits - 1));
-    const float top = __fadd_rn(__fsub_rn(val, 1.f), 0.5f), bottom = __fsub_rn(-val, 0.5f);
+__device__ __noinline__ float muppet_scale_exact(float top, float bottom, float hi, float lo) {
     const float best = fminf(fabsf(__fdiv_rn(top, hi)), fabsf(__fdiv_rn(bottom, lo)));
     const float idx = floorf(log2f(best));
     if (!(idx > 0.f)) return 1.f;
     const int e = idx > 127.f ? 128 : (int)idx;
     return e >= 128 ? __int_as_float(0x7f800000) : __int_as_float((e + 127) << 23);
 }
+// The scale is a power of two and only floor(log2) of the smaller quotient decides it, which the bit patterns tell
+// without a division: as integers, bits(a) - bits(b) has floor(log2(a / b)) above bit 23 for normal a, b > 0 (the
+// difference of the exponents, less one when the mantissa of b is the larger).  Where the quotient is within 256 units of
+// a power of two - once in ten thousand ratings - or an operand is zero or denormal, the formula itself decides, with its
+// rounded divisions and logarithm.
+__device__ __forceinline__ float muppet_scale(int bits, float hi, float lo) {
+    const float val = (float)(1 << (bits - 1));
+    const float top = __fadd_rn(__fsub_rn(val, 1.f), 0.5f), bottom = __fsub_rn(-val, 0.5f);
+    const int d = min(__float_as_int(top) - (__float_as_int(hi) & 0x7fffffff), __float_as_int(-bottom) - (__float_as_int(lo) & 0x7fffffff));
+    float s = __int_as_float((max(d, 0) & 0x7f800000) + 0x3f800000);
+    if (((d + 256) & 0x007fffff) < 512 || d >= (120 << 23)) s = (hi == 0.f && lo == 0.f) ? 1.f : muppet_scale_exact(top, bottom, hi, lo);
+    return s;
+}
 // roundf (halves away from zero) in three instructions: trunc(x + copysign(largest float below one half, x)).
 // The sum is rounded to nearest-even, which is what makes it exact: x = n + f with f < 1/2 cannot reach n + 1,
 // f >= 1/2 always does.  Equal to roundf for every one of the 2^32 float patterns (checked exhaustively on the
-// host, tests/round_check.c); the library routine costs about three times as much and these trainers call it
-// 34 times per rating and lane.
+// host, tests/round_check.c); the library routine costs about three times as much.
 __device__ __forceinline__ float round_away(float x) {
     const float h = __uint_as_float((__float_as_uint(x) & 0x80000000u) | 0x3effffffu);
     return truncf(__fadd_rn(x, h));
@@ -365,13 +374,56 @@ __device__ __forceinline__ float pow2_rev(float s) {
     return (b >= 0x00800000u && b < 0x7f000000u && !(b & 0x007fffffu)) ? __uint_as_float(0x7f000000u - b) : __fdiv_rn(1.f, s);
 }
 __device__ __forceinline__ float fix_round(float v, float s, float s_rev) { return __fmul_rn(round_away(__fmul_rn(v, s)), s_rev); }
-// Clamp to the int8 range, then to integer.  Every caller passes a value that round_away has already made
-// integral, so the one conversion instruction with saturation (truncating, which changes nothing then) equals
-// v > 127 ? 127 : (v < -128 ? -128 : (int)v).
-__device__ __forceinline__ int sat8(float v) {
-    int r;
-    asm("cvt.rzi.sat.s8.f32 %0, %1;" : "=r"(r) : "f"(v));
-    return r;
+// The eight values of a lane times a power-of-two scale, rounded like round_away - with full-rate instructions, two
+// values at a time, in place of truncations and conversions, which run at an eighth of that rate and were 64 of an
+// update's instructions.  x s is exact, so adding 1.5 * 2^23 in one multiply-add rounds it to the nearest integer, and the
+// two roundings differ at exact halves only: `odd` receives the largest distance from the integers, and a warp
+// that meets one half (rare: it takes the bits of x below the grid to be 100...0) rounds again the long way.  Results are
+// exact below 2^22, larger ones stay above 2^21, and zero is +0.
+__device__ __forceinline__ V8f quantize_near(const V8f& x, float s, float& odd) {
+    V8f o;
+    float far[4];
+    const float2 s2 = make_float2(s, s), magic = make_float2(12582912.f, 12582912.f), minus = make_float2(-12582912.f, -12582912.f);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const float2 r = __fadd2_rn(__ffma2_rn(pr(x, j), s2, magic), minus);
+        const float2 d = __ffma2_rn(pr(x, j), s2, make_float2(-r.x, -r.y));
+        far[j] = fmaxf(fabsf(d.x), fabsf(d.y));
+        set_pr(o, j, r);
+    }
+    odd = fmaxf(fmaxf(far[0], far[1]), fmaxf(far[2], far[3]));
+    return o;
+}
+__device__ __forceinline__ V8f quantize_away(const V8f& x, float s) {
+    V8f o;
+#pragma unroll
+    for (int t = 0; t < 8; t++) o.x[t] = __fadd_rn(round_away(__fmul_rn(x.x[t], s)), 0.f);
+    return o;
+}
+__device__ __forceinline__ void quantize(const V8f& p, float sp, const V8f& q, float sq, V8f& pi, V8f& qi, unsigned wmask) {
+    float odd_p, odd_q;
+    pi = quantize_near(p, sp, odd_p);
+    qi = quantize_near(q, sq, odd_q);
+    if (__any_sync(wmask, !(fmaxf(odd_p, odd_q) < 0.5f))) { pi = quantize_away(p, sp); qi = quantize_away(q, sq); }
+}
+// The int8 passes work on the integers as floats: products and sums of int8 values stay far below 2^24.
+__device__ __forceinline__ float clamp8(float v) { return v == v ? fminf(fmaxf(v, -128.f), 127.f) : 0.f; }
+__device__ __forceinline__ V8f clamp8(const V8f& x) {
+    V8f o;
+#pragma unroll
+    for (int t = 0; t < 8; t++) o.x[t] = clamp8(x.x[t]);
+    return o;
+}
+__device__ __forceinline__ float quantize8(float v, float s) { return clamp8(round_away(__fmul_rn(v, s))); }
+// A quantize()d row in binary16; what rounded to zero keeps its sign, as it does in fix_round
+__device__ __forceinline__ V8h grid_half(const V8f& r, const V8f& x, float s_rev) {
+    V8h h;
+    const float2 rev2 = make_float2(s_rev, s_rev);
+    auto signed_as = [](float v, float like) { return __uint_as_float(__float_as_uint(v) | (__float_as_uint(like) & 0x80000000u)); };
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+        h.v[t] = __float22half2_rn(__fmul2_rn(make_float2(signed_as(r.x[2 * t], x.x[2 * t]), signed_as(r.x[2 * t + 1], x.x[2 * t + 1])), rev2));
+    return h;
 }
 __device__ __forceinline__ V8h fix_round_half(const V8f& x, float s, float s_rev) {
     V8h h;
@@ -380,15 +432,39 @@ __device__ __forceinline__ V8h fix_round_half(const V8f& x, float s, float s_rev
         h.v[t] = __floats2half2_rn(fix_round(x.x[2 * t], s, s_rev), fix_round(x.x[2 * t + 1], s, s_rev));
     return h;
 }
-template <int TS> __device__ __forceinline__ float worker_min(float x, unsigned wmask) {
-#pragma unroll
-    for (int d = TS / 2; d >= 1; d >>= 1) x = fminf(x, __shfl_xor_sync(wmask, x, d));
-    return x;
+// Both quantize()d rows on their grids; `big`: some value may reach 2^21 steps of its grid
+__device__ __forceinline__ void to_grid(const V8f& p, const V8f& pi, float sp, const V8f& q, const V8f& qi, float sq, bool big, V8h& ph, V8h& qh) {
+    const float sp_rev = pow2_rev(sp), sq_rev = pow2_rev(sq);
+    if (big) { ph = fix_round_half(p, sp, sp_rev); qh = fix_round_half(q, sq, sq_rev); }
+    else { ph = grid_half(pi, p, sp_rev); qh = grid_half(qi, q, sq_rev); }
+}
+__device__ __forceinline__ float abs_max8(const V8f& x) {
+    return fmaxf(fmaxf(fmaxf(fabsf(x.x[0]), fabsf(x.x[1])), fmaxf(fabsf(x.x[2]), fabsf(x.x[3]))),
+                 fmaxf(fmaxf(fabsf(x.x[4]), fabsf(x.x[5])), fmaxf(fabsf(x.x[6]), fabsf(x.x[7]))));
 }
 template <int TS> __device__ __forceinline__ float worker_max(float x, unsigned wmask) {
 #pragma unroll
     for (int d = TS / 2; d >= 1; d >>= 1) x = fmaxf(x, __shfl_xor_sync(wmask, x, d));
     return x;
+}
+// Four maxima over a worker's lanes.  The first two steps halve what a lane holds instead of reducing all four
+// everywhere: nine shuffles (k=128) in place of sixteen.
+template <int TS> __device__ __forceinline__ void worker_max4(float (&a)[4], unsigned wmask) {
+    const int m = threadIdx.x & (TS - 1);
+    const bool up = m & (TS / 2), up2 = m & (TS / 4);
+    float r0 = fmaxf(up ? a[2] : a[0], __shfl_xor_sync(wmask, up ? a[0] : a[2], TS / 2));
+    const float r1 = fmaxf(up ? a[3] : a[1], __shfl_xor_sync(wmask, up ? a[1] : a[3], TS / 2));
+    r0 = fmaxf(up2 ? r1 : r0, __shfl_xor_sync(wmask, up2 ? r0 : r1, TS / 4));
+#pragma unroll
+    for (int d = TS / 8; d >= 1; d >>= 1) r0 = fmaxf(r0, __shfl_xor_sync(wmask, r0, d));
+#pragma unroll
+    for (int i = 0; i < 4; i++) a[i] = __shfl_sync(wmask, r0, (i >> 1) * (TS / 2) + (i & 1) * (TS / 4), TS);
+}
+__device__ __forceinline__ float max8(const V8f& x) {
+    return fmaxf(fmaxf(fmaxf(x.x[0], x.x[1]), fmaxf(x.x[2], x.x[3])), fmaxf(fmaxf(x.x[4], x.x[5]), fmaxf(x.x[6], x.x[7])));
+}
+__device__ __forceinline__ float min8(const V8f& x) {
+    return fminf(fminf(fminf(x.x[0], x.x[1]), fminf(x.x[2], x.x[3])), fminf(fminf(x.x[4], x.x[5]), fminf(x.x[6], x.x[7])));
 }
 // Squared norm of both gradients the way the reference groups it: per reference lane
 // (norm_p + norm_q), then the lane tree.  A lane here holds two (k=128) or four (k=64) reference lanes.
@@ -406,23 +482,21 @@ __device__ __forceinline__ float muppet_norm_partial(const V8f& gp, const V8f& g
 }
 
 // ---- passes shared by MuPPET and AFP ------------------------------------------------------------
-// int8 forward pass: saturated fixed-point values, exact integer dot product, one division
+// int8 forward pass: saturated fixed-point values, exact integer dot product, one division (by a power of two).
+// pi, qi: quantize()d rows, clamped if need be
 template <int TS>
-__device__ __forceinline__ float forward_int8(const V8f& p, const V8f& q, float sp, float sq, unsigned wmask) {
-    int acc = 0;
+__device__ __forceinline__ float forward_int8(const V8f& pi, const V8f& qi, float sp, float sq, unsigned wmask) {
+    float2 a = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int t = 0; t < 8; t++) acc += sat8(round_away(__fmul_rn(p.x[t], sp))) * sat8(round_away(__fmul_rn(q.x[t], sq)));
-#pragma unroll
-    for (int d = TS / 2; d >= 1; d >>= 1) acc += __shfl_xor_sync(wmask, acc, d);
-    return __fdiv_rn((float)acc, __fmul_rn(sp, sq));
+    for (int j = 0; j < 4; j++) a = __ffma2_rn(pr(pi, j), pr(qi, j), a);
+    return __fmul_rn(worker_sum<TS>(__fadd_rn(a.x, a.y), wmask), pow2_rev(__fmul_rn(sp, sq)));
 }
 // binary16 forward pass on the fixed-point grid; the two halves of the reference's half2 accumulator
 // go through the lane tree separately and meet at the end (muppet_sgd_kernel.h:170-194,
 // afp_sgd_kernel.h:252-273)
 template <int K>
-__device__ __forceinline__ float forward_half(const V8f& p, const V8f& q, float sp, float sq, unsigned wmask) {
+__device__ __forceinline__ float forward_half(const V8h& ph, const V8h& qh, unsigned wmask) {
     constexpr int TS = K / 8;
-    const V8h ph = fix_round_half(p, sp, pow2_rev(sp)), qh = fix_round_half(q, sq, pow2_rev(sq));
     __half2 xy;
     if (K == 128) {
         const __half2 xab = __hfma2(ph.v[0], qh.v[0], __hmul2_rn(ph.v[2], qh.v[2]));   // (x of lane m, x of lane m+16)
@@ -441,21 +515,19 @@ __device__ __forceinline__ float forward_half(const V8f& p, const V8f& q, float 
     return __half2float(__hadd_rn(__low2half(xy), __high2half(xy)));
 }
 // backward passes: g_p = q*e + p*(-lam), g_q = p*e + q*(-lam) in int8 or binary16 fixed point
-__device__ __forceinline__ void backward_int8(const V8f& p, const V8f& q, float ruv, float nlam, float sb, V8f& gp, V8f& gq) {
-    const float rev2 = __fdiv_rn(1.f, __fmul_rn(sb, sb));
-    const int ei = sat8(round_away(__fmul_rn(ruv, sb))), li = sat8(round_away(__fmul_rn(nlam, sb)));
+__device__ __forceinline__ void backward_int8(const V8f& pi, const V8f& qi, float ruv, float nlam, float sb, V8f& gp, V8f& gq) {
+    const float rev = pow2_rev(__fmul_rn(sb, sb)), e = quantize8(ruv, sb), l = quantize8(nlam, sb);
+    const float2 rev2 = make_float2(rev, rev), e2 = make_float2(e, e), l2 = make_float2(l, l), zero = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int t = 0; t < 8; t++) {
-        const int pi = sat8(round_away(__fmul_rn(p.x[t], sb))), qi = sat8(round_away(__fmul_rn(q.x[t], sb)));
-        gp.x[t] = __fmul_rn((float)(qi * ei + pi * li), rev2);
-        gq.x[t] = __fmul_rn((float)(pi * ei + qi * li), rev2);
+    for (int j = 0; j < 4; j++) {      // + 0: the integer sum has no negative zero
+        set_pr(gp, j, __ffma2_rn(__ffma2_rn(pr(qi, j), e2, __fmul2_rn(pr(pi, j), l2)), rev2, zero));
+        set_pr(gq, j, __ffma2_rn(__ffma2_rn(pr(pi, j), e2, __fmul2_rn(pr(qi, j), l2)), rev2, zero));
     }
 }
-__device__ __forceinline__ void backward_half(const V8f& p, const V8f& q, float ruv, float nlam, float sb, V8f& gp, V8f& gq) {
+__device__ __forceinline__ void backward_half(const V8h& ph, const V8h& qh, float ruv, float nlam, float sb, V8f& gp, V8f& gq) {
     const float sb_rev = pow2_rev(sb);
     const __half2 e2 = __half2half2(__float2half_rn(fix_round(ruv, sb, sb_rev)));
     const __half2 l2 = __half2half2(__float2half_rn(fix_round(nlam, sb, sb_rev)));
-    const V8h ph = fix_round_half(p, sb, sb_rev), qh = fix_round_half(q, sb, sb_rev);
     V8h gph, gqh;
 #pragma unroll
     for (int t = 0; t < 4; t++) {
@@ -465,35 +537,48 @@ __device__ __forceinline__ void backward_half(const V8f& p, const V8f& q, float 
     gp = widen(gph); gq = widen(gqh);
 }
 
+// Do some of the values [lo, hi] times s round to something outside the int8 range?  (The scale is chosen so that
+// hardly ever one does.)  An infinite scale (rows of nothing but tiny values) counts as outside.
+__device__ __forceinline__ bool outside8(float hi, float lo, float s) { return !(__fmul_rn(hi, s) <= 127.25f && __fmul_rn(lo, s) >= -128.25f); }
+__device__ __forceinline__ bool beyond_grid(float hi, float lo, float s) { return !(__fmul_rn(fmaxf(hi, -lo), s) < 2097152.f); }
+
 template <int K>
 __device__ __forceinline__ void muppet_update(const Consts& c, float r, V8f& p, V8f& q, V8f& gp, V8f& gq, unsigned wmask) {
     constexpr int TS = K / 8;
     const int bits = c.bits;
-    float pmin = 0.f, pmax = 0.f, qmin = 0.f, qmax = 0.f, sp = 1.f, sq = 1.f, pred;
-    if (bits != 32) {
-        pmin = pmax = p.x[0]; qmin = qmax = q.x[0];
-#pragma unroll
-        for (int t = 1; t < 8; t++) {
-            pmin = fminf(pmin, p.x[t]); pmax = fmaxf(pmax, p.x[t]);
-            qmin = fminf(qmin, q.x[t]); qmax = fmaxf(qmax, q.x[t]);
-        }
-        pmin = worker_min<TS>(pmin, wmask); pmax = worker_max<TS>(pmax, wmask);
-        qmin = worker_min<TS>(qmin, wmask); qmax = worker_max<TS>(qmax, wmask);
-        sp = muppet_scale(bits, pmax, pmin); sq = muppet_scale(bits, qmax, qmin);
-    }
-    if (bits == 8) pred = forward_int8<TS>(p, q, sp, sq, wmask);
-    else if (bits == 32) pred = worker_sum<TS>(pair_partial(p, q), wmask);
-    else pred = forward_half<K>(p, q, sp, sq, wmask);
-    const float ruv = __fsub_rn(r, pred);
     const float nlam = -c.lam;
-    float sb = 1.f;
-    if (bits != 32) {
-        const float bmin = fminf(fminf(pmin, qmin), fminf(nlam, ruv)), bmax = fmaxf(fmaxf(pmax, qmax), fmaxf(nlam, ruv));
-        sb = muppet_scale(bits, bmax, bmin);
+    if (bits == 32) {
+        const float ruv = __fsub_rn(r, worker_sum<TS>(pair_partial(p, q), wmask));
+        gp = grad(ruv, q, c.lam, p); gq = grad(ruv, p, c.lam, q);
+        p = step(c.lr, gp, p); q = step(c.lr, gq, q);
+        return;
     }
-    if (bits == 8) backward_int8(p, q, ruv, nlam, sb, gp, gq);
-    else if (bits == 32) { gp = grad(ruv, q, c.lam, p); gq = grad(ruv, p, c.lam, q); }
-    else backward_half(p, q, ruv, nlam, sb, gp, gq);
+    float a[4] = {max8(p), -min8(p), max8(q), -min8(q)};
+    worker_max4<TS>(a, wmask);
+    const float pmax = a[0], pmin = -a[1], qmax = a[2], qmin = -a[3];
+    const float sp = muppet_scale(bits, pmax, pmin), sq = muppet_scale(bits, qmax, qmin);
+    V8f pi, qi;
+    V8h ph, qh;
+    quantize(p, sp, q, sq, pi, qi, wmask);
+    float pred;
+    if (bits == 8) {
+        if (__any_sync(wmask, outside8(pmax, pmin, sp) || outside8(qmax, qmin, sq))) { pi = clamp8(pi); qi = clamp8(qi); }
+        pred = forward_int8<TS>(pi, qi, sp, sq, wmask);
+    } else {
+        to_grid(p, pi, sp, q, qi, sq, beyond_grid(pmax, pmin, sp) || beyond_grid(qmax, qmin, sq), ph, qh);
+        pred = forward_half<K>(ph, qh, wmask);
+    }
+    const float ruv = __fsub_rn(r, pred);
+    const float bmin = fminf(fminf(pmin, qmin), fminf(nlam, ruv)), bmax = fmaxf(fmaxf(pmax, qmax), fmaxf(nlam, ruv));
+    const float sb = muppet_scale(bits, bmax, bmin);
+    quantize(p, sb, q, sb, pi, qi, wmask);
+    if (bits == 8) {
+        if (__any_sync(wmask, outside8(bmax, bmin, sb))) { pi = clamp8(pi); qi = clamp8(qi); }
+        backward_int8(pi, qi, ruv, nlam, sb, gp, gq);
+    } else {
+        to_grid(p, pi, sb, q, qi, sb, beyond_grid(bmax, bmin, sb), ph, qh);
+        backward_half(ph, qh, ruv, nlam, sb, gp, gq);
+    }
     p = step(c.lr, gp, p); q = step(c.lr, gq, q);
 }
 
@@ -608,33 +693,64 @@ __device__ __noinline__ AfpSide afp_requantize(AfpSide s, float diff, float rang
     s.next += itv;
     return s;
 }
-__device__ __forceinline__ float abs_max8(const V8f& x) {
-    float m = fabsf(x.x[0]);
-#pragma unroll
-    for (int t = 1; t < 8; t++) m = fmaxf(m, fabsf(x.x[t]));
-    return m;
-}
-
+// The workers of a warp go through this together: what one of them needs (a re-estimation, the int8 or the binary16
+// pass) all of them compute, and each keeps the result if it is its own case.
 template <int K>
-__device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float r, V8f& p, V8f& q, unsigned wmask) {
+__device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float r, V8f& p, V8f& q) {
     constexpr int TS = K / 8;
+    constexpr unsigned kAll = 0xffffffffu;
     const long long cur = st.cur;
+    const bool new_user = cur == st.user.next, new_item = cur == st.item.next, new_back = cur == st.back.next;
+    const bool estimate = __any_sync(kAll, new_user || new_item || new_back);
     float pmax = 0.f, qmax = 0.f;
-    const bool need_back = cur == st.back.next;
-    if (cur == st.user.next || need_back) pmax = worker_max<TS>(abs_max8(p), wmask);
-    if (cur == st.item.next || need_back) qmax = worker_max<TS>(abs_max8(q), wmask);
-    if (cur == st.user.next) st.user = afp_requantize(st.user, afp_qem<K>(p, pmax, wmask), pmax, cur, c.afp_epoch, c.afp_init_threshold);
-    if (cur == st.item.next) st.item = afp_requantize(st.item, afp_qem<K>(q, qmax, wmask), qmax, cur, c.afp_epoch, c.afp_init_threshold);
-    const float pred = (st.user.n == 8 && st.item.n == 8) ? forward_int8<TS>(p, q, st.user.scale, st.item.scale, wmask)
-                                                          : forward_half<K>(p, q, st.user.scale, st.item.scale, wmask);
-    const float ruv = __fsub_rn(r, pred);
-    if (need_back) {
-        const float range = fmaxf(fmaxf(fmaxf(pmax, qmax), fabsf(c.lam)), fabsf(ruv));
-        st.back = afp_requantize(st.back, afp_qem_back<K>(p, q, c.lam, ruv, range, wmask), range, cur, c.afp_epoch, c.afp_init_threshold);
+    if (estimate) {
+        pmax = worker_max<TS>(abs_max8(p), kAll);
+        qmax = worker_max<TS>(abs_max8(q), kAll);
+        if (__any_sync(kAll, new_user)) {
+            const AfpSide s = afp_requantize(st.user, afp_qem<K>(p, pmax, kAll), pmax, cur, c.afp_epoch, c.afp_init_threshold);
+            if (new_user) st.user = s;
+        }
+        if (__any_sync(kAll, new_item)) {
+            const AfpSide s = afp_requantize(st.item, afp_qem<K>(q, qmax, kAll), qmax, cur, c.afp_epoch, c.afp_init_threshold);
+            if (new_item) st.item = s;
+        }
     }
+    // The formats are those of an earlier rating, so values may lie outside their range at any time.
+    const bool forward8 = st.user.n == 8 && st.item.n == 8;
+    float pred = 0.f;
+    V8f pi, qi;
+    V8h ph, qh;
+    quantize(p, st.user.scale, q, st.item.scale, pi, qi, kAll);
+    float most = fmaxf(abs_max8(pi), abs_max8(qi));
+    if (__any_sync(kAll, !forward8)) {
+        to_grid(p, pi, st.user.scale, q, qi, st.item.scale, __any_sync(kAll, !(most < 2097152.f)), ph, qh);
+        pred = forward_half<K>(ph, qh, kAll);
+    }
+    if (__any_sync(kAll, forward8)) {
+        if (__any_sync(kAll, !(most <= 127.f))) { pi = clamp8(pi); qi = clamp8(qi); }
+        const float whole = forward_int8<TS>(pi, qi, st.user.scale, st.item.scale, kAll);
+        if (forward8) pred = whole;
+    }
+    const float ruv = __fsub_rn(r, pred);
+    if (estimate && __any_sync(kAll, new_back)) {
+        const float range = fmaxf(fmaxf(fmaxf(pmax, qmax), fabsf(c.lam)), fabsf(ruv));
+        const AfpSide s = afp_requantize(st.back, afp_qem_back<K>(p, q, c.lam, ruv, range, kAll), range, cur, c.afp_epoch, c.afp_init_threshold);
+        if (new_back) st.back = s;
+    }
+    const bool back8 = st.back.n == 8;
+    quantize(p, st.back.scale, q, st.back.scale, pi, qi, kAll);
+    most = fmaxf(abs_max8(pi), abs_max8(qi));
     V8f gp, gq;
-    if (st.back.n == 8) backward_int8(p, q, ruv, -c.lam, st.back.scale, gp, gq);
-    else backward_half(p, q, ruv, -c.lam, st.back.scale, gp, gq);
+    if (__any_sync(kAll, !back8)) {
+        to_grid(p, pi, st.back.scale, q, qi, st.back.scale, __any_sync(kAll, !(most < 2097152.f)), ph, qh);
+        backward_half(ph, qh, ruv, -c.lam, st.back.scale, gp, gq);
+    }
+    if (__any_sync(kAll, back8)) {
+        if (__any_sync(kAll, !(most <= 127.f))) { pi = clamp8(pi); qi = clamp8(qi); }
+        V8f wp, wq;
+        backward_int8(pi, qi, ruv, -c.lam, st.back.scale, wp, wq);
+        if (back8) { gp = wp; gq = wq; }
+    }
     p = step(c.lr, gp, p); q = step(c.lr, gq, q);
     st.cur = cur + 1;
 }
@@ -649,7 +765,7 @@ __device__ __forceinline__ __half2 half2_of(uint32_t w) { return *reinterpret_ca
 // where they may take different branches (ROWS_DYN), each with the mask of its own lanes.
 template <int K, int KIND, int UM, int IM, bool STATS>
 __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_t uc, uint32_t ic, Raw<UM>& p_raw, Raw<IM>& q_raw,
-                                           Sample& smp, AfpState& afp, unsigned wmask, unsigned gmask) {
+                                           Sample& smp, AfpState& afp, unsigned wmask) {
     constexpr int TS = K / 8;
     if (STATS) { smp.user = false; smp.item = false; }
     if constexpr (KIND == KIND_MPT) {
@@ -673,7 +789,7 @@ __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_
         if (STATS && c.bits != 32) smp.user = true;
     } else if constexpr (KIND == KIND_AFP) {
         V8f p = as_v8f(p_raw), q = as_v8f(q_raw);
-        afp_update<K>(c, afp, __uint_as_float(rw), p, q, gmask);
+        afp_update<K>(c, afp, __uint_as_float(rw), p, q);
         put(p_raw, p); put(q_raw, q);
     } else if constexpr (KIND == KIND_MEMQUANT) {
         const V8f p = widen(as_v8h(p_raw)), q = widen(as_v8h(q_raw));
@@ -785,7 +901,7 @@ template <int K, int UM, int IM, int NS, int NSI> struct WorkerSmem {
 // The lead is kept as short as the memory latency allows: an item row that another worker updates between the
 // request and the write-back loses that update, and the chance of that grows with the lead.
 template <int K, int KIND, int UM, int IM, bool STATS, int NS, int NSI, int D, int DI>
-__global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !STATS) ? 4 : ((UM == ROWS_DYN || STATS || KIND == KIND_AFP) ? 2 : 3)) train_kernel(const KernelArgs a) {
+__global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !STATS) ? 4 : ((UM == ROWS_DYN || STATS || KIND == KIND_AFP || KIND == KIND_MUPPET) ? 2 : 3)) train_kernel(const KernelArgs a) {
     using SM = WorkerSmem<K, UM, IM, NS, NSI>;
     constexpr int TS = SM::TS;                     // lanes per worker = ratings per chunk
     constexpr unsigned kAll = 0xffffffffu;
@@ -1003,6 +1119,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     cp_wait<D - 1>();
     Raw<UM> p = lds_row<K, UM>(uring, rec.z);
 
+    constexpr int kUnroll = (KIND == KIND_AFP || KIND == KIND_MUPPET) ? 1 : NS;
     int cb = 0;                                     // buffer of the chunk in use
     while (__any_sync(kAll, cnt_cur > 0)) {
 #pragma unroll 1
@@ -1010,7 +1127,9 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
             // this group of NS records and the next one (in the other buffer at the end of a chunk)
             const unsigned r0 = s_rec + 16 * (cb * TS + jb), r1 = s_rec + 16 * ((cb * TS + jb + NS) & (2 * TS - 1));
             const unsigned q0 = s_req + 8 * (cb * TS + jb);
-#pragma unroll
+            // The fixed-point updates are some hundred instructions long: one copy of them, or the warps wait for
+            // instruction fetches (3.4 cycles per instruction with four copies of the AFP update).
+#pragma unroll(kUnroll)
             for (int t = 0; t < NS; t++) {
                 const uint32_t uc = rec.z, ic = rec.y, f = rec.x, rw = rec.w;
                 if (__any_sync(kAll, f & (F_RS | F_UDUP))) {
@@ -1039,7 +1158,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
                 cp_commit();
                 const Raw<UM> p_before = p;
                 constexpr bool kDyn = UM == ROWS_DYN || IM == ROWS_DYN;
-                update_one<K, KIND, UM, IM, STATS>(c, rw, uc, ic, p, q, smp, afp, kDyn ? gmask : kAll, gmask);
+                update_one<K, KIND, UM, IM, STATS>(c, rw, uc, ic, p, q, smp, afp, kDyn ? gmask : kAll);
                 if (a.add_user_delta) add_row_delta<K, UM>(P, uc, f & F_DROP, p, p_before);
                 else st_row_if<K, UM>(~f & F_DROP, P, uc, p);
                 if (STATS) { if (!(f & F_NONE)) record(smp, uc, ic); }

@@ -1,0 +1,64 @@
+"""The fixed-point trainers at values where their rounding and their scales can go wrong: exact halves on the grid, rows of
+zeros, tiny and denormal rows, values beyond the int8 range and beyond 2^21 steps of a grid, extremes next to a power of
+two.  Bit for bit against the sequential oracle."""
+import numpy as np
+import pytest
+
+from helpers import assert_bit_equal, random_problem
+
+pytestmark = pytest.mark.gpu
+
+KINDS = ["halves", "zeros", "zero_side", "tiny", "denormal", "mixed", "large", "powers"]
+
+
+def factors(kind, rng, rows, k):
+    x = (rng.standard_normal((rows, k)) * 0.2).astype(np.float32)
+    if kind == "halves":
+        return (np.round(x * 512) / 512 + np.float32(1 / 1024)).astype(np.float32)
+    if kind == "zeros":
+        return np.zeros_like(x)
+    if kind == "zero_side":
+        x[::2] = 0
+        return np.abs(x)
+    if kind == "tiny":
+        return x * np.float32(1e-30)
+    if kind == "denormal":
+        return x * np.float32(1e-38)
+    if kind == "mixed":
+        return x * (10.0 ** rng.integers(-6, 2, (rows, 1))).astype(np.float32)
+    if kind == "large":
+        return x * np.float32(20)
+    scale = np.float32(2.0) ** rng.integers(-8, 2, (rows, 1)).astype(np.float32)
+    x = np.clip(x, -1, 1) * scale
+    x[:, 0] = (scale * np.float32(127.5 / 128))[:, 0]                        # top / hi a power of two, exactly or by a few units
+    x[:, 1] = -(scale * np.float32(128.5 / 128))[:, 0] * (1 + rng.integers(-3, 4, rows) * np.float32(2.0 ** -23))
+    return x.astype(np.float32)
+
+
+@pytest.mark.parametrize("k", (128, 64))
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("bits", (8, 12, 16, "afp"))
+def test_extreme_values_bit_exact(mascot, oracle, k, kind, bits):
+    if kind == "denormal" and bits in (12, 16):
+        pytest.skip("the rule's own result: 0 times an infinite scale")
+    lr = 1e-6 if kind in ("mixed", "large") else 1e-3         # slow enough not to diverge
+    rng = np.random.default_rng(KINDS.index(kind))
+    n_users, n_items, n = 61, 37, 1201
+    R, _, _ = random_problem(rng, n_users, n_items, n, k)
+    P, Q = factors(kind, rng, n_users, k), factors(kind, rng, n_items, k)
+    afp = bits == "afp"
+    cfg = mascot.default_config(version=mascot.V_AFP if afp else mascot.V_MUPPET, k=k, deterministic=1, shuffle=0, epoch=50, learning_rate=lr,
+                                decay=0.1, lam=0.05, muppet_width=0 if afp else bits, sample_ratio=0.1)
+    with mascot.Engine(cfg) as eng:
+        eng.set_ratings(R, R[:10], n_users, n_items)
+        eng.set_factors(P, Q)
+        eng.train_epoch(0)
+        Pg, Qg = eng.get_factors(0)
+    rules, lrs = oracle.rules_reference(), float(np.float32(lr))
+    if afp:
+        oracle.afp_run(k, R, None, P, Q, lrs, 0.05, 0, int(np.float32(n) / np.float32(10.0)), rules)
+    else:
+        oracle.muppet_run(k, R, None, P, Q, lrs, 0.05, bits, bits, rules, first_sample_pos=n - int(np.float32(n) * np.float32(0.1)))
+    assert np.isfinite(P).all()
+    assert_bit_equal(Pg, P, "P")
+    assert_bit_equal(Qg, Q, "Q")
