@@ -14,6 +14,8 @@
 //     on with empty records.  Per-worker branches cost a warp barrier in front of every shuffle and split the update
 //     into pieces that cannot be scheduled into each other: 131 warp instructions per step of all workers of a warp
 //     before, 90 now.
+//   * what the ratings to come need (records, row copies, the vote on item rows) is done between the dependent shuffles
+//     of the dot product instead of in front of it: 8M ratings 1.39 -> 1.295 ms per epoch, fp32 rows 1.70 -> 1.52;
 //   * the rating records of a chunk (one rating per lane) are loaded one chunk ahead, tagged
 //     (repeated user, start of an item run, repeated item, dropped write-back) and put into shared memory, from where
 //     the worker reads one rating with a single 128-bit broadcast load;
@@ -31,12 +33,12 @@
 // store, once per run) every update another worker makes to that row is lost, so the loss grows with
 // (workers x lead time).  The leads are counted in ratings, and a rating takes 0.2 us where it took 0.35 when the leads
 // were three and one: the same time, and the same RMSE (0.5169 after one epoch, 0.5180 after six on the k=64
-// configuration either way).  With leads of three and two the 8M-rating configuration took 1.65 ms per epoch instead
-// of 1.39, the k=64 one 1.97 instead of 1.65; user leads of six and seven gave nothing more.
+// configuration either way).  With leads of three and two the 8M-rating configuration took 1.65 ms per epoch where it
+// took 1.39 with five and three, the k=64 one 1.97 against 1.65; user leads of six and seven gave nothing more.
 //
 // WHAT BOUNDS IT (one B200, k=128, binary16 rows).  Sets with few workers per SM (8M ratings: one warp per scheduler):
-// the chain of one update - dot product, four shuffle steps, update - and the 90 instructions around it, 2.42 -> 1.39
-// ms per epoch.  Full SMs (100M ratings, 7.17 -> 5.50 ms): the L2 and its reductions.  18.3e9 updates/s write 4.7 TB/s of
+// the chain of one update - dot product, four shuffle steps, update - and the 95 instructions around it, 2.42 -> 1.295
+// ms per epoch (3.9 cycles per instruction: 1.3 of them waits for results of fixed latency, 0.6 each for L2 and for shuffles).  Full SMs (100M ratings, 7.17 -> 5.50 ms): the L2 and its reductions.  18.3e9 updates/s write 4.7 TB/s of
 // reductions and read as much again; a kernel that does nothing but read random rows and reduce into them reaches
 // 17.6e9 rows/s on this GPU with evenly spread rows and 10.9e9 with Zipf ones (8.6e9 and 7.1e9 with fp32 rows, which is
 // what bounds the classes with fp32 user rows).
@@ -249,17 +251,25 @@ __device__ __forceinline__ float chain_partial_k128(const V8f& a, const V8f& b) 
     return __fadd_rn(c[0], c[1]);
 }
 
-template <int TS>
-__device__ __forceinline__ float worker_sum(float x, unsigned wmask) {
+// Sum over a worker's lanes.  Three or four dependent shuffles of some 25 cycles each: `mid(i)` is called while shuffle i
+// is under way, for work that does not need the sum.
+struct Nothing { __device__ __forceinline__ void operator()(int) const {} };
+template <int TS, class Mid = Nothing>
+__device__ __forceinline__ float worker_sum(float x, unsigned wmask, Mid mid = Mid()) {
 #pragma unroll
-    for (int d = TS / 2; d >= 1; d >>= 1) x = __fadd_rn(x, __shfl_xor_sync(wmask, x, d));
+    for (int d = TS / 2, i = 0; d >= 1; d >>= 1, i++) {
+        const float o = __shfl_xor_sync(wmask, x, d);
+        mid(i);
+        x = __fadd_rn(x, o);
+    }
     return x;
 }
-template <int TS>
-__device__ __forceinline__ __half2 worker_sum(__half2 x, unsigned wmask) {
+template <int TS, class Mid = Nothing>
+__device__ __forceinline__ __half2 worker_sum(__half2 x, unsigned wmask, Mid mid = Mid()) {
 #pragma unroll
-    for (int d = TS / 2; d >= 1; d >>= 1) {
+    for (int d = TS / 2, i = 0; d >= 1; d >>= 1, i++) {
         const unsigned o = __shfl_xor_sync(wmask, *reinterpret_cast<const unsigned*>(&x), d);
+        mid(i);
         x = __hadd2_rn(x, *reinterpret_cast<const __half2*>(&o));
     }
     return x;
@@ -762,16 +772,19 @@ __device__ __forceinline__ __half2 half2_of(uint32_t w) { return *reinterpret_ca
 
 // One update.  rw is the rating as its record holds it; p_raw / q_raw are the row slices in their storage precision,
 // both replaced by the updated values.  The workers of a warp come here together, with `wmask` the whole warp - or,
-// where they may take different branches (ROWS_DYN), each with the mask of its own lanes.
-template <int K, int KIND, int UM, int IM, bool STATS>
+// where they may take different branches (ROWS_DYN), each with the mask of its own lanes.  mid(0), mid(1), mid(2): what the
+// worker has to do meanwhile, done under the shuffles of the dot product.
+template <int K, int KIND, int UM, int IM, bool STATS, class Mid>
 __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_t uc, uint32_t ic, Raw<UM>& p_raw, Raw<IM>& q_raw,
-                                           Sample& smp, AfpState& afp, unsigned wmask) {
+                                           Sample& smp, AfpState& afp, unsigned wmask, Mid mid) {
     constexpr int TS = K / 8;
+    constexpr bool kAhead = KIND == KIND_MUPPET || KIND == KIND_AFP || UM == ROWS_DYN || IM == ROWS_DYN;      // no single dot product to hide under
+    if constexpr (kAhead) { mid(0); mid(1); mid(2); }
     if (STATS) { smp.user = false; smp.item = false; }
     if constexpr (KIND == KIND_MPT) {
         const V8f p = as_v8f(p_raw), q = as_v8f(q_raw);
         const V8h ph = narrow(p), qh = narrow(q);
-        const __half2 dot = worker_sum<TS>(pair_partial(ph, qh), wmask);
+        const __half2 dot = worker_sum<TS>(pair_partial(ph, qh), wmask, mid);
         const __half2 e = __hmul2_rn(c.mpt_scale, __hsub2_rn(half2_of(rw), dot));
         const V8f gp = widen(grad(e, qh, c.mpt_nlam, ph)), gq = widen(grad(e, ph, c.mpt_nlam, qh));
         V8f po, qo;
@@ -794,14 +807,16 @@ __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_
     } else if constexpr (KIND == KIND_MEMQUANT) {
         const V8f p = widen(as_v8h(p_raw)), q = widen(as_v8h(q_raw));
         const float part = (K == 128) ? chain_partial_k128(p, q) : pair_partial(p, q);
-        const float e = __fsub_rn(__uint_as_float(rw), worker_sum<TS>(part, wmask));
+        const float e = __fsub_rn(__uint_as_float(rw), worker_sum<TS>(part, wmask, mid));
         put(p_raw, narrow(step(c.lr, grad(e, q, c.lam, p), p)));
         put(q_raw, narrow(step(c.lr, grad(e, p, c.lam, q), q)));
     } else {
         const bool uf = is_f32<UM>(uc), itf = is_f32<IM>(ic);
         auto both_half = [&]() {
             const V8h p = as_v8h(p_raw), q = as_v8h(q_raw);
-            const __half2 dot = worker_sum<TS>(pair_partial(p, q), wmask);
+            __half2 dot;
+            if constexpr (kAhead) dot = worker_sum<TS>(pair_partial(p, q), wmask);
+            else dot = worker_sum<TS>(pair_partial(p, q), wmask, mid);
             const __half2 e = __hsub2_rn(kHalfRating<KIND, UM, IM> ? half2_of(rw) : __float2half2_rn(__uint_as_float(rw)), dot);
             const V8h gp = grad(e, q, c.nlam_h, p), gq = grad(e, p, c.nlam_h, q);
             put(p_raw, step(c.lr_h, gp, p));
@@ -811,7 +826,10 @@ __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_
         auto some_f32 = [&]() {
             const V8f p = uf ? as_v8f(p_raw) : widen(as_v8h(p_raw));
             const V8f q = itf ? as_v8f(q_raw) : widen(as_v8h(q_raw));
-            const float e = __fsub_rn(__uint_as_float(rw), worker_sum<TS>(pair_partial(p, q), wmask));
+            float dot;
+            if constexpr (kAhead) dot = worker_sum<TS>(pair_partial(p, q), wmask);
+            else dot = worker_sum<TS>(pair_partial(p, q), wmask, mid);
+            const float e = __fsub_rn(__uint_as_float(rw), dot);
             const V8f gp = grad(e, q, c.lam, p), gq = grad(e, p, c.lam, q);
             const V8f po = step(c.lr, gp, p), qo = step(c.lr, gq, q);
             if (uf) put(p_raw, po); else put(p_raw, narrow(po));
@@ -1118,6 +1136,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     uint4 rec = recs[0];
     cp_wait<D - 1>();
     Raw<UM> p = lds_row<K, UM>(uring, rec.z);
+    bool turn = __any_sync(kAll, rec.x & (F_RS | F_UDUP));      // does the coming rating of some worker need another item row?
 
     constexpr int kUnroll = (KIND == KIND_AFP || KIND == KIND_MUPPET) ? 1 : NS;
     int cb = 0;                                     // buffer of the chunk in use
@@ -1132,7 +1151,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
 #pragma unroll(kUnroll)
             for (int t = 0; t < NS; t++) {
                 const uint32_t uc = rec.z, ic = rec.y, f = rec.x, rw = rec.w;
-                if (__any_sync(kAll, f & (F_RS | F_UDUP))) {
+                if (turn) {
                     // a run of equal items ends for at least one of the warp's workers (or a row has to be read again)
                     cp_wait<DI - 1>();
                     const unsigned start = f & F_RS;
@@ -1146,19 +1165,26 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
                     }
                     if (start) { cur_ic = ic; have_item = (f & F_NONE) ? 0u : F_RS; }
                 }
-                // the next rating's record and user row
-                rec = lds128(t + 1 < NS ? r0 + 16 * (t + 1) : r1);
-                cp_wait<D - 2>();
-                const Raw<UM> p_next = lds_row<K, UM>(uring + ((t + 1) & (NS - 1)) * SM::kURowBytes, rec.z);
-                // requests into slots whose contents have been consumed
+                // what the ratings to come need, into slots whose contents have been consumed
+                Raw<UM> p_next;
                 uint32_t req_u, req_i;
-                asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(req_u), "=r"(req_i) : "r"(q0 + 8 * t) : "memory");
-                request_item(req_i, (t + DI) & (NSI - 1));
-                request_user(req_u, (t + D) & (NS - 1));
-                cp_commit();
+                auto meanwhile = [&](int part) {
+                    if (part == 0) {
+                        rec = lds128(t + 1 < NS ? r0 + 16 * (t + 1) : r1);
+                        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(req_u), "=r"(req_i) : "r"(q0 + 8 * t) : "memory");
+                    } else if (part == 1) {
+                        cp_wait<D - 2>();
+                        p_next = lds_row<K, UM>(uring + ((t + 1) & (NS - 1)) * SM::kURowBytes, rec.z);
+                    } else if (part == 2) {
+                        request_item(req_i, (t + DI) & (NSI - 1));
+                        request_user(req_u, (t + D) & (NS - 1));
+                        cp_commit();
+                        turn = __any_sync(kAll, rec.x & (F_RS | F_UDUP));
+                    }
+                };
                 const Raw<UM> p_before = p;
                 constexpr bool kDyn = UM == ROWS_DYN || IM == ROWS_DYN;
-                update_one<K, KIND, UM, IM, STATS>(c, rw, uc, ic, p, q, smp, afp, kDyn ? gmask : kAll);
+                update_one<K, KIND, UM, IM, STATS>(c, rw, uc, ic, p, q, smp, afp, kDyn ? gmask : kAll, meanwhile);
                 if (a.add_user_delta) add_row_delta<K, UM>(P, uc, f & F_DROP, p, p_before);
                 else st_row_if<K, UM>(~f & F_DROP, P, uc, p);
                 if (STATS) { if (!(f & F_NONE)) record(smp, uc, ic); }
