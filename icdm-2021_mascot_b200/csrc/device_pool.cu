@@ -16,6 +16,7 @@
 
 #include <mutex>
 #include <set>
+#include <vector>
 
 #include "handle.h"
 
@@ -55,7 +56,53 @@ cudaError_t current_pool(cudaMemPool_t* pool) {
     return cudaSuccess;
 }
 
+// Pinned blocks of Results: a few for the whole process, whatever number of engines and threads there are.
+constexpr size_t kBlockFloats = 16384;            // 64 KiB: block sums of 8.4M ratings
+constexpr int kBlocks = 8;
+struct PinnedBlock { float* mem; bool busy; };
+std::vector<PinnedBlock> g_blocks;
+
+float* take_block() {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    for (PinnedBlock& b : g_blocks) if (!b.busy) { b.busy = true; return b.mem; }
+    if (g_blocks.size() >= (size_t)kBlocks) return nullptr;
+    float* mem = nullptr;
+    if (cudaHostAlloc(reinterpret_cast<void**>(&mem), kBlockFloats * sizeof(float), cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    g_blocks.push_back(PinnedBlock{mem, true});
+    return mem;
+}
+
 }  // namespace
+
+Results::Results(size_t floats, cudaStream_t st) : n_(floats), st_(st) {
+    if (floats < kBlockFloats) pinned_ = take_block();
+    if (pinned_) { reinterpret_cast<uint32_t*>(pinned_)[n_] = 0; return; }
+    status_ = dev_alloc(&dev_, n_ + 1, st_);
+    if (status_ == cudaSuccess) status_ = cudaMemsetAsync(dev_ + n_, 0, sizeof(uint32_t), st_);
+}
+
+Results::~Results() {
+    dev_free(dev_, st_);
+    if (!pinned_) return;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    for (PinnedBlock& b : g_blocks) if (b.mem == pinned_) b.busy = false;
+}
+
+cudaError_t Results::wait() {
+    if (pinned_) return cudaStreamSynchronize(st_);
+    host_.resize(n_ + 1);
+    const cudaError_t e = cudaMemcpyAsync(host_.data(), dev_, sizeof(float) * (n_ + 1), cudaMemcpyDeviceToHost, st_);
+    return e == cudaSuccess ? cudaStreamSynchronize(st_) : e;
+}
+
+void release_results() {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    for (size_t j = 0; j < g_blocks.size();) {
+        if (g_blocks[j].busy) { j++; continue; }
+        cudaFreeHost(g_blocks[j].mem);
+        g_blocks.erase(g_blocks.begin() + (long)j);
+    }
+}
 
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st) {
     cudaError_t e;

@@ -87,9 +87,10 @@ cudaError_t launch_reduce_stats(float* sets, int copies, size_t copy_stride, siz
 
 // Test RMSE over a coded SoA stream; block_err has ceil(n/512) floats.
 cudaError_t launch_rmse(int K, const Stream& t, Arena P, Arena Q, float* block_err, cudaStream_t st);
-// Test RMSE over plain fp32 rows in the reference element order and AoS ratings {r,u,i}.
+// Test RMSE over plain fp32 rows in the reference element order and AoS ratings {r,u,i}.  With `bad` (may be null: ids
+// are trusted) an id outside [0, n_users) x [0, n_items) sets it and is not used as an index.
 cudaError_t launch_rmse_plain(int K, const void* d_test_aos, uint64_t n, const float* P, const float* Q,
-                              float* block_err, cudaStream_t st);
+                              uint32_t n_users, uint32_t n_items, float* block_err, uint32_t* bad, cudaStream_t st);
 
 // Set-up / conversion kernels.
 // Codes n ratings {r,u,i} into the stream arrays: optional seeded permutation + item-sorted windows, ids

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 
 #include "../../include/mascot.h"
@@ -22,56 +23,101 @@ namespace mascot {
 namespace {
 
 constexpr int kRmseBlock = 512;    // ratings per block partial (BLOCK_SIZE in rmse.h:3)
-constexpr int kRmseThreads = 256;
 
-__device__ __forceinline__ float block_tree_512(float* tmp) {
-    // tmp[j] += tmp[j+s] for s = 256 .. 1  (rmse.h:85-91 and warpReduce, rmse.h:5-24)
-    for (int s = 256; s >= 1; s >>= 1) {
-        __syncthreads();
-        for (int j = threadIdx.x; j < s; j += blockDim.x) tmp[j] = __fadd_rn(tmp[j], tmp[j + s]);
-    }
+// tmp[j] += tmp[j+s] for s = 256 .. 1  (rmse.h:85-91 and warpReduce, rmse.h:5-24), by the first eight warps: two levels
+// through shared memory, the rest in the registers of one warp (a xor butterfly adds the same pairs).
+__device__ __forceinline__ void block_tree_512(float* tmp, float* out) {
+    const int t = threadIdx.x;
     __syncthreads();
-    return tmp[0];
+    if (t < 256) tmp[t] = __fadd_rn(tmp[t], tmp[t + 256]);
+    __syncthreads();
+    if (t < 32) {
+        const float a = __fadd_rn(__fadd_rn(tmp[t], tmp[t + 128]), __fadd_rn(tmp[t + 64], tmp[t + 192]));
+        const float b = __fadd_rn(__fadd_rn(tmp[t + 32], tmp[t + 160]), __fadd_rn(tmp[t + 96], tmp[t + 224]));
+        float v = __fadd_rn(a, b);
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, d));
+        if (t == 0) *out = v;
+    }
 }
 
+// What bounds an evaluation is the latency of two dependent loads (ids, then rows) and the rows' traffic.  The ids of a
+// block come in with one coalesced load, so that all row loads of a lane can be in flight together; each team
+// takes kBatch ratings at once and reduces them together: the first steps of the lane tree exchange half of the
+// ratings instead of adding all of them in every lane, which adds the same pairs with a third of the shuffles.
+struct BlockIds {
+    float r[kRmseBlock];
+    uint32_t u[kRmseBlock], i[kRmseBlock];
+};
+
 // A lane's eight consecutive physical elements of a row as fp32 (positions: see layout.cuh).
-__device__ __forceinline__ void load8(const Arena& A, uint32_t code, int K, int tl, float* x) {
+struct Row8 { uint4 a, b; };
+template <int K>
+__device__ __forceinline__ Row8 fetch8(const Arena& A, uint32_t code, int tl) {
     const uint32_t row = code & kIdMask;
+    Row8 v;
     if (code & kPrecBit) {
-        const float4* p = reinterpret_cast<const float4*>(A.f32 + (size_t)row * K) + tl;      // two half-rows (layout.cuh)
-        const float4 v = __ldcg(p), w = __ldcg(p + K / 8);
-        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; x[4] = w.x; x[5] = w.y; x[6] = w.z; x[7] = w.w;
+        const uint4* p = reinterpret_cast<const uint4*>(A.f32 + (size_t)row * K) + tl;        // two half-rows (layout.cuh)
+        v.a = __ldcg(p); v.b = __ldcg(p + K / 8);
     } else {
-        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(A.f16 + (size_t)row * K) + tl);
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x));
-        const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
-        const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&v.z));
-        const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&v.w));
+        v.a = __ldcg(reinterpret_cast<const uint4*>(A.f16 + (size_t)row * K) + tl);
+    }
+    return v;
+}
+__device__ __forceinline__ void widen8(const Row8& v, uint32_t code, float* x) {
+    if (code & kPrecBit) {
+        x[0] = __uint_as_float(v.a.x); x[1] = __uint_as_float(v.a.y); x[2] = __uint_as_float(v.a.z); x[3] = __uint_as_float(v.a.w);
+        x[4] = __uint_as_float(v.b.x); x[5] = __uint_as_float(v.b.y); x[6] = __uint_as_float(v.b.z); x[7] = __uint_as_float(v.b.w);
+    } else {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.a.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v.a.y));
+        const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&v.a.z)), d = __half22float2(*reinterpret_cast<const __half2*>(&v.a.w));
         x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y; x[4] = c.x; x[5] = c.y; x[6] = d.x; x[7] = d.y;
     }
 }
 
+// Sums four values over a team of T lanes, xor steps T/2 .. 1; lane with index t ends with the sum of value
+// 2 * (t & T/2 set) + (t & T/4 set).
+template <int T>
+__device__ __forceinline__ float team_sum4(const float (&v)[4], int t) {
+    const bool up = t & (T / 2), up2 = t & (T / 4);
+    const float s0 = __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], T / 2), s1 = __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], T / 2);
+    const float w0 = __fadd_rn(up ? v[2] : v[0], s0), w1 = __fadd_rn(up ? v[3] : v[1], s1);
+    float x = __fadd_rn(up2 ? w1 : w0, __shfl_xor_sync(0xffffffffu, up2 ? w0 : w1, T / 4));
+#pragma unroll
+    for (int d = T / 8; d >= 1; d >>= 1) x = __fadd_rn(x, __shfl_xor_sync(0xffffffffu, x, d));
+    return x;
+}
+
 template <int K>
-__global__ void __launch_bounds__(kRmseThreads) rmse_kernel(const Stream t, const Arena P, const Arena Q, float* block_err) {
+__global__ void __launch_bounds__(512) rmse_kernel(const Stream t, const Arena P, const Arena Q, float* block_err) {
     constexpr int T = K / 8;                      // lanes per rating, eight elements each
+    constexpr int kTeams = 512 / T;
     __shared__ float tmp[kRmseBlock];
-    const int tl = threadIdx.x % T;
-    const int team = threadIdx.x / T;
-    constexpr int kTeams = kRmseThreads / T;
-    const int lane = threadIdx.x & 31;
-    const unsigned mask = ((1u << T) - 1u) << (lane - tl);
+    __shared__ BlockIds ids;
+    const int tl = threadIdx.x % T, team = threadIdx.x / T;
     const uint64_t base = (uint64_t)blockIdx.x * kRmseBlock;
-    for (int j = team; j < kRmseBlock; j += kTeams) {
-        const uint64_t idx = base + j;
-        float err2 = 0.f;
-        if (idx < t.n) {
-            const float r = __ldg(t.r + idx);
-            const uint32_t uc = __ldg(t.u + idx), ic = __ldg(t.i + idx);
+    const int left = (int)min((uint64_t)kRmseBlock, t.n - base);
+    {   // positions past the end repeat the last rating; their error counts as zero below
+        const uint64_t at = base + min((int)threadIdx.x, left - 1);
+        ids.r[threadIdx.x] = __ldg(t.r + at); ids.u[threadIdx.x] = __ldg(t.u + at); ids.i[threadIdx.x] = __ldg(t.i + at);
+    }
+    __syncthreads();
+    for (int j = team; j < kRmseBlock; j += 4 * kTeams) {      // ratings j, j + kTeams, j + 2 kTeams, j + 3 kTeams
+        Row8 rp[4], rq[4];
+        uint32_t uc[4], ic[4];
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            uc[b] = ids.u[j + b * kTeams]; ic[b] = ids.i[j + b * kTeams];
+            rp[b] = fetch8<K>(P, uc[b], tl);
+            rq[b] = fetch8<K>(Q, ic[b], tl);
+        }
+        float part[4];
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
             float p[8], q[8];
-            load8(P, uc, K, tl, p);
-            load8(Q, ic, K, tl, q);
+            widen8(rp[b], uc[b], p);
+            widen8(rq[b], ic[b], q);
             // positions 0 2 4 6 hold e0..e3, positions 1 3 5 7 hold e4..e7
-            float part;
             if (K == 128) {
                 // two reference lanes (m, m+16): product chain over four elements each (rmse.h:75),
                 // their sum is the tree's 16 step
@@ -82,56 +128,83 @@ __global__ void __launch_bounds__(kRmseThreads) rmse_kernel(const Stream t, cons
                     acc = __fmaf_rn(p[4 + h], q[4 + h], acc);
                     c[h] = __fmaf_rn(p[6 + h], q[6 + h], acc);
                 }
-                part = __fadd_rn(c[0], c[1]);
+                part[b] = __fadd_rn(c[0], c[1]);
             } else {
                 // four reference lanes (m, m+16, m+8, m+24) with two elements each: 16 step, then 8 step
                 const float f0 = __fmaf_rn(p[0], q[0], __fmul_rn(p[2], q[2]));
                 const float f1 = __fmaf_rn(p[4], q[4], __fmul_rn(p[6], q[6]));
                 const float f2 = __fmaf_rn(p[1], q[1], __fmul_rn(p[3], q[3]));
                 const float f3 = __fmaf_rn(p[5], q[5], __fmul_rn(p[7], q[7]));
-                part = __fadd_rn(__fadd_rn(f0, f1), __fadd_rn(f2, f3));
+                part[b] = __fadd_rn(__fadd_rn(f0, f1), __fadd_rn(f2, f3));
             }
-#pragma unroll
-            for (int d = T / 2; d >= 1; d >>= 1) part = __fadd_rn(part, __shfl_xor_sync(mask, part, d));
-            const float e = __fsub_rn(r, part);
-            err2 = __fmul_rn(e, e);
         }
-        if (tl == 0) tmp[j] = err2;
+        const float pred = team_sum4<T>(part, tl);
+        if ((tl & (T / 4 - 1)) == 0) {
+            const int at = j + (2 * ((tl & (T / 2)) != 0) + ((tl & (T / 4)) != 0)) * kTeams;
+            const float e = __fsub_rn(ids.r[at], pred);
+            tmp[at] = at < left ? __fmul_rn(e, e) : 0.f;
+        }
     }
-    const float s = block_tree_512(tmp);
-    if (threadIdx.x == 0) block_err[blockIdx.x] = s;
+    block_tree_512(tmp, block_err + blockIdx.x);
 }
 
 struct NodeAos { float r; uint32_t u; uint32_t i; };
 
-// Plain fp32 rows in the reference's own element order: lane l reads elements l, l+32, ...
-template <int K>
-__global__ void __launch_bounds__(kRmseThreads) rmse_plain_kernel(const NodeAos* t, uint64_t n, const float* P, const float* Q, float* block_err) {
+// Plain fp32 rows in the reference's own element order: reference lane l adds elements l, l+32, ... of a row.  Eight
+// lanes take a rating; lane t loads the 16 bytes of reference lanes 4t..4t+3 in each of the K/32 slots, so that a row
+// comes in whole 128-byte lines, and the steps 16, 8, 4 of the lane tree go across the eight lanes, 2 and 1 between
+// what they end up with: six shuffles for the four ratings of a warp.
+// The matrices may start at any float; rows off 16-byte boundaries are read float by float.
+template <bool ALIGNED> __device__ __forceinline__ float4 load4(const float* p) {
+    if (ALIGNED) return __ldg(reinterpret_cast<const float4*>(p));
+    return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+template <int K, bool ALIGNED>
+__global__ void __launch_bounds__(512) rmse_plain_kernel(const NodeAos* t, uint64_t n, const float* P, const float* Q, uint32_t n_users, uint32_t n_items,
+                                                         float* block_err, uint32_t* bad) {
+    constexpr int T = 8, kSlots = K / 32, kTeams = 512 / T, kBatch = K == 128 ? 2 : 4;
     __shared__ float tmp[kRmseBlock];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int kWarps = kRmseThreads / 32;
+    __shared__ BlockIds ids;
+    const int tl = threadIdx.x % T, team = threadIdx.x / T;
     const uint64_t base = (uint64_t)blockIdx.x * kRmseBlock;
-    for (int j = warp; j < kRmseBlock; j += kWarps) {
-        const uint64_t idx = base + j;
-        float err2 = 0.f;
-        if (idx < n) {
-            const float r = __ldg(&t[idx].r);
-            const float* p = P + (size_t)__ldg(&t[idx].u) * K;
-            const float* q = Q + (size_t)__ldg(&t[idx].i) * K;
-            float part = __fmaf_rn(p[lane], q[lane], __fmul_rn(p[lane + 32], q[lane + 32]));
-            if (K == 128) {
-                part = __fmaf_rn(p[lane + 64], q[lane + 64], part);
-                part = __fmaf_rn(p[lane + 96], q[lane + 96], part);
-            }
-#pragma unroll
-            for (int d = 16; d >= 1; d >>= 1) part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, d));
-            const float e = __fsub_rn(r, part);
-            err2 = __fmul_rn(e, e);
-        }
-        if (lane == 0) tmp[j] = err2;
+    const int left = (int)min((uint64_t)kRmseBlock, n - base);
+    {
+        const NodeAos* const nd = t + base + min((int)threadIdx.x, left - 1);
+        uint32_t u = __ldg(&nd->u), i = __ldg(&nd->i);
+        if (bad && (u >= n_users || i >= n_items)) { *bad = 1u; u = 0; i = 0; }      // never used as an index
+        ids.r[threadIdx.x] = __ldg(&nd->r); ids.u[threadIdx.x] = u; ids.i[threadIdx.x] = i;
     }
-    const float s = block_tree_512(tmp);
-    if (threadIdx.x == 0) block_err[blockIdx.x] = s;
+    __syncthreads();
+    for (int j0 = team; j0 < kRmseBlock; j0 += kBatch * kTeams) {
+        float4 p[kBatch][kSlots], q[kBatch][kSlots];
+#pragma unroll
+        for (int b = 0; b < kBatch; b++) {
+            const float* rp = P + (size_t)ids.u[j0 + b * kTeams] * K + 4 * tl;
+            const float* rq = Q + (size_t)ids.i[j0 + b * kTeams] * K + 4 * tl;
+#pragma unroll
+            for (int s = 0; s < kSlots; s++) { p[b][s] = load4<ALIGNED>(rp + 32 * s); q[b][s] = load4<ALIGNED>(rq + 32 * s); }
+        }
+#pragma unroll
+        for (int b = 0; b < kBatch; b++) {
+            auto chain = [&](auto of) {
+                float acc = __fmaf_rn(of(p[b][0]), of(q[b][0]), __fmul_rn(of(p[b][1]), of(q[b][1])));
+#pragma unroll
+                for (int s = 2; s < kSlots; s++) acc = __fmaf_rn(of(p[b][s]), of(q[b][s]), acc);
+                return acc;
+            };
+            const float v[4] = {chain([](const float4& x) { return x.x; }), chain([](const float4& x) { return x.y; }),
+                                chain([](const float4& x) { return x.z; }), chain([](const float4& x) { return x.w; })};
+            float x = team_sum4<T>(v, tl);                       // lane: reference lanes 4t + (2 up + up2), steps 16 8 4
+            x = __fadd_rn(x, __shfl_xor_sync(0xffffffffu, x, T / 2));      // step 2: values 0 + 2, 1 + 3
+            x = __fadd_rn(x, __shfl_xor_sync(0xffffffffu, x, T / 4));      // step 1
+            if (tl == 0) {
+                const int at = j0 + b * kTeams;
+                const float e = __fsub_rn(ids.r[at], x);
+                tmp[at] = at < left ? __fmul_rn(e, e) : 0.f;
+            }
+        }
+    }
+    block_tree_512(tmp, block_err + blockIdx.x);
 }
 
 }  // namespace
@@ -139,19 +212,22 @@ __global__ void __launch_bounds__(kRmseThreads) rmse_plain_kernel(const NodeAos*
 cudaError_t launch_rmse(int K, const Stream& t, Arena P, Arena Q, float* block_err, cudaStream_t st) {
     if (t.n == 0) return cudaSuccess;
     const unsigned blocks = (unsigned)((t.n + kRmseBlock - 1) / kRmseBlock);
-    if (K == 128) rmse_kernel<128><<<blocks, kRmseThreads, 0, st>>>(t, P, Q, block_err);
-    else if (K == 64) rmse_kernel<64><<<blocks, kRmseThreads, 0, st>>>(t, P, Q, block_err);
+    if (K == 128) rmse_kernel<128><<<blocks, 512, 0, st>>>(t, P, Q, block_err);
+    else if (K == 64) rmse_kernel<64><<<blocks, 512, 0, st>>>(t, P, Q, block_err);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
 
 cudaError_t launch_rmse_plain(int K, const void* d_test_aos, uint64_t n, const float* P, const float* Q,
-                              float* block_err, cudaStream_t st) {
+                              uint32_t n_users, uint32_t n_items, float* block_err, uint32_t* bad, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     const unsigned blocks = (unsigned)((n + kRmseBlock - 1) / kRmseBlock);
     const NodeAos* t = static_cast<const NodeAos*>(d_test_aos);
-    if (K == 128) rmse_plain_kernel<128><<<blocks, kRmseThreads, 0, st>>>(t, n, P, Q, block_err);
-    else if (K == 64) rmse_plain_kernel<64><<<blocks, kRmseThreads, 0, st>>>(t, n, P, Q, block_err);
+    const bool aligned = ((reinterpret_cast<uintptr_t>(P) | reinterpret_cast<uintptr_t>(Q)) & 15) == 0;
+    if (K == 128 && aligned) rmse_plain_kernel<128, true><<<blocks, 512, 0, st>>>(t, n, P, Q, n_users, n_items, block_err, bad);
+    else if (K == 128) rmse_plain_kernel<128, false><<<blocks, 512, 0, st>>>(t, n, P, Q, n_users, n_items, block_err, bad);
+    else if (K == 64 && aligned) rmse_plain_kernel<64, true><<<blocks, 512, 0, st>>>(t, n, P, Q, n_users, n_items, block_err, bad);
+    else if (K == 64) rmse_plain_kernel<64, false><<<blocks, 512, 0, st>>>(t, n, P, Q, n_users, n_items, block_err, bad);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
@@ -218,7 +294,7 @@ extern "C" int mascot_rmse_device_noalloc(const float* d_P, const float* d_Q, ui
     float* d_err = g_static_block_err_addr[dev];
     const size_t blocks = (size_t)((n_test + kRmseBlock - 1) / kRmseBlock);
     // every one of the `blocks` partials is overwritten by its block, so nothing has to be cleared
-    e = launch_rmse_plain((int)k, d_test, n_test, d_P, d_Q, d_err, nullptr);
+    e = launch_rmse_plain((int)k, d_test, n_test, d_P, d_Q, 0, 0, d_err, nullptr, nullptr);
     if (e == cudaSuccess) e = cudaMemcpy(g_static_host_partials, d_err, sizeof(float) * blocks, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) {
         snprintf(msg, sizeof msg, "evaluation failed: %s", cudaGetErrorString(e));

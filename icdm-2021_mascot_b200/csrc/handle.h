@@ -50,7 +50,6 @@ struct mascot_handle {
     uint32_t* d_umap = nullptr; uint32_t* d_imap = nullptr;
     float* d_stats = nullptr;       // stats_copies sets of: gsum_p | gsum_q | nsum_p | nsum_q
     int stats_copies = 1; size_t stats_stride = 0;
-    float* d_block_err = nullptr;
     mascot::WorkCounters counters;  // chunk counters of the update launches (all on `stream`)
     // grow-only device scratch shared by mascot_reload_train (staging of the uploaded array) and by the
     // partition of the stream by precision class; released by mascot_release_scratch / mascot_destroy
@@ -67,7 +66,6 @@ struct mascot_handle {
     std::vector<float> uerr, ierr, init_uerr, init_ierr;
     std::vector<float> lr;
     std::vector<float> h_stats;     // same layout as d_stats, gsum in LOGICAL element order
-    std::vector<float> h_block_err;
     std::vector<uint64_t> udeg_sum, ideg_sum;   // ratings per group (training set), for byte accounting
     std::vector<uint64_t> seg_off;              // training stream segments: [seg_off[s], seg_off[s+1])
     uint64_t n_train_accounted = 0;
@@ -111,6 +109,32 @@ double now_us();
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);    // from the current device's pool
 void pool_free(void* p, cudaStream_t st);
 void pool_trim();                                                  // gives the current device's idle pool memory back
+
+// Words that a kernel writes and the host reads right after it: pinned host memory that the GPU writes straight into
+// (a copy of some kilobytes costs ten microseconds of its own), or device memory and a copy where the result is
+// large or all pinned blocks are in use.  One more word behind the results is a flag, zero at first.
+class Results {
+public:
+    Results(size_t floats, cudaStream_t st);
+    ~Results();
+    Results(const Results&) = delete;
+    Results& operator=(const Results&) = delete;
+    cudaError_t status() const { return status_; }             // of the allocation
+    float* device() const { return pinned_ ? pinned_ : dev_; }
+    uint32_t* device_flag() const { return reinterpret_cast<uint32_t*>(device() + n_); }
+    cudaError_t wait();                                        // for everything queued on the stream; the results are then in
+    const float* begin() const { return pinned_ ? pinned_ : host_.data(); }
+    const float* end() const { return begin() + n_; }
+    bool flag() const { return reinterpret_cast<const uint32_t*>(begin())[n_] != 0; }
+private:
+    size_t n_;
+    cudaStream_t st_;
+    float* pinned_ = nullptr;
+    float* dev_ = nullptr;
+    std::vector<float> host_;
+    cudaError_t status_ = cudaSuccess;
+};
+void release_results();                                        // gives idle pinned blocks back
 
 template <typename T>
 cudaError_t dev_alloc(T** p, size_t count, cudaStream_t st) {

@@ -87,7 +87,7 @@ void free_ratings(mascot_handle* h) {
     dev_free(h->te_r, h->stream); dev_free(h->te_u, h->stream); dev_free(h->te_i, h->stream);
     dev_free(h->P.f16, h->stream); dev_free(h->P.f32, h->stream); dev_free(h->Q.f16, h->stream); dev_free(h->Q.f32, h->stream);
     dev_free(h->d_uprec_row, h->stream); dev_free(h->d_iprec_row, h->stream); dev_free(h->d_ugroup, h->stream); dev_free(h->d_igroup, h->stream);
-    dev_free(h->d_umap, h->stream); dev_free(h->d_imap, h->stream); dev_free(h->d_stats, h->stream); dev_free(h->d_block_err, h->stream);
+    dev_free(h->d_umap, h->stream); dev_free(h->d_imap, h->stream); dev_free(h->d_stats, h->stream);
     h->have_ratings = h->have_factors = false;
 }
 
@@ -332,7 +332,7 @@ int sort_run_windows(mascot_handle* h) {
     return reorder_segments(h, 0, h->seg_off.size() - 1, false, w);
 }
 
-float reference_rmse_from_partials(const std::vector<float>& part, uint64_t n) {
+float reference_rmse_from_partials(const Results& part, uint64_t n) {
     float sum = 0;                                  // rmse.h:183-186: float accumulation in block order
     for (float v : part) sum += v;
     return (float)std::sqrt(sum / (double)n);       // rmse.h:188, returned through a float
@@ -996,6 +996,7 @@ int mascot_release_scratch(mascot_handle* h) {
     CU(h, cudaStreamSynchronize(h->stream));
     pool_trim();
     release_copy_rings();
+    release_results();
     return MASCOT_OK;
 }
 
@@ -1019,11 +1020,12 @@ int mascot_eval_sq_error(mascot_handle* h, double* sum_sq, uint64_t* count) {
     if (!h->n_test) return MASCOT_OK;
     CU(h, cudaSetDevice(h->cfg.device));
     Stream t; t.r = h->te_r; t.u = h->te_u; t.i = h->te_i; t.n = h->n_test;
-    CU(h, launch_rmse(h->K, t, h->P, h->Q, h->d_block_err, h->stream));
-    CU(h, cudaMemcpyAsync(h->h_block_err.data(), h->d_block_err, sizeof(float) * h->h_block_err.size(), cudaMemcpyDeviceToHost, h->stream));
-    CU(h, cudaStreamSynchronize(h->stream));
+    Results sums((h->n_test + 511) / 512, h->stream);
+    CU(h, sums.status());
+    CU(h, launch_rmse(h->K, t, h->P, h->Q, sums.device(), h->stream));
+    CU(h, sums.wait());
     double s = 0;
-    for (float v : h->h_block_err) s += (double)v;
+    for (float v : sums) s += (double)v;
     *sum_sq = s;
     return MASCOT_OK;
 }
@@ -1034,10 +1036,11 @@ int mascot_eval_rmse(mascot_handle* h, double* rmse) {
     if (!h->n_test) return fail(h, MASCOT_ERR_STATE, "no test ratings were given");
     CU(h, cudaSetDevice(h->cfg.device));
     Stream t; t.r = h->te_r; t.u = h->te_u; t.i = h->te_i; t.n = h->n_test;
-    CU(h, launch_rmse(h->K, t, h->P, h->Q, h->d_block_err, h->stream));
-    CU(h, cudaMemcpyAsync(h->h_block_err.data(), h->d_block_err, sizeof(float) * h->h_block_err.size(), cudaMemcpyDeviceToHost, h->stream));
-    CU(h, cudaStreamSynchronize(h->stream));
-    *rmse = (double)reference_rmse_from_partials(h->h_block_err, h->n_test);
+    Results sums((h->n_test + 511) / 512, h->stream);
+    CU(h, sums.status());
+    CU(h, launch_rmse(h->K, t, h->P, h->Q, sums.device(), h->stream));
+    CU(h, sums.wait());
+    *rmse = (double)reference_rmse_from_partials(sums, h->n_test);
     return MASCOT_OK;
 }
 
@@ -1168,15 +1171,11 @@ int mascot_get_stream_order(mascot_handle* h, uint32_t* src_out) {
 int mascot_rmse_device(const float* d_P, const float* d_Q, uint32_t k, const mascot_rating* d_test, uint64_t n_test, double* rmse) {
     if (!d_P || !d_Q || !d_test || !rmse || !n_test) return fail(nullptr, MASCOT_ERR_BAD_ARG, "null pointer or empty test set");
     if (k != 64 && k != 128) return fail(nullptr, MASCOT_ERR_BAD_ARG, "k must be 64 or 128");
-    const size_t blocks = (size_t)((n_test + 511) / 512);
-    float* d_err = nullptr;
-    CU(nullptr, dev_alloc(&d_err, blocks, nullptr));
-    std::vector<float> part(blocks);
-    cudaError_t e = launch_rmse_plain((int)k, d_test, n_test, d_P, d_Q, d_err, nullptr);
-    if (e == cudaSuccess) e = cudaMemcpy(part.data(), d_err, sizeof(float) * blocks, cudaMemcpyDeviceToHost);
-    dev_free(d_err, nullptr);
-    CU(nullptr, e);
-    *rmse = (double)reference_rmse_from_partials(part, n_test);
+    Results sums((n_test + 511) / 512, nullptr);
+    CU(nullptr, sums.status());
+    CU(nullptr, launch_rmse_plain((int)k, d_test, n_test, d_P, d_Q, 0, 0, sums.device(), nullptr, nullptr));
+    CU(nullptr, sums.wait());
+    *rmse = (double)reference_rmse_from_partials(sums, n_test);
     return MASCOT_OK;
 }
 
@@ -1184,8 +1183,6 @@ int mascot_rmse_host(const float* P, uint32_t n_users, const float* Q, uint32_t 
                      const mascot_rating* test, uint64_t n_test, int device, double* rmse) {
     if (!P || !Q || !test || !rmse || !n_test || !n_users || !n_items) return fail(nullptr, MASCOT_ERR_BAD_ARG, "null pointer or empty input");
     if (k != 64 && k != 128) return fail(nullptr, MASCOT_ERR_BAD_ARG, "k must be 64 or 128");
-    for (uint64_t j = 0; j < n_test; j++)
-        if (test[j].u >= n_users || test[j].i >= n_items) return fail(nullptr, MASCOT_ERR_BAD_ARG, "test rating with id out of range");
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || device < 0 || device >= ndev) {
         cudaGetLastError();
@@ -1199,11 +1196,15 @@ int mascot_rmse_host(const float* P, uint32_t n_users, const float* Q, uint32_t 
     if (e == cudaSuccess) e = copy_to_device(dP, P, sizeof(float) * (size_t)n_users * k, nullptr);
     if (e == cudaSuccess) e = copy_to_device(dQ, Q, sizeof(float) * (size_t)n_items * k, nullptr);
     if (e == cudaSuccess) e = copy_to_device(dT, test, sizeof(mascot_rating) * n_test, nullptr);
-    int rc = MASCOT_OK;
-    if (e == cudaSuccess) rc = mascot_rmse_device(dP, dQ, k, dT, n_test, rmse);
+    Results sums((n_test + 511) / 512, nullptr);
+    if (e == cudaSuccess) e = sums.status();
+    if (e == cudaSuccess) e = launch_rmse_plain((int)k, dT, n_test, dP, dQ, n_users, n_items, sums.device(), sums.device_flag(), nullptr);
+    if (e == cudaSuccess) e = sums.wait();
     dev_free(dP, nullptr); dev_free(dQ, nullptr); dev_free(dT, nullptr);
     CU(nullptr, e);
-    return rc;
+    if (sums.flag()) return fail(nullptr, MASCOT_ERR_BAD_ARG, "test rating with id out of range");
+    *rmse = (double)reference_rmse_from_partials(sums, n_test);
+    return MASCOT_OK;
 }
 
 }  // extern "C"

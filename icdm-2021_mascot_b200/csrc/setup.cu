@@ -423,9 +423,6 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     CU(h, reserve(h, &h->d_stats, h->stats_stride * h->stats_copies));
     CU(h, cudaMemsetAsync(h->d_stats, 0, sizeof(float) * h->stats_stride * h->stats_copies, h->stream));
     h->h_stats.assign(stats_floats(h), 0.f);
-    const size_t blocks = (size_t)((n_test + 511) / 512);
-    CU(h, reserve(h, &h->d_block_err, blocks));
-    h->h_block_err.assign(blocks, 0.f);
     CU(h, cudaStreamSynchronize(h->stream));
     // the set-up's own use of the scratch buffer is over: the sort below may re-carve it
     const int rc_sort = sort_run_windows(h);

@@ -390,10 +390,12 @@ int mascot_shard_eval_rmse(mascot_handle* h, double* rmse) {
     double pair[2] = {0.0, (double)h->n_test};
     if (h->n_test) {
         Stream t; t.r = h->te_r; t.u = h->te_u; t.i = h->te_i; t.n = h->n_test;
-        CU(h, launch_rmse(h->K, t, h->P, h->Q, h->d_block_err, h->stream));
-        CU(h, cudaMemcpyAsync(h->h_block_err.data(), h->d_block_err, sizeof(float) * h->h_block_err.size(), cudaMemcpyDeviceToHost, h->stream));
+        Results sums((h->n_test + 511) / 512, h->stream);
+        CU(h, sums.status());
+        CU(h, launch_rmse(h->K, t, h->P, h->Q, sums.device(), h->stream));
         if ((rc = wait_stream(h, h->stream, "sharded evaluation")) != MASCOT_OK) return rc;
-        for (float v : h->h_block_err) pair[0] += (double)v;
+        CU(h, sums.wait());
+        for (float v : sums) pair[0] += (double)v;
     }
     if (S->world > 1) {
         CU(h, cudaMemcpyAsync(S->d_pair, pair, sizeof pair, cudaMemcpyHostToDevice, h->stream));
