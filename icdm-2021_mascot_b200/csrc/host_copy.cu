@@ -1,9 +1,10 @@
 // Pageable copies.  A rating array, a factor matrix or an order map comes from or goes to ordinary memory of the
 // caller, and cudaMemcpy moves such buffers with one host thread through the driver's own staging: measured on a
-// 16-core B200 host 10.5 GB/s up, 15 GB/s down into memory that has been touched and 4.6 GB/s into fresh pages, where
+// 16-core B200 host 11 GB/s up, 15 GB/s down into memory that has been touched and 4.6 GB/s into fresh pages, where
 // that thread also takes the page faults - against 55 GB/s of the link from pinned memory.  Here up to eight threads
-// each own two slots of a pinned ring: a thread fills (or empties) one slot with memcpy while the copy engine
-// works on the other, so the host side runs at several cores' bandwidth and the faults are taken in parallel.
+// move the data between the caller's memory and a pinned ring while the copy engine works on other parts of the ring, so
+// the host side runs at several cores' bandwidth and the faults are taken in parallel.  Up: 4 MB 15 -> 22 GB/s, 36 MB
+// 12 -> 41, 480 MB 11 -> 51; down into fresh pages 4.6 -> 38.
 #include "host_copy.h"
 
 #include <sched.h>
@@ -11,6 +12,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <cstdint>
 #include <cstdlib>
@@ -30,11 +32,14 @@ constexpr int kSlots = 2 * kMaxThreads;
 constexpr int kMaxRings = 2;                      // rings of a process: 2 x 16 MiB of pinned memory at most
 constexpr size_t kDirect = 192u << 10;            // below this the driver's copy is as fast
 
-// The helper threads of a ring, parked between copies: starting eight threads costs more than copying 4 MB.
+// The helper threads of a ring.  Starting eight threads costs more than copying 4 MB, and waking parked ones takes most
+// of a millisecond on a virtual machine (16 MB up: 1.3 ms after parked threads, 0.45 after awake ones).  Copies come in
+// groups - both factor matrices, then the test set - so a helper stays awake for kAwake after its last work, giving its
+// core to whoever asks for it, and parks then.
 class Team {
 public:
     ~Team() {
-        { std::lock_guard<std::mutex> lock(mu_); quit_ = true; }
+        { std::lock_guard<std::mutex> lock(mu_); quit_ = true; round_++; }
         start_.notify_all();
         for (std::thread& t : threads_) t.join();
     }
@@ -44,34 +49,44 @@ public:
         catch (...) {}                             // no more threads to be had: those that exist do the work
         const int helpers = std::min((int)threads_.size(), threads - 1);
         if (helpers > 0) {
-            { std::lock_guard<std::mutex> lock(mu_); work_ = &work; helpers_ = helpers; running_ = helpers; round_++; }
-            start_.notify_all();
+            bool parked;
+            { std::lock_guard<std::mutex> lock(mu_); work_ = &work; helpers_ = helpers; running_ = helpers; round_++; parked = parked_ > 0; }
+            if (parked) start_.notify_all();
         }
         work(0);
         while (running_.load(std::memory_order_acquire) > 0) std::this_thread::yield();
     }
 
 private:
+    static constexpr std::chrono::milliseconds kAwake{4};
     void loop(int id) {
         unsigned long seen = 0;
-        std::unique_lock<std::mutex> lock(mu_);
         for (;;) {
-            start_.wait(lock, [&] { return quit_ || (round_ != seen && id <= helpers_); });
-            if (quit_) return;
-            seen = round_;
-            const std::function<void(int)>* const work = work_;
-            lock.unlock();
+            const auto parking = std::chrono::steady_clock::now() + kAwake;
+            while (round_.load(std::memory_order_acquire) == seen && std::chrono::steady_clock::now() < parking) std::this_thread::yield();
+            const std::function<void(int)>* work = nullptr;
+            {
+                std::unique_lock<std::mutex> lock(mu_);
+                if (round_ == seen) {
+                    parked_++;
+                    start_.wait(lock, [&] { return round_ != seen; });
+                    parked_--;
+                }
+                if (quit_) return;
+                seen = round_;
+                if (id <= helpers_) work = work_;
+            }
+            if (!work) continue;
             (*work)(id);
             running_.fetch_sub(1, std::memory_order_release);
-            lock.lock();
         }
     }
     std::mutex mu_;
     std::condition_variable start_;
     std::vector<std::thread> threads_;
-    const std::function<void(int)>* work_ = nullptr;
-    int helpers_ = 0;
-    unsigned long round_ = 0;
+    const std::function<void(int)>* work_ = nullptr;      // of round `round_`, for the helpers 1 .. helpers_
+    int helpers_ = 0, parked_ = 0;
+    std::atomic<unsigned long> round_{0};
     std::atomic<int> running_{0};
     bool quit_ = false;
 };
@@ -181,27 +196,39 @@ cudaError_t copy_to_device(void* dev, const void* host, size_t bytes, cudaStream
     if (e != cudaSuccess) return e;
     Ring* const ring = bytes < kDirect || is_pinned(host) ? nullptr : take_ring(device);
     if (!ring) return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
+    // The ring is used in parts of a quarter: a copy costs the engine 4.5 us whatever its size (pieces of 256 KB: 29
+    // GB/s from pinned memory, 1 MB: 43, 4 MB: 49).  The threads fill a part together, and whoever finishes it sends it.
     const int threads = host_threads(bytes);
-    const size_t piece = std::min(kSlot, std::max<size_t>((bytes / (4 * threads) + 255) / 256 * 256, 128u << 10));
+    constexpr size_t kFill = 256u << 10, kParts = 4, kMostPart = kSlot * kSlots / kParts;
+    const size_t part = std::min(kMostPart, std::max<size_t>((bytes / kParts + kFill - 1) / kFill * kFill, 4 * kFill));
+    const size_t parts = (bytes + part - 1) / part, fills = part / kFill;
+    std::vector<std::atomic<int>> left(parts);             // pieces of each part that are still to be filled; -1: sent
+    for (size_t c = 0; c < parts; c++) left[c] = (int)((std::min(part, bytes - c * part) + kFill - 1) / kFill);
     std::atomic<size_t> next{0};
     std::atomic<int> error{0};
-    ring->team.run(threads, [&](int t) {
+    ring->team.run(threads, [&](int) {
         cudaError_t r = cudaSetDevice(device);
-        for (int use = 0; r == cudaSuccess; use++) {
-            const size_t off = next.fetch_add(1) * piece;
-            if (off >= bytes) break;
-            const size_t len = std::min(piece, bytes - off);
-            const int slot = 2 * t + (use & 1);
-            unsigned char* const mem = ring->mem + kSlot * slot;
-            r = cudaEventSynchronize(ring->done[slot]);
-            if (r != cudaSuccess) break;
-            std::memcpy(mem, static_cast<const unsigned char*>(host) + off, len);
-            r = cudaMemcpyAsync(static_cast<unsigned char*>(dev) + off, mem, len, cudaMemcpyHostToDevice, st);
-            if (r == cudaSuccess) r = cudaEventRecord(ring->done[slot], st);
+        for (size_t ready = ~(size_t)0; !error.load(std::memory_order_relaxed);) {
+            const size_t i = next.fetch_add(1), c = i / fills, in = i % fills * kFill;
+            if (c >= parts) break;
+            const size_t len = std::min(part, bytes - c * part);
+            if (in >= len) continue;
+            unsigned char* const mem = ring->mem + c % kParts * kMostPart;
+            if (c != ready) {                                   // what this quarter of the ring held before - of an earlier call, too - has to be gone
+                while (c >= kParts && left[c - kParts].load(std::memory_order_acquire) >= 0 && !error.load(std::memory_order_relaxed)) std::this_thread::yield();
+                if (r == cudaSuccess && !error.load()) r = cudaEventSynchronize(ring->done[c % kParts]);
+                ready = c;
+            }
+            if (r == cudaSuccess) std::memcpy(mem + in, static_cast<const unsigned char*>(host) + c * part + in, std::min(kFill, len - in));
+            if (r == cudaSuccess && left[c].fetch_sub(1, std::memory_order_acq_rel) == 1) {
+                r = cudaMemcpyAsync(static_cast<unsigned char*>(dev) + c * part, mem, len, cudaMemcpyHostToDevice, st);
+                if (r == cudaSuccess) r = cudaEventRecord(ring->done[c % kParts], st);
+                if (r == cudaSuccess) left[c].store(-1, std::memory_order_release);
+            }
+            if (r != cudaSuccess) error = (int)r;
         }
-        if (r != cudaSuccess) error = (int)r;
     });
-    give_ring(ring);                               // copies still in flight are waited for at the slot's next use
+    give_ring(ring);                               // copies still in flight are waited for at the next use
     return (cudaError_t)error.load();
 }
 
@@ -222,6 +249,8 @@ cudaError_t copy_to_host(const CopySpan* spans, int n_spans, cudaStream_t st) {
         return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
     }
     const int threads = host_threads(bytes);
+    for (cudaEvent_t& ev : ring->done) if (e == cudaSuccess) e = cudaEventSynchronize(ev);      // the last parts of an upload before this
+    if (e != cudaSuccess) { give_ring(ring); return e; }
     const std::vector<Piece> pieces = blocks(spans, n_spans, std::min(kSlot, std::max<size_t>(bytes / (4 * threads), 128u << 10)));
     std::atomic<size_t> next{0};
     std::atomic<int> error{0};
