@@ -828,7 +828,9 @@ int mascot_train_epoch(mascot_handle* h, uint32_t epoch, mascot_epoch_stats* out
     const bool check = muppet || ((h->grouped || (switch_only && !h->switched_to_fp32)) && is_check_epoch(h->cfg, epoch));
     uint32_t launches = 0, promoted_u = 0, promoted_i = 0;
     const uint64_t bytes_this_epoch = algorithmic_bytes(h);    // with the precisions the kernel is about to see
-    CU(h, cudaEventRecord(h->ev[0], h->stream));
+    // An epoch without statistics is its update kernels: two events time both the kernels and the whole (each event and
+    // each reading of one costs the host one to two microseconds, of the 160 of an epoch of the smallest configuration).
+    if (check) CU(h, cudaEventRecord(h->ev[0], h->stream));
     if (check) CU(h, cudaMemsetAsync(h->d_stats, 0, sizeof(float) * h->stats_stride * h->stats_copies, h->stream));   // mf_methods.cu:178-182
     CU(h, cudaEventRecord(h->ev[1], h->stream));
     LaunchShape shape;
@@ -850,18 +852,21 @@ int mascot_train_epoch(mascot_handle* h, uint32_t epoch, mascot_epoch_stats* out
         else if (switch_only) { if ((rc = switch_only_policy(h, epoch, &promoted_u, &promoted_i)) != MASCOT_OK) return rc; }
         else if ((rc = apply_stats(h, epoch, &promoted_u, &promoted_i, &launches)) != MASCOT_OK) return rc;
     }
-    CU(h, cudaEventRecord(h->ev[3], h->stream));
-    CU(h, cudaEventSynchronize(h->ev[3]));
+    if (check) CU(h, cudaEventRecord(h->ev[3], h->stream));
+    CU(h, cudaEventSynchronize(h->ev[check ? 3 : 2]));
+    float kernel_ms = 0.f, total_ms = 0.f;
+    if (cudaEventElapsedTime(&kernel_ms, h->ev[1], h->ev[2]) == cudaSuccess) h->timings.update_us += 1e3 * kernel_ms;
+    total_ms = kernel_ms;
+    if (check && out) cudaEventElapsedTime(&total_ms, h->ev[0], h->ev[3]);
     if (out) {
         std::memset(out, 0, sizeof(*out));
         out->updates = h->n_train; out->lr = lr; out->error_check = check ? 1 : 0; out->pass_bits = (uint32_t)bits_this_epoch;
         out->promoted_user_groups = promoted_u; out->promoted_item_groups = promoted_i; out->kernel_launches = launches;
         out->algorithmic_bytes = bytes_this_epoch;
         out->workers = shape.workers;
-        cudaEventElapsedTime(&out->kernel_ms, h->ev[1], h->ev[2]);
-        cudaEventElapsedTime(&out->total_ms, h->ev[0], h->ev[3]);
+        out->kernel_ms = kernel_ms;
+        out->total_ms = total_ms;
     }
-    { float kms = 0.f; if (cudaEventElapsedTime(&kms, h->ev[1], h->ev[2]) == cudaSuccess) h->timings.update_us += 1e3 * kms; }
     return MASCOT_OK;
 }
 

@@ -322,7 +322,7 @@ MASCOT_API int mascot_get_worker_count(mascot_handle* h, uint32_t* workers);
 /* Release the engine's grow-only device scratch (staging buffer of mascot_reload_train, sort buffers of
  * the set-up and of the stream partition, fp32 factors on their way in or out), the freed device memory that
  * the library keeps for its next allocations on this GPU (1 GiB at most), the pinned rings of at most
- * 2 x 16 MiB through which this process copies large pageable buffers and the pinned blocks of at most
+ * 2 x 24 MiB through which this process copies large pageable buffers and the pinned blocks of at most
  * 8 x 64 KiB into which evaluations write, as far as no call is using them.
  * All are allocated again when next needed. */
 MASCOT_API int mascot_release_scratch(mascot_handle* h);
