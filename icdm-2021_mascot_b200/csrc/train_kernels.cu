@@ -902,7 +902,7 @@ constexpr int kSpan = 8;            // consecutive chunks handed out together (t
 // user row of the rating D further on, the item row of the rating DI further on if a run starts there), then the user
 // ring, then the item ring.  A ring
 // slot is as large as the widest row its side can hold in this launch.
-template <int K, int UM, int IM, int NS, int NSI> struct WorkerSmem {
+template <int K, int UM, int IM, bool STATS, int NS, int NSI> struct WorkerSmem {
     static constexpr int TS = K / 8;
     static constexpr int kURowBytes = K * (UM == ROWS_HALF ? 2 : 4);
     static constexpr int kIRowBytes = K * (IM == ROWS_HALF ? 2 : 4);
@@ -911,7 +911,10 @@ template <int K, int UM, int IM, int NS, int NSI> struct WorkerSmem {
     // then lie in different banks.  The rings stay at multiples of 128 bytes (off them, copies and loads of rows touch
     // a line more each: 5.9 instead of 5.5 ms per epoch of the 100M-rating set).
     static constexpr int kShift = 128;
-    static constexpr int kBytes = kRecBytes + kShift + NS * kURowBytes + NSI * kIRowBytes;
+    // With statistics: the groups of both rows of every record, looked up for a whole chunk at once.  (A lookup per
+    // rating is a memory latency per rating: the sampled twentieth of an epoch took a seventh of its time.)
+    static constexpr int kGroupBytes = STATS ? 2 * TS * 4 : 0;
+    static constexpr int kBytes = kRecBytes + kShift + NS * kURowBytes + NSI * kIRowBytes + (kGroupBytes + 127) / 128 * 128;
 };
 
 // NS / NSI: slots of the user / item ring.  User rows are requested D ratings ahead, item rows DI ratings ahead; a
@@ -920,7 +923,7 @@ template <int K, int UM, int IM, int NS, int NSI> struct WorkerSmem {
 // request and the write-back loses that update, and the chance of that grows with the lead.
 template <int K, int KIND, int UM, int IM, bool STATS, int NS, int NSI, int D, int DI>
 __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !STATS) ? 4 : ((UM == ROWS_DYN || STATS || KIND == KIND_AFP || KIND == KIND_MUPPET) ? 2 : 3)) train_kernel(const KernelArgs a) {
-    using SM = WorkerSmem<K, UM, IM, NS, NSI>;
+    using SM = WorkerSmem<K, UM, IM, STATS, NS, NSI>;
     constexpr int TS = SM::TS;                     // lanes per worker = ratings per chunk
     constexpr unsigned kAll = 0xffffffffu;
     static_assert(TS % NS == 0 && (NS & (NS - 1)) == 0 && (NSI & (NSI - 1)) == 0, "the rings must divide the chunk");
@@ -941,6 +944,8 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     const unsigned s_req = s_rec + 2 * TS * 16;
     const unsigned uring = (unsigned)__cvta_generic_to_shared(mine) + SM::kRecBytes + SM::kShift + 16 * m;      // [NS][kURowBytes]
     const unsigned iring = uring + NS * SM::kURowBytes;                   // [NSI][kIRowBytes]
+    uint32_t* const groups = reinterpret_cast<uint32_t*>(mine + SM::kRecBytes + SM::kShift + NS * SM::kURowBytes + NSI * SM::kIRowBytes);
+    constexpr bool kGroups = STATS && KIND == KIND_MIXED;
     const Rows<K, UM> P(a.P, m);
     const Rows<K, IM> Q(a.Q, m);
 
@@ -1034,6 +1039,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
         const bool drop = hot && ((hot_seen + __popc(hot_set & ((2u << m) - 1u))) & hot_mask) != 0u;
         hot_seen += __popc(hot_set);
         const uint32_t u = valid ? inflight.u & kKeep : kNoRow, i = inflight.i;
+        if constexpr (kGroups) groups[b * TS + m] = valid ? (uint32_t)__ldg(a.st.ugroup + (u & kIdMask)) | (uint32_t)__ldg(a.st.igroup + (i & kIdMask)) << 16 : 0u;
         bool udup = false, idup = false, rs = false;
 #pragma unroll
         for (int d = 1; d <= (D > DI + 2 ? D + 1 : DI + 3); d++) {
@@ -1082,7 +1088,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
             if (m == 0) atomicAdd(nsum_q + acc_group, nq_acc);
         }
     };
-    auto record = [&](const Sample& smp, uint32_t uc, uint32_t ic) {
+    auto record = [&](const Sample& smp, uint32_t both_groups) {
         if constexpr (KIND == KIND_MUPPET || KIND == KIND_SWITCH) {
             // muppet_sgd_kernel.h:266-285, sgd_kernel.h:266-285: the squared norm of both gradients goes to the
             // worker's running sum, the element-wise sum of both gradients to k shared accumulators
@@ -1097,13 +1103,13 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
             return;
         }
         if (smp.user) {
-            const uint32_t g = a.st.ugroup[uc & kIdMask];
+            const uint32_t g = both_groups & 0xffffu;
             const float n = worker_sum<TS>(pair_partial(smp.gp, smp.gp), gmask);
             red_add8(gsum_p + (size_t)g * K + 8 * m, smp.gp);
             if (m == 0) atomicAdd(nsum_p + g, n);
         }
         if (smp.item) {
-            const uint32_t g = a.st.igroup[ic & kIdMask];
+            const uint32_t g = both_groups >> 16;
             const float n = worker_sum<TS>(pair_partial(smp.gq, smp.gq), gmask);
             if (g != acc_group) {
                 flush_item_stats();
@@ -1187,7 +1193,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
                 update_one<K, KIND, UM, IM, STATS>(c, rw, uc, ic, p, q, smp, afp, kDyn ? gmask : kAll, meanwhile);
                 if (a.add_user_delta) add_row_delta<K, UM>(P, uc, f & F_DROP, p, p_before);
                 else st_row_if<K, UM>(~f & F_DROP, P, uc, p);
-                if (STATS) { if (!(f & F_NONE)) record(smp, uc, ic); }
+                if (STATS) { if (!(f & F_NONE)) record(smp, kGroups ? groups[cb * TS + jb + t] : 0u); }
                 p = p_next;
             }
         }
@@ -1215,7 +1221,7 @@ template <int K, int KIND, int UM, int IM, bool STATS, int NS, int NSI, int D, i
 cudaError_t launch_ns(KernelArgs a, unsigned warps_per_sm, unsigned workers, cudaStream_t st, LaunchShape* shape, bool dry) {
     constexpr int TS = K / 8;
     constexpr int kPerWarp = 32 / TS;
-    using SM = WorkerSmem<K, UM, IM, NS, NSI>;
+    using SM = WorkerSmem<K, UM, IM, STATS, NS, NSI>;
     auto kern = train_kernel<K, KIND, UM, IM, STATS, NS, NSI, D, DI>;
     // the most dynamic shared memory a launch of this instantiation can ask for: a block of 8 warps
     constexpr size_t kSmemMax = (size_t)8 * kPerWarp * SM::kBytes;
