@@ -23,7 +23,6 @@ struct mascot_handle {
     int mup_idx = 0, mup_switched_epoch = -1, mup_violations = 0;
     float mup_max_diversity = -1.f;
     std::vector<float> mup_norms_epoch, mup_sums_epoch;
-    std::vector<uint32_t> urow_degree;           // training degree of every user row (row space of the arenas)
     bool switched_to_fp32 = false;               // whole-model switching trainer: the switch has happened
     float switch_initial_error = 1.f;            // its error at epoch index 5 (mf_methods.cu:1444, 1530)
     cudaStream_t stream = nullptr;
@@ -61,7 +60,7 @@ struct mascot_handle {
     std::vector<uint64_t> cls_off;
 
     // host
-    std::vector<uint32_t> user2sorted, item2sorted, uend, iend;
+    std::vector<uint32_t> uend, iend;
     std::vector<uint8_t> uprec, iprec;
     std::vector<float> uerr, ierr, init_uerr, init_ierr;
     std::vector<float> lr;
@@ -160,9 +159,11 @@ cudaError_t reserve(mascot_handle* h, T** p, size_t count) {
 
 // ---- mascot_api.cu ----
 void free_ratings(mascot_handle* h);
+int need_copy_stream(mascot_handle* h);                    // copy_stream and its events
 int need_scratch(mascot_handle* h, size_t bytes);           // grow-only device scratch of at least `bytes`
 bool any_fp32_group(const mascot_handle* h);
 int warm_kernels(mascot_handle* h);                        // load the update kernels the first epochs will launch
+int run_window_log2(const mascot_handle* h);               // of the resident stream; 0: none
 int sort_run_windows(mascot_handle* h);                    // item-sorted run windows of a freshly encoded resident stream
 int partition_all(mascot_handle* h);                        // (re)partition the stream by precision class when that pays
 bool is_check_epoch(const mascot_config& c, uint32_t e);

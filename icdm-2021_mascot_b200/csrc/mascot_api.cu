@@ -196,6 +196,16 @@ int need_scratch(mascot_handle* h, size_t bytes) {
     return MASCOT_OK;
 }
 
+int need_copy_stream(mascot_handle* h) {
+    if (h->copy_stream) return MASCOT_OK;
+    for (int b = 0; b < 2; b++) {
+        if (!h->ev_copied[b]) CU(h, cudaEventCreateWithFlags(&h->ev_copied[b], cudaEventDisableTiming));
+        if (!h->ev_free[b]) CU(h, cudaEventCreateWithFlags(&h->ev_free[b], cudaEventDisableTiming));
+    }
+    CU(h, cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
+    return MASCOT_OK;
+}
+
 bool any_fp32_group(const mascot_handle* h) {
     for (uint8_t p : h->uprec) if (p) return true;
     for (uint8_t p : h->iprec) if (p) return true;
@@ -472,17 +482,23 @@ int mascot_reload_train(mascot_handle* h, const mascot_rating* train, uint64_t n
         h->cls_off.clear(); h->partitioned = false;
     }
     if (!n_train) return MASCOT_OK;
-    const size_t bytes = sizeof(mascot_rating) * n_train;
-    int rc = need_scratch(h, bytes);
+    const size_t bytes = sizeof(mascot_rating) * n_train, sort_at = (bytes + 255) / 256 * 256;
+    const int run_window = run_window_log2(h), nseg = (int)h->seg_off.size() - 1;
+    const size_t sort_bytes = source_sort_bytes(n_train, h->seg_off.data(), nseg, run_window, h->irows);
+    int rc = need_scratch(h, sort_at + sort_bytes);
     if (rc != MASCOT_OK) return rc;
     CU(h, cudaMemsetAsync(h->d_err_flag, 0, sizeof(uint32_t), h->stream));
     CU(h, copy_to_device(h->d_scratch, train, bytes, h->stream));
-    CU(h, encode_segments(h, static_cast<const mascot_rating*>(h->d_scratch), h->seg_off, h->cfg.shuffle != 0,
-                          h->tr_r, h->tr_u, h->tr_i, h->tr_src));
+    if (sort_bytes)
+        CU(h, launch_source_sort(h->d_scratch, n_train, h->seg_off.data(), nseg, h->cfg.seed, run_window, h->irows, h->d_umap, h->d_imap, h->d_uprec_row, h->d_iprec_row,
+                                 h->n_users, h->n_items, h->d_err_flag, static_cast<unsigned char*>(h->d_scratch) + sort_at, h->tr_r, h->tr_u, h->tr_i, h->tr_src, h->stream));
+    else
+        CU(h, encode_segments(h, static_cast<const mascot_rating*>(h->d_scratch), h->seg_off, h->cfg.shuffle != 0,
+                              h->tr_r, h->tr_u, h->tr_i, h->tr_src));
     uint32_t bad = 0;
     CU(h, cudaMemcpyAsync(&bad, h->d_err_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
     h->cls_off.clear();
-    if ((rc = sort_run_windows(h)) != MASCOT_OK) return rc;
+    if (!sort_bytes && (rc = sort_run_windows(h)) != MASCOT_OK) return rc;
     if ((rc = partition_all(h)) != MASCOT_OK) return rc;      // the new stream carries the current precisions
     CU(h, cudaStreamSynchronize(h->stream));
     if (bad) return fail(h, MASCOT_ERR_BAD_ARG, "training rating with id out of range (replaced by zero ratings of row 0; reload a valid array)");
@@ -877,13 +893,7 @@ int mascot_train_epoch_streamed(mascot_handle* h, uint32_t epoch, const mascot_r
     if (h->shard) return fail(h, MASCOT_ERR_STATE, "this engine belongs to a sharded group: use mascot_shard_train_epoch");
     CU(h, cudaSetDevice(h->cfg.device));
     constexpr uint64_t kPiece = 8ull << 20;           // ratings per piece (96 MiB of input)
-    if (!h->copy_stream) {
-        CU(h, cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
-        for (int b = 0; b < 2; b++) {
-            CU(h, cudaEventCreateWithFlags(&h->ev_copied[b], cudaEventDisableTiming));
-            CU(h, cudaEventCreateWithFlags(&h->ev_free[b], cudaEventDisableTiming));
-        }
-    }
+    { const int rc_stream = need_copy_stream(h); if (rc_stream != MASCOT_OK) return rc_stream; }
     const uint64_t piece = std::min<uint64_t>(kPiece, std::max<uint64_t>(n_train, 1));
     if (h->stage_ratings < piece) {
         for (int b = 0; b < 2; b++) dev_free(h->d_stage[b], h->copy_stream);
@@ -1084,17 +1094,30 @@ int mascot_get_group_info(mascot_handle* h, int side, uint32_t* n_groups, uint32
     return MASCOT_OK;
 }
 
+// id -> sorted index of both sides (either may be null), from the device's id -> arena row maps
+static cudaError_t sorted_indices(mascot_handle* h, uint32_t* users, uint32_t* items) {
+    if (h->sorted_space) {
+        CopySpan spans[2];
+        int n = 0;
+        if (users) spans[n++] = CopySpan{users, h->d_umap, sizeof(uint32_t) * h->n_users};
+        if (items) spans[n++] = CopySpan{items, h->d_imap, sizeof(uint32_t) * h->n_items};
+        const cudaError_t e = copy_to_host(spans, n, h->stream);
+        if (e != cudaSuccess) return e;
+    }
+    auto finish = [&](uint32_t* v, uint32_t n, const RowLayout& L) {
+        if (!v || (h->sorted_space && L.parts <= 1)) return;           // the row is the sorted index
+        for (uint32_t e = 0; e < n; e++) v[e] = h->sorted_space ? sorted_of_row(L, v[e]) : e;
+    };
+    finish(users, h->n_users, h->ulay);
+    finish(items, h->n_items, h->ilay);
+    return cudaSuccess;
+}
+
 int mascot_get_index_maps(mascot_handle* h, uint32_t* user2sorted, uint32_t* item2sorted) {
     if (!h) return MASCOT_ERR_BAD_ARG;
     if (!h->have_ratings) return fail(h, MASCOT_ERR_STATE, "mascot_set_ratings must come first");
-    if (user2sorted) {
-        if (h->sorted_space) std::copy(h->user2sorted.begin(), h->user2sorted.end(), user2sorted);
-        else for (uint32_t e = 0; e < h->n_users; e++) user2sorted[e] = e;
-    }
-    if (item2sorted) {
-        if (h->sorted_space) std::copy(h->item2sorted.begin(), h->item2sorted.end(), item2sorted);
-        else for (uint32_t e = 0; e < h->n_items; e++) item2sorted[e] = e;
-    }
+    CU(h, cudaSetDevice(h->cfg.device));
+    CU(h, sorted_indices(h, user2sorted, item2sorted));
     return MASCOT_OK;
 }
 
@@ -1139,8 +1162,10 @@ int mascot_get_test_ratings(mascot_handle* h, mascot_rating* out, int order) {
     std::vector<uint32_t> s2u, s2i;
     if (order == 0 && h->sorted_space) {
         s2u.resize(h->n_users); s2i.resize(h->n_items);
-        for (uint32_t e = 0; e < h->n_users; e++) s2u[h->user2sorted[e]] = e;
-        for (uint32_t e = 0; e < h->n_items; e++) s2i[h->item2sorted[e]] = e;
+        std::vector<uint32_t> u2s(h->n_users), i2s(h->n_items);
+        CU(h, sorted_indices(h, u2s.data(), i2s.data()));
+        for (uint32_t e = 0; e < h->n_users; e++) s2u[u2s[e]] = e;
+        for (uint32_t e = 0; e < h->n_items; e++) s2i[i2s[e]] = e;
     }
     for (uint64_t j = 0; j < n; j++) {
         // the stream holds arena rows: back to sorted indices, then (order 0) to the caller's ids

@@ -335,6 +335,79 @@ cudaError_t launch_stream_sort(const float* r, const uint32_t* u, const uint32_t
     return cudaGetLastError();
 }
 
+// ---- the coded stream in one sort -----------------------------------------------------------------
+// encode_sorted_kernel's windows of kWindow positions only matter for what is not sorted any further.  Where run windows
+// follow - whose boundaries fall on multiples of kWindow - a stable sort of the permuted SOURCE positions by (segment, run
+// window, item row) gives the same order in one go: the block sort, the second pass over the coded arrays and the
+// copies back fall away, and the key fits 32 bits.
+__global__ void source_key_kernel(const NodeAos* src, uint64_t n, const uint64_t* seg_off, int nseg, uint64_t seed, const uint32_t* imap, uint32_t n_items,
+                                  StreamKey sk, uint32_t* key, uint32_t* val) {
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x) {
+        int lo = 0, hi = nseg - 1;                    // last segment whose offset is <= j
+        while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (seg_off[mid] <= j) lo = mid; else hi = mid - 1; }
+        const uint64_t off = seg_off[lo], s = off + permute_index(j - off, seg_off[lo + 1] - off, seed + 0x9e3779b97f4a7c15ull * (uint64_t)lo);
+        uint32_t it = src[s].i;
+        if (it >= n_items) it = 0;                    // reported when the record is read below
+        key[j] = (((uint32_t)lo << sk.window_bits | (uint32_t)(j >> sk.run_window_log2)) << sk.item_bits) | (imap ? imap[it] : it);
+        val[j] = (uint32_t)s;
+    }
+}
+__global__ void source_gather_kernel(const uint32_t* val, uint64_t n, const NodeAos* src, const uint32_t* umap, const uint32_t* imap,
+                                     const uint8_t* uprec, const uint8_t* iprec, uint32_t n_users, uint32_t n_items, uint32_t* err,
+                                     float* r, uint32_t* u, uint32_t* i, uint32_t* src_out) {
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t s = val[j];
+        const NodeAos nd = checked(src[s], n_users, n_items, err);
+        uint32_t uu = umap ? umap[nd.u] : nd.u, ii = imap ? imap[nd.i] : nd.i;
+        uu |= row_flags_to_code(uprec[uu]);
+        ii |= row_flags_to_code(iprec[ii]);
+        r[j] = nd.r; u[j] = uu; i[j] = ii; src_out[j] = s;
+    }
+}
+
+static int source_key_bits(uint64_t n, int nseg, int run_window_log2, uint32_t item_rows, StreamKey* sk) {
+    *sk = make_stream_key(n, false, run_window_log2, item_rows);
+    int seg_bits = 0;
+    while ((1ll << seg_bits) < nseg) seg_bits++;
+    return seg_bits + sk->window_bits + sk->item_bits;
+}
+
+size_t source_sort_bytes(uint64_t n, const uint64_t* seg_off, int nseg, int run_window_log2, uint32_t item_rows) {
+    StreamKey sk;
+    if (n == 0 || run_window_log2 <= 0 || source_key_bits(n, nseg, run_window_log2, item_rows, &sk) > 32) return 0;
+    for (int s = 0; s < nseg; s++) if (seg_off[s] % kWindow) return 0;
+    size_t temp = 0;
+    cub::DoubleBuffer<uint32_t> keys(nullptr, nullptr), vals(nullptr, nullptr);
+    cub::DeviceRadixSort::SortPairs(nullptr, temp, keys, vals, n, 0, 32);
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    return 4 * up(4 * n) + up(8 * (size_t)(nseg + 1)) + up(temp);
+}
+
+cudaError_t launch_source_sort(const void* d_src_aos, uint64_t n, const uint64_t* seg_off, int nseg, uint64_t seed, int run_window_log2, uint32_t item_rows,
+                               const uint32_t* user_map, const uint32_t* item_map, const uint8_t* uprec_row, const uint8_t* iprec_row,
+                               uint32_t n_users, uint32_t n_items, uint32_t* err_flag, void* space, float* r, uint32_t* u, uint32_t* i, uint32_t* src_out,
+                               cudaStream_t st) {
+    StreamKey sk;
+    const int bits = source_key_bits(n, nseg, run_window_log2, item_rows, &sk);
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    unsigned char* base = static_cast<unsigned char*>(space);
+    uint32_t* buf[4];
+    for (uint32_t*& b : buf) { b = reinterpret_cast<uint32_t*>(base); base += up(4 * n); }
+    uint64_t* d_seg = reinterpret_cast<uint64_t*>(base); base += up(8 * (size_t)(nseg + 1));
+    cudaError_t e = cudaMemcpyAsync(d_seg, seg_off, sizeof(uint64_t) * (nseg + 1), cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return e;
+    const NodeAos* src = static_cast<const NodeAos*>(d_src_aos);
+    const int g = grid_for(n, 256);
+    source_key_kernel<<<g, 256, 0, st>>>(src, n, d_seg, nseg, seed, item_map, n_items, sk, buf[0], buf[1]);
+    cub::DoubleBuffer<uint32_t> keys(buf[0], buf[2]), vals(buf[1], buf[3]);
+    size_t temp = 0;
+    e = cub::DeviceRadixSort::SortPairs(nullptr, temp, keys, vals, n, 0, bits, st);
+    if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(base, temp, keys, vals, n, 0, bits, st);
+    if (e != cudaSuccess) return e;
+    source_gather_kernel<<<g, 256, 0, st>>>(vals.Current(), n, src, user_map, item_map, uprec_row, iprec_row, n_users, n_items, err_flag, r, u, i, src_out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_scatter_factors(int K, const float* src, uint32_t rows, const uint32_t* row_map,
                                    bool round_through_half, __half* dst16, float* dst32, cudaStream_t st) {
     if (rows == 0) return cudaSuccess;

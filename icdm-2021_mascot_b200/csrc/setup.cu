@@ -9,7 +9,7 @@
 //   1. ids checked against n_users / n_items and degree histogram (atomics)            check_hist_kernel
 //   2. entities sorted by (degree, id): stable radix sort of the degrees, ids as values  cub::DeviceRadixSort
 //   3. grouping walk over the sorted degrees on the host (O(entities))                   make_groups
-//   4. id -> arena row maps, per-row group / precision tables                            host, O(entities)
+//   4. id -> arena row maps, per-row group / precision tables                            side_kernel
 //   5. sharded engines: ratings of this rank's users selected and ordered by the step of the block
 //      schedule at which their item block is here - a stable radix sort of a small key   select_key_kernel
 //   6. seeded permutation, item-sorted windows, id remap, precision tags                 launch_encode_stream
@@ -111,16 +111,70 @@ int sort_by_degree(mascot_handle* h, const uint32_t* d_deg, uint32_t n, uint32_t
     return MASCOT_OK;
 }
 
-// Host tables of one side from its sorted degrees: groups, maps, per-row flags; uploads the device copies.
-int build_side(mascot_handle* h, bool users, const std::vector<uint32_t>& s2o, const std::vector<uint32_t>& cnt_sorted,
-               const std::vector<uint32_t>& local_degree_by_id, uint64_t n_local) {
+// The tables of one side, a thread per sorted index: map[id] = arena row, and per row its group and storage flags; per
+// group the ratings of this engine's stream (byte accounting).  Consecutive indices mostly share a group, so a warp adds
+// its degrees up first.
+// A user whose ratings are so many that many workers hold its row at any time: adding up the changes of
+// that many concurrent, equally stale updates multiplies the step and can diverge.  Expected number of
+// workers inside their read-to-write span of a row: c = workers x 4 ratings x degree / n.  Measured: 23 still
+// converges as well as the reference (20M-rating configuration), 82 diverges (252M-rating one).  Above 32 the
+// row is marked, and only one in 2^shift of the updates of marked rows is written back (as a reduction, like
+// every other user row), with 2^shift the power of two that brings the c of the most popular user to 32 or
+// less (one shift per engine: the update kernel gets it as an argument); the other updates of the row are
+// dropped, which is what a plain store does to all but one of the concurrent holders - without the cost of
+// plain stores to a line every SM writes (252M-rating set at quarter size: 10.8 ms per epoch with plain stores
+// for the marked rows, 5.2 ms with reductions for every update, 4.4 ms with no write-back at all).
+// hot_workers: 0 for items.
+__global__ void side_kernel(const uint32_t* s2o, const uint32_t* local_degree, uint32_t n, RowLayout L, const uint32_t* group_end, uint32_t groups,
+                            uint8_t prec, uint64_t hot_workers, uint64_t n_local, uint32_t* map, uint16_t* group, uint8_t* flags,
+                            unsigned long long* degree_sum, uint32_t* hot_shift) {
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t s0 = blockIdx.x * blockDim.x + threadIdx.x - (threadIdx.x & 31); s0 < n; s0 += stride) {
+        const uint32_t s = s0 + (threadIdx.x & 31);
+        const bool in = s < n;
+        uint32_t g = 0;
+        unsigned long long deg = 0;
+        if (in) {
+            const uint32_t id = s2o ? s2o[s] : s, row = arena_row(L, s);
+            uint32_t hi = groups - 1;                   // first group that ends at or behind s
+            while (g < hi) { const uint32_t mid = (g + hi) >> 1; if (group_end[mid] < s) g = mid + 1; else hi = mid; }
+            deg = local_degree[id];
+            uint8_t f = prec;
+            if (deg * hot_workers > 8 * n_local) {
+                uint32_t shift = 1;
+                while (shift < 24 && ((deg * hot_workers) >> shift) > 8 * n_local) shift++;
+                f |= kRowHot;
+                atomicMax(hot_shift, shift);
+            }
+            if (map) map[id] = row;
+            group[row] = (uint16_t)g;
+            flags[row] = f;
+        }
+        const uint32_t first = __shfl_sync(0xffffffffu, g, 0);
+        if (__all_sync(0xffffffffu, !in || g == first)) {
+            for (int d = 16; d >= 1; d >>= 1) deg += __shfl_xor_sync(0xffffffffu, deg, d);
+            if ((threadIdx.x & 31) == 0) atomicAdd(degree_sum + first, deg);
+        } else if (in) {
+            atomicAdd(degree_sum + g, deg);
+        }
+    }
+}
+
+// Where side_kernel's inputs and sums live: scratch of the set-up.
+struct SideSpace {
+    uint32_t* ends;                    // [65536]
+    unsigned long long* sums;          // [65536]
+    uint32_t* shift;                   // [1]
+};
+
+// Groups of one side from its sorted degrees, and its device tables.  The sums arrive with finish_side.
+int build_side(mascot_handle* h, bool users, const uint32_t* d_s2o, const std::vector<uint32_t>& cnt_sorted, const uint32_t* d_local_degree,
+               uint64_t n_local, const SideSpace& sp) {
     const uint32_t n = users ? h->n_users : h->n_items;
     const RowLayout& L = users ? h->ulay : h->ilay;
     const uint32_t rows = layout_rows(L);
     std::vector<uint32_t>& end = users ? h->uend : h->iend;
     std::vector<uint8_t>& prec = users ? h->uprec : h->iprec;
-    std::vector<uint32_t>& o2s = users ? h->user2sorted : h->item2sorted;
-    std::vector<uint64_t>& deg_sum = users ? h->udeg_sum : h->ideg_sum;
     if (h->grouped) {
         make_groups(cnt_sorted, users ? h->cfg.user_group_num : h->cfg.item_group_num, end);
         if (end.size() > 65535) return fail(h, MASCOT_ERR_BAD_ARG, "more than 65535 groups");
@@ -129,63 +183,30 @@ int build_side(mascot_handle* h, bool users, const std::vector<uint32_t>& s2o, c
         end.assign(1, n - 1);
         prec.assign(1, (h->kind == KIND_MEMQUANT || h->kind == KIND_SWITCH) ? 0 : 1);
     }
-    // sorted position -> id (identity when ids are not sorted), id -> sorted position, id -> arena row
-    o2s.clear();
-    std::vector<uint32_t> row_of_id(n);
-    if (h->sorted_space) {
-        o2s.resize(n);
-        for (uint32_t s = 0; s < n; s++) o2s[s2o[s]] = s;
-        for (uint32_t e = 0; e < n; e++) row_of_id[e] = arena_row(L, o2s[e]);
-    } else {
-        for (uint32_t e = 0; e < n; e++) row_of_id[e] = e;
-    }
-    // per arena row: group and storage flags; ratings of this engine's stream per group (byte accounting)
-    std::vector<uint16_t> group(rows, 0);
-    std::vector<uint8_t> flags(rows, 0);
-    deg_sum.assign(end.size(), 0);
-    if (users) { h->urow_degree.assign(rows, 0); h->hot_user_shift = 0; }
-    uint32_t s = 0;
-    // A user whose ratings are so many that many workers hold its row at any time: adding up the changes of
-    // that many concurrent, equally stale updates multiplies the step and can diverge.  Expected number of
-    // workers inside their read-to-write span of a row: c = workers x 4 ratings x degree / n.  Measured: 23 still
-    // converges as well as the reference (20M-rating configuration), 82 diverges (252M-rating one).  Above 32 the
-    // row is marked, and only one in 2^shift of the updates of marked rows is written back (as a reduction, like
-    // every other user row), with 2^shift the power of two that brings the c of the most popular user to 32 or
-    // less (one shift per engine: the update kernel gets it as an argument); the other updates of the row are
-    // dropped, which is what a plain store does to all but one of the concurrent holders - without the cost of
-    // plain stores to a line every SM writes (252M-rating set at quarter size: 10.8 ms per epoch with plain stores
-    // for the marked rows, 5.2 ms with reductions for every update, 4.4 ms with no write-back at all).
-    const uint64_t w_est = std::min<uint64_t>(worker_count(h, n_local), 16384);
-    for (size_t g = 0; g < end.size(); g++) {
-        for (; s <= end[g] && s < n; s++) {
-            const uint32_t id = h->sorted_space ? s2o[s] : s;
-            const uint32_t row = arena_row(L, s);
-            const uint32_t deg = local_degree_by_id[id];
-            group[row] = (uint16_t)g;
-            flags[row] = prec[g] ? kRowPrec : 0;
-            deg_sum[g] += deg;
-            if (users) {
-                h->urow_degree[row] = deg;
-                if ((uint64_t)deg * w_est > 8 * n_local) {
-                    uint32_t shift = 1;
-                    while (shift < 24 && (((uint64_t)deg * w_est) >> shift) > 8 * n_local) shift++;
-                    flags[row] |= kRowHot;
-                    h->hot_user_shift = std::max(h->hot_user_shift, shift);
-                }
-            }
-        }
-    }
     uint16_t** dg = users ? &h->d_ugroup : &h->d_igroup;
     uint8_t** dp = users ? &h->d_uprec_row : &h->d_iprec_row;
     uint32_t** dm = users ? &h->d_umap : &h->d_imap;
     CU(h, reserve(h, dg, rows)); CU(h, reserve(h, dp, rows));
-    CU(h, cudaMemcpyAsync(*dg, group.data(), sizeof(uint16_t) * rows, cudaMemcpyHostToDevice, h->stream));
-    CU(h, cudaMemcpyAsync(*dp, flags.data(), sizeof(uint8_t) * rows, cudaMemcpyHostToDevice, h->stream));
-    if (h->sorted_space) {
-        CU(h, reserve(h, dm, n));
-        CU(h, cudaMemcpyAsync(*dm, row_of_id.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, h->stream));
+    if (h->sorted_space) CU(h, reserve(h, dm, n));
+    if (rows > n) {                    // rows that the layout leaves unused
+        CU(h, cudaMemsetAsync(*dg, 0, sizeof(uint16_t) * rows, h->stream));
+        CU(h, cudaMemsetAsync(*dp, 0, sizeof(uint8_t) * rows, h->stream));
     }
-    CU(h, cudaStreamSynchronize(h->stream));       // the host vectors above end with this call
+    CU(h, cudaMemcpyAsync(sp.ends, end.data(), sizeof(uint32_t) * end.size(), cudaMemcpyHostToDevice, h->stream));
+    CU(h, cudaMemsetAsync(sp.sums, 0, sizeof(unsigned long long) * end.size(), h->stream));
+    CU(h, cudaMemsetAsync(sp.shift, 0, sizeof(uint32_t), h->stream));
+    const uint64_t hot_workers = users ? std::min<uint64_t>(worker_count(h, n_local), 16384) : 0;
+    side_kernel<<<grid_for(n, 256), 256, 0, h->stream>>>(d_s2o, d_local_degree, n, L, sp.ends, (uint32_t)end.size(), prec[0] ? kRowPrec : 0, hot_workers,
+                                                         n_local, h->sorted_space ? *dm : nullptr, *dg, *dp, sp.sums, sp.shift);
+    CU(h, cudaGetLastError());
+    return MASCOT_OK;
+}
+
+int finish_side(mascot_handle* h, bool users, const SideSpace& sp) {
+    std::vector<uint64_t>& deg_sum = users ? h->udeg_sum : h->ideg_sum;
+    deg_sum.assign((users ? h->uend : h->iend).size(), 0);
+    CU(h, cudaMemcpyAsync(deg_sum.data(), sp.sums, sizeof(uint64_t) * deg_sum.size(), cudaMemcpyDeviceToHost, h->stream));
+    if (users) CU(h, cudaMemcpyAsync(&h->hot_user_shift, sp.shift, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
     return MASCOT_OK;
 }
 
@@ -234,64 +255,87 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     temp_bytes = std::max(temp_bytes, tb);
     cub::DeviceRadixSort::SortPairs(nullptr, tb, (const unsigned long long*)nullptr, (unsigned long long*)nullptr, (const uint32_t*)nullptr, (uint32_t*)nullptr, rq.n_test, 0, 64);
     temp_bytes = std::max(temp_bytes, tb);
-    const size_t need = Carver::up(sizeof(NodeAos) * n_big) * 2 + Carver::up(8 * n_big) * 2 + Carver::up(4 * n_big) * 2 +
-                        Carver::up(4 * (size_t)n_ent) * 6 + Carver::up(temp_bytes) + Carver::up(8 * 4100) + 4096;
-    int rc = need_scratch(h, need);
+    const uint64_t n_sel = sharded ? n_big : rq.n_test;           // ratings that are selected or sorted here
+    const size_t need = Carver::up(sizeof(NodeAos) * n_big) + Carver::up(sizeof(NodeAos) * n_sel) + Carver::up(8 * n_sel) * 2 + Carver::up(4 * n_sel) * 2 +
+                        Carver::up(4 * (size_t)n_ent) * 9 + Carver::up(temp_bytes) + Carver::up(8 * 4100) + 2 * (Carver::up(4 * 65536) + Carver::up(8 * 65536)) + 4096;
+    // the stream is built by one sort where that applies (its size and segments are known here unless the set is sharded)
+    h->seg_off = seg;
+    h->n_train = rq.n_train;
+    const int run_window = sharded ? 0 : run_window_log2(h);
+    const size_t sort_bytes = source_sort_bytes(rq.n_train, seg.data(), (int)rq.n_segments, run_window, h->irows);
+    int rc = need_scratch(h, need + sort_bytes);
     if (rc != MASCOT_OK) return rc;
     Carver cv(h->d_scratch);
     NodeAos* aos = cv.take<NodeAos>(n_big);
-    NodeAos* aos2 = cv.take<NodeAos>(n_big);
-    unsigned long long* key64_a = cv.take<unsigned long long>(n_big);      // also used as 16-bit keys
-    unsigned long long* key64_b = cv.take<unsigned long long>(n_big);
-    uint32_t* idx_a = cv.take<uint32_t>(n_big);
-    uint32_t* idx_b = cv.take<uint32_t>(n_big);
+    NodeAos* aos2 = cv.take<NodeAos>(n_sel);
+    unsigned long long* key64_a = cv.take<unsigned long long>(n_sel);      // also used as 16-bit keys
+    unsigned long long* key64_b = cv.take<unsigned long long>(n_sel);
+    uint32_t* idx_a = cv.take<uint32_t>(n_sel);
+    uint32_t* idx_b = cv.take<uint32_t>(n_sel);
     uint32_t* d_udeg = cv.take<uint32_t>(n_ent);
     uint32_t* d_ideg = cv.take<uint32_t>(n_ent);
-    uint32_t* d_sorted_deg = cv.take<uint32_t>(n_ent);
-    uint32_t* d_s2o = cv.take<uint32_t>(n_ent);
+    uint32_t* d_sorted_deg = cv.take<uint32_t>(2 * (size_t)n_ent);         // users, then items
+    uint32_t* const us2o = cv.take<uint32_t>(n_ent);
+    uint32_t* const is2o = cv.take<uint32_t>(n_ent);
     uint32_t* d_iota = cv.take<uint32_t>(n_ent);
+    uint32_t* d_given = cv.take<uint32_t>(n_ent);       // degrees the caller gave
     uint32_t* d_ldeg = cv.take<uint32_t>(n_ent);        // local degrees of the second side, see below
+    uint32_t* const side_words = cv.take<uint32_t>(64);
+    const SideSpace uspace{cv.take<uint32_t>(65536), cv.take<unsigned long long>(65536), side_words};
+    const SideSpace ispace{cv.take<uint32_t>(65536), cv.take<unsigned long long>(65536), side_words + 1};
     void* temp = cv.take<unsigned char>(temp_bytes);
     unsigned long long* d_first = cv.take<unsigned long long>(4100);
+    void* sort_space = cv.take<unsigned char>(sort_bytes);
     uint16_t* key16_a = reinterpret_cast<uint16_t*>(key64_a);
     uint16_t* key16_b = reinterpret_cast<uint16_t*>(key64_b);
 
     double t_phase = now_us();
     // ---- 1. training ratings: upload, check, degrees ----
-    if (n_all) CU(h, copy_to_device(aos, rq.train, sizeof(NodeAos) * n_all, h->stream));
     CU(h, cudaMemsetAsync(d_udeg, 0, sizeof(uint32_t) * n_users, h->stream));
     CU(h, cudaMemsetAsync(d_ideg, 0, sizeof(uint32_t) * n_items, h->stream));
-    if (n_all) {
-        check_hist_kernel<<<grid_for(n_all, 256), 256, 0, h->stream>>>(aos, n_all, n_users, n_items, d_udeg, d_ideg, h->d_err_flag);
+    // Large arrays go up piece by piece on the copy stream, and the degrees of a piece are counted while the next one is
+    // on its way (40M ratings: 1.2 ms of counting, 0.2 of it after the upload).
+    constexpr uint64_t kPiece = 8ull << 20;             // ratings, 96 MiB
+    const bool pieces = n_all > kPiece;
+    if (pieces) {
+        if ((rc = need_copy_stream(h)) != MASCOT_OK) return rc;
+        CU(h, cudaEventRecord(h->ev_free[0], h->stream));
+        CU(h, cudaStreamWaitEvent(h->copy_stream, h->ev_free[0], 0));
+    }
+    for (uint64_t off = 0; off < n_all; off += kPiece) {
+        const uint64_t len = std::min<uint64_t>(kPiece, n_all - off);
+        CU(h, copy_to_device(aos + off, rq.train + off, sizeof(NodeAos) * len, pieces ? h->copy_stream : h->stream));
+        if (pieces) {
+            CU(h, cudaEventRecord(h->ev_copied[0], h->copy_stream));
+            CU(h, cudaStreamWaitEvent(h->stream, h->ev_copied[0], 0));
+        }
+        check_hist_kernel<<<grid_for(len, 256), 256, 0, h->stream>>>(aos + off, len, n_users, n_items, d_udeg, d_ideg, h->d_err_flag);
         CU(h, cudaGetLastError());
     }
     uint32_t bad = 0;
     CU(h, cudaMemcpyAsync(&bad, h->d_err_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-    CU(h, cudaStreamSynchronize(h->stream));
-    if (bad) return fail(h, MASCOT_ERR_BAD_ARG, "training rating with id out of range");
-    // degrees that define the index space: those of the array (the whole data set for library-side
-    // sharding) or the tables a caller-sharded engine was given
-    std::vector<uint32_t> udeg_local(n_users), ideg_local(n_items);
-    CU(h, cudaMemcpyAsync(udeg_local.data(), d_udeg, sizeof(uint32_t) * n_users, cudaMemcpyDeviceToHost, h->stream));
-    CU(h, cudaMemcpyAsync(ideg_local.data(), d_ideg, sizeof(uint32_t) * n_items, cudaMemcpyDeviceToHost, h->stream));
-    if (rq.user_degree) {
-        CU(h, cudaMemcpyAsync(d_udeg, rq.user_degree, sizeof(uint32_t) * n_users, cudaMemcpyHostToDevice, h->stream));
-        CU(h, cudaMemcpyAsync(d_ideg, rq.item_degree, sizeof(uint32_t) * n_items, cudaMemcpyHostToDevice, h->stream));
-    }
 
     // ---- 2.-4. degree sort, groups, maps ----
-    std::vector<uint32_t> us2o, is2o, ucnt, icnt;
+    // degrees that define the index space: those of the array (the whole data set for library-side
+    // sharding) or the tables a caller-sharded engine was given
+    std::vector<uint32_t> ucnt, icnt;
     if (h->sorted_space) {
-        us2o.resize(n_users); ucnt.resize(n_users); is2o.resize(n_items); icnt.resize(n_items);
-        if ((rc = sort_by_degree(h, d_udeg, n_users, d_sorted_deg, d_s2o, d_iota, temp, temp_bytes)) != MASCOT_OK) return rc;
-        CU(h, cudaMemcpyAsync(us2o.data(), d_s2o, sizeof(uint32_t) * n_users, cudaMemcpyDeviceToHost, h->stream));
-        CU(h, cudaMemcpyAsync(ucnt.data(), d_sorted_deg, sizeof(uint32_t) * n_users, cudaMemcpyDeviceToHost, h->stream));
-        CU(h, cudaStreamSynchronize(h->stream));
-        if ((rc = sort_by_degree(h, d_ideg, n_items, d_sorted_deg, d_s2o, d_iota, temp, temp_bytes)) != MASCOT_OK) return rc;
-        CU(h, cudaMemcpyAsync(is2o.data(), d_s2o, sizeof(uint32_t) * n_items, cudaMemcpyDeviceToHost, h->stream));
-        CU(h, cudaMemcpyAsync(icnt.data(), d_sorted_deg, sizeof(uint32_t) * n_items, cudaMemcpyDeviceToHost, h->stream));
+        ucnt.resize(n_users); icnt.resize(n_items);
+        const uint32_t* deg[2] = {d_udeg, d_ideg};
+        const uint32_t* given[2] = {rq.user_degree, rq.item_degree};
+        for (int side = 0; side < 2; side++) {
+            const uint32_t n = side ? n_items : n_users;
+            if (given[side]) {
+                CU(h, cudaMemcpyAsync(d_given, given[side], sizeof(uint32_t) * n, cudaMemcpyHostToDevice, h->stream));
+                deg[side] = d_given;
+            }
+            if ((rc = sort_by_degree(h, deg[side], n, d_sorted_deg + (side ? n_users : 0), side ? is2o : us2o, d_iota, temp, temp_bytes)) != MASCOT_OK) return rc;
+        }
+        const CopySpan spans[2] = {{ucnt.data(), d_sorted_deg, sizeof(uint32_t) * n_users}, {icnt.data(), d_sorted_deg + n_users, sizeof(uint32_t) * n_items}};
+        CU(h, copy_to_host(spans, 2, h->stream));
     }
     CU(h, cudaStreamSynchronize(h->stream));
+    if (bad) return fail(h, MASCOT_ERR_BAD_ARG, "training rating with id out of range");
     h->timings.rating_histogram_us += now_us() - t_phase; t_phase = now_us();
 
     uint64_t n_local = n_all;
@@ -302,7 +346,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
             if (part_of_row(h->ulay, arena_row(h->ulay, s)) == (uint32_t)rq.rank) n_local += ucnt[s];
     }
     h->n_train = n_local;          // the automatic worker count and the hot-user mark follow this engine's own stream
-    if ((rc = build_side(h, true, us2o, ucnt, udeg_local, n_local)) != MASCOT_OK) return rc;
+    if ((rc = build_side(h, true, h->sorted_space ? us2o : nullptr, ucnt, d_udeg, n_local, uspace)) != MASCOT_OK) return rc;
 
     h->timings.grouping_us += now_us() - t_phase; t_phase = now_us();
     // ---- 5. sharded: keep this rank's ratings, one segment per step of the block schedule ----
@@ -310,7 +354,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     const uint32_t* src_through = nullptr;
     if (sharded) {
         // item rows are needed for the block of a rating: build the item map first (flags come later, with local degrees)
-        if ((rc = build_side(h, false, is2o, icnt, ideg_local, std::max<uint64_t>(n_local, 1))) != MASCOT_OK) return rc;
+        if ((rc = build_side(h, false, is2o, icnt, d_ideg, std::max<uint64_t>(n_local, 1), ispace)) != MASCOT_OK) return rc;
         const int kb = bits_for((uint64_t)rq.blocks + 1);
         if (n_all) {
             select_key_kernel<<<grid_for(n_all, 256), 256, 0, h->stream>>>(aos, n_all, h->d_umap, h->d_imap, h->ulay, h->ilay, (uint32_t)rq.rank,
@@ -339,11 +383,11 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
             check_hist_kernel<<<grid_for(n_local, 256), 256, 0, h->stream>>>(aos2, n_local, n_users, n_items, nullptr, d_ldeg, h->d_err_flag);
             CU(h, cudaGetLastError());
         }
-        CU(h, cudaMemcpyAsync(ideg_local.data(), d_ldeg, sizeof(uint32_t) * n_items, cudaMemcpyDeviceToHost, h->stream));
-        CU(h, cudaStreamSynchronize(h->stream));
     }
     { const double t_g = now_us();
-      if ((rc = build_side(h, false, is2o, icnt, ideg_local, std::max<uint64_t>(n_local, 1))) != MASCOT_OK) return rc;
+      if ((rc = build_side(h, false, h->sorted_space ? is2o : nullptr, icnt, sharded ? d_ldeg : d_ideg, std::max<uint64_t>(n_local, 1), ispace)) != MASCOT_OK) return rc;
+      if ((rc = finish_side(h, true, uspace)) != MASCOT_OK) return rc;
+      if ((rc = finish_side(h, false, ispace)) != MASCOT_OK) return rc;
       h->timings.grouping_us += now_us() - t_g; t_phase += now_us() - t_g; }
     h->seg_off = seg;
     h->n_train_accounted = n_local;
@@ -353,7 +397,10 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     // ---- 6. the coded training stream ----
     CU(h, reserve(h, &h->tr_r, n_local)); CU(h, reserve(h, &h->tr_u, n_local)); CU(h, reserve(h, &h->tr_i, n_local));
     CU(h, reserve(h, &h->tr_src, n_local));
-    if (n_local) {
+    if (sort_bytes) {
+        CU(h, launch_source_sort(enc_src, n_local, h->seg_off.data(), (int)rq.n_segments, h->cfg.seed, run_window, h->irows, h->d_umap, h->d_imap, h->d_uprec_row,
+                                 h->d_iprec_row, n_users, n_items, h->d_err_flag, sort_space, h->tr_r, h->tr_u, h->tr_i, h->tr_src, h->stream));
+    } else if (n_local) {
         CU(h, encode_segments(h, reinterpret_cast<const mascot_rating*>(enc_src), seg, h->cfg.shuffle != 0, h->tr_r, h->tr_u, h->tr_i, h->tr_src));
         if (src_through) {          // positions in the caller's array, not in the selected copy
             compose_kernel<<<grid_for(n_local, 256), 256, 0, h->stream>>>(h->tr_src, n_local, src_through);
@@ -364,13 +411,14 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     // ---- 7. the test set ----
     uint64_t n_test = rq.n_test;
     if (rq.n_test) {
-        CU(h, cudaStreamSynchronize(h->stream));          // aos / aos2 are reused
         CU(h, copy_to_device(aos, rq.test, sizeof(NodeAos) * rq.n_test, h->stream));
         check_hist_kernel<<<grid_for(rq.n_test, 256), 256, 0, h->stream>>>(aos, rq.n_test, n_users, n_items, nullptr, nullptr, h->d_err_flag);
         CU(h, cudaGetLastError());
-        CU(h, cudaMemcpyAsync(&bad, h->d_err_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-        CU(h, cudaStreamSynchronize(h->stream));
-        if (bad) return fail(h, MASCOT_ERR_BAD_ARG, "test rating with id out of range");
+        if (sharded) {                                    // ids are used as indices below
+            CU(h, cudaMemcpyAsync(&bad, h->d_err_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
+            CU(h, cudaStreamSynchronize(h->stream));
+            if (bad) return fail(h, MASCOT_ERR_BAD_ARG, "test rating with id out of range");
+        }
         NodeAos* cur = aos; NodeAos* other = aos2;
         if (sharded && rq.world > 1) {
             owner_key_kernel<<<grid_for(rq.n_test, 256), 256, 0, h->stream>>>(cur, rq.n_test, h->d_umap, h->ulay, (uint32_t)rq.rank, key16_a, idx_a);
@@ -405,7 +453,9 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
         CU(h, reserve(h, &h->te_r, 0)); CU(h, reserve(h, &h->te_u, 0)); CU(h, reserve(h, &h->te_i, 0));
     }
     h->n_test = n_test;
+    CU(h, cudaMemcpyAsync(&bad, h->d_err_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
+    if (bad) return fail(h, MASCOT_ERR_BAD_ARG, "test rating with id out of range");
     h->timings.reconstruction_us += now_us() - t_phase; t_phase = now_us();
 
     // ---- factor arenas and statistics ----
@@ -425,7 +475,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     h->h_stats.assign(stats_floats(h), 0.f);
     CU(h, cudaStreamSynchronize(h->stream));
     // the set-up's own use of the scratch buffer is over: the sort below may re-carve it
-    const int rc_sort = sort_run_windows(h);
+    const int rc_sort = sort_bytes ? MASCOT_OK : sort_run_windows(h);
     if (rc_sort != MASCOT_OK) return rc_sort;
     const int rc_warm = warm_kernels(h);
     if (rc_warm != MASCOT_OK) return rc_warm;
