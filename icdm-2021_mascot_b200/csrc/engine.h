@@ -107,14 +107,15 @@ cudaError_t launch_recode(uint32_t* ids, uint64_t n, const uint8_t* prec_row, cu
 // Stable re-ordering of a coded stream inside every segment, by precision class (by_class; class = 2 * (user
 // row fp32) + (item row fp32)) and / or by item inside windows of 2^run_window_log2 positions
 // (run_window_log2 > 0; item_rows = rows of the item arena, which bounds the item part of the key).
-// Inputs r/u/i/src (src may be null) stay untouched; the result goes to r2/u2/i2/src2.  key_* (n u64),
-// idx_* (n u32) and temp (stream_sort_temp_bytes) are scratch; d_first (may be null) receives, for every
+// Inputs r/u/i/src (src may be null) stay untouched; the result goes to r2/u2/i2/src2.  key_* (n keys of
+// stream_sort_key_bytes each), idx_* (n u32) and temp (stream_sort_temp_bytes) are scratch; d_first (may be null) receives, for every
 // segment * 4 + class, the first position holding it (all ones when it does not occur).  segclass_bits =
 // bits of the largest segment * 4 + class.
+size_t stream_sort_key_bytes(uint64_t n, int segclass_bits, bool by_class, int run_window_log2, uint32_t item_rows);
 size_t stream_sort_temp_bytes(uint64_t n, int segclass_bits, bool by_class, int run_window_log2, uint32_t item_rows);
 cudaError_t launch_stream_sort(const float* r, const uint32_t* u, const uint32_t* i, const uint32_t* src, uint64_t n,
                                const uint64_t* d_seg_off, int nseg, int segclass_bits, bool by_class, int run_window_log2,
-                               uint32_t item_rows, uint64_t* key_a, uint64_t* key_b, uint32_t* idx_a, uint32_t* idx_b,
+                               uint32_t item_rows, void* key_a, void* key_b, uint32_t* idx_a, uint32_t* idx_b,
                                void* temp, size_t temp_bytes, unsigned long long* d_first,
                                float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, cudaStream_t st);
 // The whole resident stream from the uploaded array: seeded permutation of every segment, item-sorted run windows, ids

@@ -169,15 +169,15 @@ cudaError_t encode_segments(mascot_handle* h, const mascot_rating* d_src, const 
     return cudaSuccess;
 }
 
-// One group fp16 -> fp32 (precision_switching.h:12-27): widen its rows into the fp32 arena and flip
+// The groups g .. last fp16 -> fp32 (precision_switching.h:12-27): widen their rows into the fp32 arena and flip
 // the per-row precision bytes; the stream ids are re-tagged afterwards by recode_side().
-int promote_group(mascot_handle* h, bool users, size_t g) {
+int promote_groups(mascot_handle* h, bool users, size_t g, size_t last) {
     const std::vector<uint32_t>& end = users ? h->uend : h->iend;
     std::vector<uint8_t>& prec = users ? h->uprec : h->iprec;
     uint8_t* prow = users ? h->d_uprec_row : h->d_iprec_row;
-    const uint32_t b = g ? end[g - 1] + 1 : 0, e = end[g] + 1;
+    const uint32_t b = g ? end[g - 1] + 1 : 0, e = end[last] + 1;
     CU(h, launch_promote_rows(h->K, users ? h->P : h->Q, prow, users ? h->ulay : h->ilay, b, e, h->stream));
-    prec[g] = 1;
+    std::fill(prec.begin() + (long)g, prec.begin() + (long)last + 1, (uint8_t)1);
     return MASCOT_OK;
 }
 
@@ -234,14 +234,14 @@ int reorder_segments(mascot_handle* h, size_t seg_first, size_t seg_count, bool 
     while ((1ull << key_bits) < seg_count * 4) key_bits++;
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t temp_bytes = stream_sort_temp_bytes(n, key_bits, by_class, run_window_log2, h->irows);
-    const size_t b_key = up(sizeof(uint64_t) * n), b_idx = up(sizeof(uint32_t) * n), b_seg = up(sizeof(uint64_t) * (seg_count + 1));
+    const size_t b_key = up(stream_sort_key_bytes(n, key_bits, by_class, run_window_log2, h->irows) * n), b_idx = up(sizeof(uint32_t) * n), b_seg = up(sizeof(uint64_t) * (seg_count + 1));
     const size_t b_first = up(sizeof(unsigned long long) * seg_count * 4);
     const size_t total = 2 * b_key + 2 * b_idx + 4 * b_idx + b_seg + b_first + up(temp_bytes);
     int rc = need_scratch(h, total);
     if (rc != MASCOT_OK) return rc;
     unsigned char* base = static_cast<unsigned char*>(h->d_scratch);
-    uint64_t* key_a = reinterpret_cast<uint64_t*>(base); base += b_key;
-    uint64_t* key_b = reinterpret_cast<uint64_t*>(base); base += b_key;
+    void* key_a = base; base += b_key;
+    void* key_b = base; base += b_key;
     uint32_t* idx_a = reinterpret_cast<uint32_t*>(base); base += b_idx;
     uint32_t* idx_b = reinterpret_cast<uint32_t*>(base); base += b_idx;
     float* r2 = reinterpret_cast<float*>(base); base += b_idx;
@@ -603,7 +603,7 @@ void muppet_policy(mascot_handle* h, uint32_t epoch) {
     }
 }
 
-int promote_group(mascot_handle* h, bool users, size_t g);
+int promote_groups(mascot_handle* h, bool users, size_t g, size_t last);
 int recode_side(mascot_handle* h, bool users);
 
 // Whole-model switching trainer after a check epoch (mf_methods.cu:1515-1545): error = squared norm of
@@ -619,8 +619,8 @@ int switch_only_policy(mascot_handle* h, uint32_t epoch, uint32_t* promoted_u, u
     if (epoch == 5) h->switch_initial_error = error;
     if (epoch > 5 && error > h->cfg.error_threshold) {
         int rc;
-        if ((rc = promote_group(h, true, 0)) != MASCOT_OK) return rc;
-        if ((rc = promote_group(h, false, 0)) != MASCOT_OK) return rc;
+        if ((rc = promote_groups(h, true, 0, 0)) != MASCOT_OK) return rc;
+        if ((rc = promote_groups(h, false, 0, 0)) != MASCOT_OK) return rc;
         if ((rc = recode_side(h, true)) != MASCOT_OK) return rc;
         if ((rc = recode_side(h, false)) != MASCOT_OK) return rc;
         h->switched_to_fp32 = true;
@@ -743,10 +743,15 @@ int apply_stats(mascot_handle* h, uint32_t epoch, uint32_t* promoted_u, uint32_t
             const std::vector<uint8_t>& prec = users ? h->uprec : h->iprec;
             const std::vector<float>& err = users ? h->uerr : h->ierr;
             uint32_t& count = users ? *promoted_u : *promoted_i;
+            // neighbouring groups are one range of rows: a launch for each run of them
             for (size_t g = 0; g < prec.size(); g++) {
-                if (!(err[g] > h->cfg.error_threshold) || prec[g]) continue;
-                if ((rc = promote_group(h, users, g)) != MASCOT_OK) return rc;
-                count++; if (launches) (*launches)++;
+                size_t last = g;
+                auto due = [&](size_t j) { return j < prec.size() && err[j] > h->cfg.error_threshold && !prec[j]; };
+                if (!due(g)) continue;
+                while (due(last + 1)) last++;
+                if ((rc = promote_groups(h, users, g, last)) != MASCOT_OK) return rc;
+                count += (uint32_t)(last - g + 1); if (launches) (*launches)++;
+                g = last;
             }
             if (count) {
                 if ((rc = recode_side(h, users)) != MASCOT_OK) return rc;
@@ -1130,7 +1135,7 @@ int mascot_promote_group(mascot_handle* h, int side, uint32_t group) {
     if (group >= prec.size()) return fail(h, MASCOT_ERR_BAD_ARG, "group index out of range");
     if (prec[group]) return MASCOT_OK;
     CU(h, cudaSetDevice(h->cfg.device));
-    int rc = promote_group(h, users, group);
+    int rc = promote_groups(h, users, group, group);
     if (rc == MASCOT_OK) rc = recode_side(h, users);
     if (rc == MASCOT_OK) rc = partition_all(h);
     if (rc != MASCOT_OK) return rc;

@@ -267,8 +267,10 @@ struct StreamKey {
     int run_window_log2;     // log2 of the window length; only read when window_bits + item_bits > 0
     int window_bits, item_bits;
 };
+// Key: 32 bits where they hold the key (stream_sort_key_bytes), else 64.
+template <class Key>
 __global__ void stream_key_kernel(const uint32_t* u, const uint32_t* i, uint64_t n, const uint64_t* seg_off, int nseg,
-                                  StreamKey sk, uint64_t* key, uint32_t* idx) {
+                                  StreamKey sk, Key* key, uint32_t* idx) {
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x) {
         int lo = 0, hi = nseg - 1;                    // last segment whose offset is <= j
         while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (seg_off[mid] <= j) lo = mid; else hi = mid - 1; }
@@ -277,7 +279,7 @@ __global__ void stream_key_kernel(const uint32_t* u, const uint32_t* i, uint64_t
         uint64_t k = (uint64_t)lo * 4 + cls;
         if (sk.window_bits + sk.item_bits > 0)
             k = (((k << sk.window_bits) | (j >> sk.run_window_log2)) << sk.item_bits) | (ic & kIdMask);
-        key[j] = k;
+        key[j] = (Key)k;
         idx[j] = (uint32_t)j;
     }
 }
@@ -291,7 +293,8 @@ __global__ void class_gather_kernel(const uint32_t* perm, uint64_t n, const floa
 }
 // first[k] = smallest position whose (segment, class) part of the key is k (entries of absent keys keep their
 // preset value)
-__global__ void class_first_kernel(const uint64_t* key_sorted, uint64_t n, int low_bits, unsigned long long* first) {
+template <class Key>
+__global__ void class_first_kernel(const Key* key_sorted, uint64_t n, int low_bits, unsigned long long* first) {
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x)
         if (j == 0 || (key_sorted[j] >> low_bits) != (key_sorted[j - 1] >> low_bits)) first[key_sorted[j] >> low_bits] = j;
 }
@@ -309,30 +312,47 @@ static StreamKey make_stream_key(uint64_t n, bool by_class, int run_window_log2,
 size_t stream_sort_temp_bytes(uint64_t n, int segclass_bits, bool by_class, int run_window_log2, uint32_t item_rows) {
     size_t bytes = 0;
     const StreamKey sk = make_stream_key(n, by_class, run_window_log2, item_rows);
-    cub::DeviceRadixSort::SortPairs(nullptr, bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr, (const uint32_t*)nullptr,
-                                    (uint32_t*)nullptr, n, 0, segclass_bits + sk.window_bits + sk.item_bits);
+    const int bits = segclass_bits + sk.window_bits + sk.item_bits;
+    if (bits <= 32) cub::DeviceRadixSort::SortPairs(nullptr, bytes, (const uint32_t*)nullptr, (uint32_t*)nullptr, (const uint32_t*)nullptr, (uint32_t*)nullptr, n, 0, bits);
+    else cub::DeviceRadixSort::SortPairs(nullptr, bytes, (const uint64_t*)nullptr, (uint64_t*)nullptr, (const uint32_t*)nullptr, (uint32_t*)nullptr, n, 0, bits);
     return bytes;
 }
 
-cudaError_t launch_stream_sort(const float* r, const uint32_t* u, const uint32_t* i, const uint32_t* src, uint64_t n,
-                               const uint64_t* d_seg_off, int nseg, int segclass_bits, bool by_class, int run_window_log2,
-                               uint32_t item_rows, uint64_t* key_a, uint64_t* key_b, uint32_t* idx_a, uint32_t* idx_b,
-                               void* temp, size_t temp_bytes, unsigned long long* d_first,
-                               float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
-    const int g = grid_for(n, 256);
+size_t stream_sort_key_bytes(uint64_t n, int segclass_bits, bool by_class, int run_window_log2, uint32_t item_rows) {
     const StreamKey sk = make_stream_key(n, by_class, run_window_log2, item_rows);
-    stream_key_kernel<<<g, 256, 0, st>>>(u, i, n, d_seg_off, nseg, sk, key_a, idx_a);
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, key_a, key_b, idx_a, idx_b, n, 0,
-                                                    segclass_bits + sk.window_bits + sk.item_bits, st);
+    return segclass_bits + sk.window_bits + sk.item_bits <= 32 ? 4 : 8;
+}
+
+template <class Key>
+static cudaError_t stream_sort(const float* r, const uint32_t* u, const uint32_t* i, const uint32_t* src, uint64_t n, const uint64_t* d_seg_off, int nseg,
+                               int bits, const StreamKey& sk, Key* key_a, Key* key_b, uint32_t* idx_a, uint32_t* idx_b, void* temp, size_t temp_bytes,
+                               unsigned long long* d_first, float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, cudaStream_t st) {
+    const int g = grid_for(n, 256);
+    stream_key_kernel<Key><<<g, 256, 0, st>>>(u, i, n, d_seg_off, nseg, sk, key_a, idx_a);
+    cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, key_a, key_b, idx_a, idx_b, n, 0, bits, st);
     if (e != cudaSuccess) return e;
     class_gather_kernel<<<g, 256, 0, st>>>(idx_b, n, r, u, i, src, r2, u2, i2, src2);
     if (d_first) {
         e = cudaMemsetAsync(d_first, 0xff, sizeof(unsigned long long) * (size_t)nseg * 4, st);
         if (e != cudaSuccess) return e;
-        class_first_kernel<<<g, 256, 0, st>>>(key_b, n, sk.window_bits + sk.item_bits, d_first);
+        class_first_kernel<Key><<<g, 256, 0, st>>>(key_b, n, sk.window_bits + sk.item_bits, d_first);
     }
     return cudaGetLastError();
+}
+
+cudaError_t launch_stream_sort(const float* r, const uint32_t* u, const uint32_t* i, const uint32_t* src, uint64_t n,
+                               const uint64_t* d_seg_off, int nseg, int segclass_bits, bool by_class, int run_window_log2,
+                               uint32_t item_rows, void* key_a, void* key_b, uint32_t* idx_a, uint32_t* idx_b,
+                               void* temp, size_t temp_bytes, unsigned long long* d_first,
+                               float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    const StreamKey sk = make_stream_key(n, by_class, run_window_log2, item_rows);
+    const int bits = segclass_bits + sk.window_bits + sk.item_bits;
+    if (bits <= 32)
+        return stream_sort(r, u, i, src, n, d_seg_off, nseg, bits, sk, static_cast<uint32_t*>(key_a), static_cast<uint32_t*>(key_b), idx_a, idx_b, temp, temp_bytes,
+                           d_first, r2, u2, i2, src2, st);
+    return stream_sort(r, u, i, src, n, d_seg_off, nseg, bits, sk, static_cast<uint64_t*>(key_a), static_cast<uint64_t*>(key_b), idx_a, idx_b, temp, temp_bytes,
+                       d_first, r2, u2, i2, src2, st);
 }
 
 // ---- the coded stream in one sort -----------------------------------------------------------------

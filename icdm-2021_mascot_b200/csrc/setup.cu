@@ -263,7 +263,10 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     h->n_train = rq.n_train;
     const int run_window = sharded ? 0 : run_window_log2(h);
     const size_t sort_bytes = source_sort_bytes(rq.n_train, seg.data(), (int)rq.n_segments, run_window, h->irows);
-    int rc = need_scratch(h, need + sort_bytes);
+    // (its buffers are free again before the selected and the test ratings need theirs: one piece of scratch for both)
+    const size_t select_bytes = Carver::up(sizeof(NodeAos) * n_sel) + Carver::up(8 * n_sel) * 2 + Carver::up(4 * n_sel) * 2;
+    const size_t more_bytes = sort_bytes > select_bytes ? sort_bytes - select_bytes : 0;
+    int rc = need_scratch(h, need + Carver::up(more_bytes));
     if (rc != MASCOT_OK) return rc;
     Carver cv(h->d_scratch);
     NodeAos* aos = cv.take<NodeAos>(n_big);
@@ -272,6 +275,8 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     unsigned long long* key64_b = cv.take<unsigned long long>(n_sel);
     uint32_t* idx_a = cv.take<uint32_t>(n_sel);
     uint32_t* idx_b = cv.take<uint32_t>(n_sel);
+    cv.take<unsigned char>(more_bytes);
+    void* const sort_space = aos2;
     uint32_t* d_udeg = cv.take<uint32_t>(n_ent);
     uint32_t* d_ideg = cv.take<uint32_t>(n_ent);
     uint32_t* d_sorted_deg = cv.take<uint32_t>(2 * (size_t)n_ent);         // users, then items
@@ -285,7 +290,6 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     const SideSpace ispace{cv.take<uint32_t>(65536), cv.take<unsigned long long>(65536), side_words + 1};
     void* temp = cv.take<unsigned char>(temp_bytes);
     unsigned long long* d_first = cv.take<unsigned long long>(4100);
-    void* sort_space = cv.take<unsigned char>(sort_bytes);
     uint16_t* key16_a = reinterpret_cast<uint16_t*>(key64_a);
     uint16_t* key16_b = reinterpret_cast<uint16_t*>(key64_b);
 
