@@ -338,6 +338,7 @@ struct KernelArgs {
     int epoch;                    // AFP: epoch index
     int add_user_delta;           // user rows are written back as reductions of the change (concurrent launches)
     unsigned workers;             // concurrent sequential workers actually launched
+    unsigned spread;              // AFP: log2 of how few of its workers a warp has, (32 / lanes of a worker) >> spread
     unsigned long long* next_chunk;   // work counter, zero at launch: chunks beyond the first two runs per
                                       // worker are handed out dynamically, so the launch never depends on
                                       // every block being resident at the same time
@@ -704,13 +705,13 @@ __device__ __noinline__ AfpSide afp_requantize(AfpSide s, float diff, float rang
     return s;
 }
 // The workers of a warp go through this together: what one of them needs (a re-estimation, the int8 or the binary16
-// pass) all of them compute, and each keeps the result if it is its own case.
+// pass) all of them compute, and each keeps the result if it is its own case.  active: is there a rating?
 template <int K>
-__device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float r, V8f& p, V8f& q) {
+__device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float r, bool active, V8f& p, V8f& q) {
     constexpr int TS = K / 8;
     constexpr unsigned kAll = 0xffffffffu;
     const long long cur = st.cur;
-    const bool new_user = cur == st.user.next, new_item = cur == st.item.next, new_back = cur == st.back.next;
+    const bool new_user = active && cur == st.user.next, new_item = active && cur == st.item.next, new_back = active && cur == st.back.next;
     const bool estimate = __any_sync(kAll, new_user || new_item || new_back);
     float pmax = 0.f, qmax = 0.f;
     if (estimate) {
@@ -732,11 +733,11 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
     V8h ph, qh;
     quantize(p, st.user.scale, q, st.item.scale, pi, qi, kAll);
     float most = fmaxf(abs_max8(pi), abs_max8(qi));
-    if (__any_sync(kAll, !forward8)) {
+    if (__any_sync(kAll, active && !forward8)) {
         to_grid(p, pi, st.user.scale, q, qi, st.item.scale, __any_sync(kAll, !(most < 2097152.f)), ph, qh);
         pred = forward_half<K>(ph, qh, kAll);
     }
-    if (__any_sync(kAll, forward8)) {
+    if (__any_sync(kAll, active && forward8)) {
         if (__any_sync(kAll, !(most <= 127.f))) { pi = clamp8(pi); qi = clamp8(qi); }
         const float whole = forward_int8<TS>(pi, qi, st.user.scale, st.item.scale, kAll);
         if (forward8) pred = whole;
@@ -751,11 +752,11 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
     quantize(p, st.back.scale, q, st.back.scale, pi, qi, kAll);
     most = fmaxf(abs_max8(pi), abs_max8(qi));
     V8f gp, gq;
-    if (__any_sync(kAll, !back8)) {
+    if (__any_sync(kAll, active && !back8)) {
         to_grid(p, pi, st.back.scale, q, qi, st.back.scale, __any_sync(kAll, !(most < 2097152.f)), ph, qh);
         backward_half(ph, qh, ruv, -c.lam, st.back.scale, gp, gq);
     }
-    if (__any_sync(kAll, back8)) {
+    if (__any_sync(kAll, active && back8)) {
         if (__any_sync(kAll, !(most <= 127.f))) { pi = clamp8(pi); qi = clamp8(qi); }
         V8f wp, wq;
         backward_int8(pi, qi, ruv, -c.lam, st.back.scale, wp, wq);
@@ -776,7 +777,7 @@ __device__ __forceinline__ __half2 half2_of(uint32_t w) { return *reinterpret_ca
 // worker has to do meanwhile, done under the shuffles of the dot product.
 template <int K, int KIND, int UM, int IM, bool STATS, class Mid>
 __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_t uc, uint32_t ic, Raw<UM>& p_raw, Raw<IM>& q_raw,
-                                           Sample& smp, AfpState& afp, unsigned wmask, Mid mid) {
+                                           Sample& smp, AfpState& afp, bool active, unsigned wmask, Mid mid) {
     constexpr int TS = K / 8;
     constexpr bool kAhead = KIND == KIND_MUPPET || KIND == KIND_AFP || UM == ROWS_DYN || IM == ROWS_DYN;      // no single dot product to hide under
     if constexpr (kAhead) { mid(0); mid(1); mid(2); }
@@ -802,7 +803,7 @@ __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_
         if (STATS && c.bits != 32) smp.user = true;
     } else if constexpr (KIND == KIND_AFP) {
         V8f p = as_v8f(p_raw), q = as_v8f(q_raw);
-        afp_update<K>(c, afp, __uint_as_float(rw), p, q);
+        afp_update<K>(c, afp, __uint_as_float(rw), active, p, q);
         put(p_raw, p); put(q_raw, q);
     } else if constexpr (KIND == KIND_MEMQUANT) {
         const V8f p = widen(as_v8h(p_raw)), q = widen(as_v8h(q_raw));
@@ -932,8 +933,12 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     const int lane = threadIdx.x & 31;
     const int m = lane % TS;
     const unsigned gmask = ((1u << TS) - 1u) << (lane - m);      // the lanes of this worker
-    const unsigned worker = (blockIdx.x * blockDim.x + threadIdx.x) / TS;
     const unsigned W = a.workers;
+    // AFP's workers may be alone in their warps (launch_ns); the other lanes then keep them company without work.
+    constexpr bool kSpread = KIND == KIND_AFP;
+    const unsigned per_warp = (32 / TS) >> a.spread, sub = lane / TS;
+    const unsigned worker = !kSpread ? (blockIdx.x * blockDim.x + threadIdx.x) / TS
+                                     : sub < per_warp ? (blockIdx.x * blockDim.x + threadIdx.x) / 32 * per_warp + sub : W;
     // fewer than 2^32 ratings, so chunks are counted in 32 bits
     const unsigned nchunks = (unsigned)((a.s.n + TS - 1) / TS);
 
@@ -1054,12 +1059,12 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
         }
         // The position after a worker's last rating starts a run of nothing, which writes the last item row back.
         const uint32_t f = valid ? (udup ? F_UDUP : 0u) | (rs ? F_RS : 0u) | ((rs && idup) ? F_IDUP : 0u) | (drop ? F_DROP : 0u)
-                                 : F_NONE | F_DROP | (m == inflight.cnt ? F_RS : 0u);
+                                 : F_NONE | F_DROP | ((!kSpread || works) && m == inflight.cnt ? F_RS : 0u);
         uint32_t rw = __float_as_uint(inflight.r);
         if constexpr (kHalfRating<KIND, UM, IM>) { const __half2 h = __float2half2_rn(inflight.r); rw = *reinterpret_cast<const uint32_t*>(&h); }
         recs[b * TS + m] = make_uint4(f, valid ? i : 0u, valid ? u : 0u, rw);
         const int pos = b * TS + m;
-        reqs[2 * ((pos - D) & (2 * TS - 1))] = valid ? u : 0u;
+        reqs[2 * ((pos - D) & (2 * TS - 1))] = valid ? u : (kSpread ? kNoRow : 0u);
         reqs[2 * ((pos - DI) & (2 * TS - 1)) + 1] = (f & F_RS) ? (valid ? i : 0u) : kNoRow;
         prev_u = u; prev_i = i;
         const int cnt = inflight.cnt;
@@ -1067,12 +1072,18 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
         __syncwarp();
         return cnt;
     };
+    if constexpr (kSpread) {
+        // lanes without work go through the updates with harmless rows, which take no slow path
+        if (!works) for (int b = 16 * m; b < NS * SM::kURowBytes + NSI * SM::kIRowBytes; b += 16 * TS)
+            *reinterpret_cast<float4*>(mine + SM::kRecBytes + SM::kShift + b) = make_float4(0.01f, 0.01f, 0.01f, 0.01f);
+    }
     int cnt_cur = publish(0), cnt_next = publish(1);
 
     // item row of the current run
     uint32_t cur_ic = 0;
     unsigned have_item = 0;                          // F_RS while there is one
     Raw<IM> q = Raw<IM>();
+    if constexpr (kSpread) put(q, V8f{{0.01f, 0.01f, 0.01f, 0.01f, 0.01f, 0.01f, 0.01f, 0.01f}});
 
     // item-side statistics of the current run of equal item groups
     V8f gq_acc; float nq_acc = 0.f; uint32_t acc_group = kNoRow;
@@ -1127,7 +1138,10 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     afp.user = AfpSide{8, 1.f, 0.f, 0}; afp.item = afp.user; afp.back = afp.user; afp.cur = 0;
 
     // requests the user row / the item row of a rating into ring slot `slot`
-    auto request_user = [&](uint32_t uc, int slot) { cp_row<K, UM>(uring + slot * SM::kURowBytes, P, uc); };
+    auto request_user = [&](uint32_t uc, int slot) {
+        if constexpr (kSpread) cp_row_if<K, UM>(uring + slot * SM::kURowBytes, P, uc);
+        else cp_row<K, UM>(uring + slot * SM::kURowBytes, P, uc);
+    };
     auto request_item = [&](uint32_t ic, int slot) { cp_row_if<K, IM>(iring + slot * SM::kIRowBytes, Q, ic); };
     // Copy groups complete in order, and every rating commits one: the item row of the rating DI ahead and the user
     // row of the rating D ahead.  Before rating j commits, the groups younger than the user row of rating j+1 are
@@ -1136,7 +1150,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
 #pragma unroll
     for (int t = 0; t < D; t++) {
         if (t >= D - DI) request_item((recs[t - (D - DI)].x & F_RS) ? recs[t - (D - DI)].y : kNoRow, (t - (D - DI)) & (NSI - 1));
-        request_user(recs[t].z, t);
+        request_user(kSpread && (recs[t].x & F_NONE) ? kNoRow : recs[t].z, t);
         cp_commit();
     }
     uint4 rec = recs[0];
@@ -1190,7 +1204,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
                 };
                 const Raw<UM> p_before = p;
                 constexpr bool kDyn = UM == ROWS_DYN || IM == ROWS_DYN;
-                update_one<K, KIND, UM, IM, STATS>(c, rw, uc, ic, p, q, smp, afp, kDyn ? gmask : kAll, meanwhile);
+                update_one<K, KIND, UM, IM, STATS>(c, rw, uc, ic, p, q, smp, afp, !(f & F_NONE), kDyn ? gmask : kAll, meanwhile);
                 if (a.add_user_delta) add_row_delta<K, UM>(P, uc, f & F_DROP, p, p_before);
                 else st_row_if<K, UM>(~f & F_DROP, P, uc, p);
                 if (STATS) { if (!(f & F_NONE)) record(smp, kGroups ? groups[cb * TS + jb + t] : 0u); }
@@ -1227,7 +1241,19 @@ cudaError_t launch_ns(KernelArgs a, unsigned warps_per_sm, unsigned workers, cud
     constexpr size_t kSmemMax = (size_t)8 * kPerWarp * SM::kBytes;
     static LaunchCache cache;                    // one per instantiation; see launch_cache.h
     int grid, block;
-    const unsigned warps = (workers + kPerWarp - 1) / kPerWarp;
+    unsigned warps = (workers + kPerWarp - 1) / kPerWarp;
+    // The workers of an AFP warp compute both passes whenever their formats differ, so few of them are spread over more
+    // warps, up to two per scheduler (4M ratings, 592 workers: 6.75 ms per epoch with two workers a warp, 5.78 with one).
+    // For the other trainers a second warp on a scheduler costs more than it gives: MPT 1.81 ms spread out 2.21, MASCOT
+    // 1.30 and 1.49, MuPPET 3.00 and 3.12.
+    constexpr unsigned kSpreadWarps = KIND == KIND_AFP ? 8 : 0;
+    unsigned spread = 0;
+    if (warps > 8) {
+        const unsigned even = (unsigned)sm_count() * warps_per_sm * kPerWarp;             // the workers of the launch
+        while ((kPerWarp >> spread) > 1 && (warps_per_sm << (spread + 1)) <= kSpreadWarps) spread++;
+        if (spread) { warps_per_sm <<= spread; warps = even / (kPerWarp >> spread); }
+    }
+    a.spread = spread;
     if (workers <= 1) a.add_user_delta = 0;      // a single worker has nobody to race with: plain stores
     unsigned blocks_per_sm = 1, warps_per_block = warps;
     if (warps > 8) {
@@ -1272,7 +1298,7 @@ cudaError_t launch_ns(KernelArgs a, unsigned warps_per_sm, unsigned workers, cud
         // no more blocks than the SM can hold at once (registers, shared memory)
         if (blocks_per_sm > (unsigned)fit) blocks_per_sm = (unsigned)fit;
         grid = (int)((unsigned)sm_count() * blocks_per_sm);
-        a.workers = (unsigned)grid * warps_per_block * kPerWarp;
+        a.workers = (unsigned)grid * warps_per_block * (kPerWarp >> spread);
     }
     if (!dry) kern<<<grid, block, smem_used, st>>>(a);      // a dry call stops here: the function is loaded and configured
     if (shape) { shape->grid = grid; shape->block = block; shape->smem = smem_used; shape->workers = a.workers; }

@@ -62,3 +62,27 @@ def test_extreme_values_bit_exact(mascot, oracle, k, kind, bits):
     assert np.isfinite(P).all()
     assert_bit_equal(Pg, P, "P")
     assert_bit_equal(Qg, Q, "Q")
+
+
+@pytest.mark.parametrize("k", (128, 64))
+@pytest.mark.parametrize("workers,n", [(40, 20011), (200, 20011), (700, 33000), (2500, 33000)])
+def test_afp_workers_alone_and_together_in_their_warps(mascot, oracle, k, workers, n):
+    """Several AFP workers, alone in a warp or not, on ratings that share no row: worker w takes the first run of 8 chunks
+    number w in order, with a format state of its own."""
+    rng = np.random.default_rng(workers)
+    R, P, Q = random_problem(rng, n, n, n, k)
+    R["u"], R["i"] = rng.permutation(n), rng.permutation(n)
+    cfg = mascot.default_config(version=mascot.V_AFP, k=k, num_workers=workers, plain_user_stores=1, seed=3, epoch=50, learning_rate=0.01, decay=0.1, lam=0.05)
+    with mascot.Engine(cfg) as eng:
+        eng.set_ratings(R, R[:10], n, n)
+        eng.set_factors(P, Q)
+        order = eng.stream_order()
+        w = eng.train_epoch(0).workers
+        Pg, Qg = eng.get_factors(0)
+    threshold = int(np.float32((n + w - 1) // w) / np.float32(10.0))
+    run = 8 * (k // 8)
+    assert w >= workers and n <= w * run, "only the first static runs"
+    for b in range(0, n, run):
+        oracle.afp_run(k, R[order[b:b + run]].copy(), None, P, Q, 0.01, 0.05, 0, threshold, oracle.rules_reference())
+    assert_bit_equal(Pg, P, "P")
+    assert_bit_equal(Qg, Q, "Q")
