@@ -1,6 +1,6 @@
 """The fixed-point trainers at values where their rounding and their scales can go wrong: exact halves on the grid, rows of
 zeros, tiny and denormal rows, values beyond the int8 range and beyond 2^21 steps of a grid, extremes next to a power of
-two.  Bit for bit against the sequential oracle."""
+two, rows on one side of zero.  Bit for bit against the sequential oracle."""
 import numpy as np
 import pytest
 
@@ -8,7 +8,7 @@ from helpers import assert_bit_equal, random_problem
 
 pytestmark = pytest.mark.gpu
 
-KINDS = ["halves", "zeros", "zero_side", "tiny", "denormal", "mixed", "large", "powers"]
+KINDS = ["halves", "zeros", "zero_side", "tiny", "denormal", "mixed", "large", "powers", "negative"]
 
 
 def factors(kind, rng, rows, k):
@@ -28,6 +28,8 @@ def factors(kind, rng, rows, k):
         return x * (10.0 ** rng.integers(-6, 2, (rows, 1))).astype(np.float32)
     if kind == "large":
         return x * np.float32(20)
+    if kind == "negative":                    # the smallest magnitude may decide the scale
+        return (-np.abs(1 + x / 40) * np.float32(0.5) ** rng.integers(0, 3, (rows, 1))).astype(np.float32)
     scale = np.float32(2.0) ** rng.integers(-8, 2, (rows, 1)).astype(np.float32)
     x = np.clip(x, -1, 1) * scale
     x[:, 0] = (scale * np.float32(127.5 / 128))[:, 0]                        # top / hi a power of two, exactly or by a few units
@@ -84,5 +86,28 @@ def test_afp_workers_alone_and_together_in_their_warps(mascot, oracle, k, worker
     assert w >= workers and n <= w * run, "only the first static runs"
     for b in range(0, n, run):
         oracle.afp_run(k, R[order[b:b + run]].copy(), None, P, Q, 0.01, 0.05, 0, threshold, oracle.rules_reference())
+    assert_bit_equal(Pg, P, "P")
+    assert_bit_equal(Qg, Q, "Q")
+
+
+@pytest.mark.parametrize("k", (128, 64))
+@pytest.mark.parametrize("bits", (8, 12, 32))
+@pytest.mark.parametrize("kind", ("mixed", "powers", "negative"))
+def test_muppet_workers_side_by_side(mascot, oracle, k, bits, kind):
+    """Two or four MuPPET workers in a warp, whose rows need different scales and some of them the exact formula: ratings that
+    share no row, so that their order does not matter."""
+    n = 20011
+    rng = np.random.default_rng(k + bits)
+    R, _, _ = random_problem(rng, n, n, n, k)
+    R["u"], R["i"] = rng.permutation(n), rng.permutation(n)
+    P, Q = factors(kind, rng, n, k), factors(kind, rng, n, k)
+    cfg = mascot.default_config(version=mascot.V_MUPPET, k=k, num_workers=200, plain_user_stores=1, epoch=50, learning_rate=1e-6, decay=0.1, lam=0.05,
+                                muppet_width=bits, sample_ratio=0.1)
+    with mascot.Engine(cfg) as eng:
+        eng.set_ratings(R, R[:10], n, n)
+        eng.set_factors(P, Q)
+        eng.train_epoch(0)
+        Pg, Qg = eng.get_factors(0)
+    oracle.muppet_run(k, R, None, P, Q, float(np.float32(1e-6)), 0.05, bits, bits, oracle.rules_reference(), first_sample_pos=n)
     assert_bit_equal(Pg, P, "P")
     assert_bit_equal(Qg, Q, "Q")
