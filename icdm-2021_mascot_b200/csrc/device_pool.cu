@@ -62,8 +62,27 @@ constexpr int kBlocks = 8;
 struct PinnedBlock { float* mem; bool busy; };
 std::vector<PinnedBlock> g_blocks;
 
+// Memory of Results whose caller gave up waiting (a group of engines that was dissolved): a kernel behind `after` still
+// writes into it.  It serves nobody else until the event has passed; without an event it never does.
+struct Abandoned { float* mem; bool pinned; cudaEvent_t after; };
+std::vector<Abandoned> g_abandoned;
+
+// With g_mutex held: pinned blocks that are free again, and device memory that may be freed now.
+void sweep_abandoned(std::vector<float*>* device) {
+    for (size_t j = 0; j < g_abandoned.size();) {
+        const Abandoned a = g_abandoned[j];
+        // freeing device memory may wait for the whole device: only where the caller asks for memory back
+        if ((!a.pinned && !device) || !a.after || cudaEventQuery(a.after) != cudaSuccess) { cudaGetLastError(); j++; continue; }
+        cudaEventDestroy(a.after);
+        if (a.pinned) { for (PinnedBlock& b : g_blocks) if (b.mem == a.mem) b.busy = false; }
+        else device->push_back(a.mem);
+        g_abandoned.erase(g_abandoned.begin() + (long)j);
+    }
+}
+
 float* take_block() {
     std::lock_guard<std::mutex> lock(g_mutex);
+    if (!g_abandoned.empty()) sweep_abandoned(nullptr);
     for (PinnedBlock& b : g_blocks) if (!b.busy) { b.busy = true; return b.mem; }
     if (g_blocks.size() >= (size_t)kBlocks) return nullptr;
     float* mem = nullptr;
@@ -82,6 +101,14 @@ Results::Results(size_t floats, cudaStream_t st) : n_(floats), st_(st) {
 }
 
 Results::~Results() {
+    if (status_ == cudaSuccess && !waited_) {      // the kernel may still be queued
+        Abandoned a{pinned_ ? pinned_ : dev_, pinned_ != nullptr, nullptr};
+        if (cudaEventCreateWithFlags(&a.after, cudaEventDisableTiming) != cudaSuccess) a.after = nullptr;
+        else if (cudaEventRecord(a.after, st_) != cudaSuccess) { cudaEventDestroy(a.after); a.after = nullptr; }
+        std::lock_guard<std::mutex> lock(g_mutex);
+        g_abandoned.push_back(a);
+        return;
+    }
     dev_free(dev_, st_);
     if (!pinned_) return;
     std::lock_guard<std::mutex> lock(g_mutex);
@@ -89,13 +116,20 @@ Results::~Results() {
 }
 
 cudaError_t Results::wait() {
-    if (pinned_) return cudaStreamSynchronize(st_);
-    host_.resize(n_ + 1);
-    const cudaError_t e = cudaMemcpyAsync(host_.data(), dev_, sizeof(float) * (n_ + 1), cudaMemcpyDeviceToHost, st_);
-    return e == cudaSuccess ? cudaStreamSynchronize(st_) : e;
+    cudaError_t e = cudaSuccess;
+    if (!pinned_) {
+        host_.resize(n_ + 1);
+        e = cudaMemcpyAsync(host_.data(), dev_, sizeof(float) * (n_ + 1), cudaMemcpyDeviceToHost, st_);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+    waited_ = e == cudaSuccess;
+    return e;
 }
 
 void release_results() {
+    std::vector<float*> device;
+    { std::lock_guard<std::mutex> lock(g_mutex); sweep_abandoned(&device); }
+    for (float*& p : device) dev_free(p, nullptr);
     std::lock_guard<std::mutex> lock(g_mutex);
     for (size_t j = 0; j < g_blocks.size();) {
         if (g_blocks[j].busy) { j++; continue; }

@@ -111,7 +111,8 @@ void pool_trim();                                                  // gives the 
 
 // Words that a kernel writes and the host reads right after it: pinned host memory that the GPU writes straight into
 // (a copy of some kilobytes costs ten microseconds of its own), or device memory and a copy where the result is
-// large or all pinned blocks are in use.  One more word behind the results is a flag, zero at first.
+// large or all pinned blocks are in use.  One more word behind the results is a flag, zero at first.  An object that goes
+// without a successful wait() leaves its memory aside until the stream has passed the kernels that were queued so far.
 class Results {
 public:
     Results(size_t floats, cudaStream_t st);
@@ -132,8 +133,9 @@ private:
     float* dev_ = nullptr;
     std::vector<float> host_;
     cudaError_t status_ = cudaSuccess;
+    bool waited_ = false;
 };
-void release_results();                                        // gives idle pinned blocks back
+void release_results();                                        // gives idle pinned blocks back, and abandoned memory that is idle by now
 
 template <typename T>
 cudaError_t dev_alloc(T** p, size_t count, cudaStream_t st) {

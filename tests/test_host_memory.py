@@ -1,0 +1,34 @@
+"""CPU tests of the memory that the library shares between calls (csrc/device_pool.cu, csrc/host_copy.cu), compiled with
+g++ against a fake CUDA runtime (fake_cudart.h) whose streams can be stuck."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "icdm-2021_mascot_b200", "csrc")
+
+
+def compile_check(tmp_path_factory, name, sources):
+    exe = str(tmp_path_factory.mktemp(name) / name)
+    cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-I", CSRC, "-I", cuda, "-x", "c++", os.path.join(ROOT, "tests", name + ".cpp")]
+                          + [os.path.join(CSRC, s) for s in sources] + ["-o", exe, "-lpthread"])
+    return exe
+
+
+@pytest.fixture(scope="module")
+def shard_timeout_check(tmp_path_factory):
+    return compile_check(tmp_path_factory, "shard_timeout_check", ["shard.cu", "device_pool.cu"])
+
+
+@pytest.mark.parametrize("n_test,gpus", [(5000, 1), (5000, 2), (512 * 20000, 1), (512 * 20000, 2)])
+def test_sums_of_an_abandoned_evaluation_go_to_nobody_else(shard_timeout_check, n_test, gpus):
+    """The all-gather in front of the evaluation kernel never ends: the call gives up after its limit, and the memory that the
+    queued kernel will write into - a pinned block or device memory - is neither freed nor handed out until it has run."""
+    out = subprocess.run([shard_timeout_check, "gather", str(n_test), str(gpus)], capture_output=True, text=True, timeout=60)
+    assert out.returncode == 0, out.stdout
+    lines = out.stdout.splitlines()
+    assert lines[1] == "hung rc -6"
+    assert lines[2] == "given away 0 alive 1" and lines[3] == "kept by a release 1"
+    assert lines[4] == "left pinned 0" and lines[5] == "left device 0"
