@@ -400,8 +400,10 @@ int mascot_shard_eval_rmse(mascot_handle* h, double* rmse) {
     if (S->world > 1) {
         CU(h, cudaMemcpyAsync(S->d_pair, pair, sizeof pair, cudaMemcpyHostToDevice, h->stream));
         NC(h, S, S->api->AllReduce(S->d_pair, S->d_pair, 2, ncclDouble, ncclSum, S->comm, h->stream));
-        CU(h, cudaMemcpyAsync(pair, S->d_pair, sizeof pair, cudaMemcpyDeviceToHost, h->stream));
+        // read back after the bounded wait: a copy into pageable memory blocks until everything before it has run
         if ((rc = wait_stream(h, h->stream, "sharded evaluation")) != MASCOT_OK) return rc;
+        CU(h, cudaMemcpyAsync(pair, S->d_pair, sizeof pair, cudaMemcpyDeviceToHost, h->stream));
+        CU(h, cudaStreamSynchronize(h->stream));
     }
     *rmse = pair[1] > 0 ? std::sqrt(pair[0] / pair[1]) : 0.0;
     return MASCOT_OK;

@@ -32,3 +32,9 @@ def test_sums_of_an_abandoned_evaluation_go_to_nobody_else(shard_timeout_check, 
     assert lines[1] == "hung rc -6"
     assert lines[2] == "given away 0 alive 1" and lines[3] == "kept by a release 1"
     assert lines[4] == "left pinned 0" and lines[5] == "left device 0"
+
+
+def test_sharded_evaluation_reads_its_result_after_the_bounded_wait(shard_timeout_check):
+    """The sum over the ranks never ends: a copy into pageable memory queued behind it would wait for good."""
+    out = subprocess.run([shard_timeout_check, "reduce", "5000", "2"], capture_output=True, text=True, timeout=60)
+    assert out.returncode == 0 and out.stdout.splitlines()[1] == "hung rc -6", out.stdout
