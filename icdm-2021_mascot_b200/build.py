@@ -40,7 +40,7 @@ def build_library(force=False, verbose=True, ptxas_verbose=False):
     srcs = [os.path.join(CSRC, s) for s in LIB_SOURCES]
     deps = srcs + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     deps.append(os.path.join(ROOT, "include", "mascot.h"))
-    if not force and not _newer(LIB, deps):
+    if not force and not _newer(LIB, deps + [os.path.abspath(__file__)]):
         return LIB
     objs = []
     for s in srcs:
@@ -49,7 +49,10 @@ def build_library(force=False, verbose=True, ptxas_verbose=False):
             cmd = ["nvcc"] + NVCC_FLAGS + (["-Xptxas", "-v"] if ptxas_verbose else []) + ["-c", s, "-o", o]
             _run(cmd, verbose)
         objs.append(o)
-    _run(["nvcc", "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB] + objs + ["-lcudart", "-ldl", "-lpthread"], verbose)
+    # nodelete: the library has threads of its own (host_copy.cu), whose code has to stay mapped when a program that
+    # loaded it with dlopen closes it again
+    _run(["nvcc", "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-Xlinker", "-z", "-Xlinker", "nodelete", "-o", LIB] + objs
+         + ["-lcudart", "-ldl", "-lpthread"], verbose)
     return LIB
 
 

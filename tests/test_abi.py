@@ -3,6 +3,8 @@ include/mascot.h declares, and fails loudly (no CPU fallback) when no GPU is usa
 import ctypes as C
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -69,3 +71,11 @@ def test_no_cpu_fallback(mascot):
         mascot.rmse_host(np.zeros((4, 64), np.float32), np.zeros((4, 64), np.float32),
                          np.zeros(3, mascot.RATING), 64)
     assert e.value.status == mascot.ERR_NO_DEVICE
+
+
+def test_library_stays_mapped_when_it_is_closed():
+    """Its helper threads would otherwise wake up in code that is no longer there."""
+    path = os.path.join(ROOT, "icdm-2021_mascot_b200", "libmascot.so")
+    code = (f"import ctypes, _ctypes; L = ctypes.CDLL({path!r}); assert L.mascot_abi_info(None, None, None) == 0; _ctypes.dlclose(L._handle); "
+            "assert 'libmascot.so' in open('/proc/self/maps').read()")
+    subprocess.run([sys.executable, "-c", code], check=True)
