@@ -4,7 +4,7 @@
 // device and - on a host that others use - now and then take milliseconds: creating, filling and destroying an
 // engine for two million ratings spent 5 of its 14 ms in them.  The pool keeps up to kKeep bytes of freed memory
 // mapped for the next allocation (of this process; beyond that, memory goes back to the system as soon as it is
-// free); mascot_release_scratch returns the rest.  The driver serialises pools internally, so engines on several
+// free); mascot_release_scratch and mascot_release_cached return the rest.  The driver serialises pools internally, so engines on several
 // threads and streams can share one; memory freed on one stream reaches another only after the work that used it.
 //
 // Buffers above kLarge still come from cudaMalloc: they live as long as an engine, would fill the pool's bound at once,
@@ -160,6 +160,23 @@ void pool_free(void* p, cudaStream_t st) {
 void pool_trim() {
     cudaMemPool_t pool = nullptr;
     if (current_pool(&pool) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+}
+
+cudaError_t pool_trim_all() {
+    int before = 0;
+    cudaError_t e = cudaSuccess;
+    bool moved = false;
+    for (int dev = 0; dev < kDevices; dev++) {
+        cudaMemPool_t pool;
+        { std::lock_guard<std::mutex> lock(g_mutex); pool = g_pools[dev]; }
+        if (!pool) continue;
+        if (!moved) { e = cudaGetDevice(&before); moved = true; }
+        if (e == cudaSuccess) e = cudaSetDevice(dev);
+        if (e == cudaSuccess) e = cudaDeviceSynchronize();      // what was freed behind queued work is idle after it
+        if (e == cudaSuccess) e = cudaMemPoolTrimTo(pool, 0);
+    }
+    if (moved) { const cudaError_t back = cudaSetDevice(before); if (e == cudaSuccess) e = back; }
+    return e;
 }
 
 }  // namespace mascot

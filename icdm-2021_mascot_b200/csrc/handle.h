@@ -108,6 +108,7 @@ double now_us();
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);    // from the current device's pool
 void pool_free(void* p, cudaStream_t st);
 void pool_trim();                                                  // gives the current device's idle pool memory back
+cudaError_t pool_trim_all();                                       // ... every device's, after all work queued there
 
 // Words that a kernel writes and the host reads right after it: pinned host memory that the GPU writes straight into
 // (a copy of some kilobytes costs ten microseconds of its own), or device memory and a copy where the result is

@@ -1020,6 +1020,13 @@ int mascot_release_scratch(mascot_handle* h) {
     return MASCOT_OK;
 }
 
+int mascot_release_cached(void) {
+    release_copy_rings();
+    release_results();
+    CU(nullptr, pool_trim_all());
+    return MASCOT_OK;
+}
+
 int mascot_sync(mascot_handle* h) {
     if (!h) return MASCOT_ERR_BAD_ARG;
     CU(h, cudaSetDevice(h->cfg.device));

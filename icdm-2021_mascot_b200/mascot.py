@@ -26,7 +26,7 @@ EXPORTS = [
     "mascot_get_test_ratings", "mascot_promote_group", "mascot_reload_train", "mascot_stream_source_index", "mascot_get_stream_order", "mascot_rmse_host", "mascot_rmse_device", "mascot_rmse_device_noalloc",
     "mascot_set_ratings_sharded", "mascot_is_check_epoch", "mascot_stats_begin", "mascot_train_segment", "mascot_stats_fetch",
     "mascot_stats_apply", "mascot_item_rows", "mascot_sync", "mascot_get_stream", "mascot_eval_sq_error", "mascot_train_epoch_streamed",
-    "mascot_release_scratch", "mascot_comm_unique_id", "mascot_shard_init", "mascot_shard_set_ratings", "mascot_shard_train_epoch",
+    "mascot_release_scratch", "mascot_release_cached", "mascot_comm_unique_id", "mascot_shard_init", "mascot_shard_set_ratings", "mascot_shard_train_epoch",
     "mascot_shard_eval_rmse", "mascot_shard_gather_factors", "mascot_shard_info", "mascot_shard_schedule", "mascot_probe_read_bandwidth", "mascot_get_timings", "mascot_get_worker_count",
 ]
 
@@ -374,6 +374,13 @@ def probe_read_bandwidth(nbytes, passes=20, device=0):
     if rc != OK:
         raise MascotError(rc, load().mascot_last_error(None).decode())
     return v.value
+
+
+def release_cached():
+    """Gives back the device memory, pinned memory and threads that the library keeps between calls."""
+    rc = load().mascot_release_cached()
+    if rc != OK:
+        raise MascotError(rc, load().mascot_last_error(None).decode())
 
 
 def rmse_host(P, Q, test, k, device=0):

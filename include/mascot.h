@@ -326,6 +326,11 @@ MASCOT_API int mascot_get_worker_count(mascot_handle* h, uint32_t* workers);
  * 8 x 64 KiB into which evaluations write, as far as no call is using them.
  * All are allocated again when next needed. */
 MASCOT_API int mascot_release_scratch(mascot_handle* h);
+/* The same for what belongs to no engine, without one: the freed device memory kept on every GPU that this process has
+ * used, the pinned rings with their helper threads (22 at most) and the pinned blocks, as far as no call is using them.  For a
+ * program that has destroyed its engines, or that only calls mascot_rmse_host or mascot_rmse_device.  Waits for the work
+ * queued on those GPUs. */
+MASCOT_API int mascot_release_cached(void);
 
 /* ---- sharded training inside the library: one engine per GPU, one host thread or process per engine,
  * NCCL between them.  No counterpart in the reference (single-GPU).  Users are pinned to a GPU with their

@@ -73,6 +73,10 @@ def test_no_cpu_fallback(mascot):
     assert e.value.status == mascot.ERR_NO_DEVICE
 
 
+def test_release_without_an_engine_needs_no_gpu(mascot):
+    mascot.release_cached()               # nothing has been kept: no GPU is touched
+
+
 def test_library_stays_mapped_when_it_is_closed():
     """Its helper threads would otherwise wake up in code that is no longer there."""
     path = os.path.join(ROOT, "icdm-2021_mascot_b200", "libmascot.so")

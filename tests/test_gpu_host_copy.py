@@ -1,6 +1,9 @@
 """Factor matrices of every size class of the staged host copies: below the direct limit, pieces of one thread, ragged
 last pieces, several blocks of whole slots, host addresses off every boundary; and buffers kept from one set of
 ratings for the next, larger or smaller."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -45,3 +48,36 @@ def test_an_engine_takes_larger_and_smaller_ratings(mascot, oracle):
         assert_bit_equal(Pg, P, "P")
         assert_bit_equal(Qg, Q, "Q")
     eng.close()
+
+
+def test_what_is_kept_between_calls_can_be_given_back_without_an_engine(mascot):
+    """A program that only evaluates, and one whose engines are gone: device memory and helper threads come back."""
+    code = """
+import importlib.util, os, sys
+import numpy as np, torch
+spec = importlib.util.spec_from_file_location("mascot_binding", sys.argv[1]); M = importlib.util.module_from_spec(spec); spec.loader.exec_module(M)
+k, n_users, n_items, n = 64, 200_000, 50_000, 100_000
+rng = np.random.default_rng(0)
+P, Q = rng.random((n_users, k), np.float32), rng.random((n_items, k), np.float32)
+R = np.empty(n, M.RATING)
+R["r"], R["u"], R["i"] = 3, rng.integers(0, n_users, n), rng.integers(0, n_items, n)
+free = lambda: torch.cuda.mem_get_info()[0]
+threads = lambda: len(os.listdir("/proc/self/task"))
+want = M.rmse_host(P, Q, R, k)
+M.release_cached()
+idle, alone = free(), threads()
+for _ in range(2):
+    assert M.rmse_host(P, Q, R, k) == want
+    kept, helped = idle - free(), threads() - alone
+    M.release_cached()
+    assert kept > 48 << 20 and idle - free() < 4 << 20, (kept, idle - free())
+    assert helped > 0 and threads() == alone, (helped, threads() - alone)
+with M.Engine(M.default_config(version=M.V_SGD, k=k)) as eng:
+    eng.set_ratings(R, R, n_users, n_items)
+    eng.set_factors(P, Q)
+    M.release_cached()                                 # under a living engine: nothing that it uses
+    assert abs(eng.eval_rmse() - want) < 1e-5 * want
+M.release_cached()
+assert idle - free() < 32 << 20 and threads() == alone      # (less the code of the update kernel)
+"""
+    subprocess.run([sys.executable, "-c", code, mascot.__file__], check=True, timeout=300)
