@@ -24,7 +24,7 @@ inline int g_gpus = 1;
 inline void fake_wait(const FakeStream* s, const char* who) {
     if (s && s->stuck) { std::printf("%s would wait for a stream that makes no progress\n", who); std::fflush(stdout); std::_Exit(3); }
 }
-inline bool any_stuck() { for (FakeStream* s : g_streams) if (s->stuck) return true; return false; }
+inline void fake_wait_all(const char* who) { for (FakeStream* s : g_streams) fake_wait(s, who); }
 
 extern "C" {
 inline cudaError_t fake_alloc(void** p, size_t n) { std::lock_guard<std::mutex> l(g_fake_mutex); *p = std::malloc(n ? n : 1); g_device.insert(*p); return cudaSuccess; }
@@ -36,7 +36,7 @@ cudaError_t cudaGetDeviceCount(int* n) { *n = g_gpus; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
 cudaError_t cudaMalloc(void** p, size_t n) { return fake_alloc(p, n); }
-cudaError_t cudaFree(void* p) { if (any_stuck()) fake_wait(*g_streams.begin(), "cudaFree"); return fake_release(p); }
+cudaError_t cudaFree(void* p) { fake_wait_all("cudaFree"); return fake_release(p); }
 cudaError_t cudaMemPoolCreate(cudaMemPool_t* pool, const cudaMemPoolProps*) { *pool = reinterpret_cast<cudaMemPool_t>(8); return cudaSuccess; }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
@@ -52,6 +52,7 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* st, unsigned) { FakeStream* 
 cudaError_t cudaStreamDestroy(cudaStream_t st) { g_streams.erase(fake(st)); return cudaSuccess; }      // events may still look at it
 cudaError_t cudaStreamQuery(cudaStream_t st) { return fake(st)->stuck ? cudaErrorNotReady : cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t st) { fake_wait(fake(st), "cudaStreamSynchronize"); return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() { fake_wait_all("cudaDeviceSynchronize"); return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) { std::memset(p, v, n); return cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t n, cudaMemcpyKind kind, cudaStream_t st) {
