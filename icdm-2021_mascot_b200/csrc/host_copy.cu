@@ -7,7 +7,6 @@
 // 12 -> 41, 480 MB 11 -> 51; down into fresh pages 4.6 -> 38.
 #include "host_copy.h"
 
-#include <sched.h>
 #include <sys/mman.h>
 
 #include <algorithm>
@@ -21,6 +20,8 @@
 #include <mutex>
 #include <thread>
 #include <vector>
+
+#include "host_cores.h"
 
 namespace mascot {
 
@@ -148,12 +149,7 @@ void give_ring(Ring* r) {
 }
 
 int host_threads(size_t bytes, int most) {
-    static const int cores = [] {
-        cpu_set_t set;
-        CPU_ZERO(&set);
-        const int n = sched_getaffinity(0, sizeof set, &set) == 0 ? CPU_COUNT(&set) : (int)std::thread::hardware_concurrency();
-        return std::max(1, n);
-    }();
+    static const int cores = usable_cores();
     // waking a thread costs about ten microseconds: half a megabyte each at least
     return (int)std::max<size_t>(1, std::min<size_t>({(size_t)cores, (size_t)most, bytes >> 19}));
 }
