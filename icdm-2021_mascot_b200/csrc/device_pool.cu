@@ -11,7 +11,8 @@
 // and unmapping 2 GB of pool memory took 40 to 80 ms where cudaFree took 6.
 //
 // Where the process sees more than one GPU, memory comes from cudaMalloc instead: programs copy item rows between
-// GPUs (mascot_item_rows), and a pool's memory is not mapped on peers.
+// GPUs (mascot_item_rows), and a pool's memory is not mapped on peers.  Where it sees one of several, another process may ask
+// for the rows, and cudaIpcGetMemHandle refuses pool memory: rows whose address a caller asks for move to cudaMalloc's.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -155,6 +156,21 @@ void pool_free(void* p, cudaStream_t st) {
     { std::lock_guard<std::mutex> lock(g_mutex); plain = g_plain.erase(p) > 0; }
     if (plain) cudaFree(p);
     else cudaFreeAsync(p, st);
+}
+
+cudaError_t pool_make_plain(void** p, size_t bytes, cudaStream_t st) {
+    { std::lock_guard<std::mutex> lock(g_mutex); if (!*p || g_plain.count(*p)) return cudaSuccess; }
+    void* own = nullptr;
+    cudaError_t e = cudaMalloc(&own, bytes);
+    if (e != cudaSuccess) return e;
+    e = cudaMemcpyAsync(own, *p, bytes, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) { cudaFree(own); return e; }
+    cudaFreeAsync(*p, st);
+    *p = own;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    g_plain.insert(own);
+    return cudaSuccess;
 }
 
 void pool_trim() {

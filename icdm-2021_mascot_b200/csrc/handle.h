@@ -107,6 +107,7 @@ double now_us();
 // ---- device_pool.cu: device memory of engines and of handle-free calls, in the order of a stream ----
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);    // from the current device's pool
 void pool_free(void* p, cudaStream_t st);
+cudaError_t pool_make_plain(void** p, size_t bytes, cudaStream_t st);   // moves a buffer out of the pool (other processes may open it then)
 void pool_trim();                                                  // gives the current device's idle pool memory back
 cudaError_t pool_trim_all();                                       // ... every device's, after all work queued there
 

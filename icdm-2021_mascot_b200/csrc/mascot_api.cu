@@ -987,6 +987,15 @@ int mascot_item_rows(mascot_handle* h, uint32_t row_begin, uint32_t row_end, voi
     if (!h->have_ratings) return fail(h, MASCOT_ERR_STATE, "mascot_set_ratings must come first");
     if (row_end > h->n_items) return fail(h, MASCOT_ERR_BAD_ARG, "item row range out of bounds");
     if (h->ilay.parts > 1) return fail(h, MASCOT_ERR_UNSUPPORTED, "the items of a sharded engine are laid out block by block, not by sorted index");
+    CU(h, cudaSetDevice(h->cfg.device));
+    const void* const before[2] = {h->Q.f16, h->Q.f32};
+    CU(h, pool_make_plain(reinterpret_cast<void**>(&h->Q.f16), h->reserved[&h->Q.f16], h->stream));
+    CU(h, pool_make_plain(reinterpret_cast<void**>(&h->Q.f32), h->reserved[&h->Q.f32], h->stream));
+    if (h->l2_window_set && (h->Q.f16 != before[0] || h->Q.f32 != before[1])) {
+        l2_window_remove(h);
+        const int rc = l2_window_install(h);
+        if (rc != MASCOT_OK) return rc;
+    }
     const size_t b = (size_t)row_begin * h->K, n = (size_t)(row_end - row_begin) * h->K;
     if (f16_ptr) *f16_ptr = h->Q.f16 ? (void*)(h->Q.f16 + b) : nullptr;
     if (f16_bytes) *f16_bytes = h->Q.f16 ? n * sizeof(__half) : 0;

@@ -301,7 +301,8 @@ MASCOT_API int mascot_stats_apply(mascot_handle* h, uint32_t epoch, const float*
                        const float* norm_sum_p, const float* norm_sum_q,
                        uint32_t* promoted_user_groups, uint32_t* promoted_item_groups);
 /* Device addresses and byte sizes of the item rows [row_begin, row_end) (sorted-index space) in the
- * binary16 and the fp32 arena (NULL / 0 for an arena the variant does not keep). */
+ * binary16 and the fp32 arena (NULL / 0 for an arena the variant does not keep).  They stay the same until the next
+ * mascot_set_ratings*, and other processes may open them (cudaIpcGetMemHandle). */
 MASCOT_API int mascot_item_rows(mascot_handle* h, uint32_t row_begin, uint32_t row_end, void** f16_ptr, uint64_t* f16_bytes,
                      void** f32_ptr, uint64_t* f32_bytes);
 /* Wait for everything queued on the engine's stream. */

@@ -1,6 +1,7 @@
 """Factor matrices of every size class of the staged host copies: below the direct limit, pieces of one thread, ragged
 last pieces, several blocks of whole slots, host addresses off every boundary; and buffers kept from one set of
 ratings for the next, larger or smaller."""
+import ctypes
 import subprocess
 import sys
 
@@ -81,3 +82,29 @@ M.release_cached()
 assert idle - free() < 32 << 20 and threads() == alone      # (less the code of the update kernel)
 """
     subprocess.run([sys.executable, "-c", code, mascot.__file__], check=True, timeout=300)
+
+
+@pytest.mark.parametrize("version", ("sgd", "mascot"))
+@pytest.mark.parametrize("window", (0, 1))
+def test_item_rows_can_be_opened_by_another_process(mascot, version, window):
+    """The driver gives out a handle for their addresses, which stay the same; the rows are the ones the engine goes on with."""
+    k, n_users, n_items, n = 64, 300, 200, 5000
+    R, P, Q = random_problem(np.random.default_rng(5), n_users, n_items, n, k)
+    cuda, got = ctypes.CDLL("libcuda.so.1"), []
+    for asked in (False, True):
+        cfg = mascot.default_config(version=mascot.V_SGD if version == "sgd" else mascot.V_MASCOT, k=k, deterministic=1, shuffle=0, l2_item_window=window)
+        with mascot.Engine(cfg) as eng:
+            eng.set_ratings(R, R[:10], n_users, n_items)
+            eng.set_factors(P, Q)
+            eng.train_epoch(0)
+            if asked:
+                (p16, b16), (p32, b32) = eng.item_rows(0, n_items)
+                assert (p16 != 0) == (version == "mascot") and p32 != 0 and b32 == 4 * n_items * k
+                for p in filter(None, (p16, p32)):
+                    handle = ctypes.create_string_buffer(64)
+                    assert cuda.cuIpcGetMemHandle(handle, ctypes.c_uint64(p)) == 0
+                assert eng.item_rows(1, 2)[1][0] == p32 + 4 * k
+            eng.train_epoch(1)
+            got.append(eng.get_factors(0))
+    assert_bit_equal(got[0][0], got[1][0], "P")
+    assert_bit_equal(got[0][1], got[1][1], "Q")
