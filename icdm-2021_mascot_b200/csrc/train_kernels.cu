@@ -1351,9 +1351,9 @@ cudaError_t launch_ns(KernelArgs a, unsigned warps_per_sm, unsigned workers, cud
     if (fit < 1) return cudaErrorLaunchOutOfResources;
     size_t smem_used = smem;
     if (warps > 8 && blocks_per_sm > (unsigned)fit && warps_per_block < 8) {
-        // The SM cannot hold as many blocks as the even split asked for: blocks of the full eight warps then put
-        // more warps on it (42 warps wanted: six blocks of seven, of which four fit = 28 warps; four blocks of
-        // eight = 32).
+        // The SM cannot hold as many blocks as the even split asked for: blocks of the full eight warps may then put
+        // more warps on it (27 warps wanted, fp32 rows on both sides: four blocks of seven, of which three fit = 21
+        // warps; three blocks of eight = 24).
         int fit8 = 0;
         const size_t smem8 = (size_t)8 * kPerWarp * SM::kBytes;
         const int rc8 = cache.lookup(
@@ -1398,6 +1398,23 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
     // are three to four times as long, and for them three and two are enough.
     constexpr bool kFixedPoint = KIND == KIND_AFP || KIND == KIND_MUPPET;
     constexpr int NS = kFixedPoint ? 4 : 8, D = kFixedPoint ? 3 : 5, DI = kFixedPoint ? 2 : 3;
+    // With fp32 rows the deep rings leave room for fewer warps than the registers do (k=128, both sides fp32: 16 per SM
+    // against 24).  The mixed-precision classes with an fp32 side want those warps: where a launch asks for more workers
+    // than the deep rings hold and rings of 4 + 2 slots hold more, it takes these, three ratings and one ahead.  Per epoch,
+    // deep rings for all classes and this rule: 40 % of the groups promoted, 40M ratings 7.17 and 6.99 ms, 63M 9.64 and 9.42,
+    // 100M (a fifth) 10.35 and 9.95; all promoted, 63M 11.25 and 10.95, k=64 at 100M 22.1 and 20.2.
+    // Where the deep rings hold the request they are faster: 20M, all promoted, 5.00 and 5.28 (k=64, 75M: 8.45 and 8.61).
+    // The other trainers gain nothing from more warps: SGD 7.73 and 7.74 ms at 63M ratings, 10.53 and 10.58 at 100M, 32.6
+    // and 34.9 at 252M (binary16 rows: 16.6 and 17.2), the same times at 16 warps per SM as at 24.  There the rate of the
+    // reductions into user rows is the limit, not the waiting of few warps.
+    constexpr bool kShortRings = KIND == KIND_MIXED && !STATS && UM != ROWS_DYN && (UM == ROWS_F32 || IM == ROWS_F32);
+    if constexpr (kShortRings) {
+        LaunchShape deep, shallow;
+        cudaError_t e = launch_ns<K, KIND, UM, IM, STATS, NS, 4, D, DI>(args, per_sm, workers, st, &deep, true);
+        if (e == cudaSuccess && deep.workers < workers) e = launch_ns<K, KIND, UM, IM, STATS, 4, 2, 3, 1>(args, per_sm, workers, st, &shallow, true);
+        if (e != cudaSuccess) return e;
+        if (shallow.workers > deep.workers) return launch_ns<K, KIND, UM, IM, STATS, 4, 2, 3, 1>(args, per_sm, workers, st, shape, dry);
+    }
     return launch_ns<K, KIND, UM, IM, STATS, NS, 4, D, DI>(args, per_sm, workers, st, shape, dry);
 }
 

@@ -65,3 +65,53 @@ def test_every_rating_once_at_any_length_and_worker_count(mascot, oracle, versio
         Po, Qo = oracle_epoch(oracle, version, k, R, P.copy(), Q.copy(), 0.01, 0.05)
         assert_bit_equal(Pg, Po, f"n {n} P")
         assert_bit_equal(Qg, Qo, f"n {n} Q")
+
+
+def promoted_model(oracle, mascot, eng, k, P, Q, users, items):
+    """Engine and oracle with every group of the given sides in fp32, and the maps from ids to sorted indices."""
+    u2s, i2s = eng.index_maps()
+    Ps, Qs = np.empty_like(P), np.empty_like(Q)
+    Ps[u2s], Qs[i2s] = P, Q
+    prec, groups = [], []
+    for side, (n, on) in enumerate(((len(P), users), (len(Q), items))):
+        end, p, _ = eng.group_info(side)
+        groups.append(np.searchsorted(end, np.arange(n), side="left").astype(np.uint32))
+        prec.append(np.zeros_like(p))
+        for g in range(len(end) if on else 0):
+            eng.promote_group(side, g)
+    model = oracle.MascotModel(k, Ps, Qs, groups[0], groups[1], *prec)
+    for name, on, p in (("u", users, prec[0]), ("i", items, prec[1])):
+        for g in range(len(p) if on else 0):
+            model.promote(name, g)
+    return model, u2s, i2s
+
+
+@pytest.mark.parametrize("k", (128, 64))
+@pytest.mark.parametrize("users,items", [(True, True), (True, False), (False, True)])
+def test_classes_with_fp32_rows_asked_for_more_workers_than_fit(mascot, oracle, k, users, items):
+    """The launch that takes short rings: rows that come back at once in the hands of the one worker that the first eight chunks
+    make, and ratings that share no row over many workers.  Plain stores, bit for bit."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for n_users, n_items, n in ((1, 1, 9), (2, 1, 33), (1, 5, 64), (3, 2, 63), (7, 7, 64), (7, 7, k), (1, 1, 1), (4097, 4097, 4097), (8191, 8191, 8191)):
+        R, P, Q = random_problem(np.random.default_rng(n + n_users), n_users, n_items, n, k)
+        if n == n_users:
+            rng = np.random.default_rng(n)
+            R["u"], R["i"] = rng.permutation(n), rng.permutation(n)
+        cfg = mascot.default_config(version=mascot.V_MASCOT, k=k, num_workers=60000, plain_user_stores=1, seed=n, epoch=50, learning_rate=0.01, decay=0.1,
+                                    lam=0.05, user_group_num=1, item_group_num=1)
+        with mascot.Engine(cfg) as eng:
+            eng.set_ratings(R, R[:1], n_users, n_items)
+            eng.set_factors(P, Q)
+            model, u2s, i2s = promoted_model(oracle, mascot, eng, k, P, Q, users, items)
+            order = eng.stream_order()
+            workers = eng.train_epoch(0).workers
+            Pg, Qg = eng.get_factors(1)
+        # deep rings: 16 warps per SM, short ones: 24, of two workers each (k=64: four)
+        assert workers > 20 * 2 * (128 // k) * sms
+        Rs = R[order].copy()
+        Rs["u"], Rs["i"] = u2s[Rs["u"]], i2s[Rs["i"]]
+        model.run(Rs, None, 0.01, 0.05, oracle.rules_reference())
+        Po, Qo = model.factors()
+        assert_bit_equal(Pg, Po, f"n {n} P")
+        assert_bit_equal(Qg, Qo, f"n {n} Q")
