@@ -1405,8 +1405,7 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
     // 100M (a fifth) 10.35 and 9.95; all promoted, 63M 11.25 and 10.95, k=64 at 100M 22.1 and 20.2.
     // Where the deep rings hold the request they are faster: 20M, all promoted, 5.00 and 5.28 (k=64, 75M: 8.45 and 8.61).
     // The other trainers gain nothing from more warps: SGD 7.73 and 7.74 ms at 63M ratings, 10.53 and 10.58 at 100M, 32.6
-    // and 34.9 at 252M (binary16 rows: 16.6 and 17.2), the same times at 16 warps per SM as at 24.  There the rate of the
-    // reductions into user rows is the limit, not the waiting of few warps.
+    // and 34.9 at 252M (binary16 rows: 16.6 and 17.2): what limits those is not the waiting of few warps.
     constexpr bool kShortRings = KIND == KIND_MIXED && !STATS && UM != ROWS_DYN && (UM == ROWS_F32 || IM == ROWS_F32);
     if constexpr (kShortRings) {
         LaunchShape deep, shallow;

@@ -37,3 +37,54 @@ def test_run_windows_sort_the_encoded_order(mascot, n, version):
             part = want[b:b + w]
             want[b:b + w] = part[np.argsort(item[part], kind="stable")]
     assert (orders[1] == want).all()
+
+
+def in_windows(order, item, seg, window):
+    """`order`, stably sorted by item inside every piece that segments and multiples of `window` cut it into."""
+    want = order.copy()
+    cuts = sorted(set(seg) | set(range(0, seg[-1], window)))
+    for b, e in zip(cuts, cuts[1:]):
+        want[b:e] = want[b:e][np.argsort(item[want[b:e]], kind="stable")]
+    return want
+
+
+@pytest.mark.parametrize("version,seg", [("sgd", [0, 8192, 40960, 100003]), ("sgd", [0, 16384, 16384, 36864]), ("sgd", [0, 4096, 4097]),
+                                         ("mascot", [0, 65536, 135168, 200704, 270001]), ("sgd", [0, 5000, 100003])])
+def test_run_windows_of_several_segments(mascot, version, seg):
+    """At the set-up and after a reload; segments that begin off the encoding step's windows take the sort of the coded stream."""
+    n_users, n_items, n, window = 700, 301, seg[-1], 1 << 14
+    R, _, _ = random_problem(np.random.default_rng(n), n_users, n_items, n, 64)
+    orders = []
+    for log2 in (12, 14):
+        cfg = mascot.default_config(version=mascot.V_SGD if version == "sgd" else mascot.V_MASCOT, k=64, num_workers=4096, seed=n, run_window_log2=log2,
+                                    sample_ratio=1.0, user_group_num=5, item_group_num=4)
+        with mascot.Engine(cfg) as eng:
+            eng.set_ratings_sharded(R, seg, R[:50], n_users, n_items)
+            item = eng.index_maps()[1][R["i"]].astype(np.int64)
+            orders.append(eng.stream_order())
+            eng.reload_train(R)
+            assert (eng.stream_order() == orders[-1]).all()
+    for b, e in zip(seg, seg[1:]):
+        assert sorted(orders[0][b:e].tolist()) == list(range(b, e))
+    assert (orders[1] == in_windows(orders[0], item, seg, window)).all()
+
+
+def test_reload_after_a_streamed_epoch_keeps_its_pieces(mascot):
+    """The pieces of a streamed epoch become the segments of the resident stream; a reload sorts each of them in run windows."""
+    n_users, n_items, piece, window = 7001, 301, 8 << 20, 1 << 14
+    n = piece + 12345
+    R, P, Q = random_problem(np.random.default_rng(3), n_users, n_items, n, 64)
+    orders = []
+    for log2 in (12, 14):
+        with mascot.Engine(mascot.default_config(version=mascot.V_SGD, k=64, num_workers=4096, run_window_log2=log2)) as eng:
+            eng.set_ratings(R, R[:50], n_users, n_items)
+            eng.set_factors(P, Q)
+            item = eng.index_maps()[1][R["i"]].astype(np.int64)
+            eng.train_epoch_streamed(0, R)
+            streamed = eng.stream_order()
+            eng.reload_train(R)
+            orders.append(eng.stream_order())
+            assert eng.train_epoch(1).updates == n
+            assert eng.train_segment(2, 1).updates == n - piece
+    assert (orders[0] == streamed).all()
+    assert (orders[1] == in_windows(streamed, item, [0, piece, n], window)).all()
