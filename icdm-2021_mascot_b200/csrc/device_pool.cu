@@ -2,13 +2,16 @@
 //
 // An engine makes about thirty allocations, and cudaMalloc and cudaFree map and unmap pages, wait for the whole
 // device and - on a host that others use - now and then take milliseconds: creating, filling and destroying an
-// engine for two million ratings spent 5 of its 14 ms in them.  The pool keeps up to kKeep bytes of freed memory
+// engine for two million ratings spent 5 of its 14 ms in them.  (A process pays once for its first pool: 7 to 10 ms.)  The pool keeps up to kKeep bytes of freed memory
 // mapped for the next allocation (of this process; beyond that, memory goes back to the system as soon as it is
 // free); mascot_release_scratch and mascot_release_cached return the rest.  The driver serialises pools internally, so engines on several
 // threads and streams can share one; memory freed on one stream reaches another only after the work that used it.
 //
-// Buffers above kLarge still come from cudaMalloc: they live as long as an engine, would fill the pool's bound at once,
-// and unmapping 2 GB of pool memory took 40 to 80 ms where cudaFree took 6.
+// Buffers above kLarge still come from cudaMalloc.  What an engine frees beyond kKeep is unmapped, and pool memory is slow
+// there: 6 ms for 1 GiB (36 on a busy host) where cudaMalloc and cudaFree together take 1.6 (3.6).  Up to kLarge the
+// buffers of one engine fit kKeep together: at 9M ratings the set-up's scratch is 256 MiB and the rest as much again.
+// One buffer beyond the line costs a job 1.0 to 1.6 ms: 4 epochs of 9M, 11M and 16M ratings from creation to factors take
+// 15.3, 16.1 and 18.4 ms, with a line of 1 GiB 14.2, 15.1 and 16.9.
 //
 // Where the process sees more than one GPU, memory comes from cudaMalloc instead: programs copy item rows between
 // GPUs (mascot_item_rows), and a pool's memory is not mapped on peers.  Where it sees one of several, another process may ask

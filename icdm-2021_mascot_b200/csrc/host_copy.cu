@@ -2,9 +2,11 @@
 // caller, and cudaMemcpy moves such buffers with one host thread through the driver's own staging: measured on a
 // 16-core B200 host 11 GB/s up, 15 GB/s down into memory that has been touched and 4.6 GB/s into fresh pages, where
 // that thread also takes the page faults - against 55 GB/s of the link from pinned memory.  Here up to eight threads
-// move the data between the caller's memory and a pinned ring while the copy engine works on other parts of the ring, so
-// the host side runs at several cores' bandwidth and the faults are taken in parallel.  Up: 4 MB 15 -> 22 GB/s, 36 MB
-// 12 -> 41, 480 MB 11 -> 51; down into fresh pages 4.6 -> 38.
+// (down, above 64 MB, twelve) move the data between the caller's memory and a pinned ring while the copy engine works on
+// other parts of the ring, so the host side runs at several cores' bandwidth and the faults are taken in parallel.  Up:
+// 4 MB 15 -> 22 GB/s, 36 MB 12 -> 41, 480 MB 11 -> 51; down into fresh pages 4.6 -> 38.
+//
+// The first large copy of a process makes the ring: 24 MiB touched in 4 to 5 ms, registered in 1 to 10.
 #include "host_copy.h"
 
 #include <sys/mman.h>
@@ -37,7 +39,7 @@ constexpr size_t kDirect = 192u << 10;            // below this the driver's cop
 // The helper threads of a ring.  Starting eight threads costs more than copying 4 MB, and waking parked ones takes most
 // of a millisecond on a virtual machine (16 MB up: 1.3 ms after parked threads, 0.45 after awake ones).  Copies come in
 // groups - both factor matrices, then the test set - so a helper stays awake for kAwake after its last work, giving its
-// core to whoever asks for it, and parks then.
+// core to whoever asks for it, and parks then.  (Under a CPU quota there are no more helpers than it pays for.)
 class Team {
 public:
     ~Team() {

@@ -2,8 +2,8 @@
 //
 // One handle = one GPU, one stream, one host control thread (like the reference: a single thread
 // driving the default stream with a synchronisation after each epoch, mf_methods.cu:239).  The
-// m-quantization set-up (degree sort, grouping, id maps) runs once on the host; everything per
-// epoch runs on the device and only the small group statistics travel back on check epochs.
+// m-quantization set-up (degree sort, maps, coded stream: setup.cu) and everything per epoch run on the device; the host
+// cuts the groups from the sorted degrees, and the small group statistics travel back on check epochs.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -278,10 +278,10 @@ int reorder_segments(mascot_handle* h, size_t seg_first, size_t seg_count, bool 
 // one promoted group, and sizes the sort key and the 32-bit permutation can express.
 bool wants_partition(const mascot_handle* h) {
     if (!(h->grouped && !h->cfg.deterministic && any_fp32_group(h) && h->n_train < (1ull << 32) && (h->seg_off.size() - 1) * 4 <= 65536)) return false;
-    // Measured on one B200 with promoted groups: 100M-rating set 7.6 ms per epoch with one launch per class (14.0 ms
-    // before the run windows) against 15.2 ms for one launch that reads each id's precision bit; 252M-rating set,
-    // 40 epochs: 1,126 ms against 1,365 ms (the launch of the all-binary16 class keeps its 32 warps per SM, the
-    // per-rating instantiation runs 16).
+    // Measured on one B200, ms per epoch with one launch per class and with one that reads each id's precision bit: 100M
+    // ratings, a fifth of the groups promoted 9.9 and 13.6 to 14.2; 252M, 40 % of them 34.0 and 36 to 40.  In between the one
+    // launch is faster - 63M, 40 % promoted 9.8 and 9.0; 40M 6.9 and 5.5; k=64, 100M 12.7 and 7.2 - but leaves a test RMSE
+    // that is 0.1 % higher after four epochs (0.57343 against 0.57262 at 40M).
     return h->cfg.no_class_partition != 1;
 }
 

@@ -4,15 +4,17 @@
 // The reference does this part with a device histogram and a thrust sort, then host loops over the
 // entities (user_item_rating_histogram, split_group_based_equal_size_not_strict_ret_end_idx,
 // matrix_reconstruction; preprocess_utils.h:54-255), after a host std::map pass over every rating
-// (io_utils.h:30-240).  Here one host->device copy of the rating array is followed by kernels only; the
-// host touches per-ENTITY tables (degrees, groups, maps: a few MB), never the ratings:
-//   1. ids checked against n_users / n_items and degree histogram (atomics)            check_hist_kernel
+// (io_utils.h:30-240).  Here the rating array is copied to the device once, and everything is kernels; the host
+// only walks the sorted degrees (a few MB) to cut the groups, and never sees the ratings:
+//   1. ids checked against n_users / n_items and degree histogram (atomics), piece by piece under the copy of the
+//      next piece                                                                        check_hist_kernel
 //   2. entities sorted by (degree, id): stable radix sort of the degrees, ids as values  cub::DeviceRadixSort
 //   3. grouping walk over the sorted degrees on the host (O(entities))                   make_groups
 //   4. id -> arena row maps, per-row group / precision tables                            side_kernel
 //   5. sharded engines: ratings of this rank's users selected and ordered by the step of the block
 //      schedule at which their item block is here - a stable radix sort of a small key   select_key_kernel
-//   6. seeded permutation, item-sorted windows, id remap, precision tags                 launch_encode_stream
+//   6. the coded stream: seeded permutation, item-sorted run windows, id remap and precision tags in one sort
+//      (launch_source_sort); where that does not apply, launch_encode_stream and launch_stream_sort after it
 //   7. test set: same check, (sharded: this rank's users), sorted by (user, item) like test_set_preprocess
 //      (preprocess_utils.h:38-52) with a stable 64-bit radix sort, then coded without shuffling.
 #include <algorithm>

@@ -13,7 +13,7 @@
 //     predicated, chunks are fetched and tickets drawn without branches, and a worker that has run out of ratings goes
 //     on with empty records.  Per-worker branches cost a warp barrier in front of every shuffle and split the update
 //     into pieces that cannot be scheduled into each other: 131 warp instructions per step of all workers of a warp
-//     before, 90 now.
+//     before, 91 now.
 //   * what the ratings to come need (records, row copies, the vote on item rows) is done between the dependent shuffles
 //     of the dot product instead of in front of it: 8M ratings 1.39 -> 1.295 ms per epoch, fp32 rows 1.70 -> 1.52;
 //   * the rating records of a chunk (one rating per lane) are loaded one chunk ahead, tagged
@@ -36,12 +36,13 @@
 // configuration either way).  With leads of three and two the 8M-rating configuration took 1.65 ms per epoch where it
 // took 1.39 with five and three, the k=64 one 1.97 against 1.65; user leads of six and seven gave nothing more.
 //
-// WHAT BOUNDS IT (one B200, k=128, binary16 rows).  Sets with few workers per SM (8M ratings: one warp per scheduler):
-// the chain of one update - dot product, four shuffle steps, update - and the 95 instructions around it, 2.42 -> 1.295
-// ms per epoch (3.9 cycles per instruction: 1.3 of them waits for results of fixed latency, 0.6 each for L2 and for shuffles).  Full SMs (100M ratings, 7.17 -> 5.50 ms): the L2 and its reductions.  18.3e9 updates/s write 4.7 TB/s of
-// reductions and read as much again; a kernel that does nothing but read random rows and reduce into them reaches
-// 17.6e9 rows/s on this GPU with evenly spread rows and 10.9e9 with Zipf ones (8.6e9 and 7.1e9 with fp32 rows, which is
-// what bounds the classes with fp32 user rows).
+// WHAT BOUNDS IT (one B200, k=128).  Sets with few workers per SM (8M ratings: one warp per scheduler): the chain of one
+// update - dot product, four shuffle steps, update - and the 91 instructions around it, 2.42 -> 1.295 ms per epoch (3.9
+// cycles per instruction: 1.3 of them waits for results of fixed latency, 0.6 each for L2 and for shuffles).  Full SMs
+// (100M ratings, 7.17 -> 5.50 ms): the traffic between SMs and L2.  The launches that fill the GPU all move 9.9 to 10.1
+// TB/s of row reads, stores and reductions (reads alone: 16 to 17.7), whatever else they do: 100M and 126M ratings with
+// binary16 rows (541 and 621 bytes an update), 63M with fp32 rows on both sides (SGD, 1,230 bytes; the fp32 class of a
+// promoted set), with 71 down to 35 % of the issue slots busy and 16 to 28 warps per SM.
 //
 // ELEMENT ORDER.  layout.cuh stores rows permuted so that lane m of a worker holds the elements of
 // reference lanes m and m+16 (k=128) or m, m+16, m+8, m+24 (k=64).  With pair products
