@@ -3,17 +3,17 @@
 // WORKERS.  The reference runs `-wg` warps, each applying one rating at a time; the number of such
 // sequential workers decides how many updates of a popular row are lost to races, i.e. how fast the
 // model converges per epoch.  This engine keeps that meaning of `-wg` - a worker is a group of
-// K/8 lanes (16 for k=128, 8 for k=64; two or four workers per warp) that applies its ratings
-// strictly one after the other - and gets its speed from making each worker fast instead of adding
-// workers:
+// K/8 lanes (16 for k=128, 8 for k=64; two or four workers per warp), or of K/4 lanes where there are few of them
+// (launch_one), that applies its ratings strictly one after the other - and gets its speed from making each worker fast
+// instead of adding workers:
 //   * every lane holds eight consecutive physical elements of a row (one 128-bit access for
-//     binary16 storage, two for fp32);
+//     binary16 storage, two for fp32), or four of them (one access);
 //   * the workers of a warp go through their ratings in step, with whole-warp shuffles, and the loop has no branch
 //     that they could take differently: what only some of them do (a new item row, a dropped write-back) is
 //     predicated, chunks are fetched and tickets drawn without branches, and a worker that has run out of ratings goes
 //     on with empty records.  Per-worker branches cost a warp barrier in front of every shuffle and split the update
 //     into pieces that cannot be scheduled into each other: 131 warp instructions per step of all workers of a warp
-//     before, 91 now.
+//     before, 91 now (K/8 lanes a worker, binary16 rows).
 //   * what the ratings to come need (records, row copies, the vote on item rows) is done between the dependent shuffles
 //     of the dot product instead of in front of it: 8M ratings 1.39 -> 1.295 ms per epoch, fp32 rows 1.70 -> 1.52;
 //   * the rating records of a chunk (one rating per lane) are loaded one chunk ahead, tagged
@@ -38,11 +38,14 @@
 //
 // WHAT BOUNDS IT (one B200, k=128).  Sets with few workers per SM (8M ratings: one warp per scheduler): the chain of one
 // update - dot product, four shuffle steps, update - and the 91 instructions around it, 2.42 -> 1.295 ms per epoch (3.9
-// cycles per instruction: 1.3 of them waits for results of fixed latency, 0.6 each for L2 and for shuffles).  Full SMs
+// cycles per instruction: 1.3 of them waits for results of fixed latency, 0.6 each for L2 and for shuffles); with fp32
+// rows or arithmetic half of a row per lane shortens that (1.52 -> 1.31 ms; 4M ratings of AFP 5.69 -> 4.43).  Full SMs
 // (100M ratings, 7.17 -> 5.50 ms): the traffic between SMs and L2.  The launches that fill the GPU all move 9.9 to 10.1
 // TB/s of row reads, stores and reductions (reads alone: 16 to 17.7), whatever else they do: 100M and 126M ratings with
 // binary16 rows (541 and 621 bytes an update), 63M with fp32 rows on both sides (SGD, 1,230 bytes; the fp32 class of a
-// promoted set), with 71 down to 35 % of the issue slots busy and 16 to 28 warps per SM.
+// promoted set), with 71 down to 35 % of the issue slots busy and 16 to 28 warps per SM.  Nothing but random rows read with
+// cp.async and reduced runs at 17.4e9 binary16 or 9.0e9 fp32 rows/s (20 MB of rows; 16.8 and 8.4 with 127 MB), a reduction
+// alone at 24.5e9 and 12.0e9: the 100M-rating set, 18.1e9 updates/s, is there.
 //
 // ELEMENT ORDER.  layout.cuh stores rows permuted so that lane m of a worker holds the elements of
 // reference lanes m and m+16 (k=128) or m, m+16, m+8, m+24 (k=64).  With pair products
@@ -74,19 +77,33 @@ namespace {
 
 constexpr uint32_t kNoRow = 0xffffffffu;     // never a valid stream id
 
-struct V8h { __half2 v[4]; };                // eight binary16 values, physical order
-struct V8f { float x[8]; };
+template <int N> struct Vh { __half2 v[N / 2]; };      // a lane's values, physical order
+template <int N> struct Vf { float x[N]; };
+typedef Vh<8> V8h;
+typedef Vf<8> V8f;
 
 // How the rows of one side are stored in a launch.  Known on the host, so the common cases carry no
 // per-rating precision test, no unused registers and no oversized ring slots.  The mixed-precision
 // trainer keeps its stream partitioned by (user precision, item precision), and every part runs the
 // instantiation made for it; ROWS_DYN (precision read from bit 31 of the id, per rating) remains for
 // the deterministic single-worker mode, which must follow the stream in its original order.
-enum RowMode { ROWS_HALF = 0, ROWS_F32 = 1, ROWS_DYN = 2 };
+// ROWS_HALFQ, ROWS_F32Q: a lane holds four elements of a row instead of eight, so that a worker has K/4 lanes.  Lane m and lane
+// m + K/8 of a worker share the eight elements that lane m of the wider form would hold: the first has (e0, e4, e1, e5),
+// the second (e2, e6, e3, e7) (layout.cuh).  Of an fp32 row lane l thus holds the 16 bytes at 16 l.
+enum RowMode { ROWS_HALF = 0, ROWS_F32 = 1, ROWS_DYN = 2, ROWS_HALFQ = 3, ROWS_F32Q = 4 };
+template <int MODE> constexpr int kElems = MODE == ROWS_HALFQ || MODE == ROWS_F32Q ? 4 : 8;      // per lane
+template <int MODE> constexpr bool kHalfRows = MODE == ROWS_HALF || MODE == ROWS_HALFQ;
+template <int MODE> constexpr bool kTwoParts = MODE == ROWS_F32 || MODE == ROWS_DYN;             // a second access for (some) rows
+// where a lane's part of a row begins, in bytes
+template <int K, int MODE> __device__ __forceinline__ int lane_at(int m) {
+    return MODE == ROWS_HALFQ ? 16 * (m & (K / 8 - 1)) + (m & (K / 8) ? 8 : 0) : 16 * m;
+}
 
-// A lane's slice of a row as fetched: 16 bytes for binary16 storage, 32 bytes for fp32 storage.
+// A lane's slice of a row as fetched: 16 bytes for binary16 storage, 32 bytes for fp32 storage, half of that with four elements.
 template <int MODE> struct Raw { uint4 a, b; };
 template <> struct Raw<ROWS_HALF> { uint4 a; };
+template <> struct Raw<ROWS_F32Q> { uint4 a; };
+template <> struct Raw<ROWS_HALFQ> { uint2 a; };
 
 __device__ __forceinline__ V8h v8h_of(const uint4& a) {
     V8h h;
@@ -100,38 +117,48 @@ __device__ __forceinline__ V8f v8f_of(const uint4& a, const uint4& b) {
     f.x[4] = __uint_as_float(b.x); f.x[5] = __uint_as_float(b.y); f.x[6] = __uint_as_float(b.z); f.x[7] = __uint_as_float(b.w);
     return f;
 }
-template <int MODE> __device__ __forceinline__ V8h as_v8h(const Raw<MODE>& r) { return v8h_of(r.a); }
-template <int MODE> __device__ __forceinline__ V8f as_v8f(const Raw<MODE>& r) {
-    if constexpr (MODE != ROWS_HALF) return v8f_of(r.a, r.b); else return v8f_of(r.a, r.a);   // fp32 rows never occur in ROWS_HALF
+template <int MODE> __device__ __forceinline__ Vh<kElems<MODE>> as_vh(const Raw<MODE>& r) {
+    if constexpr (kElems<MODE> == 8) return v8h_of(r.a);
+    else {                                            // binary16 rows never occur in ROWS_F32Q
+        Vh<4> h;
+        h.v[0] = *reinterpret_cast<const __half2*>(&r.a.x); h.v[1] = *reinterpret_cast<const __half2*>(&r.a.y);
+        return h;
+    }
+}
+template <int MODE> __device__ __forceinline__ Vf<kElems<MODE>> as_vf(const Raw<MODE>& r) {
+    if constexpr (MODE == ROWS_HALFQ) return Vf<4>{{0.f, 0.f, 0.f, 0.f}};      // fp32 rows never occur here
+    else if constexpr (MODE == ROWS_F32Q) return Vf<4>{{__uint_as_float(r.a.x), __uint_as_float(r.a.y), __uint_as_float(r.a.z), __uint_as_float(r.a.w)}};
+    else if constexpr (MODE != ROWS_HALF) return v8f_of(r.a, r.b);
+    else return v8f_of(r.a, r.a);                     // fp32 rows never occur in ROWS_HALF
 }
 
-template <int MODE> __device__ __forceinline__ void put(Raw<MODE>& r, const V8h& h) {
+template <int MODE> __device__ __forceinline__ void put(Raw<MODE>& r, const Vh<kElems<MODE>>& h) {
     r.a.x = *reinterpret_cast<const unsigned*>(&h.v[0]); r.a.y = *reinterpret_cast<const unsigned*>(&h.v[1]);
-    r.a.z = *reinterpret_cast<const unsigned*>(&h.v[2]); r.a.w = *reinterpret_cast<const unsigned*>(&h.v[3]);
+    if constexpr (kElems<MODE> == 8) { r.a.z = *reinterpret_cast<const unsigned*>(&h.v[2]); r.a.w = *reinterpret_cast<const unsigned*>(&h.v[3]); }
 }
-template <int MODE> __device__ __forceinline__ void put(Raw<MODE>& r, const V8f& f) {
-    if constexpr (MODE != ROWS_HALF) {
+template <int MODE> __device__ __forceinline__ void put(Raw<MODE>& r, const Vf<kElems<MODE>>& f) {
+    if constexpr (!kHalfRows<MODE>) {
         r.a = make_uint4(__float_as_uint(f.x[0]), __float_as_uint(f.x[1]), __float_as_uint(f.x[2]), __float_as_uint(f.x[3]));
-        r.b = make_uint4(__float_as_uint(f.x[4]), __float_as_uint(f.x[5]), __float_as_uint(f.x[6]), __float_as_uint(f.x[7]));
+        if constexpr (kTwoParts<MODE>) r.b = make_uint4(__float_as_uint(f.x[4]), __float_as_uint(f.x[5]), __float_as_uint(f.x[6]), __float_as_uint(f.x[7]));
     }
 }
 
-__device__ __forceinline__ V8f widen(const V8h& h) {
-    V8f f;
+template <int N> __device__ __forceinline__ Vf<N> widen(const Vh<N>& h) {
+    Vf<N> f;
 #pragma unroll
-    for (int s = 0; s < 4; s++) { const float2 t = __half22float2(h.v[s]); f.x[2 * s] = t.x; f.x[2 * s + 1] = t.y; }
+    for (int s = 0; s < N / 2; s++) { const float2 t = __half22float2(h.v[s]); f.x[2 * s] = t.x; f.x[2 * s + 1] = t.y; }
     return f;
 }
-__device__ __forceinline__ V8h narrow(const V8f& f) {
-    V8h h;
+template <int N> __device__ __forceinline__ Vh<N> narrow(const Vf<N>& f) {
+    Vh<N> h;
 #pragma unroll
-    for (int s = 0; s < 4; s++) h.v[s] = __halves2half2(__float2half_rn(f.x[2 * s]), __float2half_rn(f.x[2 * s + 1]));
+    for (int s = 0; s < N / 2; s++) h.v[s] = __halves2half2(__float2half_rn(f.x[2 * s]), __float2half_rn(f.x[2 * s + 1]));
     return h;
 }
 
 // Is the row behind this stream id stored in fp32?
 template <int MODE> __device__ __forceinline__ bool is_f32(uint32_t code) {
-    return MODE == ROWS_F32 || (MODE == ROWS_DYN && (code & kPrecBit));
+    return MODE == ROWS_F32 || MODE == ROWS_F32Q || (MODE == ROWS_DYN && (code & kPrecBit));
 }
 
 // The rows of one side as a lane sees them: addresses of its slice of row 0 in the two arenas.  (One multiply-add
@@ -140,10 +167,10 @@ template <int K, int MODE> struct Rows {
     const unsigned char* b16;
     const unsigned char* b32;
     __device__ __forceinline__ Rows(const Arena& A, int m)
-        : b16(reinterpret_cast<const unsigned char*>(A.f16) + 16 * m), b32(reinterpret_cast<const unsigned char*>(A.f32) + 16 * m) {}
+        : b16(reinterpret_cast<const unsigned char*>(A.f16) + lane_at<K, MODE>(m)), b32(reinterpret_cast<const unsigned char*>(A.f32) + lane_at<K, MODE>(m)) {}
     __device__ __forceinline__ const unsigned char* at(uint32_t code) const {
-        if constexpr (MODE == ROWS_HALF) return b16 + (uint64_t)code * (2u * K);
-        else if constexpr (MODE == ROWS_F32) return b32 + (uint64_t)code * (4u * K);
+        if constexpr (kHalfRows<MODE>) return b16 + (uint64_t)code * (2u * K);
+        else if constexpr (MODE == ROWS_F32 || MODE == ROWS_F32Q) return b32 + (uint64_t)code * (4u * K);
         else return (code & kPrecBit) ? b32 + (uint64_t)(code & kIdMask) * (4u * K) : b16 + (uint64_t)(code & kIdMask) * (2u * K);
     }
 };
@@ -153,7 +180,7 @@ template <int MODE> __device__ __forceinline__ unsigned second_half(unsigned go,
     return MODE == ROWS_DYN ? ((code & kPrecBit) ? go : 0u) : go;
 }
 
-// Predicated accesses to a lane's 16 bytes: the code around them stays free of branches, which two or four workers of
+// Predicated accesses to a lane's 16 bytes (8 of ROWS_HALFQ): the code around them stays free of branches, which two or four workers of
 // a warp would take one after the other.
 template <int OFF> __device__ __forceinline__ void ldg_if(unsigned go, uint4& v, const unsigned char* p) {
     asm volatile("{ .reg .pred g; setp.ne.u32 g, %4, 0; @g ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%5 + %6]; }" : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
@@ -162,6 +189,15 @@ template <int OFF> __device__ __forceinline__ void ldg_if(unsigned go, uint4& v,
 template <int OFF> __device__ __forceinline__ void stg_if(unsigned go, const unsigned char* p, const uint4& v) {
     asm volatile("{ .reg .pred g; setp.ne.u32 g, %4, 0; @g st.global.cg.v4.u32 [%5 + %6], {%0, %1, %2, %3}; }" ::"r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w),
                  "r"(go), "l"(p), "n"(OFF) : "memory");
+}
+template <int OFF> __device__ __forceinline__ void ldg_if(unsigned go, uint2& v, const unsigned char* p) {
+    asm volatile("{ .reg .pred g; setp.ne.u32 g, %2, 0; @g ld.global.cg.v2.u32 {%0, %1}, [%3 + %4]; }" : "+r"(v.x), "+r"(v.y) : "r"(go), "l"(p), "n"(OFF) : "memory");
+}
+template <int OFF> __device__ __forceinline__ void stg_if(unsigned go, const unsigned char* p, const uint2& v) {
+    asm volatile("{ .reg .pred g; setp.ne.u32 g, %2, 0; @g st.global.cg.v2.u32 [%3 + %4], {%0, %1}; }" ::"r"(v.x), "r"(v.y), "r"(go), "l"(p), "n"(OFF) : "memory");
+}
+template <int OFF> __device__ __forceinline__ void lds_if(unsigned go, uint2& v, unsigned addr) {
+    asm volatile("{ .reg .pred g; setp.ne.u32 g, %2, 0; @g ld.shared.v2.u32 {%0, %1}, [%3 + %4]; }" : "+r"(v.x), "+r"(v.y) : "r"(go), "r"(addr), "n"(OFF) : "memory");
 }
 template <int OFF> __device__ __forceinline__ void lds_if(unsigned go, uint4& v, unsigned addr) {
     asm volatile("{ .reg .pred g; setp.ne.u32 g, %4, 0; @g ld.shared.v4.u32 {%0, %1, %2, %3}, [%5 + %6]; }" : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
@@ -173,13 +209,13 @@ template <int K, int MODE>
 __device__ __forceinline__ void ld_row_if(unsigned go, Raw<MODE>& r, const Rows<K, MODE>& A, uint32_t code) {
     const unsigned char* p = A.at(code);
     ldg_if<0>(go, r.a, p);
-    if constexpr (MODE != ROWS_HALF) ldg_if<2 * K>(second_half<MODE>(go, code), r.b, p);
+    if constexpr (kTwoParts<MODE>) ldg_if<2 * K>(second_half<MODE>(go, code), r.b, p);
 }
 template <int K, int MODE>
 __device__ __forceinline__ void st_row_if(unsigned go, const Rows<K, MODE>& A, uint32_t code, const Raw<MODE>& r) {
     const unsigned char* p = A.at(code);
     stg_if<0>(go, p, r.a);
-    if constexpr (MODE != ROWS_HALF) stg_if<2 * K>(second_half<MODE>(go, code), p, r.b);
+    if constexpr (kTwoParts<MODE>) stg_if<2 * K>(second_half<MODE>(go, code), p, r.b);
 }
 
 // Adds (now - before) to a row, unless `skip`, instead of storing `now`: with several workers on the same row at the
@@ -195,16 +231,23 @@ template <int K, int MODE>
 __device__ __forceinline__ void add_row_delta(const Rows<K, MODE>& A, uint32_t code, unsigned skip, const Raw<MODE>& now, const Raw<MODE>& before) {
     const unsigned char* p = A.at(code);
     if (is_f32<MODE>(code)) {
-        if constexpr (MODE != ROWS_HALF) {
-            const V8f n = v8f_of(now.a, now.b), o = v8f_of(before.a, before.b);
+        if constexpr (!kHalfRows<MODE>) {
+            constexpr int N = kElems<MODE>;
+            const Vf<N> n = as_vf(now), o = as_vf(before);
             const float2 minus = make_float2(-1.f, -1.f);      // n - o as fma(-1, o, n): the same single rounding, two lanes at once
-            float2 d[4];
+            float2 d[N / 2];
 #pragma unroll
-            for (int j = 0; j < 4; j++) d[j] = __ffma2_rn(minus, make_float2(o.x[2 * j], o.x[2 * j + 1]), make_float2(n.x[2 * j], n.x[2 * j + 1]));
+            for (int j = 0; j < N / 2; j++) d[j] = __ffma2_rn(minus, make_float2(o.x[2 * j], o.x[2 * j + 1]), make_float2(n.x[2 * j], n.x[2 * j + 1]));
             red_f32x4<0>(p, skip, d[0].x, d[0].y, d[1].x, d[1].y);
-            red_f32x4<2 * K>(p, skip, d[2].x, d[2].y, d[3].x, d[3].y);
+            if constexpr (kTwoParts<MODE>) red_f32x4<2 * K>(p, skip, d[2].x, d[2].y, d[3].x, d[3].y);
         }
-    } else {
+    } else if constexpr (MODE == ROWS_HALFQ) {
+        const Vh<4> n = as_vh(now), o = as_vh(before);
+        unsigned d[2];
+#pragma unroll
+        for (int t = 0; t < 2; t++) { const __half2 x = __hsub2(n.v[t], o.v[t]); d[t] = *reinterpret_cast<const unsigned*>(&x); }
+        asm volatile("{ .reg .pred s; setp.ne.u32 s, %3, 0; @!s red.global.add.noftz.v2.f16x2 [%0], {%1, %2}; }" ::"l"(p), "r"(d[0]), "r"(d[1]), "r"(skip) : "memory");
+    } else if constexpr (MODE != ROWS_F32Q) {
         const V8h n = v8h_of(now.a), o = v8h_of(before.a);
         unsigned d[4];
 #pragma unroll
@@ -221,8 +264,8 @@ __device__ __forceinline__ void add_row_delta(const Rows<K, MODE>& A, uint32_t c
 // fp32 arithmetic runs on the packed two-lane instructions of sm_100 (fma / mul / add .f32x2): each lane
 // is rounded on its own, exactly like the scalar instruction, and a row slice needs half as many issue
 // slots - which is what bounds this kernel.
-__device__ __forceinline__ float2 pr(const V8f& v, int j) { return make_float2(v.x[2 * j], v.x[2 * j + 1]); }
-__device__ __forceinline__ void set_pr(V8f& v, int j, float2 t) { v.x[2 * j] = t.x; v.x[2 * j + 1] = t.y; }
+template <int N> __device__ __forceinline__ float2 pr(const Vf<N>& v, int j) { return make_float2(v.x[2 * j], v.x[2 * j + 1]); }
+template <int N> __device__ __forceinline__ void set_pr(Vf<N>& v, int j, float2 t) { v.x[2 * j] = t.x; v.x[2 * j + 1] = t.y; }
 
 __device__ __forceinline__ float pair_partial(const V8f& a, const V8f& b) {
     // (f0, f2) = (a0 b0 + a2 b2, a1 b1 + a3 b3), (f1, f3) likewise from positions 4..7
@@ -276,31 +319,81 @@ __device__ __forceinline__ __half2 worker_sum(__half2 x, unsigned wmask, Mid mid
     return x;
 }
 
+// Dot product of two rows over a worker's lanes.  With four elements a lane, the two lanes that make up a lane of the wider
+// form have (f_0, f_2) and (f_1, f_3): both get the other's pair, and the lane partial and its butterfly follow as above.
+template <int TS, class Mid = Nothing>
+__device__ __forceinline__ float worker_dot(const V8f& a, const V8f& b, unsigned wmask, Mid mid = Mid()) { return worker_sum<TS>(pair_partial(a, b), wmask, mid); }
+template <int TS, class Mid = Nothing>
+__device__ __forceinline__ __half2 worker_dot(const V8h& a, const V8h& b, unsigned wmask, Mid mid = Mid()) { return worker_sum<TS>(pair_partial(a, b), wmask, mid); }
+template <class Mid> struct After {           // the steps of `mid` from the second on
+    Mid mid;
+    __device__ __forceinline__ void operator()(int i) const { mid(i + 1); }
+};
+template <int TS, class Mid = Nothing>
+__device__ __forceinline__ float worker_dot(const Vf<4>& a, const Vf<4>& b, unsigned wmask, Mid mid = Mid()) {
+    const float2 f = __ffma2_rn(pr(a, 0), pr(b, 0), __fmul2_rn(pr(a, 1), pr(b, 1)));
+    const float2 o = make_float2(__shfl_xor_sync(wmask, f.x, TS / 2), __shfl_xor_sync(wmask, f.y, TS / 2));
+    mid(0);
+    const float2 t = __fadd2_rn(f, o);
+    return worker_sum<TS / 2>(__fadd_rn(t.x, t.y), wmask, After<Mid>{mid});
+}
+template <int TS, class Mid = Nothing>
+__device__ __forceinline__ __half2 worker_dot(const Vh<4>& a, const Vh<4>& b, unsigned wmask, Mid mid = Mid()) {
+    const __half2 f = __hfma2(a.v[0], b.v[0], __hmul2_rn(a.v[1], b.v[1]));
+    const unsigned o = __shfl_xor_sync(wmask, *reinterpret_cast<const unsigned*>(&f), TS / 2);
+    mid(0);
+    const __half2 t = __hadd2_rn(f, *reinterpret_cast<const __half2*>(&o));
+    return worker_sum<TS / 2>(__hadd2_rn(__low2half2(t), __high2half2(t)), wmask, After<Mid>{mid});
+}
+
+// The chain over four lanes' worth of elements where a lane has two of each: the lanes with e0, e1 begin, those with e2, e3 go on;
+// the lane tree goes through the latter, and its last step brings the sum to all.
+template <int TS, class Mid>
+__device__ __forceinline__ float worker_chain_k128(const Vf<4>& a, const Vf<4>& b, unsigned wmask, Mid mid) {
+    const int m = threadIdx.x & (TS - 1);
+    const bool up = m & (TS / 2);
+    float c[2], begun[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) begun[h] = __shfl_xor_sync(wmask, __fmaf_rn(a.x[h], b.x[h], __fmul_rn(a.x[2 + h], b.x[2 + h])), TS / 2);
+    mid(0);
+#pragma unroll
+    for (int h = 0; h < 2; h++) c[h] = __fmaf_rn(a.x[2 + h], b.x[2 + h], __fmaf_rn(a.x[h], b.x[h], begun[h]));
+    float x = __fadd_rn(c[0], c[1]);
+#pragma unroll
+    for (int d = TS / 4, i = 1; d >= 2; d >>= 1, i++) {
+        const float o = __shfl_xor_sync(wmask, x, d);
+        mid(i);
+        x = __fadd_rn(x, o);
+    }
+    const float o = __shfl_sync(wmask, x, (m ^ 1) | (TS / 2), TS), own = __shfl_sync(wmask, x, m | (TS / 2), TS);
+    return __fadd_rn(up ? x : own, o);
+}
+
 // t = fma(e, y, -(lam*x)) and x' = fma(lr, t, x), element-wise
-__device__ __forceinline__ V8f grad(float e, const V8f& y, float lam, const V8f& x) {
-    V8f g;
+template <int N> __device__ __forceinline__ Vf<N> grad(float e, const Vf<N>& y, float lam, const Vf<N>& x) {
+    Vf<N> g;
     const float2 e2 = make_float2(e, e), nlam2 = make_float2(-lam, -lam);      // (-lam) * x == -(lam * x), bit for bit
 #pragma unroll
-    for (int j = 0; j < 4; j++) set_pr(g, j, __ffma2_rn(e2, pr(y, j), __fmul2_rn(nlam2, pr(x, j))));
+    for (int j = 0; j < N / 2; j++) set_pr(g, j, __ffma2_rn(e2, pr(y, j), __fmul2_rn(nlam2, pr(x, j))));
     return g;
 }
-__device__ __forceinline__ V8h grad(__half2 e, const V8h& y, __half2 nlam, const V8h& x) {
-    V8h g;
+template <int N> __device__ __forceinline__ Vh<N> grad(__half2 e, const Vh<N>& y, __half2 nlam, const Vh<N>& x) {
+    Vh<N> g;
 #pragma unroll
-    for (int s = 0; s < 4; s++) g.v[s] = __hfma2(e, y.v[s], __hmul2_rn(nlam, x.v[s]));     // (-lam) * x == -(lam * x), bit for bit
+    for (int s = 0; s < N / 2; s++) g.v[s] = __hfma2(e, y.v[s], __hmul2_rn(nlam, x.v[s]));     // (-lam) * x == -(lam * x), bit for bit
     return g;
 }
-__device__ __forceinline__ V8f step(float lr, const V8f& g, const V8f& x) {
-    V8f o;
+template <int N> __device__ __forceinline__ Vf<N> step(float lr, const Vf<N>& g, const Vf<N>& x) {
+    Vf<N> o;
     const float2 lr2 = make_float2(lr, lr);
 #pragma unroll
-    for (int j = 0; j < 4; j++) set_pr(o, j, __ffma2_rn(lr2, pr(g, j), pr(x, j)));
+    for (int j = 0; j < N / 2; j++) set_pr(o, j, __ffma2_rn(lr2, pr(g, j), pr(x, j)));
     return o;
 }
-__device__ __forceinline__ V8h step(__half2 lr, const V8h& g, const V8h& x) {
-    V8h o;
+template <int N> __device__ __forceinline__ Vh<N> step(__half2 lr, const Vh<N>& g, const Vh<N>& x) {
+    Vh<N> o;
 #pragma unroll
-    for (int s = 0; s < 4; s++) o.v[s] = __hfma2(lr, g.v[s], x.v[s]);
+    for (int s = 0; s < N / 2; s++) o.v[s] = __hfma2(lr, g.v[s], x.v[s]);
     return o;
 }
 
@@ -336,14 +429,14 @@ struct Consts {
 // order; here the user side does the same per rating, while the item side - whose ratings arrive in
 // runs of the same group, because shuffle windows are item-sorted - is summed in registers over a run
 // of equal item groups and flushed once per run, which removes the contention on popular items.
-struct Sample {
-    V8f gp, gq;
+template <int N> struct Sample {
+    Vf<N> gp, gq;
     bool user, item;      // which sides of this rating contribute (binary16-stored rows only)
 };
 
-__device__ __forceinline__ void red_add8(float* dst, const V8f& g) {
+template <int N> __device__ __forceinline__ void red_add(float* dst, const Vf<N>& g) {
     atomicAdd(reinterpret_cast<float4*>(dst), make_float4(g.x[0], g.x[1], g.x[2], g.x[3]));
-    atomicAdd(reinterpret_cast<float4*>(dst) + 1, make_float4(g.x[4], g.x[5], g.x[6], g.x[7]));
+    if constexpr (N == 8) atomicAdd(reinterpret_cast<float4*>(dst) + 1, make_float4(g.x[4], g.x[5], g.x[6], g.x[7]));
 }
 
 struct KernelArgs {
@@ -415,33 +508,34 @@ __device__ __forceinline__ float pow2_rev(float s) {
     return (b >= 0x00800000u && b < 0x7f000000u && !(b & 0x007fffffu)) ? __uint_as_float(0x7f000000u - b) : __fdiv_rn(1.f, s);
 }
 __device__ __forceinline__ float fix_round(float v, float s, float s_rev) { return __fmul_rn(round_away(__fmul_rn(v, s)), s_rev); }
-// The eight values of a lane times a power-of-two scale, rounded like round_away - with full-rate instructions, two
+// The values of a lane times a power-of-two scale, rounded like round_away - with full-rate instructions, two
 // values at a time, in place of truncations and conversions, which run at an eighth of that rate and were 64 of an
 // update's instructions.  x s is exact, so adding 1.5 * 2^23 in one multiply-add rounds it to the nearest integer, and the
 // two roundings differ at exact halves only: `odd` receives the largest distance from the integers, and a warp
 // that meets one half (rare: it takes the bits of x below the grid to be 100...0) rounds again the long way.  Results are
 // exact below 2^22, larger ones stay above 2^21, and zero is +0.
-__device__ __forceinline__ V8f quantize_near(const V8f& x, float s, float& odd) {
-    V8f o;
-    float far[4];
+template <int N> __device__ __forceinline__ Vf<N> quantize_near(const Vf<N>& x, float s, float& odd) {
+    Vf<N> o;
+    float far[N / 2];
     const float2 s2 = make_float2(s, s), magic = make_float2(12582912.f, 12582912.f), minus = make_float2(-12582912.f, -12582912.f);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < N / 2; j++) {
         const float2 r = __fadd2_rn(__ffma2_rn(pr(x, j), s2, magic), minus);
         const float2 d = __ffma2_rn(pr(x, j), s2, make_float2(-r.x, -r.y));
         far[j] = fmaxf(fabsf(d.x), fabsf(d.y));
         set_pr(o, j, r);
     }
-    odd = fmaxf(fmaxf(far[0], far[1]), fmaxf(far[2], far[3]));
+    odd = fmaxf(far[0], far[1]);
+    if constexpr (N == 8) odd = fmaxf(odd, fmaxf(far[2], far[3]));
     return o;
 }
-__device__ __forceinline__ V8f quantize_away(const V8f& x, float s) {
-    V8f o;
+template <int N> __device__ __forceinline__ Vf<N> quantize_away(const Vf<N>& x, float s) {
+    Vf<N> o;
 #pragma unroll
-    for (int t = 0; t < 8; t++) o.x[t] = __fadd_rn(round_away(__fmul_rn(x.x[t], s)), 0.f);
+    for (int t = 0; t < N; t++) o.x[t] = __fadd_rn(round_away(__fmul_rn(x.x[t], s)), 0.f);
     return o;
 }
-__device__ __forceinline__ void quantize(const V8f& p, float sp, const V8f& q, float sq, V8f& pi, V8f& qi, unsigned wmask) {
+template <int N> __device__ __forceinline__ void quantize(const Vf<N>& p, float sp, const Vf<N>& q, float sq, Vf<N>& pi, Vf<N>& qi, unsigned wmask) {
     float odd_p, odd_q;
     pi = quantize_near(p, sp, odd_p);
     qi = quantize_near(q, sq, odd_q);
@@ -449,14 +543,14 @@ __device__ __forceinline__ void quantize(const V8f& p, float sp, const V8f& q, f
 }
 // The int8 passes work on the integers as floats: products and sums of int8 values stay far below 2^24.
 __device__ __forceinline__ float clamp8(float v) { return v == v ? fminf(fmaxf(v, -128.f), 127.f) : 0.f; }
-__device__ __forceinline__ V8f clamp8(const V8f& x) {
-    V8f o;
+template <int N> __device__ __forceinline__ Vf<N> clamp8(const Vf<N>& x) {
+    Vf<N> o;
 #pragma unroll
-    for (int t = 0; t < 8; t++) o.x[t] = clamp8(x.x[t]);
+    for (int t = 0; t < N; t++) o.x[t] = clamp8(x.x[t]);
     return o;
 }
 // quantize() to int8 values; `outside`: may some value leave their range?
-__device__ __forceinline__ void quantize_int8(const V8f& p, float sp, const V8f& q, float sq, bool outside, V8f& pi, V8f& qi, unsigned wmask) {
+template <int N> __device__ __forceinline__ void quantize_int8(const Vf<N>& p, float sp, const Vf<N>& q, float sq, bool outside, Vf<N>& pi, Vf<N>& qi, unsigned wmask) {
     float odd_p, odd_q;
     pi = quantize_near(p, sp, odd_p);
     qi = quantize_near(q, sq, odd_q);
@@ -464,31 +558,33 @@ __device__ __forceinline__ void quantize_int8(const V8f& p, float sp, const V8f&
 }
 __device__ __forceinline__ float quantize8(float v, float s) { return clamp8(round_away(__fmul_rn(v, s))); }
 // A quantize()d row in binary16; what rounded to zero keeps its sign, as it does in fix_round
-__device__ __forceinline__ V8h grid_half(const V8f& r, const V8f& x, float s_rev) {
-    V8h h;
+template <int N> __device__ __forceinline__ Vh<N> grid_half(const Vf<N>& r, const Vf<N>& x, float s_rev) {
+    Vh<N> h;
     const float2 rev2 = make_float2(s_rev, s_rev);
     auto signed_as = [](float v, float like) { return __uint_as_float(__float_as_uint(v) | (__float_as_uint(like) & 0x80000000u)); };
 #pragma unroll
-    for (int t = 0; t < 4; t++)
+    for (int t = 0; t < N / 2; t++)
         h.v[t] = __float22half2_rn(__fmul2_rn(make_float2(signed_as(r.x[2 * t], x.x[2 * t]), signed_as(r.x[2 * t + 1], x.x[2 * t + 1])), rev2));
     return h;
 }
-__device__ __forceinline__ V8h fix_round_half(const V8f& x, float s, float s_rev) {
-    V8h h;
+template <int N> __device__ __forceinline__ Vh<N> fix_round_half(const Vf<N>& x, float s, float s_rev) {
+    Vh<N> h;
 #pragma unroll
-    for (int t = 0; t < 4; t++)
+    for (int t = 0; t < N / 2; t++)
         h.v[t] = __floats2half2_rn(fix_round(x.x[2 * t], s, s_rev), fix_round(x.x[2 * t + 1], s, s_rev));
     return h;
 }
 // Both quantize()d rows on their grids; `big`: some value may reach 2^21 steps of its grid
-__device__ __forceinline__ void to_grid(const V8f& p, const V8f& pi, float sp, const V8f& q, const V8f& qi, float sq, bool big, V8h& ph, V8h& qh) {
+template <int N>
+__device__ __forceinline__ void to_grid(const Vf<N>& p, const Vf<N>& pi, float sp, const Vf<N>& q, const Vf<N>& qi, float sq, bool big, Vh<N>& ph, Vh<N>& qh) {
     const float sp_rev = pow2_rev(sp), sq_rev = pow2_rev(sq);
     if (big) { ph = fix_round_half(p, sp, sp_rev); qh = fix_round_half(q, sq, sq_rev); }
     else { ph = grid_half(pi, p, sp_rev); qh = grid_half(qi, q, sq_rev); }
 }
-__device__ __forceinline__ float abs_max8(const V8f& x) {
-    return fmaxf(fmaxf(fmaxf(fabsf(x.x[0]), fabsf(x.x[1])), fmaxf(fabsf(x.x[2]), fabsf(x.x[3]))),
-                 fmaxf(fmaxf(fabsf(x.x[4]), fabsf(x.x[5])), fmaxf(fabsf(x.x[6]), fabsf(x.x[7]))));
+template <int N> __device__ __forceinline__ float abs_max(const Vf<N>& x) {
+    const float m = fmaxf(fmaxf(fabsf(x.x[0]), fabsf(x.x[1])), fmaxf(fabsf(x.x[2]), fabsf(x.x[3])));
+    if constexpr (N == 4) return m;
+    else return fmaxf(m, fmaxf(fmaxf(fabsf(x.x[4]), fabsf(x.x[5])), fmaxf(fabsf(x.x[6]), fabsf(x.x[7]))));
 }
 template <int TS> __device__ __forceinline__ float worker_max(float x, unsigned wmask) {
 #pragma unroll
@@ -508,14 +604,33 @@ template <int TS> __device__ __forceinline__ void worker_max4(float (&a)[4], uns
 #pragma unroll
     for (int i = 0; i < 4; i++) a[i] = __shfl_sync(wmask, r0, (i >> 1) * (TS / 2) + (i & 1) * (TS / 4), TS);
 }
-__device__ __forceinline__ float max8(const V8f& x) {
-    return fmaxf(fmaxf(fmaxf(x.x[0], x.x[1]), fmaxf(x.x[2], x.x[3])), fmaxf(fmaxf(x.x[4], x.x[5]), fmaxf(x.x[6], x.x[7])));
+template <int N> __device__ __forceinline__ float max_of(const Vf<N>& x) {
+    const float m = fmaxf(fmaxf(x.x[0], x.x[1]), fmaxf(x.x[2], x.x[3]));
+    if constexpr (N == 4) return m;
+    else return fmaxf(m, fmaxf(fmaxf(x.x[4], x.x[5]), fmaxf(x.x[6], x.x[7])));
 }
-__device__ __forceinline__ float min8(const V8f& x) {
-    return fminf(fminf(fminf(x.x[0], x.x[1]), fminf(x.x[2], x.x[3])), fminf(fminf(x.x[4], x.x[5]), fminf(x.x[6], x.x[7])));
+template <int N> __device__ __forceinline__ float min_of(const Vf<N>& x) {
+    const float m = fminf(fminf(x.x[0], x.x[1]), fminf(x.x[2], x.x[3]));
+    if constexpr (N == 4) return m;
+    else return fminf(m, fminf(fminf(x.x[4], x.x[5]), fminf(x.x[6], x.x[7])));
 }
 // Squared norm of both gradients the way the reference groups it: per reference lane
-// (norm_p + norm_q), then the lane tree.  A lane here holds two (k=128) or four (k=64) reference lanes.
+// (norm_p + norm_q), then the lane tree.  A lane here holds two (k=128) or four (k=64) reference lanes; with four elements a
+// lane it holds half of each (k=128) or two of them (k=64), and muppet_norm_join adds what lane l ^ K/8 holds.
+template <int K> __device__ __forceinline__ float4 muppet_norm_parts(const Vf<4>& gp, const Vf<4>& gq) {
+    auto sq = [](const Vf<4>& g, int a, int b) { return __fmaf_rn(g.x[a], g.x[a], __fmul_rn(g.x[b], g.x[b])); };
+    const float4 s = make_float4(sq(gp, 0, 2), sq(gp, 1, 3), sq(gq, 0, 2), sq(gq, 1, 3));
+    return K == 128 ? s : make_float4(__fadd_rn(s.x, s.z), __fadd_rn(s.y, s.w), 0.f, 0.f);
+}
+template <int K> __device__ __forceinline__ float muppet_norm_join(const float4& s) {
+    auto both = [](float v) { return __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, K / 8)); };
+    if (K == 128) {
+        const float a = both(s.x), b = both(s.y), c = both(s.z), d = both(s.w);
+        return __fadd_rn(__fadd_rn(a, c), __fadd_rn(b, d));
+    }
+    const float a = both(s.x), b = both(s.y);
+    return __fadd_rn(a, b);
+}
 template <int K>
 __device__ __forceinline__ float muppet_norm_partial(const V8f& gp, const V8f& gq) {
     auto sq = [](const V8f& g, int a, int b) { return __fmaf_rn(g.x[a], g.x[a], __fmul_rn(g.x[b], g.x[b])); };
@@ -533,11 +648,11 @@ __device__ __forceinline__ float muppet_norm_partial(const V8f& gp, const V8f& g
 // int8 forward pass: saturated fixed-point values, exact integer dot product, one division (by a power of two).
 // pi, qi: quantize()d rows, clamped if need be.  A lane's sum stays below 2^18, the whole one below 2^22, so both pass
 // between integer and float in the low bits of 1.5 * 2^23 + x.
-template <int TS>
-__device__ __forceinline__ float forward_int8(const V8f& pi, const V8f& qi, float sp, float sq) {
+template <int TS, int N>
+__device__ __forceinline__ float forward_int8(const Vf<N>& pi, const Vf<N>& qi, float sp, float sq) {
     float2 a = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int j = 0; j < 4; j++) a = __ffma2_rn(pr(pi, j), pr(qi, j), a);
+    for (int j = 0; j < N / 2; j++) a = __ffma2_rn(pr(pi, j), pr(qi, j), a);
     const int whole = worker_add<TS>(__float_as_int(__fadd_rn(__fadd_rn(a.x, a.y), 12582912.f)) - 0x4b400000);
     return __fmul_rn(__fsub_rn(__int_as_float(whole + 0x4b400000), 12582912.f), pow2_rev(__fmul_rn(sp, sq)));
 }
@@ -564,23 +679,46 @@ __device__ __forceinline__ float forward_half(const V8h& ph, const V8h& qh, unsi
     }
     return __half2float(__hadd_rn(__low2half(xy), __high2half(xy)));
 }
+// The same with four elements a lane.  K=128: the lanes with (e2, e6, e3, e7) hand their products to those that have the first
+// terms of the sums, and in the last step of the tree every lane takes both values from them.  K=64: both lanes add both products.
+template <int K>
+__device__ __forceinline__ float forward_half(const Vh<4>& ph, const Vh<4>& qh, unsigned wmask) {
+    constexpr int TS = K / 4;
+    auto from = [&](const __half2& v, int lane_of) {
+        const unsigned o = __shfl_sync(wmask, *reinterpret_cast<const unsigned*>(&v), lane_of, TS);
+        return *reinterpret_cast<const __half2*>(&o);
+    };
+    const int l = threadIdx.x & (TS - 1);
+    const __half2 m0 = __hmul2_rn(ph.v[0], qh.v[0]), m1 = __hmul2_rn(ph.v[1], qh.v[1]);
+    const __half2 o0 = from(m0, l ^ (TS / 2)), o1 = from(m1, l ^ (TS / 2));
+    __half2 xab, yab;
+    if (K == 128) { xab = __hfma2(ph.v[0], qh.v[0], o0); yab = __hfma2(ph.v[1], qh.v[1], o1); }
+    else { xab = __hadd2_rn(m0, o0); yab = __hadd2_rn(m1, o1); }
+    __half2 xy = __hadd2_rn(__lows2half2(xab, yab), __highs2half2(xab, yab));
+#pragma unroll
+    for (int d = TS / 4; d >= 2; d >>= 1) xy = __hadd2_rn(xy, from(xy, l ^ d));
+    const int low = l & (TS / 2 - 1);
+    const __half2 last = from(xy, low ^ 1);
+    xy = __hadd2_rn(K == 128 ? from(xy, low) : xy, last);
+    return __half2float(__hadd_rn(__low2half(xy), __high2half(xy)));
+}
 // backward passes: g_p = q*e + p*(-lam), g_q = p*e + q*(-lam) in int8 or binary16 fixed point
-__device__ __forceinline__ void backward_int8(const V8f& pi, const V8f& qi, float ruv, float nlam, float sb, V8f& gp, V8f& gq) {
+template <int N> __device__ __forceinline__ void backward_int8(const Vf<N>& pi, const Vf<N>& qi, float ruv, float nlam, float sb, Vf<N>& gp, Vf<N>& gq) {
     const float rev = pow2_rev(__fmul_rn(sb, sb)), e = quantize8(ruv, sb), l = quantize8(nlam, sb);
     const float2 rev2 = make_float2(rev, rev), e2 = make_float2(e, e), l2 = make_float2(l, l), zero = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {      // + 0: the integer sum has no negative zero
+    for (int j = 0; j < N / 2; j++) {      // + 0: the integer sum has no negative zero
         set_pr(gp, j, __ffma2_rn(__ffma2_rn(pr(qi, j), e2, __fmul2_rn(pr(pi, j), l2)), rev2, zero));
         set_pr(gq, j, __ffma2_rn(__ffma2_rn(pr(pi, j), e2, __fmul2_rn(pr(qi, j), l2)), rev2, zero));
     }
 }
-__device__ __forceinline__ void backward_half(const V8h& ph, const V8h& qh, float ruv, float nlam, float sb, V8f& gp, V8f& gq) {
+template <int N> __device__ __forceinline__ void backward_half(const Vh<N>& ph, const Vh<N>& qh, float ruv, float nlam, float sb, Vf<N>& gp, Vf<N>& gq) {
     const float sb_rev = pow2_rev(sb);
     const __half2 e2 = __half2half2(__float2half_rn(fix_round(ruv, sb, sb_rev)));
     const __half2 l2 = __half2half2(__float2half_rn(fix_round(nlam, sb, sb_rev)));
-    V8h gph, gqh;
+    Vh<N> gph, gqh;
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
+    for (int t = 0; t < N / 2; t++) {
         gph.v[t] = __hadd2_rn(__hmul2_rn(qh.v[t], e2), __hmul2_rn(ph.v[t], l2));
         gqh.v[t] = __hadd2_rn(__hmul2_rn(ph.v[t], e2), __hmul2_rn(qh.v[t], l2));
     }
@@ -608,20 +746,20 @@ template <int TS> __device__ __noinline__ float muppet_back_scale_exact(int bits
 // hundred workers that chain is the epoch, so what shortens it counts: keys in place of four extremes, warp-wide
 // integer reductions in place of shuffles, one vote a pass, the norm of the rating before on the side.  2M ratings, 592
 // workers: 2.98 -> 2.25 ms per epoch.
-template <int K, class Mid>
-__device__ __forceinline__ void muppet_update(const Consts& c, float r, V8f& p, V8f& q, V8f& gp, V8f& gq, Mid mid) {
-    constexpr int TS = K / 8;
+template <int K, int N, class Mid>
+__device__ __forceinline__ void muppet_update(const Consts& c, float r, Vf<N>& p, Vf<N>& q, Vf<N>& gp, Vf<N>& gq, Mid mid) {
+    constexpr int TS = K / N;
     constexpr unsigned kAll = 0xffffffffu;
     const int bits = c.bits;
     const float nlam = -c.lam;
     if (bits == 32) {
-        const float ruv = __fsub_rn(r, worker_sum<TS>(pair_partial(p, q), kAll, mid));
+        const float ruv = __fsub_rn(r, worker_dot<TS>(p, q, kAll, mid));
         gp = grad(ruv, q, c.lam, p); gq = grad(ruv, p, c.lam, q);
         p = step(c.lr, gp, p); q = step(c.lr, gq, q);
         return;
     }
     const int2 bound = scale_bounds(bits);
-    const float phi = max8(p), plo = min8(p), qhi = max8(q), qlo = min8(q);
+    const float phi = max_of(p), plo = min_of(p), qhi = max_of(q), qlo = min_of(q);
     mid(0);
     const int kp = worker_min<TS>(scale_key(bound, phi, plo)), kq = worker_min<TS>(scale_key(bound, qhi, qlo));
     mid(1);
@@ -630,8 +768,8 @@ __device__ __forceinline__ void muppet_update(const Consts& c, float r, V8f& p, 
         const float2 s = muppet_scales_exact<TS>(bits, phi, plo, qhi, qlo);
         sp = s.x; sq = s.y;
     }
-    V8f pi, qi;
-    V8h ph, qh;
+    Vf<N> pi, qi;
+    Vh<N> ph, qh;
     float pred;
     if (bits == 8) {
         quantize_int8(p, sp, q, sq, outside8(phi, plo, sp) || outside8(qhi, qlo, sq), pi, qi, kAll);
@@ -651,9 +789,11 @@ __device__ __forceinline__ void muppet_update(const Consts& c, float r, V8f& p, 
     if (__any_sync(kAll, scale_unsure(bound, kb))) sb = muppet_back_scale_exact<TS>(bits, hi, lo, nlam, ruv);
     if (bits == 8) {
         quantize_int8(p, sb, q, sb, outside8(hi, lo, sb), pi, qi, kAll);
+        mid(4);
         backward_int8(pi, qi, ruv, nlam, sb, gp, gq);
     } else {
         quantize(p, sb, q, sb, pi, qi, kAll);
+        mid(4);
         to_grid(p, pi, sb, q, qi, sb, beyond_grid(hi, lo, sb), ph, qh);
         backward_half(ph, qh, ruv, nlam, sb, gp, gq);
     }
@@ -696,6 +836,20 @@ __device__ __forceinline__ int ceil_log2_rounded(float x) {
     const int j = 31 - __clz((int)a);
     const uint32_t limit = j <= 1 ? 0u : (j == 2 ? 1u : (j == 3 ? 2u : (j == 4 ? 5u : (j == 5 ? 11u : (j == 6 ? 22u : 44u)))));
     return M <= limit ? E : E + 1;
+}
+
+// The eight elements of lane l mod K/8 of the wider form, from the two lanes that hold four of them each
+template <int K> __device__ __forceinline__ const V8f& eight(const V8f& x) { return x; }
+template <int K> __device__ __forceinline__ V8f eight(const Vf<4>& x) {
+    const bool up = threadIdx.x & (K / 8);
+    V8f o;
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        const float other = __shfl_xor_sync(0xffffffffu, x.x[t], K / 8);
+        o.x[t] = up ? other : x.x[t];
+        o.x[4 + t] = up ? x.x[t] : other;
+    }
+    return o;
 }
 
 // 2^|ceil(log2(range / (2^(bits-1) - 1)))| (afp_sgd_kernel.h:8-16, 112-118); exponent capped at 126
@@ -773,33 +927,33 @@ __device__ __noinline__ AfpSide afp_requantize(AfpSide s, float diff, float rang
 }
 // The workers of a warp go through this together: what one of them needs (a re-estimation, the int8 or the binary16
 // pass) all of them compute, and each keeps the result if it is its own case.  active: is there a rating?
-template <int K>
-__device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float r, bool active, V8f& p, V8f& q) {
-    constexpr int TS = K / 8;
+template <int K, int N>
+__device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float r, bool active, Vf<N>& p, Vf<N>& q) {
+    constexpr int TS = K / N;
     constexpr unsigned kAll = 0xffffffffu;
     const long long cur = st.cur;
     const bool new_user = active && cur == st.user.next, new_item = active && cur == st.item.next, new_back = active && cur == st.back.next;
     const bool estimate = __any_sync(kAll, new_user || new_item || new_back);
     float pmax = 0.f, qmax = 0.f;
     if (estimate) {
-        pmax = worker_max<TS>(abs_max8(p), kAll);
-        qmax = worker_max<TS>(abs_max8(q), kAll);
+        pmax = worker_max<TS>(abs_max(p), kAll);
+        qmax = worker_max<TS>(abs_max(q), kAll);
         if (__any_sync(kAll, new_user)) {
-            const AfpSide s = afp_requantize(st.user, afp_qem<K>(p, pmax, kAll), pmax, cur, c.afp_epoch, c.afp_init_threshold);
+            const AfpSide s = afp_requantize(st.user, afp_qem<K>(eight<K>(p), pmax, kAll), pmax, cur, c.afp_epoch, c.afp_init_threshold);
             if (new_user) st.user = s;
         }
         if (__any_sync(kAll, new_item)) {
-            const AfpSide s = afp_requantize(st.item, afp_qem<K>(q, qmax, kAll), qmax, cur, c.afp_epoch, c.afp_init_threshold);
+            const AfpSide s = afp_requantize(st.item, afp_qem<K>(eight<K>(q), qmax, kAll), qmax, cur, c.afp_epoch, c.afp_init_threshold);
             if (new_item) st.item = s;
         }
     }
     // The formats are those of an earlier rating, so values may lie outside their range at any time.
     const bool forward8 = st.user.n == 8 && st.item.n == 8;
     float pred = 0.f;
-    V8f pi, qi;
-    V8h ph, qh;
+    Vf<N> pi, qi;
+    Vh<N> ph, qh;
     quantize(p, st.user.scale, q, st.item.scale, pi, qi, kAll);
-    float most = fmaxf(abs_max8(pi), abs_max8(qi));
+    float most = fmaxf(abs_max(pi), abs_max(qi));
     if (__any_sync(kAll, active && !forward8)) {
         to_grid(p, pi, st.user.scale, q, qi, st.item.scale, __any_sync(kAll, !(most < 2097152.f)), ph, qh);
         pred = forward_half<K>(ph, qh, kAll);
@@ -812,20 +966,20 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
     const float ruv = __fsub_rn(r, pred);
     if (estimate && __any_sync(kAll, new_back)) {
         const float range = fmaxf(fmaxf(fmaxf(pmax, qmax), fabsf(c.lam)), fabsf(ruv));
-        const AfpSide s = afp_requantize(st.back, afp_qem_back<K>(p, q, c.lam, ruv, range, kAll), range, cur, c.afp_epoch, c.afp_init_threshold);
+        const AfpSide s = afp_requantize(st.back, afp_qem_back<K>(eight<K>(p), eight<K>(q), c.lam, ruv, range, kAll), range, cur, c.afp_epoch, c.afp_init_threshold);
         if (new_back) st.back = s;
     }
     const bool back8 = st.back.n == 8;
     quantize(p, st.back.scale, q, st.back.scale, pi, qi, kAll);
-    most = fmaxf(abs_max8(pi), abs_max8(qi));
-    V8f gp, gq;
+    most = fmaxf(abs_max(pi), abs_max(qi));
+    Vf<N> gp, gq;
     if (__any_sync(kAll, active && !back8)) {
         to_grid(p, pi, st.back.scale, q, qi, st.back.scale, __any_sync(kAll, !(most < 2097152.f)), ph, qh);
         backward_half(ph, qh, ruv, -c.lam, st.back.scale, gp, gq);
     }
     if (__any_sync(kAll, active && back8)) {
         if (__any_sync(kAll, !(most <= 127.f))) { pi = clamp8(pi); qi = clamp8(qi); }
-        V8f wp, wq;
+        Vf<N> wp, wq;
         backward_int8(pi, qi, ruv, -c.lam, st.back.scale, wp, wq);
         if (back8) { gp = wp; gq = wq; }
     }
@@ -835,7 +989,7 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
 
 // Does a launch work with binary16 ratings?  Its records then hold the converted value in both halves of a word.
 template <int KIND, int UM, int IM> constexpr bool kHalfRating =
-    KIND == KIND_MPT || ((KIND == KIND_MIXED || KIND == KIND_SWITCH) && UM == ROWS_HALF && IM == ROWS_HALF);
+    KIND == KIND_MPT || ((KIND == KIND_MIXED || KIND == KIND_SWITCH) && kHalfRows<UM> && kHalfRows<IM>);
 __device__ __forceinline__ __half2 half2_of(uint32_t w) { return *reinterpret_cast<const __half2*>(&w); }
 
 // One update.  rw is the rating as its record holds it; p_raw / q_raw are the row slices in their storage precision,
@@ -844,67 +998,71 @@ __device__ __forceinline__ __half2 half2_of(uint32_t w) { return *reinterpret_ca
 // worker has to do meanwhile, done under the shuffles of the dot product.
 template <int K, int KIND, int UM, int IM, bool STATS, class Mid>
 __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_t uc, uint32_t ic, Raw<UM>& p_raw, Raw<IM>& q_raw,
-                                           Sample& smp, AfpState& afp, bool active, unsigned wmask, Mid mid) {
-    constexpr int TS = K / 8;
+                                           Sample<kElems<UM>>& smp, AfpState& afp, bool active, unsigned wmask, Mid mid) {
+    constexpr int N = kElems<UM>, TS = K / N;
+    static_assert(N == kElems<IM>, "both rows are spread over the worker's lanes the same way");
     constexpr bool kAhead = KIND == KIND_AFP || UM == ROWS_DYN || IM == ROWS_DYN;      // no single dot product to hide under
     if constexpr (kAhead) { mid(0); mid(1); mid(2); }
     if (STATS) { smp.user = false; smp.item = false; }
     if constexpr (KIND == KIND_MPT) {
-        const V8f p = as_v8f(p_raw), q = as_v8f(q_raw);
-        const V8h ph = narrow(p), qh = narrow(q);
-        const __half2 dot = worker_sum<TS>(pair_partial(ph, qh), wmask, mid);
+        const Vf<N> p = as_vf(p_raw), q = as_vf(q_raw);
+        const Vh<N> ph = narrow(p), qh = narrow(q);
+        const __half2 dot = worker_dot<TS>(ph, qh, wmask, mid);
         const __half2 e = __hmul2_rn(c.mpt_scale, __hsub2_rn(half2_of(rw), dot));
-        const V8f gp = widen(grad(e, qh, c.mpt_nlam, ph)), gq = widen(grad(e, ph, c.mpt_nlam, qh));
-        V8f po, qo;
+        const Vf<N> gp = widen(grad(e, qh, c.mpt_nlam, ph)), gq = widen(grad(e, ph, c.mpt_nlam, qh));
+        Vf<N> po, qo;
         const float2 lr2 = make_float2(c.lr, c.lr), rev2 = make_float2(c.mpt_rev, c.mpt_rev);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
+        for (int j = 0; j < N / 2; j++) {
             set_pr(po, j, __ffma2_rn(lr2, __fmul2_rn(rev2, pr(gp, j)), pr(p, j)));
             set_pr(qo, j, __ffma2_rn(lr2, __fmul2_rn(rev2, pr(gq, j)), pr(q, j)));
         }
         put(p_raw, po); put(q_raw, qo);
     } else if constexpr (KIND == KIND_MUPPET) {
-        V8f p = as_v8f(p_raw), q = as_v8f(q_raw);
+        Vf<N> p = as_vf(p_raw), q = as_vf(q_raw);
         muppet_update<K>(c, __uint_as_float(rw), p, q, smp.gp, smp.gq, mid);
         put(p_raw, p); put(q_raw, q);
         if (STATS && c.bits != 32) smp.user = true;
     } else if constexpr (KIND == KIND_AFP) {
-        V8f p = as_v8f(p_raw), q = as_v8f(q_raw);
+        Vf<N> p = as_vf(p_raw), q = as_vf(q_raw);
         afp_update<K>(c, afp, __uint_as_float(rw), active, p, q);
         put(p_raw, p); put(q_raw, q);
     } else if constexpr (KIND == KIND_MEMQUANT) {
-        const V8f p = widen(as_v8h(p_raw)), q = widen(as_v8h(q_raw));
-        const float part = (K == 128) ? chain_partial_k128(p, q) : pair_partial(p, q);
-        const float e = __fsub_rn(__uint_as_float(rw), worker_sum<TS>(part, wmask, mid));
+        const Vf<N> p = widen(as_vh(p_raw)), q = widen(as_vh(q_raw));
+        float dot;
+        if constexpr (K == 64) dot = worker_dot<TS>(p, q, wmask, mid);
+        else if constexpr (N == 4) dot = worker_chain_k128<TS>(p, q, wmask, mid);
+        else dot = worker_sum<TS>(chain_partial_k128(p, q), wmask, mid);
+        const float e = __fsub_rn(__uint_as_float(rw), dot);
         put(p_raw, narrow(step(c.lr, grad(e, q, c.lam, p), p)));
         put(q_raw, narrow(step(c.lr, grad(e, p, c.lam, q), q)));
     } else {
         const bool uf = is_f32<UM>(uc), itf = is_f32<IM>(ic);
         auto both_half = [&]() {
-            const V8h p = as_v8h(p_raw), q = as_v8h(q_raw);
+            const Vh<N> p = as_vh(p_raw), q = as_vh(q_raw);
             __half2 dot;
-            if constexpr (kAhead) dot = worker_sum<TS>(pair_partial(p, q), wmask);
-            else dot = worker_sum<TS>(pair_partial(p, q), wmask, mid);
+            if constexpr (kAhead) dot = worker_dot<TS>(p, q, wmask);
+            else dot = worker_dot<TS>(p, q, wmask, mid);
             const __half2 e = __hsub2_rn(kHalfRating<KIND, UM, IM> ? half2_of(rw) : __float2half2_rn(__uint_as_float(rw)), dot);
-            const V8h gp = grad(e, q, c.nlam_h, p), gq = grad(e, p, c.nlam_h, q);
+            const Vh<N> gp = grad(e, q, c.nlam_h, p), gq = grad(e, p, c.nlam_h, q);
             put(p_raw, step(c.lr_h, gp, p));
             put(q_raw, step(c.lr_h, gq, q));
             if (STATS) { smp.gp = widen(gp); smp.gq = widen(gq); smp.user = true; smp.item = true; }
         };
         auto some_f32 = [&]() {
-            const V8f p = uf ? as_v8f(p_raw) : widen(as_v8h(p_raw));
-            const V8f q = itf ? as_v8f(q_raw) : widen(as_v8h(q_raw));
+            const Vf<N> p = uf ? as_vf(p_raw) : widen(as_vh(p_raw));
+            const Vf<N> q = itf ? as_vf(q_raw) : widen(as_vh(q_raw));
             float dot;
-            if constexpr (kAhead) dot = worker_sum<TS>(pair_partial(p, q), wmask);
-            else dot = worker_sum<TS>(pair_partial(p, q), wmask, mid);
+            if constexpr (kAhead) dot = worker_dot<TS>(p, q, wmask);
+            else dot = worker_dot<TS>(p, q, wmask, mid);
             const float e = __fsub_rn(__uint_as_float(rw), dot);
-            const V8f gp = grad(e, q, c.lam, p), gq = grad(e, p, c.lam, q);
-            const V8f po = step(c.lr, gp, p), qo = step(c.lr, gq, q);
+            const Vf<N> gp = grad(e, q, c.lam, p), gq = grad(e, p, c.lam, q);
+            const Vf<N> po = step(c.lr, gp, p), qo = step(c.lr, gq, q);
             if (uf) put(p_raw, po); else put(p_raw, narrow(po));
             if (itf) put(q_raw, qo); else put(q_raw, narrow(qo));
             if (STATS) { smp.gp = gp; smp.gq = gq; smp.user = !uf; smp.item = !itf; }
         };
-        if constexpr (UM == ROWS_HALF && IM == ROWS_HALF) both_half();
+        if constexpr (kHalfRows<UM> && kHalfRows<IM>) both_half();
         else if constexpr (UM != ROWS_DYN && IM != ROWS_DYN) some_f32();
         else { if (!uf && !itf) both_half(); else some_f32(); }
     }
@@ -934,23 +1092,27 @@ __device__ __forceinline__ uint4 lds128(unsigned addr) {
 // every lane (layout.cuh), so that neither the 128-bit shared-memory accesses of neighbouring lanes collide
 // on a bank nor the global accesses of a worker touch partial sectors.  `slot` includes the lane's 16 m.
 template <int K, int MODE>
+__device__ __forceinline__ void cp_row_if(unsigned slot, const Rows<K, MODE>& A, uint32_t code) {      // kNoRow: nothing
+    const unsigned char* g = A.at(code);
+    // copies are of 16 bytes: of binary16 rows the first half of the lanes fetches what both halves hold
+    if constexpr (MODE == ROWS_HALFQ) code = threadIdx.x & (K / 8) ? kNoRow : code;
+    cp16_if_row<0>(code, slot, g);
+    if constexpr (MODE == ROWS_F32) cp16_if_row<2 * K>(code, slot, g);
+    if constexpr (MODE == ROWS_DYN) cp16_if_row<2 * K>((code & kPrecBit) ? code : kNoRow, slot, g);
+}
+template <int K, int MODE>
 __device__ __forceinline__ void cp_row(unsigned slot, const Rows<K, MODE>& A, uint32_t code) {
+    if constexpr (MODE == ROWS_HALFQ) { cp_row_if<K, MODE>(slot, A, code); return; }
     const unsigned char* g = A.at(code);
     cp16<0>(slot, g);
     if constexpr (MODE == ROWS_F32) cp16<2 * K>(slot, g);                                   // second half of the row
     if constexpr (MODE == ROWS_DYN) cp16_if_row<2 * K>((code & kPrecBit) ? 0u : kNoRow, slot, g);
 }
 template <int K, int MODE>
-__device__ __forceinline__ void cp_row_if(unsigned slot, const Rows<K, MODE>& A, uint32_t code) {      // kNoRow: nothing
-    const unsigned char* g = A.at(code);
-    cp16_if_row<0>(code, slot, g);
-    if constexpr (MODE == ROWS_F32) cp16_if_row<2 * K>(code, slot, g);
-    if constexpr (MODE == ROWS_DYN) cp16_if_row<2 * K>((code & kPrecBit) ? code : kNoRow, slot, g);
-}
-template <int K, int MODE>
 __device__ __forceinline__ Raw<MODE> lds_row(unsigned slot, uint32_t code) {
     Raw<MODE> r;
-    r.a = lds128(slot);
+    if constexpr (MODE == ROWS_HALFQ) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.a.x), "=r"(r.a.y) : "r"(slot) : "memory");
+    else r.a = lds128(slot);
     if constexpr (MODE == ROWS_F32) r.b = lds128(slot + 2 * K);
     if constexpr (MODE == ROWS_DYN) { if (is_f32<MODE>(code)) r.b = lds128(slot + 2 * K); }
     return r;
@@ -964,16 +1126,15 @@ constexpr uint32_t F_IDUP = 4u;     // run start whose item also occurs shortly 
 constexpr uint32_t F_DROP = 8u;     // the user row is not written back (an update of a very popular user, or no rating at all)
 constexpr uint32_t F_NONE = 16u;    // there is no rating at this position
 
-constexpr int kSpan = 8;            // consecutive chunks handed out together (the longest run of one ticket)
 
 // Shared memory of one worker: two chunks of records, what to request while each of them is processed (8 bytes: the
 // user row of the rating D further on, the item row of the rating DI further on if a run starts there), then the user
 // ring, then the item ring.  A ring
 // slot is as large as the widest row its side can hold in this launch.
 template <int K, int UM, int IM, bool STATS, int NS, int NSI> struct WorkerSmem {
-    static constexpr int TS = K / 8;
-    static constexpr int kURowBytes = K * (UM == ROWS_HALF ? 2 : 4);
-    static constexpr int kIRowBytes = K * (IM == ROWS_HALF ? 2 : 4);
+    static constexpr int TS = K / kElems<UM>;
+    static constexpr int kURowBytes = K * (kHalfRows<UM> ? 2 : 4);
+    static constexpr int kIRowBytes = K * (kHalfRows<IM> ? 2 : 4);
     static constexpr int kRecBytes = 2 * TS * 16 + 2 * TS * 8;
     // The records of the workers of a warp are shifted by 16 bytes from worker to worker: those read at the same time
     // then lie in different banks.  The rings stay at multiples of 128 bytes (off them, copies and loads of rows touch
@@ -990,16 +1151,18 @@ template <int K, int UM, int IM, bool STATS, int NS, int NSI> struct WorkerSmem 
 // The lead is kept as short as the memory latency allows: an item row that another worker updates between the
 // request and the write-back loses that update, and the chance of that grows with the lead.
 template <int K, int KIND, int UM, int IM, bool STATS, int NS, int NSI, int D, int DI>
-__global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !STATS) ? 4 : ((UM == ROWS_DYN || STATS || KIND == KIND_AFP || KIND == KIND_MUPPET) ? 2 : 3)) train_kernel(const KernelArgs a) {
+__global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS) ? 4 : ((UM == ROWS_DYN || STATS || KIND == KIND_AFP || KIND == KIND_MUPPET) ? 2 : 3)) train_kernel(const KernelArgs a) {
     using SM = WorkerSmem<K, UM, IM, STATS, NS, NSI>;
     constexpr int TS = SM::TS;                     // lanes per worker = ratings per chunk
+    constexpr int N = kElems<UM>;                  // elements per lane
+    constexpr unsigned kSpan = K / TS;             // consecutive chunks handed out together: K ratings, the longest run of one ticket
     constexpr unsigned kAll = 0xffffffffu;
     static_assert(TS % NS == 0 && (NS & (NS - 1)) == 0 && (NSI & (NSI - 1)) == 0, "the rings must divide the chunk");
     static_assert(DI >= 1 && D >= 2 && DI <= D && D < NS && DI < NSI && NSI <= NS, "leads must fit the rings");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int m = lane % TS;
-    const unsigned gmask = ((1u << TS) - 1u) << (lane - m);      // the lanes of this worker
+    const unsigned gmask = (0xffffffffu >> (32 - TS)) << (lane - m);      // the lanes of this worker
     const unsigned W = a.workers;
     // AFP's workers may be alone in their warps (launch_ns); the other lanes then keep them company without work.
     constexpr bool kSpread = KIND == KIND_AFP;
@@ -1014,8 +1177,9 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     uint32_t* const reqs = reinterpret_cast<uint32_t*>(recs + 2 * TS);          // [2][TS][user, item]
     const unsigned s_rec = (unsigned)__cvta_generic_to_shared(recs);
     const unsigned s_req = s_rec + 2 * TS * 16;
-    const unsigned uring = (unsigned)__cvta_generic_to_shared(mine) + SM::kRecBytes + SM::kShift + 16 * m;      // [NS][kURowBytes]
-    const unsigned iring = uring + NS * SM::kURowBytes;                   // [NSI][kIRowBytes]
+    const unsigned rings = (unsigned)__cvta_generic_to_shared(mine) + SM::kRecBytes + SM::kShift;
+    const unsigned uring = rings + lane_at<K, UM>(m);                            // [NS][kURowBytes]
+    const unsigned iring = rings + NS * SM::kURowBytes + lane_at<K, IM>(m);      // [NSI][kIRowBytes]
     uint32_t* const groups = reinterpret_cast<uint32_t*>(mine + SM::kRecBytes + SM::kShift + NS * SM::kURowBytes + NSI * SM::kIRowBytes);
     constexpr bool kGroups = STATS && KIND == KIND_MIXED;
     const Rows<K, UM> P(a.P, m);
@@ -1051,7 +1215,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     const unsigned share_log2 = 32 - __clz(2 * W - 1);              // 2 W rounded up to a power of two
     auto run_length = [&](unsigned seen) -> unsigned {
         const unsigned g = (dyn_chunks > seen ? dyn_chunks - seen : 0) >> share_log2;
-        return min(max(g, 1u), (unsigned)kSpan);
+        return min(max(g, 1u), kSpan);
     };
     // lane 0 of a worker takes `len` chunks off the shared counter
     auto draw_ticket = [&](bool go, unsigned len) -> unsigned {
@@ -1150,19 +1314,25 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     uint32_t cur_ic = 0;
     unsigned have_item = 0;                          // F_RS while there is one
     Raw<IM> q = Raw<IM>();
-    if constexpr (kSpread) put(q, V8f{{0.01f, 0.01f, 0.01f, 0.01f, 0.01f, 0.01f, 0.01f, 0.01f}});
+    if constexpr (kSpread) {
+        Vf<N> harmless;
+#pragma unroll
+        for (int t = 0; t < N; t++) harmless.x[t] = 0.01f;
+        put(q, harmless);
+    }
 
     // item-side statistics of the current run of equal item groups
-    V8f gq_acc; float nq_acc = 0.f; uint32_t acc_group = kNoRow;
+    const int stat_at = N == 8 ? 8 * m : 8 * (m & (TS / 2 - 1)) + (m & (TS / 2) ? 4 : 0);      // the lane's first element in physical order
+    Vf<N> gq_acc; float nq_acc = 0.f; uint32_t acc_group = kNoRow;
 #pragma unroll
-    for (int t = 0; t < 8; t++) gq_acc.x[t] = 0.f;
+    for (int t = 0; t < N; t++) gq_acc.x[t] = 0.f;
     // this block's private set of accumulators (fewer workers per address, less serialisation)
     const size_t my_set = STATS ? (size_t)(blockIdx.x % (unsigned)a.st.copies) * a.st.copy_stride : 0;
     float* const gsum_p = a.st.gsum_p + my_set; float* const gsum_q = a.st.gsum_q + my_set;
     float* const nsum_p = a.st.nsum_p + my_set; float* const nsum_q = a.st.nsum_q + my_set;
     auto flush_item_stats = [&]() {
         if (acc_group != kNoRow) {
-            red_add8(gsum_q + (size_t)acc_group * K + 8 * m, gq_acc);
+            red_add(gsum_q + (size_t)acc_group * K + stat_at, gq_acc);
             if (m == 0) atomicAdd(nsum_q + acc_group, nq_acc);
         }
     };
@@ -1171,40 +1341,43 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     // norm of a rating goes through the worker's lanes during the next rating (`norm_step`), in the same order as at once.
     constexpr bool kWhole = STATS && (KIND == KIND_MUPPET || KIND == KIND_SWITCH);
     float norm = 0.f;
+    float4 norm_parts = make_float4(0.f, 0.f, 0.f, 0.f);      // with four elements a lane: what the first step joins
     auto norm_step = [&](int part) {
-        if (kWhole && (TS / 2) >> part) norm = __fadd_rn(norm, __shfl_xor_sync(kAll, norm, (TS / 2) >> part));
+        if (kWhole && N == 4 && part == 0) norm = muppet_norm_join<K>(norm_parts);
+        else if (kWhole && (TS / 2) >> part) norm = __fadd_rn(norm, __shfl_xor_sync(kAll, norm, (TS / 2) >> part));
     };
-    auto record_whole = [&](const Sample& smp, bool there) {
+    auto record_whole = [&](const Sample<N>& smp, bool there) {
         if (!smp.user) return;                                 // all ratings of a launch, or none
         nq_acc = __fadd_rn(nq_acc, norm);
-        norm = there ? muppet_norm_partial<K>(smp.gp, smp.gq) : 0.f;
+        if constexpr (N == 4) norm_parts = there ? muppet_norm_parts<K>(smp.gp, smp.gq) : make_float4(0.f, 0.f, 0.f, 0.f);
+        else norm = there ? muppet_norm_partial<K>(smp.gp, smp.gq) : 0.f;
         if (there) {
 #pragma unroll
-            for (int t = 0; t < 8; t++) gq_acc.x[t] = __fadd_rn(gq_acc.x[t], __fadd_rn(smp.gp.x[t], smp.gq.x[t]));
+            for (int t = 0; t < N; t++) gq_acc.x[t] = __fadd_rn(gq_acc.x[t], __fadd_rn(smp.gp.x[t], smp.gq.x[t]));
         }
     };
-    auto record = [&](const Sample& smp, uint32_t both_groups) {
+    auto record = [&](const Sample<N>& smp, uint32_t both_groups) {
         if (smp.user) {
             const uint32_t g = both_groups & 0xffffu;
-            const float n = worker_sum<TS>(pair_partial(smp.gp, smp.gp), gmask);
-            red_add8(gsum_p + (size_t)g * K + 8 * m, smp.gp);
+            const float n = worker_dot<TS>(smp.gp, smp.gp, gmask);
+            red_add(gsum_p + (size_t)g * K + stat_at, smp.gp);
             if (m == 0) atomicAdd(nsum_p + g, n);
         }
         if (smp.item) {
             const uint32_t g = both_groups >> 16;
-            const float n = worker_sum<TS>(pair_partial(smp.gq, smp.gq), gmask);
+            const float n = worker_dot<TS>(smp.gq, smp.gq, gmask);
             if (g != acc_group) {
                 flush_item_stats();
                 acc_group = g; nq_acc = 0.f;
 #pragma unroll
-                for (int t = 0; t < 8; t++) gq_acc.x[t] = 0.f;
+                for (int t = 0; t < N; t++) gq_acc.x[t] = 0.f;
             }
 #pragma unroll
-            for (int t = 0; t < 8; t++) gq_acc.x[t] = __fadd_rn(gq_acc.x[t], smp.gq.x[t]);
+            for (int t = 0; t < N; t++) gq_acc.x[t] = __fadd_rn(gq_acc.x[t], smp.gq.x[t]);
             nq_acc = __fadd_rn(nq_acc, n);
         }
     };
-    Sample smp;
+    Sample<N> smp;
     AfpState afp;
     afp.user = AfpSide{8, 1.f, 0.f, 0}; afp.item = afp.user; afp.back = afp.user; afp.cur = 0;
 
@@ -1214,6 +1387,16 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
         else cp_row<K, UM>(uring + slot * SM::kURowBytes, P, uc);
     };
     auto request_item = [&](uint32_t ic, int slot) { cp_row_if<K, IM>(iring + slot * SM::kIRowBytes, Q, ic); };
+    // Binary16 rows over K/4 lanes: copies are of 16 bytes, so the first half of the lanes fetches the user row and the second
+    // half the item row, with one instruction.
+    constexpr bool kOneRequest = UM == ROWS_HALFQ && IM == ROWS_HALFQ;
+    const bool second = m & (TS / 2);
+    const unsigned char* const one_base = reinterpret_cast<const unsigned char*>(second ? a.Q.f16 : a.P.f16) + 16 * (m & (TS / 2 - 1));
+    const unsigned one_ring = rings + (second ? NS * SM::kURowBytes : 0) + 16 * (m & (TS / 2 - 1));
+    auto request_one = [&](uint32_t uc, int uslot, uint32_t ic, int islot) {
+        const uint32_t code = second ? ic : uc;
+        cp16_if_row<0>(code, one_ring + (second ? islot * SM::kIRowBytes : uslot * SM::kURowBytes), one_base + (uint64_t)code * (2u * K));
+    };
     // Copy groups complete in order, and every rating commits one: the item row of the rating DI ahead and the user
     // row of the rating D ahead.  Before rating j commits, the groups younger than the user row of rating j+1 are
     // D - 2, those younger than the item row of rating j are DI - 1: waiting for exactly that many to remain
@@ -1249,7 +1432,7 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
                     st_row_if<K, IM>(start & have_item, Q, cur_ic, q);
                     const unsigned slot = iring + (t & (NSI - 1)) * SM::kIRowBytes;
                     lds_if<0>(start, q.a, slot);
-                    if constexpr (IM != ROWS_HALF) lds_if<2 * K>(second_half<IM>(start, ic), q.b, slot);
+                    if constexpr (kTwoParts<IM>) lds_if<2 * K>(second_half<IM>(start, ic), q.b, slot);
                     if (__any_sync(kAll, f & (F_IDUP | F_UDUP))) {
                         ld_row_if<K, IM>(f & F_IDUP, q, Q, ic);
                         ld_row_if<K, UM>(f & F_UDUP, p, P, uc);
@@ -1268,8 +1451,11 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
                         cp_wait<D - 2>();
                         p_next = lds_row<K, UM>(uring + ((t + 1) & (NS - 1)) * SM::kURowBytes, rec.z);
                     } else if (part == 2) {
-                        request_item(req_i, (t + DI) & (NSI - 1));
-                        request_user(req_u, (t + D) & (NS - 1));
+                        if constexpr (kOneRequest) request_one(req_u, (t + D) & (NS - 1), req_i, (t + DI) & (NSI - 1));
+                        else {
+                            request_item(req_i, (t + DI) & (NSI - 1));
+                            request_user(req_u, (t + D) & (NS - 1));
+                        }
                         cp_commit();
                         turn = __any_sync(kAll, rec.x & (F_RS | F_UDUP));
                     }
@@ -1292,8 +1478,10 @@ __global__ void __launch_bounds__(256, (UM == ROWS_HALF && IM == ROWS_HALF && !S
     st_row_if<K, IM>(have_item, Q, cur_ic, q);
     if (STATS) {
         if constexpr (kWhole) {
-            nq_acc = __fadd_rn(nq_acc, worker_sum<TS>(norm, kAll));
-            red_add8(gsum_p + 8 * m, gq_acc);
+            // the norm of the last rating
+            if constexpr (N == 4) nq_acc = __fadd_rn(nq_acc, worker_sum<TS / 2>(muppet_norm_join<K>(norm_parts), kAll));
+            else nq_acc = __fadd_rn(nq_acc, worker_sum<TS>(norm, kAll));
+            red_add(gsum_p + stat_at, gq_acc);
             if (m == 0) atomicAdd(nsum_p, nq_acc);
         }
         else flush_item_stats();
@@ -1310,7 +1498,7 @@ __global__ void reduce_stats_kernel(float* sets, int copies, size_t stride, size
 
 template <int K, int KIND, int UM, int IM, bool STATS, int NS, int NSI, int D, int DI>
 cudaError_t launch_ns(KernelArgs a, unsigned warps_per_sm, unsigned workers, cudaStream_t st, LaunchShape* shape, bool dry) {
-    constexpr int TS = K / 8;
+    constexpr int TS = K / kElems<UM>;
     constexpr int kPerWarp = 32 / TS;
     using SM = WorkerSmem<K, UM, IM, STATS, NS, NSI>;
     auto kern = train_kernel<K, KIND, UM, IM, STATS, NS, NSI, D, DI>;
@@ -1320,7 +1508,7 @@ cudaError_t launch_ns(KernelArgs a, unsigned warps_per_sm, unsigned workers, cud
     int grid, block;
     unsigned warps = (workers + kPerWarp - 1) / kPerWarp;
     // The workers of an AFP warp compute both passes whenever their formats differ, so few of them are spread over more
-    // warps, up to two per scheduler (4M ratings, 592 workers: 6.75 ms per epoch with two workers a warp, 5.78 with one).
+    // warps, up to two per scheduler (K/8 lanes, 4M ratings, 592 workers: 6.75 ms per epoch with two workers a warp, 5.78 with one).
     // For the other trainers a second warp on a scheduler costs more than it gives: MPT 1.81 ms spread out 2.21, MASCOT
     // 1.30 and 1.49, MuPPET 3.00 and 3.12.
     constexpr unsigned kSpreadWarps = KIND == KIND_AFP ? 8 : 0;
@@ -1399,6 +1587,22 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
     // are three to four times as long, and for them three and two are enough.
     constexpr bool kFixedPoint = KIND == KIND_AFP || KIND == KIND_MUPPET;
     constexpr int NS = kFixedPoint ? 4 : 8, D = kFixedPoint ? 3 : 5, DI = kFixedPoint ? 2 : 3;
+    // A step of few warps is a chain of some ninety instructions.  With K/4 lanes a worker the warp has half of the row work
+    // and one worker fewer to wait for: shorter steps, on twice as many warps - as long as the schedulers can take those.  ms per
+    // epoch with K/8 and K/4 lanes, by warps of the narrow form per SM: AFP 4M ratings (4) 5.69 and 4.43, 12M (10) 8.94 and 6.30; MuPPET
+    // 2M (4) 2.25 and 1.71, 14M (12) 5.73 and 5.04; MPT 8M (8) 1.81 and 1.50, 16M (14) 2.39 and 2.13; SGD 8M (8) 1.52 and 1.31, 16M (14)
+    // 2.08 and 2.05, k=64 0.8M (6) 0.132 and 0.105, 20M (10) 2.04 and 1.69; fp16 storage 8M 1.64 and 1.47, 16M (14) 2.13 and 2.04; MASCOT
+    // k=64 8M (4) 1.44 and 1.23, 20M (10) 1.56 and 1.45, 30M (14) 1.73 and 1.70, 40 % promoted, 16M (14) 3.67 and 3.57.  At 18 and more
+    // the narrow form gives nothing more (SGD 20M 2.45 and 2.46) or loses (fp16 storage 20M 2.08 and 2.23).  Binary16 rows
+    // with packed binary16 arithmetic have the shortest steps and stop gaining earlier: k=128, 2M (4) 0.637 and 0.590, 6M (6) 1.28
+    // and 1.255, 8M (8) 1.302 and 1.300, 20M (18) 1.68 and 1.94.
+    if constexpr (UM != ROWS_DYN) {
+        constexpr int UQ = UM == ROWS_HALF ? ROWS_HALFQ : ROWS_F32Q, IQ = IM == ROWS_HALF ? ROWS_HALFQ : ROWS_F32Q;
+        constexpr unsigned kMost = K == 128 && kHalfRating<KIND, UM, IM> && KIND != KIND_MPT && !STATS ? 8 : 16;      // warps per SM
+        // (a single block has exactly the workers that were asked for: they have to fit it in this form, too)
+        if (2 * per_sm <= kMost && (warps > 8 || 2 * workers <= 8 * kPerWarp))
+            return launch_ns<K, KIND, UQ, IQ, STATS, NS, 4, D, DI>(args, 2 * per_sm, workers, st, shape, dry);
+    }
     // With fp32 rows the deep rings leave room for fewer warps than the registers do (k=128, both sides fp32: 16 per SM
     // against 24).  The mixed-precision classes with an fp32 side want those warps: where a launch asks for more workers
     // than the deep rings hold and rings of 4 + 2 slots hold more, it takes these, three ratings and one ahead.  Per epoch,

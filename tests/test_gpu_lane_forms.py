@@ -1,0 +1,73 @@
+"""Workers of K/4 lanes (four elements each) and of K/8 lanes (eight), on both sides of the launch rule: ratings few enough for
+the first run of one worker, in which rows come back at once, so that the sequential oracle has every bit of the result
+and of the sampled statistics."""
+import numpy as np
+import pytest
+
+from helpers import assert_bit_equal, random_problem
+from test_gpu_update_edges import oracle_epoch, promoted_model
+
+pytestmark = pytest.mark.gpu
+
+# workers -> form: 1 to 8 (k=64: 16) of a single block and a few warps per SM are narrow; 9 to 16 (17 to 32), which fit a single block of
+# the wide form only, and a full GPU are wide
+WORKERS = (2, 8, 12, 16, 31, 300, 60000)
+
+
+@pytest.mark.parametrize("k", (128, 64))
+@pytest.mark.parametrize("workers", WORKERS)
+@pytest.mark.parametrize("version", ["sgd", "mpt", "memquant", "muppet8", "muppet12", "muppet32", "afp"])
+def test_both_lane_forms_follow_the_oracle(mascot, oracle, k, workers, version):
+    for n_users, n_items, n in ((1, 1, 9), (3, 2, k // 2 + 1), (17, 5, k)):
+        R, P, Q = random_problem(np.random.default_rng(n + n_users), n_users, n_items, n, k, scale=0.2)
+        muppet = version.startswith("muppet")
+        v = dict(sgd=mascot.V_SGD, mpt=mascot.V_MPT, memquant=mascot.V_MEMQUANT, afp=mascot.V_AFP).get(version, mascot.V_MUPPET)
+        width = int(version[6:]) if muppet else 0
+        cfg = mascot.default_config(version=v, k=k, num_workers=workers, plain_user_stores=1, shuffle=0, epoch=50, learning_rate=0.01, decay=0.1, lam=0.05,
+                                    muppet_width=width, sample_ratio=0.3)
+        with mascot.Engine(cfg) as eng:
+            eng.set_ratings(R, R[:1], n_users, n_items)
+            eng.set_factors(P, Q)
+            w = eng.train_epoch(0).workers
+            Pg, Qg = eng.get_factors(0)
+            gp, _, norms, _ = eng.sample_stats()
+        rules = oracle.rules_reference()
+        if muppet:
+            first = n - int(np.float32(n) * np.float32(0.3))
+            sums, norm = oracle.muppet_run(k, R, None, P, Q, float(np.float32(0.01)), 0.05, width, width, rules, first_sample_pos=first)
+            if width != 32:
+                assert_bit_equal(gp[:k], sums, "sum of gradients")
+                assert_bit_equal(norms[:1], np.float32(norm), "sum of norms")
+        elif version == "afp":
+            oracle.afp_run(k, R, None, P, Q, 0.01, 0.05, 0, int(np.float32((n + w - 1) // w) / np.float32(10.0)), rules)
+        else:
+            P, Q = oracle_epoch(oracle, version, k, R, P, Q, 0.01, 0.05)
+        assert_bit_equal(Pg, P, f"n {n} P")
+        assert_bit_equal(Qg, Q, f"n {n} Q")
+
+
+@pytest.mark.parametrize("k", (128, 64))
+@pytest.mark.parametrize("workers", WORKERS)
+@pytest.mark.parametrize("users,items", [(False, False), (True, True), (True, False), (False, True)])
+def test_both_lane_forms_of_the_precision_classes(mascot, oracle, k, workers, users, items):
+    for n_users, n_items, n in ((1, 1, 9), (3, 2, k // 2 + 1), (17, 5, k)):
+        R, P, Q = random_problem(np.random.default_rng(n + n_users), n_users, n_items, n, k, scale=0.2)
+        cfg = mascot.default_config(version=mascot.V_MASCOT, k=k, num_workers=workers, plain_user_stores=1, shuffle=0, epoch=50, learning_rate=0.01, decay=0.1,
+                                    lam=0.05, user_group_num=1, item_group_num=1, sample_ratio=0.3, interval=1, error_threshold=1e30)
+        with mascot.Engine(cfg) as eng:
+            eng.set_ratings(R, R[:1], n_users, n_items)
+            eng.set_factors(P, Q)
+            model, u2s, i2s = promoted_model(oracle, mascot, eng, k, P, Q, users, items)
+            assert eng.train_epoch(5).error_check
+            Pg, Qg = eng.get_factors(1)
+            got = eng.sample_stats()
+        Rs = R.copy()
+        Rs["u"], Rs["i"] = u2s[R["u"]], i2s[R["i"]]
+        lr = float(oracle.lr_schedule(0.01, 0.1, 50)[5])
+        first = n - int(np.float32(n) * np.float32(0.3))
+        want = model.run(Rs, None, lr, 0.05, oracle.rules_reference(), first_sample_pos=first, stats=True, item_stats_by_run=True)
+        for a, b, what in zip(got, want, ("gsum_p", "gsum_q", "nsum_p", "nsum_q")):
+            assert_bit_equal(a, b, f"n {n} {what}")
+        Po, Qo = model.factors()
+        assert_bit_equal(Pg, Po, f"n {n} P")
+        assert_bit_equal(Qg, Qo, f"n {n} Q")
