@@ -77,6 +77,10 @@ namespace {
 
 constexpr uint32_t kNoRow = 0xffffffffu;     // never a valid stream id
 
+// MuPPET's trainer is three kernels: passes of 8 bits (KIND_MUPPET), of 12 to 16 bits (this one), and the fp32 trainer's at 32
+constexpr int kMuppetHalf = 100;
+template <int KIND> constexpr bool kMuppet = KIND == KIND_MUPPET || KIND == kMuppetHalf;
+
 template <int N> struct Vh { __half2 v[N / 2]; };      // a lane's values, physical order
 template <int N> struct Vf { float x[N]; };
 typedef Vh<8> V8h;
@@ -535,12 +539,6 @@ template <int N> __device__ __forceinline__ Vf<N> quantize_away(const Vf<N>& x, 
     for (int t = 0; t < N; t++) o.x[t] = __fadd_rn(round_away(__fmul_rn(x.x[t], s)), 0.f);
     return o;
 }
-template <int N> __device__ __forceinline__ void quantize(const Vf<N>& p, float sp, const Vf<N>& q, float sq, Vf<N>& pi, Vf<N>& qi, unsigned wmask) {
-    float odd_p, odd_q;
-    pi = quantize_near(p, sp, odd_p);
-    qi = quantize_near(q, sq, odd_q);
-    if (__any_sync(wmask, !(fmaxf(odd_p, odd_q) < 0.5f))) { pi = quantize_away(p, sp); qi = quantize_away(q, sq); }
-}
 // The int8 passes work on the integers as floats: products and sums of int8 values stay far below 2^24.
 __device__ __forceinline__ float clamp8(float v) { return v == v ? fminf(fmaxf(v, -128.f), 127.f) : 0.f; }
 template <int N> __device__ __forceinline__ Vf<N> clamp8(const Vf<N>& x) {
@@ -549,15 +547,8 @@ template <int N> __device__ __forceinline__ Vf<N> clamp8(const Vf<N>& x) {
     for (int t = 0; t < N; t++) o.x[t] = clamp8(x.x[t]);
     return o;
 }
-// quantize() to int8 values; `outside`: may some value leave their range?
-template <int N> __device__ __forceinline__ void quantize_int8(const Vf<N>& p, float sp, const Vf<N>& q, float sq, bool outside, Vf<N>& pi, Vf<N>& qi, unsigned wmask) {
-    float odd_p, odd_q;
-    pi = quantize_near(p, sp, odd_p);
-    qi = quantize_near(q, sq, odd_q);
-    if (__any_sync(wmask, outside || !(fmaxf(odd_p, odd_q) < 0.5f))) { pi = clamp8(quantize_away(p, sp)); qi = clamp8(quantize_away(q, sq)); }
-}
 __device__ __forceinline__ float quantize8(float v, float s) { return clamp8(round_away(__fmul_rn(v, s))); }
-// A quantize()d row in binary16; what rounded to zero keeps its sign, as it does in fix_round
+// A rounded row in binary16; what rounded to zero keeps its sign, as it does in fix_round
 template <int N> __device__ __forceinline__ Vh<N> grid_half(const Vf<N>& r, const Vf<N>& x, float s_rev) {
     Vh<N> h;
     const float2 rev2 = make_float2(s_rev, s_rev);
@@ -574,11 +565,11 @@ template <int N> __device__ __forceinline__ Vh<N> fix_round_half(const Vf<N>& x,
         h.v[t] = __floats2half2_rn(fix_round(x.x[2 * t], s, s_rev), fix_round(x.x[2 * t + 1], s, s_rev));
     return h;
 }
-// Both quantize()d rows on their grids; `big`: some value may reach 2^21 steps of its grid
+// Both rounded rows on their grids; `big`: some value may reach 2^21 steps of its grid
 template <int N>
-__device__ __forceinline__ void to_grid(const Vf<N>& p, const Vf<N>& pi, float sp, const Vf<N>& q, const Vf<N>& qi, float sq, bool big, Vh<N>& ph, Vh<N>& qh) {
-    const float sp_rev = pow2_rev(sp), sq_rev = pow2_rev(sq);
-    if (big) { ph = fix_round_half(p, sp, sp_rev); qh = fix_round_half(q, sq, sq_rev); }
+__device__ __forceinline__ void to_grid(const Vf<N>& p, const Vf<N>& pi, float sp, float sp_rev, const Vf<N>& q, const Vf<N>& qi, float sq, float sq_rev, bool big,
+                                        Vh<N>& ph, Vh<N>& qh) {
+    if (__builtin_expect(big, 0)) { ph = fix_round_half(p, sp, sp_rev); qh = fix_round_half(q, sq, sq_rev); }
     else { ph = grid_half(pi, p, sp_rev); qh = grid_half(qi, q, sq_rev); }
 }
 template <int N> __device__ __forceinline__ float abs_max(const Vf<N>& x) {
@@ -646,15 +637,15 @@ __device__ __forceinline__ float muppet_norm_partial(const V8f& gp, const V8f& g
 
 // ---- passes shared by MuPPET and AFP ------------------------------------------------------------
 // int8 forward pass: saturated fixed-point values, exact integer dot product, one division (by a power of two).
-// pi, qi: quantize()d rows, clamped if need be.  A lane's sum stays below 2^18, the whole one below 2^22, so both pass
+// pi, qi: rounded rows, clamped if need be; rev: 1 / (product of their scales).  A lane's sum stays below 2^18, the whole one below 2^22, so both pass
 // between integer and float in the low bits of 1.5 * 2^23 + x.
 template <int TS, int N>
-__device__ __forceinline__ float forward_int8(const Vf<N>& pi, const Vf<N>& qi, float sp, float sq) {
+__device__ __forceinline__ float forward_int8(const Vf<N>& pi, const Vf<N>& qi, float rev) {
     float2 a = make_float2(0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < N / 2; j++) a = __ffma2_rn(pr(pi, j), pr(qi, j), a);
     const int whole = worker_add<TS>(__float_as_int(__fadd_rn(__fadd_rn(a.x, a.y), 12582912.f)) - 0x4b400000);
-    return __fmul_rn(__fsub_rn(__int_as_float(whole + 0x4b400000), 12582912.f), pow2_rev(__fmul_rn(sp, sq)));
+    return __fmul_rn(__fsub_rn(__int_as_float(whole + 0x4b400000), 12582912.f), rev);
 }
 // binary16 forward pass on the fixed-point grid; the two halves of the reference's half2 accumulator
 // go through the lane tree separately and meet at the end (muppet_sgd_kernel.h:170-194,
@@ -702,9 +693,9 @@ __device__ __forceinline__ float forward_half(const Vh<4>& ph, const Vh<4>& qh, 
     xy = __hadd2_rn(K == 128 ? from(xy, low) : xy, last);
     return __half2float(__hadd_rn(__low2half(xy), __high2half(xy)));
 }
-// backward passes: g_p = q*e + p*(-lam), g_q = p*e + q*(-lam) in int8 or binary16 fixed point
-template <int N> __device__ __forceinline__ void backward_int8(const Vf<N>& pi, const Vf<N>& qi, float ruv, float nlam, float sb, Vf<N>& gp, Vf<N>& gq) {
-    const float rev = pow2_rev(__fmul_rn(sb, sb)), e = quantize8(ruv, sb), l = quantize8(nlam, sb);
+// backward passes: g_p = q*e + p*(-lam), g_q = p*e + q*(-lam) in int8 or binary16 fixed point; l, l2: -lam on the grid, rev: 1 / (sb sb)
+template <int N> __device__ __forceinline__ void backward_int8(const Vf<N>& pi, const Vf<N>& qi, float ruv, float l, float sb, float rev, Vf<N>& gp, Vf<N>& gq) {
+    const float e = quantize8(ruv, sb);
     const float2 rev2 = make_float2(rev, rev), e2 = make_float2(e, e), l2 = make_float2(l, l), zero = make_float2(0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < N / 2; j++) {      // + 0: the integer sum has no negative zero
@@ -712,10 +703,8 @@ template <int N> __device__ __forceinline__ void backward_int8(const Vf<N>& pi, 
         set_pr(gq, j, __ffma2_rn(__ffma2_rn(pr(pi, j), e2, __fmul2_rn(pr(qi, j), l2)), rev2, zero));
     }
 }
-template <int N> __device__ __forceinline__ void backward_half(const Vh<N>& ph, const Vh<N>& qh, float ruv, float nlam, float sb, Vf<N>& gp, Vf<N>& gq) {
-    const float sb_rev = pow2_rev(sb);
+template <int N> __device__ __forceinline__ void backward_half(const Vh<N>& ph, const Vh<N>& qh, float ruv, __half2 l2, float sb, float sb_rev, Vf<N>& gp, Vf<N>& gq) {
     const __half2 e2 = __half2half2(__float2half_rn(fix_round(ruv, sb, sb_rev)));
-    const __half2 l2 = __half2half2(__float2half_rn(fix_round(nlam, sb, sb_rev)));
     Vh<N> gph, gqh;
 #pragma unroll
     for (int t = 0; t < N / 2; t++) {
@@ -746,39 +735,40 @@ template <int TS> __device__ __noinline__ float muppet_back_scale_exact(int bits
 // hundred workers that chain is the epoch, so what shortens it counts: keys in place of four extremes, warp-wide
 // integer reductions in place of shuffles, one vote a pass, the norm of the rating before on the side.  2M ratings, 592
 // workers: 2.98 -> 2.25 ms per epoch.
-template <int K, int N, class Mid>
+// A pass has one vote: is there a scale that the keys leave open, an exact half, a value outside the int8 range (or at 2^21
+// steps of its grid)?  The rows are rounded with the scale of the keys before that is known, and again where it is so.
+// INT8: passes of 8 bits; else 12 to 16 bits on a binary16 grid.
+template <int K, bool INT8, int N, class Mid>
 __device__ __forceinline__ void muppet_update(const Consts& c, float r, Vf<N>& p, Vf<N>& q, Vf<N>& gp, Vf<N>& gq, Mid mid) {
     constexpr int TS = K / N;
     constexpr unsigned kAll = 0xffffffffu;
-    const int bits = c.bits;
+    const int bits = INT8 ? 8 : c.bits;
     const float nlam = -c.lam;
-    if (bits == 32) {
-        const float ruv = __fsub_rn(r, worker_dot<TS>(p, q, kAll, mid));
-        gp = grad(ruv, q, c.lam, p); gq = grad(ruv, p, c.lam, q);
-        p = step(c.lr, gp, p); q = step(c.lr, gq, q);
-        return;
-    }
     const int2 bound = scale_bounds(bits);
     const float phi = max_of(p), plo = min_of(p), qhi = max_of(q), qlo = min_of(q);
     mid(0);
     const int kp = worker_min<TS>(scale_key(bound, phi, plo)), kq = worker_min<TS>(scale_key(bound, qhi, qlo));
     mid(1);
-    float sp = scale_of(kp), sq = scale_of(kq);
-    if (__any_sync(kAll, scale_unsure(bound, kp) || scale_unsure(bound, kq))) {
-        const float2 s = muppet_scales_exact<TS>(bits, phi, plo, qhi, qlo);
-        sp = s.x; sq = s.y;
+    float sp = scale_of(kp), sq = scale_of(kq), odd_p, odd_q;
+    Vf<N> pi = quantize_near(p, sp, odd_p), qi = quantize_near(q, sq, odd_q);
+    auto outside = [](float hi, float lo, float s) { return INT8 ? outside8(hi, lo, s) : beyond_grid(hi, lo, s); };
+    bool big = false;
+    if (__builtin_expect(__any_sync(kAll, scale_unsure(bound, kp) || scale_unsure(bound, kq) || outside(phi, plo, sp) || outside(qhi, qlo, sq)
+                                          || !(fmaxf(odd_p, odd_q) < 0.5f)), 0)) {
+        if (__any_sync(kAll, scale_unsure(bound, kp) || scale_unsure(bound, kq))) {
+            const float2 s = muppet_scales_exact<TS>(bits, phi, plo, qhi, qlo);
+            sp = s.x; sq = s.y;
+        }
+        pi = quantize_away(p, sp); qi = quantize_away(q, sq);
+        if (INT8) { pi = clamp8(pi); qi = clamp8(qi); }
+        else big = beyond_grid(phi, plo, sp) || beyond_grid(qhi, qlo, sq);
     }
-    Vf<N> pi, qi;
+    mid(2);
     Vh<N> ph, qh;
     float pred;
-    if (bits == 8) {
-        quantize_int8(p, sp, q, sq, outside8(phi, plo, sp) || outside8(qhi, qlo, sq), pi, qi, kAll);
-        mid(2);
-        pred = forward_int8<TS>(pi, qi, sp, sq);
-    } else {
-        quantize(p, sp, q, sq, pi, qi, kAll);
-        mid(2);
-        to_grid(p, pi, sp, q, qi, sq, beyond_grid(phi, plo, sp) || beyond_grid(qhi, qlo, sq), ph, qh);
+    if constexpr (INT8) pred = forward_int8<TS>(pi, qi, pow2_rev(__fmul_rn(sp, sq)));
+    else {
+        to_grid(p, pi, sp, pow2_rev(sp), q, qi, sq, pow2_rev(sq), big, ph, qh);
         pred = forward_half<K>(ph, qh, kAll);
     }
     mid(3);
@@ -786,16 +776,20 @@ __device__ __forceinline__ void muppet_update(const Consts& c, float r, Vf<N>& p
     const float hi = fmaxf(phi, qhi), lo = fminf(plo, qlo);
     const int kb = min(min(kp, kq), scale_key(bound, fmaxf(nlam, ruv), fminf(nlam, ruv)));
     float sb = scale_of(kb);
-    if (__any_sync(kAll, scale_unsure(bound, kb))) sb = muppet_back_scale_exact<TS>(bits, hi, lo, nlam, ruv);
-    if (bits == 8) {
-        quantize_int8(p, sb, q, sb, outside8(hi, lo, sb), pi, qi, kAll);
-        mid(4);
-        backward_int8(pi, qi, ruv, nlam, sb, gp, gq);
-    } else {
-        quantize(p, sb, q, sb, pi, qi, kAll);
-        mid(4);
-        to_grid(p, pi, sb, q, qi, sb, beyond_grid(hi, lo, sb), ph, qh);
-        backward_half(ph, qh, ruv, nlam, sb, gp, gq);
+    pi = quantize_near(p, sb, odd_p); qi = quantize_near(q, sb, odd_q);
+    big = false;
+    if (__builtin_expect(__any_sync(kAll, scale_unsure(bound, kb) || outside(hi, lo, sb) || !(fmaxf(odd_p, odd_q) < 0.5f)), 0)) {
+        if (__any_sync(kAll, scale_unsure(bound, kb))) sb = muppet_back_scale_exact<TS>(bits, hi, lo, nlam, ruv);
+        pi = quantize_away(p, sb); qi = quantize_away(q, sb);
+        if (INT8) { pi = clamp8(pi); qi = clamp8(qi); }
+        else big = beyond_grid(hi, lo, sb);
+    }
+    mid(4);
+    if constexpr (INT8) backward_int8(pi, qi, ruv, quantize8(nlam, sb), sb, pow2_rev(__fmul_rn(sb, sb)), gp, gq);
+    else {
+        const float sb_rev = pow2_rev(sb);
+        to_grid(p, pi, sb, sb_rev, q, qi, sb, sb_rev, big, ph, qh);
+        backward_half(ph, qh, ruv, __half2half2(__float2half_rn(fix_round(nlam, sb, sb_rev))), sb, sb_rev, gp, gq);
     }
     p = step(c.lr, gp, p); q = step(c.lr, gq, q);
 }
@@ -804,7 +798,15 @@ __device__ __forceinline__ void muppet_update(const Consts& c, float r, Vf<N>& p
 // One side's quantization parameters and the rating count at which they are estimated next.  The
 // reference keeps three of these per warp for a whole kernel launch; here per worker.
 struct AfpSide { int n; float scale; float mov_avg; long long next; };
-struct AfpState { AfpSide user, item, back; long long cur; };
+// Parameters change once in many ratings, so what follows from them is kept beside them.
+struct AfpState {
+    AfpSide user, item, back;
+    unsigned cur;                             // ratings of this worker so far
+    unsigned due;                             // ratings until one of the warp's workers estimates a parameter again
+    bool forward16, forward8, back16, back8;  // passes that some worker of the warp needs
+    float user_rev, item_rev, both_rev, back_rev, back2_rev, lam8;      // 1 / scales and products of two; -lam on the int8 grid
+    __half2 lam16;                            // -lam on the binary16 grid
+};
 
 // log2 in double precision, rounded once to float: the CPU restatement computes it the same way, so
 // both take identical re-estimation decisions (it runs only when parameters are re-estimated).
@@ -927,15 +929,17 @@ __device__ __noinline__ AfpSide afp_requantize(AfpSide s, float diff, float rang
 }
 // The workers of a warp go through this together: what one of them needs (a re-estimation, the int8 or the binary16
 // pass) all of them compute, and each keeps the result if it is its own case.  active: is there a rating?
+// What passes there are and when the next estimate is due only changes with an estimate, so a rating without one has two votes: is
+// there an exact half, or a value outside the int8 range (2^21 steps of the grid)?
 template <int K, int N>
 __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float r, bool active, Vf<N>& p, Vf<N>& q) {
     constexpr int TS = K / N;
     constexpr unsigned kAll = 0xffffffffu;
-    const long long cur = st.cur;
-    const bool new_user = active && cur == st.user.next, new_item = active && cur == st.item.next, new_back = active && cur == st.back.next;
-    const bool estimate = __any_sync(kAll, new_user || new_item || new_back);
+    const unsigned cur = st.cur;
+    const bool estimate = st.due == 0;
     float pmax = 0.f, qmax = 0.f;
-    if (estimate) {
+    if (__builtin_expect(estimate, 0)) {
+        const bool new_user = active && cur == st.user.next, new_item = active && cur == st.item.next;
         pmax = worker_max<TS>(abs_max(p), kAll);
         qmax = worker_max<TS>(abs_max(q), kAll);
         if (__any_sync(kAll, new_user)) {
@@ -946,42 +950,69 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
             const AfpSide s = afp_requantize(st.item, afp_qem<K>(eight<K>(q), qmax, kAll), qmax, cur, c.afp_epoch, c.afp_init_threshold);
             if (new_item) st.item = s;
         }
+        const bool mine8 = st.user.n == 8 && st.item.n == 8;
+        st.forward16 = __any_sync(kAll, active && !mine8);
+        st.forward8 = !st.forward16 || __any_sync(kAll, active && mine8);
+        st.user_rev = pow2_rev(st.user.scale); st.item_rev = pow2_rev(st.item.scale);
+        st.both_rev = pow2_rev(__fmul_rn(st.user.scale, st.item.scale));
     }
     // The formats are those of an earlier rating, so values may lie outside their range at any time.
-    const bool forward8 = st.user.n == 8 && st.item.n == 8;
-    float pred = 0.f;
-    Vf<N> pi, qi;
+    float pred = 0.f, odd_p, odd_q;
+    Vf<N> pi = quantize_near(p, st.user.scale, odd_p), qi = quantize_near(q, st.item.scale, odd_q);
     Vh<N> ph, qh;
-    quantize(p, st.user.scale, q, st.item.scale, pi, qi, kAll);
-    float most = fmaxf(abs_max(pi), abs_max(qi));
-    if (__any_sync(kAll, active && !forward8)) {
-        to_grid(p, pi, st.user.scale, q, qi, st.item.scale, __any_sync(kAll, !(most < 2097152.f)), ph, qh);
+    bool big = false, clamp = false;
+    auto check = [&](float sp, float sq, bool some8) {
+        float most = fmaxf(abs_max(pi), abs_max(qi));
+        if (__builtin_expect(__any_sync(kAll, !(fmaxf(odd_p, odd_q) < 0.5f) || !(most <= (some8 ? 127.f : 2097151.f))), 0)) {
+            pi = quantize_away(p, sp); qi = quantize_away(q, sq);
+            most = fmaxf(abs_max(pi), abs_max(qi));
+            big = __any_sync(kAll, !(most < 2097152.f));
+            clamp = __any_sync(kAll, !(most <= 127.f));
+        }
+    };
+    check(st.user.scale, st.item.scale, st.forward8);
+    if (st.forward16) {
+        to_grid(p, pi, st.user.scale, st.user_rev, q, qi, st.item.scale, st.item_rev, big, ph, qh);
         pred = forward_half<K>(ph, qh, kAll);
     }
-    if (__any_sync(kAll, active && forward8)) {
-        if (__any_sync(kAll, !(most <= 127.f))) { pi = clamp8(pi); qi = clamp8(qi); }
-        const float whole = forward_int8<TS>(pi, qi, st.user.scale, st.item.scale);
-        if (forward8) pred = whole;
+    if (st.forward8) {
+        if (__builtin_expect(clamp, 0)) { pi = clamp8(pi); qi = clamp8(qi); }
+        const float whole = forward_int8<TS>(pi, qi, st.both_rev);
+        if (st.user.n == 8 && st.item.n == 8) pred = whole;
     }
     const float ruv = __fsub_rn(r, pred);
-    if (estimate && __any_sync(kAll, new_back)) {
-        const float range = fmaxf(fmaxf(fmaxf(pmax, qmax), fabsf(c.lam)), fabsf(ruv));
-        const AfpSide s = afp_requantize(st.back, afp_qem_back<K>(eight<K>(p), eight<K>(q), c.lam, ruv, range, kAll), range, cur, c.afp_epoch, c.afp_init_threshold);
-        if (new_back) st.back = s;
+    if (__builtin_expect(estimate, 0)) {
+        const bool new_back = active && cur == st.back.next;
+        if (__any_sync(kAll, new_back)) {
+            const float range = fmaxf(fmaxf(fmaxf(pmax, qmax), fabsf(c.lam)), fabsf(ruv));
+            const AfpSide s = afp_requantize(st.back, afp_qem_back<K>(eight<K>(p), eight<K>(q), c.lam, ruv, range, kAll), range, cur, c.afp_epoch, c.afp_init_threshold);
+            if (new_back) st.back = s;
+        }
+        const bool mine8 = st.back.n == 8;
+        st.back16 = __any_sync(kAll, active && !mine8);
+        st.back8 = !st.back16 || __any_sync(kAll, active && mine8);
+        st.back_rev = pow2_rev(st.back.scale); st.back2_rev = pow2_rev(__fmul_rn(st.back.scale, st.back.scale));
+        st.lam8 = quantize8(-c.lam, st.back.scale);
+        st.lam16 = __half2half2(__float2half_rn(fix_round(-c.lam, st.back.scale, st.back_rev)));
+        // an estimate whose time has passed never comes again
+        auto wait = [&](long long next) { const long long d = next - cur - 1; return d < 0 || d > 0x7fffffff ? 0x7fffffff : (int)d; };
+        st.due = (unsigned)__reduce_min_sync(kAll, min(min(wait(st.user.next), wait(st.item.next)), wait(st.back.next)));
+    } else {
+        st.due--;
     }
-    const bool back8 = st.back.n == 8;
-    quantize(p, st.back.scale, q, st.back.scale, pi, qi, kAll);
-    most = fmaxf(abs_max(pi), abs_max(qi));
+    pi = quantize_near(p, st.back.scale, odd_p); qi = quantize_near(q, st.back.scale, odd_q);
+    big = clamp = false;
+    check(st.back.scale, st.back.scale, st.back8);
     Vf<N> gp, gq;
-    if (__any_sync(kAll, active && !back8)) {
-        to_grid(p, pi, st.back.scale, q, qi, st.back.scale, __any_sync(kAll, !(most < 2097152.f)), ph, qh);
-        backward_half(ph, qh, ruv, -c.lam, st.back.scale, gp, gq);
+    if (st.back16) {
+        to_grid(p, pi, st.back.scale, st.back_rev, q, qi, st.back.scale, st.back_rev, big, ph, qh);
+        backward_half(ph, qh, ruv, st.lam16, st.back.scale, st.back_rev, gp, gq);
     }
-    if (__any_sync(kAll, active && back8)) {
-        if (__any_sync(kAll, !(most <= 127.f))) { pi = clamp8(pi); qi = clamp8(qi); }
+    if (st.back8) {
+        if (__builtin_expect(clamp, 0)) { pi = clamp8(pi); qi = clamp8(qi); }
         Vf<N> wp, wq;
-        backward_int8(pi, qi, ruv, -c.lam, st.back.scale, wp, wq);
-        if (back8) { gp = wp; gq = wq; }
+        backward_int8(pi, qi, ruv, st.lam8, st.back.scale, st.back2_rev, wp, wq);
+        if (!st.back16 || st.back.n == 8) { gp = wp; gq = wq; }
     }
     p = step(c.lr, gp, p); q = step(c.lr, gq, q);
     st.cur = cur + 1;
@@ -1018,11 +1049,11 @@ __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_
             set_pr(qo, j, __ffma2_rn(lr2, __fmul2_rn(rev2, pr(gq, j)), pr(q, j)));
         }
         put(p_raw, po); put(q_raw, qo);
-    } else if constexpr (KIND == KIND_MUPPET) {
+    } else if constexpr (KIND == KIND_MUPPET || KIND == kMuppetHalf) {
         Vf<N> p = as_vf(p_raw), q = as_vf(q_raw);
-        muppet_update<K>(c, __uint_as_float(rw), p, q, smp.gp, smp.gq, mid);
+        muppet_update<K, KIND == KIND_MUPPET>(c, __uint_as_float(rw), p, q, smp.gp, smp.gq, mid);
         put(p_raw, p); put(q_raw, q);
-        if (STATS && c.bits != 32) smp.user = true;
+        if (STATS) smp.user = true;
     } else if constexpr (KIND == KIND_AFP) {
         Vf<N> p = as_vf(p_raw), q = as_vf(q_raw);
         afp_update<K>(c, afp, __uint_as_float(rw), active, p, q);
@@ -1151,7 +1182,7 @@ template <int K, int UM, int IM, bool STATS, int NS, int NSI> struct WorkerSmem 
 // The lead is kept as short as the memory latency allows: an item row that another worker updates between the
 // request and the write-back loses that update, and the chance of that grows with the lead.
 template <int K, int KIND, int UM, int IM, bool STATS, int NS, int NSI, int D, int DI>
-__global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS) ? 4 : ((UM == ROWS_DYN || STATS || KIND == KIND_AFP || KIND == KIND_MUPPET) ? 2 : 3)) train_kernel(const KernelArgs a) {
+__global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS) ? 4 : ((UM == ROWS_DYN || STATS || KIND == KIND_AFP || kMuppet<KIND>) ? 2 : 3)) train_kernel(const KernelArgs a) {
     using SM = WorkerSmem<K, UM, IM, STATS, NS, NSI>;
     constexpr int TS = SM::TS;                     // lanes per worker = ratings per chunk
     constexpr int N = kElems<UM>;                  // elements per lane
@@ -1339,7 +1370,7 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
     // MuPPET, whole-model switching (muppet_sgd_kernel.h:266-285, sgd_kernel.h:266-285): the element-wise sum of both
     // gradients and the sum of their squared norms, one set for all groups, over the ratings of the worker.  The
     // norm of a rating goes through the worker's lanes during the next rating (`norm_step`), in the same order as at once.
-    constexpr bool kWhole = STATS && (KIND == KIND_MUPPET || KIND == KIND_SWITCH);
+    constexpr bool kWhole = STATS && (kMuppet<KIND> || KIND == KIND_SWITCH);
     float norm = 0.f;
     float4 norm_parts = make_float4(0.f, 0.f, 0.f, 0.f);      // with four elements a lane: what the first step joins
     auto norm_step = [&](int part) {
@@ -1347,7 +1378,6 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
         else if (kWhole && (TS / 2) >> part) norm = __fadd_rn(norm, __shfl_xor_sync(kAll, norm, (TS / 2) >> part));
     };
     auto record_whole = [&](const Sample<N>& smp, bool there) {
-        if (!smp.user) return;                                 // all ratings of a launch, or none
         nq_acc = __fadd_rn(nq_acc, norm);
         if constexpr (N == 4) norm_parts = there ? muppet_norm_parts<K>(smp.gp, smp.gq) : make_float4(0.f, 0.f, 0.f, 0.f);
         else norm = there ? muppet_norm_partial<K>(smp.gp, smp.gq) : 0.f;
@@ -1379,7 +1409,7 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
     };
     Sample<N> smp;
     AfpState afp;
-    afp.user = AfpSide{8, 1.f, 0.f, 0}; afp.item = afp.user; afp.back = afp.user; afp.cur = 0;
+    afp.user = AfpSide{8, 1.f, 0.f, 0}; afp.item = afp.user; afp.back = afp.user; afp.cur = 0; afp.due = 0;
 
     // requests the user row / the item row of a rating into ring slot `slot`
     auto request_user = [&](uint32_t uc, int slot) {
@@ -1412,7 +1442,7 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
     Raw<UM> p = lds_row<K, UM>(uring, rec.z);
     bool turn = __any_sync(kAll, rec.x & (F_RS | F_UDUP));      // does the coming rating of some worker need another item row?
 
-    constexpr int kUnroll = (KIND == KIND_AFP || KIND == KIND_MUPPET) ? 1 : NS;
+    constexpr int kUnroll = (KIND == KIND_AFP || kMuppet<KIND>) ? 1 : NS;
     int cb = 0;                                     // buffer of the chunk in use
     while (__any_sync(kAll, cnt_cur > 0)) {
 #pragma unroll 1
@@ -1585,7 +1615,7 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
     // at 0.2 us a rating.  Three and two ahead cost the small configurations 5 to 20 % (8M ratings: 1.30 -> 1.57 ms per
     // epoch; four and two 1.40) and the 100M-rating one nothing; six and seven gain nothing.  The fixed-point updates
     // are three to four times as long, and for them three and two are enough.
-    constexpr bool kFixedPoint = KIND == KIND_AFP || KIND == KIND_MUPPET;
+    constexpr bool kFixedPoint = KIND == KIND_AFP || kMuppet<KIND>;
     constexpr int NS = kFixedPoint ? 4 : 8, D = kFixedPoint ? 3 : 5, DI = kFixedPoint ? 2 : 3;
     // A step of few warps is a chain of some ninety instructions.  With K/4 lanes a worker the warp has half of the row work
     // and one worker fewer to wait for: shorter steps, on twice as many warps - as long as the schedulers can take those.  ms per
@@ -1644,7 +1674,11 @@ cudaError_t launch_k(TrainKind kind, const KernelArgs& a, bool stats, RowClass c
         case KIND_MEMQUANT: return launch_one<K, KIND_MEMQUANT, ROWS_HALF, ROWS_HALF, false>(a, workers, st, sh, dry);
         case KIND_AFP: return launch_one<K, KIND_AFP, ROWS_F32, ROWS_F32, false>(a, workers, st, sh, dry);
         case KIND_SWITCH: return launch_st<K, KIND_SWITCH, ROWS_HALF, ROWS_HALF>(a, stats, workers, st, sh, dry);
-        case KIND_MUPPET: return launch_st<K, KIND_MUPPET, ROWS_F32, ROWS_F32>(a, stats, workers, st, sh, dry);
+        case KIND_MUPPET:
+            // at 32 bits MuPPET is plain fp32 SGD and samples nothing: 2M ratings 0.81 ms per epoch in a kernel for all widths, XXX
+            if (a.bits == 32) return launch_one<K, KIND_FP32, ROWS_F32, ROWS_F32, false>(a, workers, st, sh, dry);
+            if (a.bits == 8) return launch_st<K, KIND_MUPPET, ROWS_F32, ROWS_F32>(a, stats, workers, st, sh, dry);
+            return launch_st<K, kMuppetHalf, ROWS_F32, ROWS_F32>(a, stats, workers, st, sh, dry);
     }
     return cudaErrorInvalidValue;
 }
