@@ -496,7 +496,10 @@ __device__ __forceinline__ int scale_key(int2 bound, float hi, float lo) {
     return min(bound.x - max(__float_as_int(hi), 0), bound.y - max(__float_as_int(-lo), 0));
 }
 __device__ __forceinline__ float scale_of(int key) { return __int_as_float((max(key, 0) & 0x7f800000) + 0x3f800000); }
-__device__ __forceinline__ bool scale_unsure(int2 bound, int key) { return ((key + 256) & 0x007fffff) < 512 + bound.y - bound.x || key >= (120 << 23); }
+// (From 2^60 on, the formula too: below that the reciprocal of a product of two scales is a normal number, and comes from the bits.)
+__device__ __forceinline__ bool scale_unsure(int2 bound, int key) { return ((key + 256) & 0x007fffff) < 512 + bound.y - bound.x || key >= (60 << 23); }
+__device__ __forceinline__ float near_rev(float s) { return __int_as_float(0x7f000000 - __float_as_int(s)); }
+__device__ __forceinline__ float near_rev(float s, float t) { return __int_as_float((int)0xbe800000u - __float_as_int(s) - __float_as_int(t)); }
 // roundf (halves away from zero) in three instructions: trunc(x + copysign(largest float below one half, x)).
 // The sum is rounded to nearest-even, which is what makes it exact: x = n + f with f < 1/2 cannot reach n + 1,
 // f >= 1/2 always does.  Equal to roundf for every one of the 2^32 float patterns (checked exhaustively on the
@@ -532,6 +535,13 @@ template <int N> __device__ __forceinline__ Vf<N> quantize_near(const Vf<N>& x, 
     odd = fmaxf(far[0], far[1]);
     if constexpr (N == 8) odd = fmaxf(odd, fmaxf(far[2], far[3]));
     return o;
+}
+// The same for two values that all lanes have
+__device__ __forceinline__ float2 quantize_near(float2 x, float s, float& odd) {
+    const float2 s2 = make_float2(s, s), magic = make_float2(12582912.f, 12582912.f), minus = make_float2(-12582912.f, -12582912.f);
+    const float2 r = __fadd2_rn(__ffma2_rn(x, s2, magic), minus), d = __ffma2_rn(x, s2, make_float2(-r.x, -r.y));
+    odd = fmaxf(fabsf(d.x), fabsf(d.y));
+    return r;
 }
 template <int N> __device__ __forceinline__ Vf<N> quantize_away(const Vf<N>& x, float s) {
     Vf<N> o;
@@ -693,9 +703,8 @@ __device__ __forceinline__ float forward_half(const Vh<4>& ph, const Vh<4>& qh, 
     xy = __hadd2_rn(K == 128 ? from(xy, low) : xy, last);
     return __half2float(__hadd_rn(__low2half(xy), __high2half(xy)));
 }
-// backward passes: g_p = q*e + p*(-lam), g_q = p*e + q*(-lam) in int8 or binary16 fixed point; l, l2: -lam on the grid, rev: 1 / (sb sb)
-template <int N> __device__ __forceinline__ void backward_int8(const Vf<N>& pi, const Vf<N>& qi, float ruv, float l, float sb, float rev, Vf<N>& gp, Vf<N>& gq) {
-    const float e = quantize8(ruv, sb);
+// backward passes: g_p = q*e + p*(-lam), g_q = p*e + q*(-lam) in int8 or binary16 fixed point; e, l: error and -lam on the grid, rev: 1 / (sb sb)
+template <int N> __device__ __forceinline__ void backward_int8(const Vf<N>& pi, const Vf<N>& qi, float e, float l, float rev, Vf<N>& gp, Vf<N>& gq) {
     const float2 rev2 = make_float2(rev, rev), e2 = make_float2(e, e), l2 = make_float2(l, l), zero = make_float2(0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < N / 2; j++) {      // + 0: the integer sum has no negative zero
@@ -703,8 +712,7 @@ template <int N> __device__ __forceinline__ void backward_int8(const Vf<N>& pi, 
         set_pr(gq, j, __ffma2_rn(__ffma2_rn(pr(pi, j), e2, __fmul2_rn(pr(qi, j), l2)), rev2, zero));
     }
 }
-template <int N> __device__ __forceinline__ void backward_half(const Vh<N>& ph, const Vh<N>& qh, float ruv, __half2 l2, float sb, float sb_rev, Vf<N>& gp, Vf<N>& gq) {
-    const __half2 e2 = __half2half2(__float2half_rn(fix_round(ruv, sb, sb_rev)));
+template <int N> __device__ __forceinline__ void backward_half(const Vh<N>& ph, const Vh<N>& qh, __half2 e2, __half2 l2, Vf<N>& gp, Vf<N>& gq) {
     Vh<N> gph, gqh;
 #pragma unroll
     for (int t = 0; t < N / 2; t++) {
@@ -752,12 +760,14 @@ __device__ __forceinline__ void muppet_update(const Consts& c, float r, Vf<N>& p
     float sp = scale_of(kp), sq = scale_of(kq), odd_p, odd_q;
     Vf<N> pi = quantize_near(p, sp, odd_p), qi = quantize_near(q, sq, odd_q);
     auto outside = [](float hi, float lo, float s) { return INT8 ? outside8(hi, lo, s) : beyond_grid(hi, lo, s); };
+    float sp_rev = near_rev(sp), sq_rev = near_rev(sq), both_rev = near_rev(sp, sq);
     bool big = false;
     if (__builtin_expect(__any_sync(kAll, scale_unsure(bound, kp) || scale_unsure(bound, kq) || outside(phi, plo, sp) || outside(qhi, qlo, sq)
                                           || !(fmaxf(odd_p, odd_q) < 0.5f)), 0)) {
         if (__any_sync(kAll, scale_unsure(bound, kp) || scale_unsure(bound, kq))) {
             const float2 s = muppet_scales_exact<TS>(bits, phi, plo, qhi, qlo);
             sp = s.x; sq = s.y;
+            sp_rev = pow2_rev(sp); sq_rev = pow2_rev(sq); both_rev = pow2_rev(__fmul_rn(sp, sq));
         }
         pi = quantize_away(p, sp); qi = quantize_away(q, sq);
         if (INT8) { pi = clamp8(pi); qi = clamp8(qi); }
@@ -766,30 +776,38 @@ __device__ __forceinline__ void muppet_update(const Consts& c, float r, Vf<N>& p
     mid(2);
     Vh<N> ph, qh;
     float pred;
-    if constexpr (INT8) pred = forward_int8<TS>(pi, qi, pow2_rev(__fmul_rn(sp, sq)));
+    if constexpr (INT8) pred = forward_int8<TS>(pi, qi, both_rev);
     else {
-        to_grid(p, pi, sp, pow2_rev(sp), q, qi, sq, pow2_rev(sq), big, ph, qh);
+        to_grid(p, pi, sp, sp_rev, q, qi, sq, sq_rev, big, ph, qh);
         pred = forward_half<K>(ph, qh, kAll);
     }
     mid(3);
     const float ruv = __fsub_rn(r, pred);
-    const float hi = fmaxf(phi, qhi), lo = fminf(plo, qlo);
-    const int kb = min(min(kp, kq), scale_key(bound, fmaxf(nlam, ruv), fminf(nlam, ruv)));
-    float sb = scale_of(kb);
+    const float ehi = fmaxf(nlam, ruv), elo = fminf(nlam, ruv), hi = fmaxf(fmaxf(phi, qhi), ehi), lo = fminf(fminf(plo, qlo), elo);
+    const int kb = min(min(kp, kq), scale_key(bound, ehi, elo));
+    float sb = scale_of(kb), odd_e;
     pi = quantize_near(p, sb, odd_p); qi = quantize_near(q, sb, odd_q);
+    float2 el = quantize_near(make_float2(ruv, nlam), sb, odd_e);      // error and -lam on the grid
+    float sb_rev = near_rev(sb), sb2_rev = near_rev(sb, sb);
     big = false;
-    if (__builtin_expect(__any_sync(kAll, scale_unsure(bound, kb) || outside(hi, lo, sb) || !(fmaxf(odd_p, odd_q) < 0.5f)), 0)) {
-        if (__any_sync(kAll, scale_unsure(bound, kb))) sb = muppet_back_scale_exact<TS>(bits, hi, lo, nlam, ruv);
+    if (__builtin_expect(__any_sync(kAll, scale_unsure(bound, kb) || outside(hi, lo, sb) || !(fmaxf(odd_p, odd_q) < 0.5f) || !(odd_e < 0.5f)), 0)) {
+        if (__any_sync(kAll, scale_unsure(bound, kb))) {
+            sb = muppet_back_scale_exact<TS>(bits, hi, lo, nlam, ruv);
+            sb_rev = pow2_rev(sb); sb2_rev = pow2_rev(__fmul_rn(sb, sb));
+        }
         pi = quantize_away(p, sb); qi = quantize_away(q, sb);
         if (INT8) { pi = clamp8(pi); qi = clamp8(qi); }
         else big = beyond_grid(hi, lo, sb);
+        el = make_float2(round_away(__fmul_rn(ruv, sb)), round_away(__fmul_rn(nlam, sb)));
+        if (INT8) el = make_float2(clamp8(el.x), clamp8(el.y));
     }
     mid(4);
-    if constexpr (INT8) backward_int8(pi, qi, ruv, quantize8(nlam, sb), sb, pow2_rev(__fmul_rn(sb, sb)), gp, gq);
+    if constexpr (INT8) backward_int8(pi, qi, el.x, el.y, sb2_rev, gp, gq);
     else {
-        const float sb_rev = pow2_rev(sb);
         to_grid(p, pi, sb, sb_rev, q, qi, sb, sb_rev, big, ph, qh);
-        backward_half(ph, qh, ruv, __half2half2(__float2half_rn(fix_round(nlam, sb, sb_rev))), sb, sb_rev, gp, gq);
+        // (a value that rounds to zero keeps its sign)
+        backward_half(ph, qh, __half2half2(__float2half_rn(__fmul_rn(copysignf(el.x, ruv), sb_rev))), __half2half2(__float2half_rn(__fmul_rn(copysignf(el.y, nlam), sb_rev))),
+                      gp, gq);
     }
     p = step(c.lr, gp, p); q = step(c.lr, gq, q);
 }
@@ -961,16 +979,18 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
     Vf<N> pi = quantize_near(p, st.user.scale, odd_p), qi = quantize_near(q, st.item.scale, odd_q);
     Vh<N> ph, qh;
     bool big = false, clamp = false;
-    auto check = [&](float sp, float sq, bool some8) {
-        float most = fmaxf(abs_max(pi), abs_max(qi));
-        if (__builtin_expect(__any_sync(kAll, !(fmaxf(odd_p, odd_q) < 0.5f) || !(most <= (some8 ? 127.f : 2097151.f))), 0)) {
+    auto check = [&](float sp, float sq, bool some8, float also, float odd_also) {
+        float most = fmaxf(fmaxf(abs_max(pi), abs_max(qi)), fabsf(also));
+        const bool again = __any_sync(kAll, !(fmaxf(odd_p, odd_q) < 0.5f) || !(odd_also < 0.5f) || !(most <= (some8 ? 127.f : 2097151.f)));
+        if (__builtin_expect(again, 0)) {
             pi = quantize_away(p, sp); qi = quantize_away(q, sq);
             most = fmaxf(abs_max(pi), abs_max(qi));
             big = __any_sync(kAll, !(most < 2097152.f));
             clamp = __any_sync(kAll, !(most <= 127.f));
         }
+        return again;
     };
-    check(st.user.scale, st.item.scale, st.forward8);
+    check(st.user.scale, st.item.scale, st.forward8, 0.f, 0.f);
     if (st.forward16) {
         to_grid(p, pi, st.user.scale, st.user_rev, q, qi, st.item.scale, st.item_rev, big, ph, qh);
         pred = forward_half<K>(ph, qh, kAll);
@@ -1001,17 +1021,19 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
         st.due--;
     }
     pi = quantize_near(p, st.back.scale, odd_p); qi = quantize_near(q, st.back.scale, odd_q);
+    float odd_e;
+    float2 e = quantize_near(make_float2(ruv, ruv), st.back.scale, odd_e);      // the error on the two grids
     big = clamp = false;
-    check(st.back.scale, st.back.scale, st.back8);
+    if (__builtin_expect(check(st.back.scale, st.back.scale, st.back8, e.x, odd_e), 0)) e = make_float2(quantize8(ruv, st.back.scale), round_away(__fmul_rn(ruv, st.back.scale)));
     Vf<N> gp, gq;
     if (st.back16) {
         to_grid(p, pi, st.back.scale, st.back_rev, q, qi, st.back.scale, st.back_rev, big, ph, qh);
-        backward_half(ph, qh, ruv, st.lam16, st.back.scale, st.back_rev, gp, gq);
+        backward_half(ph, qh, __half2half2(__float2half_rn(__fmul_rn(copysignf(e.y, ruv), st.back_rev))), st.lam16, gp, gq);
     }
     if (st.back8) {
         if (__builtin_expect(clamp, 0)) { pi = clamp8(pi); qi = clamp8(qi); }
         Vf<N> wp, wq;
-        backward_int8(pi, qi, ruv, st.lam8, st.back.scale, st.back2_rev, wp, wq);
+        backward_int8(pi, qi, e.x, st.lam8, st.back2_rev, wp, wq);
         if (!st.back16 || st.back.n == 8) { gp = wp; gq = wq; }
     }
     p = step(c.lr, gp, p); q = step(c.lr, gq, q);
@@ -1442,7 +1464,7 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
     Raw<UM> p = lds_row<K, UM>(uring, rec.z);
     bool turn = __any_sync(kAll, rec.x & (F_RS | F_UDUP));      // does the coming rating of some worker need another item row?
 
-    constexpr int kUnroll = (KIND == KIND_AFP || kMuppet<KIND>) ? 1 : NS;
+    constexpr int kUnroll = (KIND == KIND_AFP || KIND == KIND_MUPPET) ? 1 : KIND == kMuppetHalf ? 2 : NS;
     int cb = 0;                                     // buffer of the chunk in use
     while (__any_sync(kAll, cnt_cur > 0)) {
 #pragma unroll 1
@@ -1675,7 +1697,7 @@ cudaError_t launch_k(TrainKind kind, const KernelArgs& a, bool stats, RowClass c
         case KIND_AFP: return launch_one<K, KIND_AFP, ROWS_F32, ROWS_F32, false>(a, workers, st, sh, dry);
         case KIND_SWITCH: return launch_st<K, KIND_SWITCH, ROWS_HALF, ROWS_HALF>(a, stats, workers, st, sh, dry);
         case KIND_MUPPET:
-            // at 32 bits MuPPET is plain fp32 SGD and samples nothing: 2M ratings 0.81 ms per epoch in a kernel for all widths, XXX
+            // at 32 bits MuPPET is plain fp32 SGD and samples nothing (2M ratings: 0.81 ms per epoch in a kernel for all widths, 0.64 in this one)
             if (a.bits == 32) return launch_one<K, KIND_FP32, ROWS_F32, ROWS_F32, false>(a, workers, st, sh, dry);
             if (a.bits == 8) return launch_st<K, KIND_MUPPET, ROWS_F32, ROWS_F32>(a, stats, workers, st, sh, dry);
             return launch_st<K, kMuppetHalf, ROWS_F32, ROWS_F32>(a, stats, workers, st, sh, dry);
