@@ -104,20 +104,25 @@ cudaError_t launch_encode_stream(const void* d_src_aos, uint64_t n, bool shuffle
                                  float* r, uint32_t* u, uint32_t* i, uint32_t* src_out, uint32_t src_base,
                                  cudaStream_t st);
 cudaError_t launch_recode(uint32_t* ids, uint64_t n, const uint8_t* prec_row, cudaStream_t st);
-// Stable re-ordering of a coded stream inside every segment, by precision class (by_class; class = 2 * (user
-// row fp32) + (item row fp32)) and / or by item inside windows of 2^run_window_log2 positions
-// (run_window_log2 > 0; item_rows = rows of the item arena, which bounds the item part of the key).
-// Inputs r/u/i/src (src may be null) stay untouched; the result goes to r2/u2/i2/src2.  key_* (n keys of
-// stream_sort_key_bytes each), idx_* (n u32) and temp (stream_sort_temp_bytes) are scratch; d_first (may be null) receives, for every
-// segment * 4 + class, the first position holding it (all ones when it does not occur).  segclass_bits =
-// bits of the largest segment * 4 + class.
-size_t stream_sort_key_bytes(uint64_t n, int segclass_bits, bool by_class, int run_window_log2, uint32_t item_rows);
-size_t stream_sort_temp_bytes(uint64_t n, int segclass_bits, bool by_class, int run_window_log2, uint32_t item_rows);
+// Stable re-ordering of a coded stream inside every segment by item, in windows of 2^run_window_log2 positions (item_rows =
+// rows of the item arena, which bounds the item part of the key).  Inputs r/u/i/src (src may be null) stay untouched; the
+// result goes to r2/u2/i2/src2.  key_* (n keys of stream_sort_key_bytes each), idx_* (n u32) and temp (stream_sort_temp_bytes)
+// are scratch.  seg_bits = bits of the largest segment number.
+size_t stream_sort_key_bytes(uint64_t n, int seg_bits, int run_window_log2, uint32_t item_rows);
+size_t stream_sort_temp_bytes(uint64_t n, int seg_bits, int run_window_log2, uint32_t item_rows);
 cudaError_t launch_stream_sort(const float* r, const uint32_t* u, const uint32_t* i, const uint32_t* src, uint64_t n,
-                               const uint64_t* d_seg_off, int nseg, int segclass_bits, bool by_class, int run_window_log2,
-                               uint32_t item_rows, void* key_a, void* key_b, uint32_t* idx_a, uint32_t* idx_b,
-                               void* temp, size_t temp_bytes, unsigned long long* d_first,
+                               const uint64_t* d_seg_off, int nseg, int seg_bits, int run_window_log2, uint32_t item_rows,
+                               void* key_a, void* key_b, uint32_t* idx_a, uint32_t* idx_b, void* temp, size_t temp_bytes,
                                float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, cudaStream_t st);
+// Partition of a coded stream, inside every segment, by precision class = 2 * (user row fp32) + (item row fp32); inside a class the
+// ratings are in the order in which the stream was coded.  pos: where each rating was then (null: where it is now); pos2, which may
+// be key_a (or null), receives the same for the new order.  key_*, idx_* (n u32) and temp are scratch; key_bits = bits of the largest
+// segment * 4 + class; d_first receives, for every segment * 4 + class, the first position holding it (all ones when it does not occur).
+size_t class_partition_temp_bytes(uint64_t n, int key_bits);
+cudaError_t launch_class_partition(const float* r, const uint32_t* u, const uint32_t* i, const uint32_t* src, const uint32_t* pos, uint64_t n,
+                                   const uint64_t* d_seg_off, int nseg, int key_bits, uint32_t* key_a, uint32_t* key_b, uint32_t* idx_a, uint32_t* idx_b,
+                                   void* temp, size_t temp_bytes, unsigned long long* d_first, float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, uint32_t* pos2,
+                                   cudaStream_t st);
 // The whole resident stream from the uploaded array: seeded permutation of every segment, item-sorted run windows, ids
 // coded - the order that launch_encode_stream and launch_stream_sort give, in one sort.  source_sort_bytes: the scratch it
 // wants, or 0 where it does not apply (no run windows, segments that begin off the encoding step's windows, keys beyond 32

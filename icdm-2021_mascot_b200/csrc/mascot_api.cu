@@ -83,7 +83,7 @@ int mascot::fail(mascot_handle* h, int code, const std::string& msg) {
 namespace mascot {
 
 void free_ratings(mascot_handle* h) {
-    dev_free(h->tr_r, h->stream); dev_free(h->tr_u, h->stream); dev_free(h->tr_i, h->stream); dev_free(h->tr_src, h->stream);
+    dev_free(h->tr_r, h->stream); dev_free(h->tr_u, h->stream); dev_free(h->tr_i, h->stream); dev_free(h->tr_src, h->stream); dev_free(h->tr_pos, h->stream);
     dev_free(h->te_r, h->stream); dev_free(h->te_u, h->stream); dev_free(h->te_i, h->stream);
     dev_free(h->P.f16, h->stream); dev_free(h->P.f32, h->stream); dev_free(h->Q.f16, h->stream); dev_free(h->Q.f32, h->stream);
     dev_free(h->d_uprec_row, h->stream); dev_free(h->d_iprec_row, h->stream); dev_free(h->d_ugroup, h->stream); dev_free(h->d_igroup, h->stream);
@@ -212,64 +212,87 @@ bool any_fp32_group(const mascot_handle* h) {
     return false;
 }
 
-// Re-orders the segments [seg_first, seg_first + seg_count) of the coded stream, stably, inside each segment:
-//   by_class: the ratings of one precision class become contiguous (the order inside a class is the order
-//     before) and the class boundaries are recorded.  Called after the precision bits of the ids changed
-//     (promotion + recode) or after a stream was encoded while promoted groups exist.
-//   run_window_log2 > 0: every window of 2^run_window_log2 positions is sorted by item (longer runs of equal
-//     items).  Called once after a stream was encoded.
-// The single-worker deterministic mode keeps the caller's order and does neither.
-int reorder_segments(mascot_handle* h, size_t seg_first, size_t seg_count, bool by_class, int run_window_log2) {
-    const size_t nseg_all = h->seg_off.size() - 1;
-    if (by_class && h->cls_off.size() != nseg_all * 5) {
-        h->cls_off.assign(nseg_all * 5, 0);
-        for (size_t sg = 0; sg < nseg_all; sg++) {          // everything in the first class
-            h->cls_off[sg * 5] = h->seg_off[sg];
-            for (int c = 1; c <= 4; c++) h->cls_off[sg * 5 + c] = h->seg_off[sg + 1];
-        }
-    }
-    const uint64_t begin = h->seg_off[seg_first], end = h->seg_off[seg_first + seg_count], n = end - begin;
-    if (n == 0) return MASCOT_OK;
-    int key_bits = 2;
-    while ((1ull << key_bits) < seg_count * 4) key_bits++;
+// Scratch of a re-ordering: keys and indices of a radix sort, the re-ordered arrays, the segment offsets.
+struct SortSpace {
+    void *key_a, *key_b, *temp;
+    uint32_t *idx_a, *idx_b, *u, *i, *src;
+    float* r;
+    uint64_t* seg;
+    unsigned long long* first;         // four per segment
+};
+static int sort_space(mascot_handle* h, size_t key_bytes, size_t temp_bytes, SortSpace* sp) {
+    const size_t n = h->n_train, nseg = h->seg_off.size() - 1;
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    const size_t temp_bytes = stream_sort_temp_bytes(n, key_bits, by_class, run_window_log2, h->irows);
-    const size_t b_key = up(stream_sort_key_bytes(n, key_bits, by_class, run_window_log2, h->irows) * n), b_idx = up(sizeof(uint32_t) * n), b_seg = up(sizeof(uint64_t) * (seg_count + 1));
-    const size_t b_first = up(sizeof(unsigned long long) * seg_count * 4);
-    const size_t total = 2 * b_key + 2 * b_idx + 4 * b_idx + b_seg + b_first + up(temp_bytes);
-    int rc = need_scratch(h, total);
+    const size_t b_key = up(key_bytes * n), b_idx = up(sizeof(uint32_t) * n), b_seg = up(sizeof(uint64_t) * (nseg + 1)), b_first = up(sizeof(unsigned long long) * nseg * 4);
+    const int rc = need_scratch(h, 2 * b_key + 6 * b_idx + b_seg + b_first + up(temp_bytes));
     if (rc != MASCOT_OK) return rc;
     unsigned char* base = static_cast<unsigned char*>(h->d_scratch);
-    void* key_a = base; base += b_key;
-    void* key_b = base; base += b_key;
-    uint32_t* idx_a = reinterpret_cast<uint32_t*>(base); base += b_idx;
-    uint32_t* idx_b = reinterpret_cast<uint32_t*>(base); base += b_idx;
-    float* r2 = reinterpret_cast<float*>(base); base += b_idx;
-    uint32_t* u2 = reinterpret_cast<uint32_t*>(base); base += b_idx;
-    uint32_t* i2 = reinterpret_cast<uint32_t*>(base); base += b_idx;
-    uint32_t* s2 = reinterpret_cast<uint32_t*>(base); base += b_idx;
-    uint64_t* d_seg = reinterpret_cast<uint64_t*>(base); base += b_seg;
-    unsigned long long* d_first = reinterpret_cast<unsigned long long*>(base); base += b_first;
-    void* temp = base;
-    std::vector<uint64_t> rel(seg_count + 1);
-    for (size_t j = 0; j <= seg_count; j++) rel[j] = h->seg_off[seg_first + j] - begin;
-    CU(h, cudaMemcpyAsync(d_seg, rel.data(), sizeof(uint64_t) * rel.size(), cudaMemcpyHostToDevice, h->stream));
-    uint32_t* src = h->tr_src ? h->tr_src + begin : nullptr;
-    CU(h, launch_stream_sort(h->tr_r + begin, h->tr_u + begin, h->tr_i + begin, src, n, d_seg, (int)seg_count, key_bits, by_class,
-                             run_window_log2, h->irows, key_a, key_b, idx_a, idx_b, temp, temp_bytes, by_class ? d_first : nullptr,
-                             r2, u2, i2, s2, h->stream));
-    CU(h, cudaMemcpyAsync(h->tr_r + begin, r2, sizeof(float) * n, cudaMemcpyDeviceToDevice, h->stream));
-    CU(h, cudaMemcpyAsync(h->tr_u + begin, u2, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
-    CU(h, cudaMemcpyAsync(h->tr_i + begin, i2, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
-    if (src) CU(h, cudaMemcpyAsync(src, s2, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
-    std::vector<unsigned long long> first(seg_count * 4);
-    if (by_class) CU(h, cudaMemcpyAsync(first.data(), d_first, sizeof(unsigned long long) * first.size(), cudaMemcpyDeviceToHost, h->stream));
-    CU(h, cudaStreamSynchronize(h->stream));          // `rel` and `first` are host buffers of this call
-    if (!by_class) return MASCOT_OK;
-    for (size_t j = 0; j < seg_count; j++) {
-        uint64_t* off = &h->cls_off[(seg_first + j) * 5];
-        off[4] = h->seg_off[seg_first + j + 1];
-        for (int c = 3; c >= 0; c--) off[c] = first[j * 4 + c] == ~0ull ? off[c + 1] : begin + first[j * 4 + c];
+    auto take = [&](size_t bytes) { unsigned char* p = base; base += bytes; return p; };
+    sp->key_a = take(b_key); sp->key_b = take(b_key);
+    sp->idx_a = reinterpret_cast<uint32_t*>(take(b_idx)); sp->idx_b = reinterpret_cast<uint32_t*>(take(b_idx));
+    sp->r = reinterpret_cast<float*>(take(b_idx)); sp->u = reinterpret_cast<uint32_t*>(take(b_idx));
+    sp->i = reinterpret_cast<uint32_t*>(take(b_idx)); sp->src = reinterpret_cast<uint32_t*>(take(b_idx));
+    sp->seg = reinterpret_cast<uint64_t*>(take(b_seg)); sp->first = reinterpret_cast<unsigned long long*>(take(b_first));
+    sp->temp = base;
+    CU(h, cudaMemcpyAsync(sp->seg, h->seg_off.data(), sizeof(uint64_t) * (nseg + 1), cudaMemcpyHostToDevice, h->stream));
+    return MASCOT_OK;
+}
+static int take_reordered(mascot_handle* h, const SortSpace& sp) {
+    const size_t n = h->n_train;
+    CU(h, cudaMemcpyAsync(h->tr_r, sp.r, sizeof(float) * n, cudaMemcpyDeviceToDevice, h->stream));
+    CU(h, cudaMemcpyAsync(h->tr_u, sp.u, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
+    CU(h, cudaMemcpyAsync(h->tr_i, sp.i, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
+    if (h->tr_src) CU(h, cudaMemcpyAsync(h->tr_src, sp.src, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
+    return MASCOT_OK;
+}
+
+// Sorts every window of 2^run_window_log2 positions of the coded stream by item (longer runs of equal items), inside each
+// segment.  Called once after a stream was encoded.  The single-worker deterministic mode keeps the caller's order.
+static int sort_windows(mascot_handle* h, int run_window_log2) {
+    const uint64_t n = h->n_train;
+    const int nseg = (int)h->seg_off.size() - 1;
+    int seg_bits = 0;
+    while ((1ll << seg_bits) < nseg) seg_bits++;
+    const size_t temp_bytes = stream_sort_temp_bytes(n, seg_bits, run_window_log2, h->irows);
+    SortSpace sp;
+    int rc = sort_space(h, stream_sort_key_bytes(n, seg_bits, run_window_log2, h->irows), temp_bytes, &sp);
+    if (rc != MASCOT_OK) return rc;
+    CU(h, launch_stream_sort(h->tr_r, h->tr_u, h->tr_i, h->tr_src, n, sp.seg, nseg, seg_bits, run_window_log2, h->irows, sp.key_a, sp.key_b, sp.idx_a, sp.idx_b,
+                             sp.temp, temp_bytes, sp.r, sp.u, sp.i, sp.src, h->stream));
+    if ((rc = take_reordered(h, sp)) != MASCOT_OK) return rc;
+    CU(h, cudaStreamSynchronize(h->stream));
+    return MASCOT_OK;
+}
+
+// Makes the ratings of each precision class contiguous inside every segment and records the class boundaries.  Called after the
+// precision bits of the ids changed (promotion + recode) or after a stream was encoded while promoted groups exist.
+static int partition_by_class(mascot_handle* h) {
+    const uint64_t n = h->n_train;
+    const size_t nseg = h->seg_off.size() - 1;
+    h->cls_off.assign(nseg * 5, 0);
+    if (n == 0) return MASCOT_OK;
+    int key_bits = 2;
+    while ((1ull << key_bits) < nseg * 4) key_bits++;
+    const size_t temp_bytes = class_partition_temp_bytes(n, key_bits);
+    SortSpace sp;
+    int rc = sort_space(h, sizeof(uint32_t), temp_bytes, &sp);
+    if (rc != MASCOT_OK) return rc;
+    // Without memory for the positions the classes keep the order that the last partition gave them.
+    if (!h->moved && reserve(h, &h->tr_pos, n) != cudaSuccess) { cudaGetLastError(); dev_free(h->tr_pos, h->stream); }
+    uint32_t* const pos2 = h->tr_pos ? static_cast<uint32_t*>(sp.key_a) : nullptr;
+    CU(h, launch_class_partition(h->tr_r, h->tr_u, h->tr_i, h->tr_src, h->moved ? h->tr_pos : nullptr, n, sp.seg, (int)nseg, key_bits,
+                                 static_cast<uint32_t*>(sp.key_a), static_cast<uint32_t*>(sp.key_b), sp.idx_a, sp.idx_b, sp.temp, temp_bytes, sp.first,
+                                 sp.r, sp.u, sp.i, sp.src, pos2, h->stream));
+    if ((rc = take_reordered(h, sp)) != MASCOT_OK) return rc;
+    if (pos2) CU(h, cudaMemcpyAsync(h->tr_pos, pos2, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
+    std::vector<unsigned long long> first(nseg * 4);
+    CU(h, cudaMemcpyAsync(first.data(), sp.first, sizeof(unsigned long long) * first.size(), cudaMemcpyDeviceToHost, h->stream));
+    CU(h, cudaStreamSynchronize(h->stream));
+    h->moved = pos2 != nullptr;
+    for (size_t j = 0; j < nseg; j++) {
+        uint64_t* off = &h->cls_off[j * 5];
+        off[4] = h->seg_off[j + 1];
+        for (int c = 3; c >= 0; c--) off[c] = first[j * 4 + c] == ~0ull ? off[c + 1] : first[j * 4 + c];
     }
     return MASCOT_OK;
 }
@@ -279,16 +302,15 @@ int reorder_segments(mascot_handle* h, size_t seg_first, size_t seg_count, bool 
 bool wants_partition(const mascot_handle* h) {
     if (!(h->grouped && !h->cfg.deterministic && any_fp32_group(h) && h->n_train < (1ull << 32) && (h->seg_off.size() - 1) * 4 <= 65536)) return false;
     // Measured on one B200, ms per epoch with one launch per class and with one that reads each id's precision bit: 100M
-    // ratings, a fifth of the groups promoted 9.9 and 13.6 to 14.2; 252M, 40 % of them 34.0 and 36 to 40.  In between the one
-    // launch is faster - 63M, 40 % promoted 9.8 and 9.0; 40M 6.9 and 5.5; k=64, 100M 12.7 and 7.2 - but leaves a test RMSE
-    // that is 0.1 % higher after four epochs (0.57343 against 0.57262 at 40M).
+    // ratings, a fifth of the groups promoted 8.6 and 13.6; 40 % of them, 63M 7.1 and 9.0, 40M 4.1 and 5.5, k=64, 100M 6.6 and
+    // 7.2.  Both leave the same test RMSE (0.57333 and 0.57346 after four epochs at 40M).
     return h->cfg.no_class_partition != 1;
 }
 
 int partition_all(mascot_handle* h) {
     h->partitioned = false;
     if (!wants_partition(h)) return MASCOT_OK;
-    const int rc = reorder_segments(h, 0, h->seg_off.size() - 1, true, 0);
+    const int rc = partition_by_class(h);
     if (rc == MASCOT_OK) h->partitioned = true;
     return rc;
 }
@@ -339,7 +361,7 @@ int sort_run_windows(mascot_handle* h) {
     const int w = run_window_log2(h);
     if (w == 0 || h->n_train == 0) return MASCOT_OK;
     NvtxRange range("mascot: item-sorted run windows");
-    return reorder_segments(h, 0, h->seg_off.size() - 1, false, w);
+    return sort_windows(h, w);
 }
 
 float reference_rmse_from_partials(const Results& part, uint64_t n) {
@@ -479,7 +501,7 @@ int mascot_reload_train(mascot_handle* h, const mascot_rating* train, uint64_t n
         CU(h, reserve(h, &h->tr_src, n_train));
         h->n_train = n_train;
         h->seg_off.assign({0, n_train});           // a stream of another length is one segment
-        h->cls_off.clear(); h->partitioned = false;
+        h->stream_is_new();
     }
     if (!n_train) return MASCOT_OK;
     const size_t bytes = sizeof(mascot_rating) * n_train, sort_at = (bytes + 255) / 256 * 256;
@@ -497,7 +519,7 @@ int mascot_reload_train(mascot_handle* h, const mascot_rating* train, uint64_t n
                               h->tr_r, h->tr_u, h->tr_i, h->tr_src));
     uint32_t bad = 0;
     CU(h, cudaMemcpyAsync(&bad, h->d_err_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-    h->cls_off.clear();
+    h->stream_is_new();
     if (!sort_bytes && (rc = sort_run_windows(h)) != MASCOT_OK) return rc;
     if ((rc = partition_all(h)) != MASCOT_OK) return rc;      // the new stream carries the current precisions
     CU(h, cudaStreamSynchronize(h->stream));
@@ -919,8 +941,7 @@ int mascot_train_epoch_streamed(mascot_handle* h, uint32_t epoch, const mascot_r
     // The pieces are not partitioned by precision class: finding the class boundaries needs a read-back,
     // i.e. a host wait per piece, which would stall the upload pipeline.  With promoted groups every piece
     // runs the instantiation that reads each id's precision bit; its extra cost hides behind the upload.
-    h->cls_off.clear();
-    h->partitioned = false;
+    h->stream_is_new();
 
     const float lr = epoch < h->lr.size() ? h->lr[epoch] : lr_at(h->cfg, epoch);
     const bool muppet = h->kind == KIND_MUPPET;

@@ -236,7 +236,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     l2_window_remove(h);
     h->have_ratings = h->have_factors = false;       // the buffers stay and are used again where they are large enough
     h->n_users = n_users; h->n_items = n_items; h->n_test = 0; h->n_train = 0;
-    h->cls_off.clear(); h->partitioned = false;
+    h->stream_is_new();
     h->sorted_space = h->grouped || sharded;
     if (!h->sorted_space) { dev_free(h->d_umap, h->stream); dev_free(h->d_imap, h->stream); }      // identity
     h->ulay = RowLayout(); h->ilay = RowLayout();

@@ -1656,13 +1656,12 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
             return launch_ns<K, KIND, UQ, IQ, STATS, NS, 4, D, DI>(args, 2 * per_sm, workers, st, shape, dry);
     }
     // With fp32 rows the deep rings leave room for fewer warps than the registers do (k=128, both sides fp32: 16 per SM
-    // against 24).  The mixed-precision classes with an fp32 side want those warps: where a launch asks for more workers
-    // than the deep rings hold and rings of 4 + 2 slots hold more, it takes these, three ratings and one ahead.  Per epoch,
-    // deep rings for all classes and this rule: 40 % of the groups promoted, 40M ratings 7.17 and 6.99 ms, 63M 9.64 and 9.42,
-    // 100M (a fifth) 10.35 and 9.95; all promoted, 63M 11.25 and 10.95, k=64 at 100M 22.1 and 20.2.
-    // Where the deep rings hold the request they are faster: 20M, all promoted, 5.00 and 5.28 (k=64, 75M: 8.45 and 8.61).
-    // The other trainers gain nothing from more warps: SGD 7.73 and 7.74 ms at 63M ratings, 10.53 and 10.58 at 100M, 32.6
-    // and 34.9 at 252M (binary16 rows: 16.6 and 17.2): what limits those is not the waiting of few warps.
+    // against 24).  Where a launch of a mixed-precision class with an fp32 side asks for more workers than the deep rings hold and
+    // rings of 4 + 2 slots hold more, it takes these, three ratings and one ahead, and has the workers.  The time is the same
+    // within a hundredth - ms per epoch, deep rings for all classes and this rule: 40 % of the groups promoted, 40M ratings 4.11 and
+    // 4.14, 63M 7.09 and 7.17, 252M 30.3 to 32.1 and 30.7 to 32.0, k=64 100M 6.56 and 6.54; 100M (a fifth) 8.60 and 8.57; all
+    // promoted, 63M 7.42 and 7.49 - as for the other trainers, which do without (SGD 7.73 and 7.74 at 63M, 10.53 and 10.58 at
+    // 100M): full GPUs are bound by what the rows' traffic allows.
     constexpr bool kShortRings = KIND == KIND_MIXED && !STATS && UM != ROWS_DYN && (UM == ROWS_F32 || IM == ROWS_F32);
     if constexpr (kShortRings) {
         LaunchShape deep, shallow;

@@ -88,3 +88,36 @@ def test_reload_after_a_streamed_epoch_keeps_its_pieces(mascot):
             assert eng.train_segment(2, 1).updates == n - piece
     assert (orders[0] == streamed).all()
     assert (orders[1] == in_windows(streamed, item, [0, piece, n], window)).all()
+
+
+@pytest.mark.parametrize("seg,shuffle", [([0, 100003], 1), ([0, 5000, 5000, 40960, 60001], 1), ([0, 3001], 0), ([0, 1], 1)])
+def test_classes_keep_the_coded_order(mascot, seg, shuffle):
+    """Inside a precision class the ratings stay in the order in which the stream was coded, also after several promotions one
+    after the other, after a reload and after a streamed epoch (whose piece is a stream of its own)."""
+    n_users, n_items, n = 700, 301, seg[-1]
+    R, P, Q = random_problem(np.random.default_rng(n), n_users, n_items, n, 64)
+    cfg = mascot.default_config(version=mascot.V_MASCOT, k=64, num_workers=4096, shuffle=shuffle, sample_ratio=1.0, user_group_num=6, item_group_num=5)
+    with mascot.Engine(cfg) as eng:
+        eng.set_ratings_sharded(R, seg, R[:1], n_users, n_items)
+        eng.set_factors(P, Q)
+        rows = [m[ids] for m, ids in zip(eng.index_maps(), (R["u"], R["i"]))]
+        ends = [eng.group_info(side)[0] for side in (0, 1)]
+
+        def expected(order, cuts):
+            fp32 = [eng.group_info(side)[1][np.searchsorted(ends[side], rows[side], side="left")] != 0 for side in (0, 1)]
+            cls = 2 * fp32[0] + fp32[1]
+            return np.concatenate([order[b:e][np.argsort(cls[order[b:e]], kind="stable")] for b, e in zip(cuts, cuts[1:])])
+
+        coded = eng.stream_order()
+        for side, group in ((0, len(ends[0]) - 1), (1, 0), (0, 0), (1, len(ends[1]) - 1)):
+            eng.promote_group(side, min(group, len(ends[side]) - 1))
+            assert (eng.stream_order() == expected(coded, seg)).all()
+        eng.reload_train(R)
+        assert (eng.stream_order() == expected(coded, seg)).all()
+        eng.promote_group(0, min(1, len(ends[0]) - 1))
+        assert (eng.stream_order() == expected(coded, seg)).all()
+        eng.train_epoch_streamed(0, R)
+        piece = eng.stream_order()
+        eng.promote_group(1, min(1, len(ends[1]) - 1))
+        eng.promote_group(0, min(2, len(ends[0]) - 1))
+        assert (eng.stream_order() == expected(piece, [0, n])).all()
