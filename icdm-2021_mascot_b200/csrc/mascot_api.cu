@@ -212,31 +212,22 @@ bool any_fp32_group(const mascot_handle* h) {
     return false;
 }
 
-// Scratch of a re-ordering: keys and indices of a radix sort, the re-ordered arrays, the segment offsets.
+// Scratch of a re-ordering: pieces that are carved off one after the other.  The first call sizes it (base null), the second lays it out.
 struct SortSpace {
-    void *key_a, *key_b, *temp;
-    uint32_t *idx_a, *idx_b, *u, *i, *src;
-    float* r;
-    uint64_t* seg;
-    unsigned long long* first;         // four per segment
+    unsigned char* base = nullptr;
+    size_t off = 0;
+    float* r; uint32_t *u, *i, *src;       // the re-ordered arrays
+    uint64_t* seg;                         // the segment offsets
+    template <typename T> T* take(size_t count) {
+        T* const p = reinterpret_cast<T*>(base + off);
+        off += (sizeof(T) * count + 255) / 256 * 256;
+        return p;
+    }
+    void arrays(size_t n, size_t nseg) {
+        r = take<float>(n); u = take<uint32_t>(n); i = take<uint32_t>(n); src = take<uint32_t>(n);
+        seg = take<uint64_t>(nseg + 1);
+    }
 };
-static int sort_space(mascot_handle* h, size_t key_bytes, size_t temp_bytes, SortSpace* sp) {
-    const size_t n = h->n_train, nseg = h->seg_off.size() - 1;
-    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    const size_t b_key = up(key_bytes * n), b_idx = up(sizeof(uint32_t) * n), b_seg = up(sizeof(uint64_t) * (nseg + 1)), b_first = up(sizeof(unsigned long long) * nseg * 4);
-    const int rc = need_scratch(h, 2 * b_key + 6 * b_idx + b_seg + b_first + up(temp_bytes));
-    if (rc != MASCOT_OK) return rc;
-    unsigned char* base = static_cast<unsigned char*>(h->d_scratch);
-    auto take = [&](size_t bytes) { unsigned char* p = base; base += bytes; return p; };
-    sp->key_a = take(b_key); sp->key_b = take(b_key);
-    sp->idx_a = reinterpret_cast<uint32_t*>(take(b_idx)); sp->idx_b = reinterpret_cast<uint32_t*>(take(b_idx));
-    sp->r = reinterpret_cast<float*>(take(b_idx)); sp->u = reinterpret_cast<uint32_t*>(take(b_idx));
-    sp->i = reinterpret_cast<uint32_t*>(take(b_idx)); sp->src = reinterpret_cast<uint32_t*>(take(b_idx));
-    sp->seg = reinterpret_cast<uint64_t*>(take(b_seg)); sp->first = reinterpret_cast<unsigned long long*>(take(b_first));
-    sp->temp = base;
-    CU(h, cudaMemcpyAsync(sp->seg, h->seg_off.data(), sizeof(uint64_t) * (nseg + 1), cudaMemcpyHostToDevice, h->stream));
-    return MASCOT_OK;
-}
 static int take_reordered(mascot_handle* h, const SortSpace& sp) {
     const size_t n = h->n_train;
     CU(h, cudaMemcpyAsync(h->tr_r, sp.r, sizeof(float) * n, cudaMemcpyDeviceToDevice, h->stream));
@@ -253,12 +244,25 @@ static int sort_windows(mascot_handle* h, int run_window_log2) {
     const int nseg = (int)h->seg_off.size() - 1;
     int seg_bits = 0;
     while ((1ll << seg_bits) < nseg) seg_bits++;
-    const size_t temp_bytes = stream_sort_temp_bytes(n, seg_bits, run_window_log2, h->irows);
+    const size_t temp_bytes = stream_sort_temp_bytes(n, seg_bits, run_window_log2, h->irows), key_bytes = stream_sort_key_bytes(n, seg_bits, run_window_log2, h->irows);
     SortSpace sp;
-    int rc = sort_space(h, stream_sort_key_bytes(n, seg_bits, run_window_log2, h->irows), temp_bytes, &sp);
+    unsigned char *key_a, *key_b, *temp;
+    uint32_t *idx_a, *idx_b;
+    auto lay_out = [&]() {
+        sp.off = 0;
+        key_a = sp.take<unsigned char>(key_bytes * n); key_b = sp.take<unsigned char>(key_bytes * n);
+        idx_a = sp.take<uint32_t>(n); idx_b = sp.take<uint32_t>(n);
+        sp.arrays(n, nseg);
+        temp = sp.take<unsigned char>(temp_bytes);
+    };
+    lay_out();
+    int rc = need_scratch(h, sp.off);
     if (rc != MASCOT_OK) return rc;
-    CU(h, launch_stream_sort(h->tr_r, h->tr_u, h->tr_i, h->tr_src, n, sp.seg, nseg, seg_bits, run_window_log2, h->irows, sp.key_a, sp.key_b, sp.idx_a, sp.idx_b,
-                             sp.temp, temp_bytes, sp.r, sp.u, sp.i, sp.src, h->stream));
+    sp.base = static_cast<unsigned char*>(h->d_scratch);
+    lay_out();
+    CU(h, cudaMemcpyAsync(sp.seg, h->seg_off.data(), sizeof(uint64_t) * (nseg + 1), cudaMemcpyHostToDevice, h->stream));
+    CU(h, launch_stream_sort(h->tr_r, h->tr_u, h->tr_i, h->tr_src, n, sp.seg, nseg, seg_bits, run_window_log2, h->irows, key_a, key_b, idx_a, idx_b,
+                             temp, temp_bytes, sp.r, sp.u, sp.i, sp.src, h->stream));
     if ((rc = take_reordered(h, sp)) != MASCOT_OK) return rc;
     CU(h, cudaStreamSynchronize(h->stream));
     return MASCOT_OK;
@@ -271,28 +275,41 @@ static int partition_by_class(mascot_handle* h) {
     const size_t nseg = h->seg_off.size() - 1;
     h->cls_off.assign(nseg * 5, 0);
     if (n == 0) return MASCOT_OK;
-    int key_bits = 2;
-    while ((1ull << key_bits) < nseg * 4) key_bits++;
-    const size_t temp_bytes = class_partition_temp_bytes(n, key_bits);
+    std::vector<uint32_t> first_tile(nseg + 1), first(nseg * 4);
+    const uint32_t tiles = class_tiles(h->seg_off.data(), (int)nseg, first_tile.data());
+    const size_t temp_bytes = class_partition_temp_bytes(tiles);
     SortSpace sp;
-    int rc = sort_space(h, sizeof(uint32_t), temp_bytes, &sp);
+    uint32_t *d_first_tile, *d_first, *place, *pos2, *counts, *starts;
+    uint8_t* cls;
+    unsigned char* temp;
+    auto lay_out = [&]() {
+        sp.off = 0;
+        sp.arrays(n, nseg);
+        d_first_tile = sp.take<uint32_t>(nseg + 1); d_first = sp.take<uint32_t>(nseg * 4);
+        place = sp.take<uint32_t>(n); pos2 = sp.take<uint32_t>(n); cls = sp.take<uint8_t>(n);
+        counts = sp.take<uint32_t>(4 * (size_t)tiles); starts = sp.take<uint32_t>(4 * (size_t)tiles);
+        temp = sp.take<unsigned char>(temp_bytes);
+    };
+    lay_out();
+    int rc = need_scratch(h, sp.off);
     if (rc != MASCOT_OK) return rc;
+    sp.base = static_cast<unsigned char*>(h->d_scratch);
+    lay_out();
     // Without memory for the positions the classes keep the order that the last partition gave them.
     if (!h->moved && reserve(h, &h->tr_pos, n) != cudaSuccess) { cudaGetLastError(); dev_free(h->tr_pos, h->stream); }
-    uint32_t* const pos2 = h->tr_pos ? static_cast<uint32_t*>(sp.key_a) : nullptr;
-    CU(h, launch_class_partition(h->tr_r, h->tr_u, h->tr_i, h->tr_src, h->moved ? h->tr_pos : nullptr, n, sp.seg, (int)nseg, key_bits,
-                                 static_cast<uint32_t*>(sp.key_a), static_cast<uint32_t*>(sp.key_b), sp.idx_a, sp.idx_b, sp.temp, temp_bytes, sp.first,
-                                 sp.r, sp.u, sp.i, sp.src, pos2, h->stream));
+    if (!h->tr_pos) pos2 = nullptr;
+    CU(h, cudaMemcpyAsync(sp.seg, h->seg_off.data(), sizeof(uint64_t) * (nseg + 1), cudaMemcpyHostToDevice, h->stream));
+    CU(h, cudaMemcpyAsync(d_first_tile, first_tile.data(), sizeof(uint32_t) * (nseg + 1), cudaMemcpyHostToDevice, h->stream));
+    CU(h, launch_class_partition(h->tr_r, h->tr_u, h->tr_i, h->tr_src, h->moved ? h->tr_pos : nullptr, n, sp.seg, d_first_tile, (int)nseg, tiles, cls, place,
+                                 counts, starts, temp, temp_bytes, d_first, sp.r, sp.u, sp.i, sp.src, pos2, h->stream));
     if ((rc = take_reordered(h, sp)) != MASCOT_OK) return rc;
     if (pos2) CU(h, cudaMemcpyAsync(h->tr_pos, pos2, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
-    std::vector<unsigned long long> first(nseg * 4);
-    CU(h, cudaMemcpyAsync(first.data(), sp.first, sizeof(unsigned long long) * first.size(), cudaMemcpyDeviceToHost, h->stream));
+    CU(h, cudaMemcpyAsync(first.data(), d_first, sizeof(uint32_t) * first.size(), cudaMemcpyDeviceToHost, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
     h->moved = pos2 != nullptr;
     for (size_t j = 0; j < nseg; j++) {
-        uint64_t* off = &h->cls_off[j * 5];
-        off[4] = h->seg_off[j + 1];
-        for (int c = 3; c >= 0; c--) off[c] = first[j * 4 + c] == ~0ull ? off[c + 1] : first[j * 4 + c];
+        for (int c = 0; c < 4; c++) h->cls_off[j * 5 + c] = first[j * 4 + c];
+        h->cls_off[j * 5 + 4] = h->seg_off[j + 1];
     }
     return MASCOT_OK;
 }
