@@ -350,6 +350,89 @@ __device__ __forceinline__ __half2 worker_dot(const Vh<4>& a, const Vh<4>& b, un
     return worker_sum<TS / 2>(__hadd2_rn(__low2half2(t), __high2half2(t)), wmask, After<Mid>{mid});
 }
 
+// The same sum through shared memory: every lane puts its partial down and reads all of them, and adds them up in the order of
+// the butterfly - half of the shuffles' latency at as many instructions.  slot: room for the worker's partials, 2 or 4
+// bytes each; steps take two of them in turn, so that one warp barrier a step keeps what is read from what is written next.
+__device__ __forceinline__ uint4 lds128(unsigned addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+template <int P, class Mid>
+__device__ __forceinline__ __half2 tree_sum(__half2 x, unsigned slot, Mid mid) {      // x: the partial in both halves
+    static_assert(P == 16 || P == 8, "partials of a worker");
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(slot + 2 * (threadIdx.x & (P - 1))), "h"(__half_as_ushort(__low2half(x))) : "memory");
+    __syncwarp();
+    mid(0);
+    auto h2 = [](uint32_t w) { return *reinterpret_cast<const __half2*>(&w); };
+    const uint4 a = lds128(slot);
+    __half2 c;
+    if constexpr (P == 16) {
+        const uint4 b = lds128(slot + 16);
+        mid(1); mid(2);
+        const __half2 s0 = __hadd2_rn(h2(a.x), h2(b.x)), s1 = __hadd2_rn(h2(a.y), h2(b.y)), s2 = __hadd2_rn(h2(a.z), h2(b.z)), s3 = __hadd2_rn(h2(a.w), h2(b.w));
+        c = __hadd2_rn(__hadd2_rn(s0, s2), __hadd2_rn(s1, s3));
+    } else {
+        mid(1); mid(2);
+        c = __hadd2_rn(__hadd2_rn(h2(a.x), h2(a.z)), __hadd2_rn(h2(a.y), h2(a.w)));
+    }
+    return __hadd2_rn(__low2half2(c), __high2half2(c));
+}
+template <int P, class Mid>
+__device__ __forceinline__ float tree_sum(float x, unsigned slot, Mid mid) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 4 * (threadIdx.x & (P - 1))), "f"(x) : "memory");
+    __syncwarp();
+    mid(0);
+    auto f2 = [](uint32_t lo, uint32_t hi) { return make_float2(__uint_as_float(lo), __uint_as_float(hi)); };
+    const uint4 a = lds128(slot), b = lds128(slot + 16);
+    float2 s0, s1;                                     // sums of the partials 0 1 and 2 3 modulo 4
+    if constexpr (P == 16) {
+        const uint4 c = lds128(slot + 32), d = lds128(slot + 48);
+        mid(1); mid(2);
+        s0 = __fadd2_rn(__fadd2_rn(f2(a.x, a.y), f2(c.x, c.y)), __fadd2_rn(f2(b.x, b.y), f2(d.x, d.y)));
+        s1 = __fadd2_rn(__fadd2_rn(f2(a.z, a.w), f2(c.z, c.w)), __fadd2_rn(f2(b.z, b.w), f2(d.z, d.w)));
+    } else {
+        mid(1); mid(2);
+        s0 = __fadd2_rn(f2(a.x, a.y), f2(b.x, b.y));
+        s1 = __fadd2_rn(f2(a.z, a.w), f2(b.z, b.w));
+    }
+    const float2 s = __fadd2_rn(s0, s1);
+    return __fadd_rn(s.x, s.y);
+}
+// The same for pairs of binary16 sums; who: lanes that have a partial
+template <int P> __device__ __forceinline__ __half2 tree_sum2(__half2 x, bool who, unsigned slot) {
+    if (who) asm volatile("st.shared.u32 [%0], %1;" ::"r"(slot + 4 * (threadIdx.x & (P - 1))), "r"(*reinterpret_cast<const unsigned*>(&x)) : "memory");
+    __syncwarp();
+    auto h2 = [](uint32_t w) { return *reinterpret_cast<const __half2*>(&w); };
+    uint4 v[P / 4];
+#pragma unroll
+    for (int j = 0; j < P / 4; j++) v[j] = lds128(slot + 16 * j);
+    __half2 s[4];                                      // sums of the partials 0, 1, 2, 3 modulo 4
+    if constexpr (P == 16) {
+        s[0] = __hadd2_rn(__hadd2_rn(h2(v[0].x), h2(v[2].x)), __hadd2_rn(h2(v[1].x), h2(v[3].x)));
+        s[1] = __hadd2_rn(__hadd2_rn(h2(v[0].y), h2(v[2].y)), __hadd2_rn(h2(v[1].y), h2(v[3].y)));
+        s[2] = __hadd2_rn(__hadd2_rn(h2(v[0].z), h2(v[2].z)), __hadd2_rn(h2(v[1].z), h2(v[3].z)));
+        s[3] = __hadd2_rn(__hadd2_rn(h2(v[0].w), h2(v[2].w)), __hadd2_rn(h2(v[1].w), h2(v[3].w)));
+    } else {
+        s[0] = __hadd2_rn(h2(v[0].x), h2(v[1].x)); s[1] = __hadd2_rn(h2(v[0].y), h2(v[1].y));
+        s[2] = __hadd2_rn(h2(v[0].z), h2(v[1].z)); s[3] = __hadd2_rn(h2(v[0].w), h2(v[1].w));
+    }
+    return __hadd2_rn(__hadd2_rn(s[0], s[2]), __hadd2_rn(s[1], s[3]));
+}
+// Dot product with that sum
+template <int K, class Mid> __device__ __forceinline__ float tree_dot(const Vf<4>& a, const Vf<4>& b, unsigned slot, Mid mid) {
+    const float2 f = __ffma2_rn(pr(a, 0), pr(b, 0), __fmul2_rn(pr(a, 1), pr(b, 1)));
+    const float2 o = make_float2(__shfl_xor_sync(0xffffffffu, f.x, K / 8), __shfl_xor_sync(0xffffffffu, f.y, K / 8));
+    const float2 t = __fadd2_rn(f, o);
+    return tree_sum<K / 8>(__fadd_rn(t.x, t.y), slot, mid);
+}
+template <int K, class Mid> __device__ __forceinline__ __half2 tree_dot(const Vh<4>& a, const Vh<4>& b, unsigned slot, Mid mid) {
+    const __half2 f = __hfma2(a.v[0], b.v[0], __hmul2_rn(a.v[1], b.v[1]));
+    const unsigned o = __shfl_xor_sync(0xffffffffu, *reinterpret_cast<const unsigned*>(&f), K / 8);
+    const __half2 t = __hadd2_rn(f, *reinterpret_cast<const __half2*>(&o));
+    return tree_sum<K / 8>(__hadd2_rn(__low2half2(t), __high2half2(t)), slot, mid);
+}
+
 // The chain over four lanes' worth of elements where a lane has two of each: the lanes with e0, e1 begin, those with e2, e3 go on;
 // the lane tree goes through the latter, and its last step brings the sum to all.
 template <int TS, class Mid>
@@ -661,7 +744,7 @@ __device__ __forceinline__ float forward_int8(const Vf<N>& pi, const Vf<N>& qi, 
 // go through the lane tree separately and meet at the end (muppet_sgd_kernel.h:170-194,
 // afp_sgd_kernel.h:252-273)
 template <int K>
-__device__ __forceinline__ float forward_half(const V8h& ph, const V8h& qh, unsigned wmask) {
+__device__ __forceinline__ float forward_half(const V8h& ph, const V8h& qh, unsigned wmask, unsigned) {
     constexpr int TS = K / 8;
     __half2 xy;
     if (K == 128) {
@@ -681,26 +764,19 @@ __device__ __forceinline__ float forward_half(const V8h& ph, const V8h& qh, unsi
     return __half2float(__hadd_rn(__low2half(xy), __high2half(xy)));
 }
 // The same with four elements a lane.  K=128: the lanes with (e2, e6, e3, e7) hand their products to those that have the first
-// terms of the sums, and in the last step of the tree every lane takes both values from them.  K=64: both lanes add both products.
+// terms of the sums.  K=64: both lanes add both products.
 template <int K>
-__device__ __forceinline__ float forward_half(const Vh<4>& ph, const Vh<4>& qh, unsigned wmask) {
-    constexpr int TS = K / 4;
-    auto from = [&](const __half2& v, int lane_of) {
-        const unsigned o = __shfl_sync(wmask, *reinterpret_cast<const unsigned*>(&v), lane_of, TS);
+__device__ __forceinline__ float forward_half(const Vh<4>& ph, const Vh<4>& qh, unsigned wmask, unsigned slot) {
+    auto other = [&](const __half2& v) {
+        const unsigned o = __shfl_xor_sync(wmask, *reinterpret_cast<const unsigned*>(&v), K / 8);
         return *reinterpret_cast<const __half2*>(&o);
     };
-    const int l = threadIdx.x & (TS - 1);
     const __half2 m0 = __hmul2_rn(ph.v[0], qh.v[0]), m1 = __hmul2_rn(ph.v[1], qh.v[1]);
-    const __half2 o0 = from(m0, l ^ (TS / 2)), o1 = from(m1, l ^ (TS / 2));
+    const __half2 o0 = other(m0), o1 = other(m1);
     __half2 xab, yab;
     if (K == 128) { xab = __hfma2(ph.v[0], qh.v[0], o0); yab = __hfma2(ph.v[1], qh.v[1], o1); }
     else { xab = __hadd2_rn(m0, o0); yab = __hadd2_rn(m1, o1); }
-    __half2 xy = __hadd2_rn(__lows2half2(xab, yab), __highs2half2(xab, yab));
-#pragma unroll
-    for (int d = TS / 4; d >= 2; d >>= 1) xy = __hadd2_rn(xy, from(xy, l ^ d));
-    const int low = l & (TS / 2 - 1);
-    const __half2 last = from(xy, low ^ 1);
-    xy = __hadd2_rn(K == 128 ? from(xy, low) : xy, last);
+    const __half2 xy = tree_sum2<K / 8>(__hadd2_rn(__lows2half2(xab, yab), __highs2half2(xab, yab)), !(threadIdx.x & (K / 8)), slot);
     return __half2float(__hadd_rn(__low2half(xy), __high2half(xy)));
 }
 // backward passes: g_p = q*e + p*(-lam), g_q = p*e + q*(-lam) in int8 or binary16 fixed point; e, l: error and -lam on the grid, rev: 1 / (sb sb)
@@ -747,7 +823,7 @@ template <int TS> __device__ __noinline__ float muppet_back_scale_exact(int bits
 // steps of its grid)?  The rows are rounded with the scale of the keys before that is known, and again where it is so.
 // INT8: passes of 8 bits; else 12 to 16 bits on a binary16 grid.
 template <int K, bool INT8, int N, class Mid>
-__device__ __forceinline__ void muppet_update(const Consts& c, float r, Vf<N>& p, Vf<N>& q, Vf<N>& gp, Vf<N>& gq, Mid mid) {
+__device__ __forceinline__ void muppet_update(const Consts& c, float r, Vf<N>& p, Vf<N>& q, Vf<N>& gp, Vf<N>& gq, unsigned slot, Mid mid) {
     constexpr int TS = K / N;
     constexpr unsigned kAll = 0xffffffffu;
     const int bits = INT8 ? 8 : c.bits;
@@ -779,7 +855,7 @@ __device__ __forceinline__ void muppet_update(const Consts& c, float r, Vf<N>& p
     if constexpr (INT8) pred = forward_int8<TS>(pi, qi, both_rev);
     else {
         to_grid(p, pi, sp, sp_rev, q, qi, sq, sq_rev, big, ph, qh);
-        pred = forward_half<K>(ph, qh, kAll);
+        pred = forward_half<K>(ph, qh, kAll, slot);
     }
     mid(3);
     const float ruv = __fsub_rn(r, pred);
@@ -950,7 +1026,7 @@ __device__ __noinline__ AfpSide afp_requantize(AfpSide s, float diff, float rang
 // What passes there are and when the next estimate is due only changes with an estimate, so a rating without one has two votes: is
 // there an exact half, or a value outside the int8 range (2^21 steps of the grid)?
 template <int K, int N>
-__device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float r, bool active, Vf<N>& p, Vf<N>& q) {
+__device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float r, bool active, Vf<N>& p, Vf<N>& q, unsigned slot) {
     constexpr int TS = K / N;
     constexpr unsigned kAll = 0xffffffffu;
     const unsigned cur = st.cur;
@@ -993,7 +1069,7 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
     check(st.user.scale, st.item.scale, st.forward8, 0.f, 0.f);
     if (st.forward16) {
         to_grid(p, pi, st.user.scale, st.user_rev, q, qi, st.item.scale, st.item_rev, big, ph, qh);
-        pred = forward_half<K>(ph, qh, kAll);
+        pred = forward_half<K>(ph, qh, kAll, slot);
     }
     if (st.forward8) {
         if (__builtin_expect(clamp, 0)) { pi = clamp8(pi); qi = clamp8(qi); }
@@ -1040,6 +1116,10 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
     st.cur = cur + 1;
 }
 
+// Does a launch add its dot products up through shared memory?  It shortens the chain of a rating, which bounds the narrow form; the
+// statistics use the steps of the shuffles.  A GPU full of K/8-lane workers has better uses for the shared memory (100M ratings 5.56 ->
+// 5.81 ms per epoch).
+template <int KIND, int UM, int IM, bool STATS> constexpr bool kTreeSum = !STATS && kElems<UM> == 4 && KIND != KIND_AFP && !kMuppet<KIND>;
 // Does a launch work with binary16 ratings?  Its records then hold the converted value in both halves of a word.
 template <int KIND, int UM, int IM> constexpr bool kHalfRating =
     KIND == KIND_MPT || ((KIND == KIND_MIXED || KIND == KIND_SWITCH) && kHalfRows<UM> && kHalfRows<IM>);
@@ -1051,16 +1131,19 @@ __device__ __forceinline__ __half2 half2_of(uint32_t w) { return *reinterpret_ca
 // worker has to do meanwhile, done under the shuffles of the dot product.
 template <int K, int KIND, int UM, int IM, bool STATS, class Mid>
 __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_t uc, uint32_t ic, Raw<UM>& p_raw, Raw<IM>& q_raw,
-                                           Sample<kElems<UM>>& smp, AfpState& afp, bool active, unsigned wmask, Mid mid) {
+                                           Sample<kElems<UM>>& smp, AfpState& afp, bool active, unsigned wmask, unsigned slot, Mid mid) {
     constexpr int N = kElems<UM>, TS = K / N;
     static_assert(N == kElems<IM>, "both rows are spread over the worker's lanes the same way");
     constexpr bool kAhead = KIND == KIND_AFP || UM == ROWS_DYN || IM == ROWS_DYN;      // no single dot product to hide under
+    constexpr bool kTree = kTreeSum<KIND, UM, IM, STATS>;
     if constexpr (kAhead) { mid(0); mid(1); mid(2); }
     if (STATS) { smp.user = false; smp.item = false; }
     if constexpr (KIND == KIND_MPT) {
         const Vf<N> p = as_vf(p_raw), q = as_vf(q_raw);
         const Vh<N> ph = narrow(p), qh = narrow(q);
-        const __half2 dot = worker_dot<TS>(ph, qh, wmask, mid);
+        __half2 dot;
+        if constexpr (kTree) dot = tree_dot<K>(ph, qh, slot, mid);
+        else dot = worker_dot<TS>(ph, qh, wmask, mid);
         const __half2 e = __hmul2_rn(c.mpt_scale, __hsub2_rn(half2_of(rw), dot));
         const Vf<N> gp = widen(grad(e, qh, c.mpt_nlam, ph)), gq = widen(grad(e, ph, c.mpt_nlam, qh));
         Vf<N> po, qo;
@@ -1073,19 +1156,20 @@ __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_
         put(p_raw, po); put(q_raw, qo);
     } else if constexpr (KIND == KIND_MUPPET || KIND == kMuppetHalf) {
         Vf<N> p = as_vf(p_raw), q = as_vf(q_raw);
-        muppet_update<K, KIND == KIND_MUPPET>(c, __uint_as_float(rw), p, q, smp.gp, smp.gq, mid);
+        muppet_update<K, KIND == KIND_MUPPET>(c, __uint_as_float(rw), p, q, smp.gp, smp.gq, slot, mid);
         put(p_raw, p); put(q_raw, q);
         if (STATS) smp.user = true;
     } else if constexpr (KIND == KIND_AFP) {
         Vf<N> p = as_vf(p_raw), q = as_vf(q_raw);
-        afp_update<K>(c, afp, __uint_as_float(rw), active, p, q);
+        afp_update<K>(c, afp, __uint_as_float(rw), active, p, q, slot);
         put(p_raw, p); put(q_raw, q);
     } else if constexpr (KIND == KIND_MEMQUANT) {
         const Vf<N> p = widen(as_vh(p_raw)), q = widen(as_vh(q_raw));
         float dot;
-        if constexpr (K == 64) dot = worker_dot<TS>(p, q, wmask, mid);
-        else if constexpr (N == 4) dot = worker_chain_k128<TS>(p, q, wmask, mid);
-        else dot = worker_sum<TS>(chain_partial_k128(p, q), wmask, mid);
+        if constexpr (K == 128 && N == 4) dot = worker_chain_k128<TS>(p, q, wmask, mid);
+        else if constexpr (K == 128) dot = worker_sum<TS>(chain_partial_k128(p, q), wmask, mid);
+        else if constexpr (kTree) dot = tree_dot<K>(p, q, slot, mid);
+        else dot = worker_dot<TS>(p, q, wmask, mid);
         const float e = __fsub_rn(__uint_as_float(rw), dot);
         put(p_raw, narrow(step(c.lr, grad(e, q, c.lam, p), p)));
         put(q_raw, narrow(step(c.lr, grad(e, p, c.lam, q), q)));
@@ -1094,7 +1178,8 @@ __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_
         auto both_half = [&]() {
             const Vh<N> p = as_vh(p_raw), q = as_vh(q_raw);
             __half2 dot;
-            if constexpr (kAhead) dot = worker_dot<TS>(p, q, wmask);
+            if constexpr (kTree) dot = tree_dot<K>(p, q, slot, mid);
+            else if constexpr (kAhead) dot = worker_dot<TS>(p, q, wmask);
             else dot = worker_dot<TS>(p, q, wmask, mid);
             const __half2 e = __hsub2_rn(kHalfRating<KIND, UM, IM> ? half2_of(rw) : __float2half2_rn(__uint_as_float(rw)), dot);
             const Vh<N> gp = grad(e, q, c.nlam_h, p), gq = grad(e, p, c.nlam_h, q);
@@ -1106,7 +1191,8 @@ __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_
             const Vf<N> p = uf ? as_vf(p_raw) : widen(as_vh(p_raw));
             const Vf<N> q = itf ? as_vf(q_raw) : widen(as_vh(q_raw));
             float dot;
-            if constexpr (kAhead) dot = worker_dot<TS>(p, q, wmask);
+            if constexpr (kTree) dot = tree_dot<K>(p, q, slot, mid);
+            else if constexpr (kAhead) dot = worker_dot<TS>(p, q, wmask);
             else dot = worker_dot<TS>(p, q, wmask, mid);
             const float e = __fsub_rn(__uint_as_float(rw), dot);
             const Vf<N> gp = grad(e, q, c.lam, p), gq = grad(e, p, c.lam, q);
@@ -1135,12 +1221,6 @@ template <int OFF> __device__ __forceinline__ void cp16_if_row(uint32_t row, uns
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ uint4 lds128(unsigned addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-
 // Slot layout = row layout: the first 16 bytes of every lane, then (fp32 rows) the second 16 bytes of
 // every lane (layout.cuh), so that neither the 128-bit shared-memory accesses of neighbouring lanes collide
 // on a bank nor the global accesses of a worker touch partial sectors.  `slot` includes the lane's 16 m.
@@ -1192,7 +1272,11 @@ template <int K, int UM, int IM, bool STATS, int NS, int NSI> struct WorkerSmem 
     // The records of the workers of a warp are shifted by 16 bytes from worker to worker: those read at the same time
     // then lie in different banks.  The rings stay at multiples of 128 bytes (off them, copies and loads of rows touch
     // a line more each: 5.9 instead of 5.5 ms per epoch of the 100M-rating set).
-    static constexpr int kShift = 128;
+    // Behind the records of the narrow form follow two slots for the partials of a dot product (tree_sum): 64 bytes, which the shift
+    // leaves of its 128 - or 128, and as much room more, for partials of four bytes at k=128.
+    static constexpr bool kWideSlots = K == 128 && kElems<UM> == 4 && !(kHalfRows<UM> && kHalfRows<IM>);
+    static constexpr int kSlotBytes = kWideSlots ? 64 : 32;
+    static constexpr int kShift = kWideSlots ? 256 : 128;
     // With statistics: the groups of both rows of every record, looked up for a whole chunk at once.  (A lookup per
     // rating is a memory latency per rating: the sampled twentieth of an epoch took a seventh of its time.)
     static constexpr int kGroupBytes = STATS ? 2 * TS * 4 : 0;
@@ -1230,6 +1314,7 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
     uint32_t* const reqs = reinterpret_cast<uint32_t*>(recs + 2 * TS);          // [2][TS][user, item]
     const unsigned s_rec = (unsigned)__cvta_generic_to_shared(recs);
     const unsigned s_req = s_rec + 2 * TS * 16;
+    const unsigned slots = s_req + 2 * TS * 8;
     const unsigned rings = (unsigned)__cvta_generic_to_shared(mine) + SM::kRecBytes + SM::kShift;
     const unsigned uring = rings + lane_at<K, UM>(m);                            // [NS][kURowBytes]
     const unsigned iring = rings + NS * SM::kURowBytes + lane_at<K, IM>(m);      // [NSI][kIRowBytes]
@@ -1514,7 +1599,7 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
                 };
                 const Raw<UM> p_before = p;
                 constexpr bool kDyn = UM == ROWS_DYN || IM == ROWS_DYN;
-                update_one<K, KIND, UM, IM, STATS>(c, rw, uc, ic, p, q, smp, afp, !(f & F_NONE), kDyn ? gmask : kAll, meanwhile);
+                update_one<K, KIND, UM, IM, STATS>(c, rw, uc, ic, p, q, smp, afp, !(f & F_NONE), kDyn ? gmask : kAll, slots + (t & 1) * SM::kSlotBytes, meanwhile);
                 if (a.add_user_delta) add_row_delta<K, UM>(P, uc, f & F_DROP, p, p_before);
                 else st_row_if<K, UM>(~f & F_DROP, P, uc, p);
                 if constexpr (kWhole) record_whole(smp, !(f & F_NONE));
@@ -1641,16 +1726,16 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
     constexpr int NS = kFixedPoint ? 4 : 8, D = kFixedPoint ? 3 : 5, DI = kFixedPoint ? 2 : 3;
     // A step of few warps is a chain of some ninety instructions.  With K/4 lanes a worker the warp has half of the row work
     // and one worker fewer to wait for: shorter steps, on twice as many warps - as long as the schedulers can take those.  ms per
-    // epoch with K/8 and K/4 lanes, by warps of the narrow form per SM: AFP 4M ratings (4) 5.69 and 4.43, 12M (10) 8.94 and 6.30; MuPPET
-    // 2M (4) 2.25 and 1.71, 14M (12) 5.73 and 5.04; MPT 8M (8) 1.81 and 1.50, 16M (14) 2.39 and 2.13; SGD 8M (8) 1.52 and 1.31, 16M (14)
-    // 2.08 and 2.05, k=64 0.8M (6) 0.132 and 0.105, 20M (10) 2.04 and 1.69; fp16 storage 8M 1.64 and 1.47, 16M (14) 2.13 and 2.04; MASCOT
-    // k=64 8M (4) 1.44 and 1.23, 20M (10) 1.56 and 1.45, 30M (14) 1.73 and 1.70, 40 % promoted, 16M (14) 3.67 and 3.57.  At 18 and more
-    // the narrow form gives nothing more (SGD 20M 2.45 and 2.46) or loses (fp16 storage 20M 2.08 and 2.23).  Binary16 rows
-    // with packed binary16 arithmetic have the shortest steps and stop gaining earlier: k=128, 2M (4) 0.637 and 0.590, 6M (6) 1.28
-    // and 1.255, 8M (8) 1.302 and 1.300, 20M (18) 1.68 and 1.94.
+    // epoch with K/8 and K/4 lanes, by warps of the narrow form per SM: AFP 4M ratings (4) 5.69 and 3.37, 12M (10) 8.94 and 5.17; MuPPET,
+    // 8 bits, 2M (4) 2.25 and 1.13, 14M (12) 5.73 and 4.08; MPT 8M (8) 1.81 and 1.37, 18M (16) 2.38 and 2.16; SGD 8M (8) 1.52 and
+    // 1.24, 16M (14) 2.08 and 1.92, k=64 0.8M (6) 0.132 and 0.100, 20M (10) 2.04 and 1.64; fp16 storage 8M 1.64 and 1.47, 16M (14) 2.13 and
+    // 2.04; MASCOT k=64 8M (4) 1.44 and 1.19, 20M (10) 1.56 and 1.41, 30M (14) 1.73 and 1.66, 40 % promoted, 16M (14) 2.25 and 2.18.  At 18 and
+    // more the narrow form gives nothing more (SGD 20M 2.32 and 2.32) or loses (fp16 storage 20M 2.08 and 2.23).  Binary16 rows with
+    // packed binary16 arithmetic have the shortest steps and stop gaining earlier: k=128, 2M (4) 0.637 and 0.531, 8M (8) 1.302 and
+    // 1.184, 14M (12) 1.646 and 1.565, 16M (14) 1.659 and 1.671, 20M (18) 1.66 and 1.91.
     if constexpr (UM != ROWS_DYN) {
         constexpr int UQ = UM == ROWS_HALF ? ROWS_HALFQ : ROWS_F32Q, IQ = IM == ROWS_HALF ? ROWS_HALFQ : ROWS_F32Q;
-        constexpr unsigned kMost = K == 128 && kHalfRating<KIND, UM, IM> && KIND != KIND_MPT && !STATS ? 8 : 16;      // warps per SM
+        constexpr unsigned kMost = K == 128 && kHalfRating<KIND, UM, IM> && KIND != KIND_MPT && !STATS ? 12 : 16;      // warps per SM
         // (a single block has exactly the workers that were asked for: they have to fit it in this form, too)
         if (2 * per_sm <= kMost && (warps > 8 || 2 * workers <= 8 * kPerWarp))
             return launch_ns<K, KIND, UQ, IQ, STATS, NS, 4, D, DI>(args, 2 * per_sm, workers, st, shape, dry);
