@@ -521,6 +521,15 @@ template <int N> struct Sample {
     bool user, item;      // which sides of this rating contribute (binary16-stored rows only)
 };
 
+// ... unless `skip`
+template <int N> __device__ __forceinline__ void red_add_if_not(unsigned skip, float* dst, const Vf<N>& g) {
+    const unsigned char* const p = reinterpret_cast<const unsigned char*>(dst);
+    red_f32x4<0>(p, skip, g.x[0], g.x[1], g.x[2], g.x[3]);
+    if constexpr (N == 8) red_f32x4<16>(p, skip, g.x[4], g.x[5], g.x[6], g.x[7]);
+}
+__device__ __forceinline__ void red_add_if_not(unsigned skip, float* dst, float x) {
+    asm volatile("{ .reg .pred s; setp.ne.u32 s, %2, 0; @!s red.global.add.f32 [%0], %1; }" ::"l"(dst), "f"(x), "r"(skip) : "memory");
+}
 template <int N> __device__ __forceinline__ void red_add(float* dst, const Vf<N>& g) {
     atomicAdd(reinterpret_cast<float4*>(dst), make_float4(g.x[0], g.x[1], g.x[2], g.x[3]));
     if constexpr (N == 8) atomicAdd(reinterpret_cast<float4*>(dst) + 1, make_float4(g.x[4], g.x[5], g.x[6], g.x[7]));
@@ -1480,8 +1489,62 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
     constexpr bool kWhole = STATS && (kMuppet<KIND> || KIND == KIND_SWITCH);
     float norm = 0.f;
     float4 norm_parts = make_float4(0.f, 0.f, 0.f, 0.f);      // with four elements a lane: what the first step joins
+    // MASCOT: the same for the norms of both sides, each with the group it belongs to.  Nothing of it branches where the workers of
+    // a warp could differ, and the two sums run under the next rating's dot product: a sampled rating took four times as
+    // long as another one (check epoch of 8M ratings 1.353 -> 1.302 ms, k=64 20M 1.594 -> 1.531; 100M: no change, there the sums are traffic).
+    constexpr bool kDefer = kGroups && UM != ROWS_DYN && IM != ROWS_DYN;
+    constexpr bool kUserStats = kHalfRows<UM>, kItemStats = kHalfRows<IM>;
+    float norm_q = 0.f;
+    uint32_t late_groups = 0;
+    bool late = false;                               // is there a rating before whose norms are to be added?
+    auto late_step = [&](int part) {
+        auto add = [&](float v) { return __fadd_rn(v, __shfl_xor_sync(kAll, v, (TS / 2) >> part)); };
+        if (N == 4 && part == 0) {
+            if (kUserStats) norm = __fadd_rn(add(norm_parts.x), add(norm_parts.y));
+            if (kItemStats) norm_q = __fadd_rn(add(norm_parts.z), add(norm_parts.w));
+        } else if ((TS / 2) >> part) {
+            if (kUserStats) norm = add(norm);
+            if (kItemStats) norm_q = add(norm_q);
+        }
+    };
+    auto late_norms = [&]() {
+        if (kUserStats) red_add_if_not(!late || m != 0, nsum_p + (late_groups & 0xffffu), norm);
+        if (kItemStats && late) nq_acc = __fadd_rn(nq_acc, norm_q);
+    };
+    auto record_deferred = [&](const Sample<N>& smp, uint32_t both_groups, bool there) {
+        late_norms();
+        if (kUserStats) red_add_if_not(!there, gsum_p + (size_t)(both_groups & 0xffffu) * K + stat_at, smp.gp);
+        if (kItemStats) {
+            const uint32_t g = both_groups >> 16;
+            const bool other = there && g != acc_group;
+            if (__any_sync(kAll, other)) {
+                const unsigned skip = !other || acc_group == kNoRow;
+                const uint32_t to = skip ? 0u : acc_group;
+                red_add_if_not(skip, gsum_q + (size_t)to * K + stat_at, gq_acc);
+                red_add_if_not(skip || m != 0, nsum_q + to, nq_acc);
+                if (other) {
+                    acc_group = g; nq_acc = 0.f;
+#pragma unroll
+                    for (int t = 0; t < N; t++) gq_acc.x[t] = 0.f;
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < N; t++) gq_acc.x[t] = there ? __fadd_rn(gq_acc.x[t], smp.gq.x[t]) : gq_acc.x[t];
+        }
+        late = there; late_groups = both_groups;
+        if constexpr (N == 4) {
+            float2 p2 = make_float2(0.f, 0.f), q2 = p2;
+            if (kUserStats) p2 = __ffma2_rn(pr(smp.gp, 0), pr(smp.gp, 0), __fmul2_rn(pr(smp.gp, 1), pr(smp.gp, 1)));
+            if (kItemStats) q2 = __ffma2_rn(pr(smp.gq, 0), pr(smp.gq, 0), __fmul2_rn(pr(smp.gq, 1), pr(smp.gq, 1)));
+            norm_parts = make_float4(p2.x, p2.y, q2.x, q2.y);
+        } else {
+            if (kUserStats) norm = pair_partial(smp.gp, smp.gp);
+            if (kItemStats) norm_q = pair_partial(smp.gq, smp.gq);
+        }
+    };
     auto norm_step = [&](int part) {
-        if (kWhole && N == 4 && part == 0) norm = muppet_norm_join<K>(norm_parts);
+        if (kDefer) late_step(part);
+        else if (kWhole && N == 4 && part == 0) norm = muppet_norm_join<K>(norm_parts);
         else if (kWhole && (TS / 2) >> part) norm = __fadd_rn(norm, __shfl_xor_sync(kAll, norm, (TS / 2) >> part));
     };
     auto record_whole = [&](const Sample<N>& smp, bool there) {
@@ -1603,6 +1666,7 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
                 if (a.add_user_delta) add_row_delta<K, UM>(P, uc, f & F_DROP, p, p_before);
                 else st_row_if<K, UM>(~f & F_DROP, P, uc, p);
                 if constexpr (kWhole) record_whole(smp, !(f & F_NONE));
+                else if constexpr (kDefer) record_deferred(smp, groups[cb * TS + jb + t], !(f & F_NONE));
                 else if (STATS) { if (!(f & F_NONE)) record(smp, kGroups ? groups[cb * TS + jb + t] : 0u); }
                 p = p_next;
             }
@@ -1621,7 +1685,14 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
             red_add(gsum_p + stat_at, gq_acc);
             if (m == 0) atomicAdd(nsum_p, nq_acc);
         }
-        else flush_item_stats();
+        else {
+            if constexpr (kDefer) {
+#pragma unroll
+                for (int part = 0; (TS / 2) >> part; part++) late_step(part);
+                late_norms();
+            }
+            flush_item_stats();
+        }
     }
 }
 
