@@ -118,3 +118,13 @@ def test_integer_ceil_log2_equals_the_double_precision_formula(tmp_path):
     subprocess.check_call(["gcc", "-O2", "-fopenmp", os.path.join(ROOT, "tests", "ceil_log2_check.c"), "-o", exe, "-lm"])
     out = subprocess.run([exe], capture_output=True, text=True, timeout=600)
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout
+
+
+def test_permutation_with_ready_keys_is_the_same(tmp_path):
+    exe = str(tmp_path / "permutation_check")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-I", CSRC, os.path.join(ROOT, "tests", "permutation_check.cpp"), "-o", exe])
+    cases = [(1, 3), (2, 3), (3, 0), (4, 9), (5, 2 ** 64 - 1), (17, 0), (4096, 7), (4097, 2 ** 40 + 5), (8 << 20, 1), (100_480_507, 42), (2 ** 30, 5), (2 ** 30 + 1, 5),
+             (2 ** 32 - 1, 6)]
+    out = subprocess.run([exe] + [str(x) for c in cases for x in c], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout
+    assert int(out.stdout) > 250_000
