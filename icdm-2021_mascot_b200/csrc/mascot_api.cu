@@ -951,9 +951,24 @@ int mascot_train_epoch_streamed(mascot_handle* h, uint32_t epoch, const mascot_r
         h->n_train = n_train;
     }
     CU(h, cudaMemsetAsync(h->d_err_flag, 0, sizeof(uint32_t), h->stream));
-    // the pieces become the segments of the resident stream (seeded permutation inside each piece)
+    // The pieces become the segments of the resident stream (seeded permutation inside each piece).  Beyond two of them some are
+    // smaller (multiples of 4096, the encoding kernel's windows).  Binary16 rows are coded and trained in 0.6 of the time of their
+    // copy: what follows the end of the copy counts, and the last pieces are halves of what is left (27M ratings, MASCOT 6.91 -> 6.37 ms
+    // per epoch, k=64 6.65 -> 6.07, fp16 storage 6.90 -> 6.35).  MuPPET takes longer than the copy: what comes before its start counts,
+    // and its first pieces are an eighth, a quarter and a half (9.50 -> 9.02).  Trainers with fp32 rows take about as long as the copy
+    // and lose in more launches what they gain (SGD 7.63, either way or both 7.60 to 7.73; promoted groups 7.78 and 7.86).
+    const bool binary16 = (h->kind == KIND_MIXED || h->kind == KIND_MEMQUANT || h->kind == KIND_SWITCH) && !any_fp32_group(h);
     h->seg_off.clear();
-    for (uint64_t off = 0; off < n_train; off += piece) h->seg_off.push_back(off);
+    for (uint64_t off = 0, c = 0; off < n_train; c++) {
+        h->seg_off.push_back(off);
+        const uint64_t left = n_train - off;
+        uint64_t len = std::min(piece, left);
+        if (n_train > 2 * piece && !h->cfg.deterministic) {
+            if (h->kind == KIND_MUPPET && c < 3) len = piece >> (3 - c);
+            else if (binary16 && left <= 2 * piece && left > piece / 4) len = (left / 2 + 4095) / 4096 * 4096;
+        }
+        off += len;
+    }
     h->seg_off.push_back(n_train);
     // The pieces are not partitioned by precision class: finding the class boundaries needs a read-back,
     // i.e. a host wait per piece, which would stall the upload pipeline.  With promoted groups every piece

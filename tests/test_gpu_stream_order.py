@@ -121,3 +121,24 @@ def test_classes_keep_the_coded_order(mascot, seg, shuffle):
         eng.promote_group(1, min(1, len(ends[1]) - 1))
         eng.promote_group(0, min(2, len(ends[0]) - 1))
         assert (eng.stream_order() == expected(piece, [0, n])).all()
+
+
+@pytest.mark.parametrize("version,parts", [("mascot", [64, 34, 17, 8.5, 8.5]), ("muppet", [8, 16, 32, 64, 12]), ("sgd", [64, 64, 4])])
+def test_pieces_of_a_long_streamed_epoch(mascot, version, parts):
+    """Beyond two pieces the first or the last ones are smaller (sizes in 64ths of a piece); each is a permutation of its own range, and all are trained."""
+    n_users, n_items, n = 7001, 301, (8 << 20) // 64 * int(sum(parts)) + 77
+    R, P, Q = random_problem(np.random.default_rng(4), n_users, n_items, n, 64)
+    v = dict(mascot=mascot.V_MASCOT, muppet=mascot.V_MUPPET, sgd=mascot.V_SGD)[version]
+    with mascot.Engine(mascot.default_config(version=v, k=64, num_workers=4096, learning_rate=1e-4)) as eng:
+        eng.set_ratings(R[:1000], R[:50], n_users, n_items)
+        eng.set_factors(P, Q)
+        assert eng.train_epoch_streamed(0, R).updates == n
+        order = eng.stream_order()
+        sizes = [eng.train_segment(1, s).updates for s in range(len(parts))]
+        with pytest.raises(mascot.MascotError):
+            eng.train_segment(1, len(parts))
+    assert sum(sizes) == n and all(abs(s - e * (8 << 20) / 64) <= 4096 for s, e in zip(sizes, parts))
+    at = 0
+    for s in sizes:
+        assert at % 4096 == 0 and (np.bincount(order[at:at + s] - at, minlength=s) == 1).all()
+        at += s
