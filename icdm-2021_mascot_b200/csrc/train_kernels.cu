@@ -379,8 +379,8 @@ __device__ __forceinline__ __half2 tree_sum(__half2 x, unsigned slot, Mid mid) {
     return __hadd2_rn(__low2half2(c), __high2half2(c));
 }
 template <int P, class Mid>
-__device__ __forceinline__ float tree_sum(float x, unsigned slot, Mid mid) {
-    asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 4 * (threadIdx.x & (P - 1))), "f"(x) : "memory");
+__device__ __forceinline__ float tree_sum(float x, unsigned slot, Mid mid, bool who = true) {      // who: lanes that have a partial
+    if (who) asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 4 * (threadIdx.x & (P - 1))), "f"(x) : "memory");
     __syncwarp();
     mid(0);
     auto f2 = [](uint32_t lo, uint32_t hi) { return make_float2(__uint_as_float(lo), __uint_as_float(hi)); };
@@ -433,27 +433,17 @@ template <int K, class Mid> __device__ __forceinline__ __half2 tree_dot(const Vh
     return tree_sum<K / 8>(__hadd2_rn(__low2half2(t), __high2half2(t)), slot, mid);
 }
 
-// The chain over four lanes' worth of elements where a lane has two of each: the lanes with e0, e1 begin, those with e2, e3 go on;
-// the lane tree goes through the latter, and its last step brings the sum to all.
-template <int TS, class Mid>
-__device__ __forceinline__ float worker_chain_k128(const Vf<4>& a, const Vf<4>& b, unsigned wmask, Mid mid) {
-    const int m = threadIdx.x & (TS - 1);
-    const bool up = m & (TS / 2);
-    float c[2], begun[2];
+// The chain over four lanes' worth of elements where a lane has two of each: the lanes with e0, e1 begin, those with e2, e3 go on,
+// and put down what is added up.
+template <int K, class Mid>
+__device__ __forceinline__ float tree_chain_k128(const Vf<4>& a, const Vf<4>& b, unsigned slot, Mid mid) {
+    float c[2];
 #pragma unroll
-    for (int h = 0; h < 2; h++) begun[h] = __shfl_xor_sync(wmask, __fmaf_rn(a.x[h], b.x[h], __fmul_rn(a.x[2 + h], b.x[2 + h])), TS / 2);
-    mid(0);
-#pragma unroll
-    for (int h = 0; h < 2; h++) c[h] = __fmaf_rn(a.x[2 + h], b.x[2 + h], __fmaf_rn(a.x[h], b.x[h], begun[h]));
-    float x = __fadd_rn(c[0], c[1]);
-#pragma unroll
-    for (int d = TS / 4, i = 1; d >= 2; d >>= 1, i++) {
-        const float o = __shfl_xor_sync(wmask, x, d);
-        mid(i);
-        x = __fadd_rn(x, o);
+    for (int h = 0; h < 2; h++) {
+        const float begun = __shfl_xor_sync(0xffffffffu, __fmaf_rn(a.x[h], b.x[h], __fmul_rn(a.x[2 + h], b.x[2 + h])), K / 8);
+        c[h] = __fmaf_rn(a.x[2 + h], b.x[2 + h], __fmaf_rn(a.x[h], b.x[h], begun));
     }
-    const float o = __shfl_sync(wmask, x, (m ^ 1) | (TS / 2), TS), own = __shfl_sync(wmask, x, m | (TS / 2), TS);
-    return __fadd_rn(up ? x : own, o);
+    return tree_sum<K / 8>(__fadd_rn(c[0], c[1]), slot, mid, threadIdx.x & (K / 8));
 }
 
 // t = fma(e, y, -(lam*x)) and x' = fma(lr, t, x), element-wise
@@ -1175,7 +1165,7 @@ __device__ __forceinline__ void update_one(const Consts& c, uint32_t rw, uint32_
     } else if constexpr (KIND == KIND_MEMQUANT) {
         const Vf<N> p = widen(as_vh(p_raw)), q = widen(as_vh(q_raw));
         float dot;
-        if constexpr (K == 128 && N == 4) dot = worker_chain_k128<TS>(p, q, wmask, mid);
+        if constexpr (K == 128 && N == 4) dot = tree_chain_k128<K>(p, q, slot, mid);
         else if constexpr (K == 128) dot = worker_sum<TS>(chain_partial_k128(p, q), wmask, mid);
         else if constexpr (kTree) dot = tree_dot<K>(p, q, slot, mid);
         else dot = worker_dot<TS>(p, q, wmask, mid);
@@ -1273,7 +1263,7 @@ constexpr uint32_t F_NONE = 16u;    // there is no rating at this position
 // user row of the rating D further on, the item row of the rating DI further on if a run starts there), then the user
 // ring, then the item ring.  A ring
 // slot is as large as the widest row its side can hold in this launch.
-template <int K, int UM, int IM, bool STATS, int NS, int NSI> struct WorkerSmem {
+template <int K, int KIND, int UM, int IM, bool STATS, int NS, int NSI> struct WorkerSmem {
     static constexpr int TS = K / kElems<UM>;
     static constexpr int kURowBytes = K * (kHalfRows<UM> ? 2 : 4);
     static constexpr int kIRowBytes = K * (kHalfRows<IM> ? 2 : 4);
@@ -1283,7 +1273,7 @@ template <int K, int UM, int IM, bool STATS, int NS, int NSI> struct WorkerSmem 
     // a line more each: 5.9 instead of 5.5 ms per epoch of the 100M-rating set).
     // Behind the records of the narrow form follow two slots for the partials of a dot product (tree_sum): 64 bytes, which the shift
     // leaves of its 128 - or 128, and as much room more, for partials of four bytes at k=128.
-    static constexpr bool kWideSlots = K == 128 && kElems<UM> == 4 && !(kHalfRows<UM> && kHalfRows<IM>);
+    static constexpr bool kWideSlots = K == 128 && kElems<UM> == 4 && (!(kHalfRows<UM> && kHalfRows<IM>) || KIND == KIND_MEMQUANT);
     static constexpr int kSlotBytes = kWideSlots ? 64 : 32;
     static constexpr int kShift = kWideSlots ? 256 : 128;
     // With statistics: the groups of both rows of every record, looked up for a whole chunk at once.  (A lookup per
@@ -1298,7 +1288,7 @@ template <int K, int UM, int IM, bool STATS, int NS, int NSI> struct WorkerSmem 
 // request and the write-back loses that update, and the chance of that grows with the lead.
 template <int K, int KIND, int UM, int IM, bool STATS, int NS, int NSI, int D, int DI>
 __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS) ? 4 : ((UM == ROWS_DYN || STATS || KIND == KIND_AFP || kMuppet<KIND>) ? 2 : 3)) train_kernel(const KernelArgs a) {
-    using SM = WorkerSmem<K, UM, IM, STATS, NS, NSI>;
+    using SM = WorkerSmem<K, KIND, UM, IM, STATS, NS, NSI>;
     constexpr int TS = SM::TS;                     // lanes per worker = ratings per chunk
     constexpr int N = kElems<UM>;                  // elements per lane
     constexpr unsigned kSpan = K / TS;             // consecutive chunks handed out together: K ratings, the longest run of one ticket
@@ -1708,7 +1698,7 @@ template <int K, int KIND, int UM, int IM, bool STATS, int NS, int NSI, int D, i
 cudaError_t launch_ns(KernelArgs a, unsigned warps_per_sm, unsigned workers, cudaStream_t st, LaunchShape* shape, bool dry) {
     constexpr int TS = K / kElems<UM>;
     constexpr int kPerWarp = 32 / TS;
-    using SM = WorkerSmem<K, UM, IM, STATS, NS, NSI>;
+    using SM = WorkerSmem<K, KIND, UM, IM, STATS, NS, NSI>;
     auto kern = train_kernel<K, KIND, UM, IM, STATS, NS, NSI, D, DI>;
     // the most dynamic shared memory a launch of this instantiation can ask for: a block of 8 warps
     constexpr size_t kSmemMax = (size_t)8 * kPerWarp * SM::kBytes;
