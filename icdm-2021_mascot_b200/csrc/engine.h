@@ -129,10 +129,12 @@ cudaError_t launch_class_partition(const float* r, const uint32_t* u, const uint
 // coded - the order that launch_encode_stream and launch_stream_sort give, in one sort.  source_sort_bytes: the scratch it
 // wants, or 0 where it does not apply (no run windows, segments that begin off the encoding step's windows, keys beyond 32
 // bits).  seg_off: nseg + 1 offsets in host memory.
+// source_sort_items: a part of that scratch in which the caller may leave the item ids of the array alone (`items`, else null).
 size_t source_sort_bytes(uint64_t n, const uint64_t* seg_off, int nseg, int run_window_log2, uint32_t item_rows);
+uint32_t* source_sort_items(void* space, uint64_t n);
 cudaError_t launch_source_sort(const void* d_src_aos, uint64_t n, const uint64_t* seg_off, int nseg, uint64_t seed, int run_window_log2, uint32_t item_rows,
                                const uint32_t* user_map, const uint32_t* item_map, const uint8_t* uprec_row, const uint8_t* iprec_row,
-                               uint32_t n_users, uint32_t n_items, uint32_t* err_flag, void* space, float* r, uint32_t* u, uint32_t* i, uint32_t* src_out,
+                               uint32_t n_users, uint32_t n_items, uint32_t* err_flag, void* space, const uint32_t* items, float* r, uint32_t* u, uint32_t* i, uint32_t* src_out,
                                cudaStream_t st);
 cudaError_t launch_scatter_factors(int K, const float* src, uint32_t rows, const uint32_t* row_map,
                                    bool round_through_half, __half* dst16, float* dst32, cudaStream_t st);

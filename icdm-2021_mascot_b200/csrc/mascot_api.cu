@@ -530,7 +530,7 @@ int mascot_reload_train(mascot_handle* h, const mascot_rating* train, uint64_t n
     CU(h, copy_to_device(h->d_scratch, train, bytes, h->stream));
     if (sort_bytes)
         CU(h, launch_source_sort(h->d_scratch, n_train, h->seg_off.data(), nseg, h->cfg.seed, run_window, h->irows, h->d_umap, h->d_imap, h->d_uprec_row, h->d_iprec_row,
-                                 h->n_users, h->n_items, h->d_err_flag, static_cast<unsigned char*>(h->d_scratch) + sort_at, h->tr_r, h->tr_u, h->tr_i, h->tr_src, h->stream));
+                                 h->n_users, h->n_items, h->d_err_flag, static_cast<unsigned char*>(h->d_scratch) + sort_at, nullptr, h->tr_r, h->tr_u, h->tr_i, h->tr_src, h->stream));
     else
         CU(h, encode_segments(h, static_cast<const mascot_rating*>(h->d_scratch), h->seg_off, h->cfg.shuffle != 0,
                               h->tr_r, h->tr_u, h->tr_i, h->tr_src));

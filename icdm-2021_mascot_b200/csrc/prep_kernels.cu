@@ -472,13 +472,13 @@ cudaError_t launch_class_partition(const float* r, const uint32_t* u, const uint
 // follow - whose boundaries fall on multiples of kWindow - a stable sort of the permuted SOURCE positions by (segment, run
 // window, item row) gives the same order in one go: the block sort, the second pass over the coded arrays and the
 // copies back fall away, and the key fits 32 bits.
-__global__ void source_key_kernel(const NodeAos* src, uint64_t n, const uint64_t* seg_off, int nseg, uint64_t seed, Permutation first, const uint32_t* imap, uint32_t n_items,
+__global__ void source_key_kernel(const NodeAos* src, const uint32_t* items, uint64_t n, const uint64_t* seg_off, int nseg, uint64_t seed, Permutation first, const uint32_t* imap, uint32_t n_items,
                                   StreamKey sk, uint32_t* key, uint32_t* val) {
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x) {
         const int lo = segment_of(j, seg_off, nseg);
         const uint64_t off = seg_off[lo], seg_seed = seed + 0x9e3779b97f4a7c15ull * (uint64_t)lo;
         const uint32_t s = (uint32_t)off + permute(nseg == 1 ? first : make_permutation(seg_off[lo + 1] - off, seg_seed), (uint32_t)(j - off));
-        uint32_t it = src[s].i;
+        uint32_t it = items ? items[s] : src[s].i;
         if (it >= n_items) it = 0;                    // reported when the record is read below
         key[j] = (((uint32_t)lo << sk.window_bits | (uint32_t)(j >> sk.run_window_log2)) << sk.item_bits) | (imap ? imap[it] : it);
         val[j] = s;
@@ -515,10 +515,13 @@ size_t source_sort_bytes(uint64_t n, const uint64_t* seg_off, int nseg, int run_
     return 4 * up(4 * n) + up(8 * (size_t)(nseg + 1)) + up(temp);
 }
 
+// The last of the four buffers is not written before the keys, which are made from the item ids, are there.
+uint32_t* source_sort_items(void* space, uint64_t n) { return reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(space) + 3 * ((4 * n + 255) / 256 * 256)); }
+
 cudaError_t launch_source_sort(const void* d_src_aos, uint64_t n, const uint64_t* seg_off, int nseg, uint64_t seed, int run_window_log2, uint32_t item_rows,
                                const uint32_t* user_map, const uint32_t* item_map, const uint8_t* uprec_row, const uint8_t* iprec_row,
-                               uint32_t n_users, uint32_t n_items, uint32_t* err_flag, void* space, float* r, uint32_t* u, uint32_t* i, uint32_t* src_out,
-                               cudaStream_t st) {
+                               uint32_t n_users, uint32_t n_items, uint32_t* err_flag, void* space, const uint32_t* items, float* r, uint32_t* u, uint32_t* i,
+                               uint32_t* src_out, cudaStream_t st) {
     StreamKey sk;
     const int bits = source_key_bits(n, nseg, run_window_log2, item_rows, &sk);
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
@@ -530,7 +533,7 @@ cudaError_t launch_source_sort(const void* d_src_aos, uint64_t n, const uint64_t
     if (e != cudaSuccess) return e;
     const NodeAos* src = static_cast<const NodeAos*>(d_src_aos);
     const int g = grid_for(n, 256);
-    source_key_kernel<<<g, 256, 0, st>>>(src, n, d_seg, nseg, seed, make_permutation(n, seed), item_map, n_items, sk, buf[0], buf[1]);
+    source_key_kernel<<<g, 256, 0, st>>>(src, items, n, d_seg, nseg, seed, make_permutation(n, seed), item_map, n_items, sk, buf[0], buf[1]);
     cub::DoubleBuffer<uint32_t> keys(buf[0], buf[2]), vals(buf[1], buf[3]);
     size_t temp = 0;
     e = cub::DeviceRadixSort::SortPairs(nullptr, temp, keys, vals, n, 0, bits, st);

@@ -38,10 +38,13 @@ inline int grid_for(uint64_t n, int block) {
 }
 
 // An id out of range raises the flag and is NOT used as an index.
+// items (may be null): the item ids alone, for what reads them in another order (40M ratings: 160 MB, most of which stay in L2, in place
+// of 480 MB of records: 0.4 of the 13.6 ms of a set-up).
 __global__ void check_hist_kernel(const NodeAos* R, uint64_t n, uint32_t n_users, uint32_t n_items,
-                                  uint32_t* udeg, uint32_t* ideg, uint32_t* err) {
+                                  uint32_t* udeg, uint32_t* ideg, uint32_t* err, uint32_t* items) {
     for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t u = R[j].u, i = R[j].i;
+        if (items) items[j] = i;
         if (u >= n_users || i >= n_items) { atomicOr(err, 1u); continue; }
         if (udeg) atomicAdd(udeg + u, 1u);
         if (ideg) atomicAdd(ideg + i, 1u);
@@ -308,6 +311,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
         CU(h, cudaEventRecord(h->ev_free[0], h->stream));
         CU(h, cudaStreamWaitEvent(h->copy_stream, h->ev_free[0], 0));
     }
+    uint32_t* const items = sort_bytes ? source_sort_items(sort_space, n_all) : nullptr;
     for (uint64_t off = 0; off < n_all; off += kPiece) {
         const uint64_t len = std::min<uint64_t>(kPiece, n_all - off);
         CU(h, copy_to_device(aos + off, rq.train + off, sizeof(NodeAos) * len, pieces ? h->copy_stream : h->stream));
@@ -315,7 +319,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
             CU(h, cudaEventRecord(h->ev_copied[0], h->copy_stream));
             CU(h, cudaStreamWaitEvent(h->stream, h->ev_copied[0], 0));
         }
-        check_hist_kernel<<<grid_for(len, 256), 256, 0, h->stream>>>(aos + off, len, n_users, n_items, d_udeg, d_ideg, h->d_err_flag);
+        check_hist_kernel<<<grid_for(len, 256), 256, 0, h->stream>>>(aos + off, len, n_users, n_items, d_udeg, d_ideg, h->d_err_flag, items ? items + off : nullptr);
         CU(h, cudaGetLastError());
     }
     uint32_t bad = 0;
@@ -386,7 +390,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
         // local item degrees of the kept ratings, for the byte accounting of the item groups
         CU(h, cudaMemsetAsync(d_ldeg, 0, sizeof(uint32_t) * n_items, h->stream));
         if (n_local) {
-            check_hist_kernel<<<grid_for(n_local, 256), 256, 0, h->stream>>>(aos2, n_local, n_users, n_items, nullptr, d_ldeg, h->d_err_flag);
+            check_hist_kernel<<<grid_for(n_local, 256), 256, 0, h->stream>>>(aos2, n_local, n_users, n_items, nullptr, d_ldeg, h->d_err_flag, nullptr);
             CU(h, cudaGetLastError());
         }
     }
@@ -405,7 +409,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     CU(h, reserve(h, &h->tr_src, n_local));
     if (sort_bytes) {
         CU(h, launch_source_sort(enc_src, n_local, h->seg_off.data(), (int)rq.n_segments, h->cfg.seed, run_window, h->irows, h->d_umap, h->d_imap, h->d_uprec_row,
-                                 h->d_iprec_row, n_users, n_items, h->d_err_flag, sort_space, h->tr_r, h->tr_u, h->tr_i, h->tr_src, h->stream));
+                                 h->d_iprec_row, n_users, n_items, h->d_err_flag, sort_space, items, h->tr_r, h->tr_u, h->tr_i, h->tr_src, h->stream));
     } else if (n_local) {
         CU(h, encode_segments(h, reinterpret_cast<const mascot_rating*>(enc_src), seg, h->cfg.shuffle != 0, h->tr_r, h->tr_u, h->tr_i, h->tr_src));
         if (src_through) {          // positions in the caller's array, not in the selected copy
@@ -418,7 +422,7 @@ int setup_ratings(mascot_handle* h, const SetupRequest& rq) {
     uint64_t n_test = rq.n_test;
     if (rq.n_test) {
         CU(h, copy_to_device(aos, rq.test, sizeof(NodeAos) * rq.n_test, h->stream));
-        check_hist_kernel<<<grid_for(rq.n_test, 256), 256, 0, h->stream>>>(aos, rq.n_test, n_users, n_items, nullptr, nullptr, h->d_err_flag);
+        check_hist_kernel<<<grid_for(rq.n_test, 256), 256, 0, h->stream>>>(aos, rq.n_test, n_users, n_items, nullptr, nullptr, h->d_err_flag, nullptr);
         CU(h, cudaGetLastError());
         if (sharded) {                                    // ids are used as indices below
             CU(h, cudaMemcpyAsync(&bad, h->d_err_flag, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
