@@ -1479,17 +1479,18 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
     constexpr bool kWhole = STATS && (kMuppet<KIND> || KIND == KIND_SWITCH);
     float norm = 0.f;
     float4 norm_parts = make_float4(0.f, 0.f, 0.f, 0.f);      // with four elements a lane: what the first step joins
-    // MASCOT: the same for the norms of both sides, each with the group it belongs to.  Nothing of it branches where the workers of
-    // a warp could differ, and the two sums run under the next rating's dot product: a sampled rating took four times as
-    // long as another one (check epoch of 8M ratings 1.353 -> 1.302 ms, k=64 20M 1.594 -> 1.531; 100M: no change, there the sums are traffic).
-    constexpr bool kDefer = kGroups && UM != ROWS_DYN && IM != ROWS_DYN;
+    // MASCOT, few workers: the same for the norms of both sides, each with the group it belongs to.  Nothing of it branches where the
+    // workers of a warp could differ, and the two sums run under the next rating's dot product: a sampled rating took four times as long as
+    // another one (check epoch of 8M ratings 1.353 -> 1.302 ms, k=64 20M 1.594 -> 1.531).  With K/8 lanes a worker the sums at once are
+    // faster (20M 1.92 and 1.97, 40M 2.81 and 2.82; 100M equal: there the statistics are traffic).
+    constexpr bool kDefer = kGroups && N == 4;
     constexpr bool kUserStats = kHalfRows<UM>, kItemStats = kHalfRows<IM>;
     float norm_q = 0.f;
     uint32_t late_groups = 0;
     bool late = false;                               // is there a rating before whose norms are to be added?
     auto late_step = [&](int part) {
         auto add = [&](float v) { return __fadd_rn(v, __shfl_xor_sync(kAll, v, (TS / 2) >> part)); };
-        if (N == 4 && part == 0) {
+        if (part == 0) {
             if (kUserStats) norm = __fadd_rn(add(norm_parts.x), add(norm_parts.y));
             if (kItemStats) norm_q = __fadd_rn(add(norm_parts.z), add(norm_parts.w));
         } else if ((TS / 2) >> part) {
@@ -1522,15 +1523,10 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
             for (int t = 0; t < N; t++) gq_acc.x[t] = there ? __fadd_rn(gq_acc.x[t], smp.gq.x[t]) : gq_acc.x[t];
         }
         late = there; late_groups = both_groups;
-        if constexpr (N == 4) {
-            float2 p2 = make_float2(0.f, 0.f), q2 = p2;
-            if (kUserStats) p2 = __ffma2_rn(pr(smp.gp, 0), pr(smp.gp, 0), __fmul2_rn(pr(smp.gp, 1), pr(smp.gp, 1)));
-            if (kItemStats) q2 = __ffma2_rn(pr(smp.gq, 0), pr(smp.gq, 0), __fmul2_rn(pr(smp.gq, 1), pr(smp.gq, 1)));
-            norm_parts = make_float4(p2.x, p2.y, q2.x, q2.y);
-        } else {
-            if (kUserStats) norm = pair_partial(smp.gp, smp.gp);
-            if (kItemStats) norm_q = pair_partial(smp.gq, smp.gq);
-        }
+        float2 p2 = make_float2(0.f, 0.f), q2 = p2;
+        if (kUserStats) p2 = __ffma2_rn(pr(smp.gp, 0), pr(smp.gp, 0), __fmul2_rn(pr(smp.gp, 1), pr(smp.gp, 1)));
+        if (kItemStats) q2 = __ffma2_rn(pr(smp.gq, 0), pr(smp.gq, 0), __fmul2_rn(pr(smp.gq, 1), pr(smp.gq, 1)));
+        norm_parts = make_float4(p2.x, p2.y, q2.x, q2.y);
     };
     auto norm_step = [&](int part) {
         if (kDefer) late_step(part);
