@@ -1793,9 +1793,13 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
     if constexpr (UM != ROWS_DYN) {
         constexpr int UQ = UM == ROWS_HALF ? ROWS_HALFQ : ROWS_F32Q, IQ = IM == ROWS_HALF ? ROWS_HALFQ : ROWS_F32Q;
         constexpr unsigned kMost = K == 128 && kHalfRating<KIND, UM, IM> && KIND != KIND_MPT && !STATS ? 12 : 16;      // warps per SM
+        // Binary16 rows: steps of 0.16 to 0.2 us, a fifth shorter than those the leads were made for, so one rating more each - the same
+        // time ahead (k=64, 20M 1.42 -> 1.395, 8M 1.191 -> 1.160; k=128, 2M 0.530 -> 0.517, 8M 1.182 -> 1.176).  Seven and five are slower
+        // again, and MPT loses by it (1.370 and 1.383).
+        constexpr bool kLonger = kHalfRows<UM> && kHalfRows<IM>;
         // (a single block has exactly the workers that were asked for: they have to fit it in this form, too)
         if (2 * per_sm <= kMost && (warps > 8 || 2 * workers <= 8 * kPerWarp))
-            return launch_ns<K, KIND, UQ, IQ, STATS, NS, 4, D, DI>(args, 2 * per_sm, workers, st, shape, dry);
+            return launch_ns<K, KIND, UQ, IQ, STATS, NS, kLonger ? 8 : 4, kLonger ? 6 : D, kLonger ? 4 : DI>(args, 2 * per_sm, workers, st, shape, dry);
     }
     // With fp32 rows the deep rings leave room for fewer warps than the registers do (k=128, both sides fp32: 16 per SM
     // against 24).  Where a launch of a mixed-precision class with an fp32 side asks for more workers than the deep rings hold and
