@@ -16,7 +16,7 @@ CLI = os.path.join(HERE, "cli")
 LIB = os.path.join(HERE, "libmascot.so")
 BIN = os.path.join(HERE, "bin")
 
-NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
+NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "--no-compress",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 
 LIB_SOURCES = ["mascot_api.cu", "setup.cu", "shard.cu", "train_kernels.cu", "eval_kernels.cu", "prep_kernels.cu", "host_copy.cu", "device_pool.cu", "probe.cu"]
