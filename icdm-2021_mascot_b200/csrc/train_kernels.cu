@@ -1798,7 +1798,11 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
         // again, and MPT loses by it (1.370 and 1.383).
         constexpr bool kLonger = kHalfRows<UM> && kHalfRows<IM>;
         // (a single block has exactly the workers that were asked for: they have to fit it in this form, too)
-        if (2 * per_sm <= kMost && (warps > 8 || 2 * workers <= 8 * kPerWarp))
+        // Grids whose workers have less than two of their first runs each keep the wide form: such a launch is over before its steps count for
+        // much (160,000 ratings, 2,368 workers: 0.046 and 0.037 ms), and what its races leave hangs on how the steps of a single
+        // run fall together - the item factors of two forms differed four times as much as those of two passes of one.
+        const bool worth = STATS || args.s.n >= 2ull * K * workers;
+        if (2 * per_sm <= kMost && (warps > 8 ? worth : 2 * workers <= 8 * kPerWarp))
             return launch_ns<K, KIND, UQ, IQ, STATS, NS, kLonger ? 8 : 4, kLonger ? 6 : D, kLonger ? 4 : DI>(args, 2 * per_sm, workers, st, shape, dry);
     }
     // With fp32 rows the deep rings leave room for fewer warps than the registers do (k=128, both sides fp32: 16 per SM
@@ -1832,7 +1836,7 @@ cudaError_t launch_k(TrainKind kind, const KernelArgs& a, bool stats, RowClass c
                 case ROWCLASS_HH: return launch_st<K, KIND_MIXED, ROWS_HALF, ROWS_HALF>(a, stats, workers, st, sh, dry);
                 case ROWCLASS_HF: return launch_st<K, KIND_MIXED, ROWS_HALF, ROWS_F32>(a, stats, workers, st, sh, dry);
                 case ROWCLASS_FH: return launch_st<K, KIND_MIXED, ROWS_F32, ROWS_HALF>(a, stats, workers, st, sh, dry);
-                case ROWCLASS_FF: return launch_st<K, KIND_MIXED, ROWS_F32, ROWS_F32>(a, stats, workers, st, sh, dry);
+                case ROWCLASS_FF: return launch_one<K, KIND_MIXED, ROWS_F32, ROWS_F32, false>(a, workers, st, sh, dry);      // fp32 groups are not sampled
                 case ROWCLASS_ANY: return launch_st<K, KIND_MIXED, ROWS_DYN, ROWS_DYN>(a, stats, workers, st, sh, dry);
             }
             return cudaErrorInvalidValue;

@@ -9,8 +9,8 @@ from test_gpu_update_edges import oracle_epoch, promoted_model
 
 pytestmark = pytest.mark.gpu
 
-# workers -> form: 1 to 8 (k=64: 16) of a single block and a few warps per SM are narrow; 9 to 16 (17 to 32), which fit a single block of
-# the wide form only, and a full GPU are wide
+# workers -> form: 1 to 8 (k=64: 16) of a single block are narrow; 9 to 16 (17 to 32), which fit a single block of the wide form only,
+# and grids with less than two runs a worker are wide (their statistics are not, up to 16 warps per SM)
 WORKERS = (2, 8, 12, 16, 31, 300, 60000)
 
 
@@ -71,3 +71,37 @@ def test_both_lane_forms_of_the_precision_classes(mascot, oracle, k, workers, us
         Po, Qo = model.factors()
         assert_bit_equal(Pg, Po, f"n {n} P")
         assert_bit_equal(Qg, Qo, f"n {n} Q")
+
+
+@pytest.mark.parametrize("k", (128, 64))
+@pytest.mark.parametrize("version", ["sgd", "mpt", "memquant", "muppet8", "muppet12", "afp"])
+def test_a_grid_of_narrow_workers(mascot, oracle, k, version):
+    """Two full runs a worker on ratings that share no row, and a remainder; AFP's workers follow the oracle run by run."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    workers = 2 * (128 // k) * sms                      # one warp per SM with K/8 lanes, two with K/4
+    n = 2 * k * workers + (0 if version == "afp" else 37)
+    rng = np.random.default_rng(k)
+    R, P, Q = random_problem(rng, n, n, n, k, scale=0.2)
+    R["u"], R["i"] = rng.permutation(n), rng.permutation(n)
+    muppet = version.startswith("muppet")
+    v = dict(sgd=mascot.V_SGD, mpt=mascot.V_MPT, memquant=mascot.V_MEMQUANT, afp=mascot.V_AFP).get(version, mascot.V_MUPPET)
+    width = int(version[6:]) if muppet else 0
+    cfg = mascot.default_config(version=v, k=k, num_workers=workers, plain_user_stores=1, shuffle=0, epoch=50, learning_rate=0.01, decay=0.1, lam=0.05,
+                                muppet_width=width, sample_ratio=0.0)
+    with mascot.Engine(cfg) as eng:
+        eng.set_ratings(R, R[:1], n, n)
+        eng.set_factors(P, Q)
+        assert eng.train_epoch(0).workers == workers
+        Pg, Qg = eng.get_factors(0)
+    rules = oracle.rules_reference()
+    if muppet:
+        oracle.muppet_run(k, R, None, P, Q, float(np.float32(0.01)), 0.05, width, width, rules, first_sample_pos=n)
+    elif version == "afp":
+        for w in range(workers):                        # runs w and w + workers, one after the other
+            mine = np.concatenate([R[w * k:(w + 1) * k], R[(w + workers) * k:(w + workers + 1) * k]])
+            oracle.afp_run(k, mine, None, P, Q, 0.01, 0.05, 0, int(np.float32((n + workers - 1) // workers) / np.float32(10.0)), rules)
+    else:
+        P, Q = oracle_epoch(oracle, version, k, R, P, Q, 0.01, 0.05)
+    assert_bit_equal(Pg, P, "P")
+    assert_bit_equal(Qg, Q, "Q")
