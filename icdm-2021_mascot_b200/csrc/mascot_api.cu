@@ -799,7 +799,7 @@ int apply_stats(mascot_handle* h, uint32_t epoch, uint32_t* promoted_u, uint32_t
         }
         if (*promoted_u + *promoted_i) {
             if ((rc = partition_all(h)) != MASCOT_OK) return rc;
-            if (launches && h->partitioned) (*launches) += 4;
+            if (launches && h->partitioned) (*launches) += 5;
             CU(h, cudaStreamSynchronize(h->stream));
         }
         h->timings.precision_switching_us += now_us() - t_sw;

@@ -274,8 +274,8 @@ MASCOT_API int mascot_set_ratings_sharded(mascot_handle* h, const mascot_rating*
                                const mascot_rating* test, uint64_t n_test, uint32_t n_users, uint32_t n_items,
                                const uint32_t* user_degree, const uint32_t* item_degree);
 /* One epoch over a rating array that is still in HOST memory (pinned memory for a real overlap):
- * the array is uploaded in pieces of 8Mi ratings on a copy stream while the piece before it is
- * encoded and trained, so the epoch costs max(upload, updates) instead of their sum.  The seeded
+ * the array is uploaded in pieces of 8Mi ratings (beyond two of them the first or the last ones are smaller) on a copy
+ * stream while the piece before it is encoded and trained, so the epoch costs max(upload, updates) instead of their sum.  The seeded
  * permutation and the item-sorted windows stay inside a piece; afterwards the pieces are the
  * segments of the resident stream, as after mascot_reload_train.  Ids must be those given to
  * mascot_set_ratings (same users/items; checked on the device, MASCOT_ERR_BAD_ARG as for
