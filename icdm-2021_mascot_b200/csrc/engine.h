@@ -115,16 +115,15 @@ cudaError_t launch_stream_sort(const float* r, const uint32_t* u, const uint32_t
                                void* key_a, void* key_b, uint32_t* idx_a, uint32_t* idx_b, void* temp, size_t temp_bytes,
                                float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, cudaStream_t st);
 // Partition of a coded stream, inside every segment, by precision class = 2 * (user row fp32) + (item row fp32); inside a class the
-// ratings are in the order in which the stream was coded.  pos: where each rating was then (null: where it is now); pos2 (may be
-// null) receives the same for the new order.  class_tiles: number of tiles, and per segment (nseg + 1) the tiles before it, which go
-// to d_first_tile.  cls (n), place (n), counts and starts (4 * tiles each) and temp are scratch; d_first receives, for every
-// segment * 4 + class, the first position of the class (that of the class after it where there is none).
+// ratings stay in the order in which they are.  class_tiles: number of tiles, and per segment (nseg + 1) the tiles before it, which go
+// to d_first_tile.  counts and starts (4 * tiles each) and temp are scratch; d_first receives, for every segment * 4 + class, the
+// first position of the class (that of the class after it where there is none).
 uint32_t class_tiles(const uint64_t* seg_off, int nseg, uint32_t* first);
 size_t class_partition_temp_bytes(uint32_t tiles);
-cudaError_t launch_class_partition(const float* r, const uint32_t* u, const uint32_t* i, const uint32_t* src, const uint32_t* pos, uint64_t n,
-                                   const uint64_t* d_seg_off, const uint32_t* d_first_tile, int nseg, uint32_t tiles, uint8_t* cls, uint32_t* place,
+cudaError_t launch_class_partition(const float* r, const uint32_t* u, const uint32_t* i, const uint32_t* src, uint64_t n,
+                                   const uint64_t* d_seg_off, const uint32_t* d_first_tile, int nseg, uint32_t tiles,
                                    uint32_t* counts, uint32_t* starts, void* temp, size_t temp_bytes, uint32_t* d_first,
-                                   float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, uint32_t* pos2, cudaStream_t st);
+                                   float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, cudaStream_t st);
 // The whole resident stream from the uploaded array: seeded permutation of every segment, item-sorted run windows, ids
 // coded - the order that launch_encode_stream and launch_stream_sort give, in one sort.  source_sort_bytes: the scratch it
 // wants, or 0 where it does not apply (no run windows, segments that begin off the encoding step's windows, keys beyond 32

@@ -58,9 +58,7 @@ struct mascot_handle {
     // five stream positions per segment: the starts of the classes and the end of the segment.
     bool partitioned = false;
     std::vector<uint64_t> cls_off;
-    uint32_t* tr_pos = nullptr;     // position of each stream entry when the stream was coded, while `moved`
-    bool moved = false;             // some partition has moved the ratings since then
-    void stream_is_new() { cls_off.clear(); partitioned = moved = false; }
+    void stream_is_new() { cls_off.clear(); partitioned = false; }
 
     // host
     std::vector<uint32_t> uend, iend;

@@ -83,7 +83,7 @@ int mascot::fail(mascot_handle* h, int code, const std::string& msg) {
 namespace mascot {
 
 void free_ratings(mascot_handle* h) {
-    dev_free(h->tr_r, h->stream); dev_free(h->tr_u, h->stream); dev_free(h->tr_i, h->stream); dev_free(h->tr_src, h->stream); dev_free(h->tr_pos, h->stream);
+    dev_free(h->tr_r, h->stream); dev_free(h->tr_u, h->stream); dev_free(h->tr_i, h->stream); dev_free(h->tr_src, h->stream);
     dev_free(h->te_r, h->stream); dev_free(h->te_u, h->stream); dev_free(h->te_i, h->stream);
     dev_free(h->P.f16, h->stream); dev_free(h->P.f32, h->stream); dev_free(h->Q.f16, h->stream); dev_free(h->Q.f32, h->stream);
     dev_free(h->d_uprec_row, h->stream); dev_free(h->d_iprec_row, h->stream); dev_free(h->d_ugroup, h->stream); dev_free(h->d_igroup, h->stream);
@@ -268,7 +268,8 @@ static int sort_windows(mascot_handle* h, int run_window_log2) {
     return MASCOT_OK;
 }
 
-// Makes the ratings of each precision class contiguous inside every segment and records the class boundaries.  Called after the
+// Makes the ratings of each precision class contiguous inside every segment - the order inside a class is the order before - and
+// records the class boundaries.  Called after the
 // precision bits of the ids changed (promotion + recode) or after a stream was encoded while promoted groups exist.
 static int partition_by_class(mascot_handle* h) {
     const uint64_t n = h->n_train;
@@ -279,14 +280,12 @@ static int partition_by_class(mascot_handle* h) {
     const uint32_t tiles = class_tiles(h->seg_off.data(), (int)nseg, first_tile.data());
     const size_t temp_bytes = class_partition_temp_bytes(tiles);
     SortSpace sp;
-    uint32_t *d_first_tile, *d_first, *place, *pos2, *counts, *starts;
-    uint8_t* cls;
+    uint32_t *d_first_tile, *d_first, *counts, *starts;
     unsigned char* temp;
     auto lay_out = [&]() {
         sp.off = 0;
         sp.arrays(n, nseg);
         d_first_tile = sp.take<uint32_t>(nseg + 1); d_first = sp.take<uint32_t>(nseg * 4);
-        place = sp.take<uint32_t>(n); pos2 = sp.take<uint32_t>(n); cls = sp.take<uint8_t>(n);
         counts = sp.take<uint32_t>(4 * (size_t)tiles); starts = sp.take<uint32_t>(4 * (size_t)tiles);
         temp = sp.take<unsigned char>(temp_bytes);
     };
@@ -295,18 +294,13 @@ static int partition_by_class(mascot_handle* h) {
     if (rc != MASCOT_OK) return rc;
     sp.base = static_cast<unsigned char*>(h->d_scratch);
     lay_out();
-    // Without memory for the positions the classes keep the order that the last partition gave them.
-    if (!h->moved && reserve(h, &h->tr_pos, n) != cudaSuccess) { cudaGetLastError(); dev_free(h->tr_pos, h->stream); }
-    if (!h->tr_pos) pos2 = nullptr;
     CU(h, cudaMemcpyAsync(sp.seg, h->seg_off.data(), sizeof(uint64_t) * (nseg + 1), cudaMemcpyHostToDevice, h->stream));
     CU(h, cudaMemcpyAsync(d_first_tile, first_tile.data(), sizeof(uint32_t) * (nseg + 1), cudaMemcpyHostToDevice, h->stream));
-    CU(h, launch_class_partition(h->tr_r, h->tr_u, h->tr_i, h->tr_src, h->moved ? h->tr_pos : nullptr, n, sp.seg, d_first_tile, (int)nseg, tiles, cls, place,
-                                 counts, starts, temp, temp_bytes, d_first, sp.r, sp.u, sp.i, sp.src, pos2, h->stream));
+    CU(h, launch_class_partition(h->tr_r, h->tr_u, h->tr_i, h->tr_src, n, sp.seg, d_first_tile, (int)nseg, tiles,
+                                 counts, starts, temp, temp_bytes, d_first, sp.r, sp.u, sp.i, sp.src, h->stream));
     if ((rc = take_reordered(h, sp)) != MASCOT_OK) return rc;
-    if (pos2) CU(h, cudaMemcpyAsync(h->tr_pos, pos2, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
     CU(h, cudaMemcpyAsync(first.data(), d_first, sizeof(uint32_t) * first.size(), cudaMemcpyDeviceToHost, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
-    h->moved = pos2 != nullptr;
     for (size_t j = 0; j < nseg; j++) {
         for (int c = 0; c < 4; c++) h->cls_off[j * 5 + c] = first[j * 4 + c];
         h->cls_off[j * 5 + 4] = h->seg_off[j + 1];
@@ -319,8 +313,9 @@ static int partition_by_class(mascot_handle* h) {
 bool wants_partition(const mascot_handle* h) {
     if (!(h->grouped && !h->cfg.deterministic && any_fp32_group(h) && h->n_train < (1ull << 32) && (h->seg_off.size() - 1) * 4 <= 65536)) return false;
     // Measured on one B200, ms per epoch with one launch per class and with one that reads each id's precision bit: 100M
-    // ratings, a fifth of the groups promoted 8.6 and 13.6; 40 % of them, 63M 7.1 and 9.0, 40M 4.1 and 5.5, k=64, 100M 6.6 and
-    // 7.2.  Both leave the same test RMSE (0.57333 and 0.57346 after four epochs at 40M).
+    // ratings, a fifth of the groups promoted 9.9 and 13.6 to 14.2; 252M, 40 % of them 34.0 and 36 to 40.  In between the one
+    // launch is faster - 63M, 40 % promoted 9.8 and 9.0; 40M 6.9 and 5.5; k=64, 100M 12.7 and 7.2 - but leaves a test RMSE
+    // that is 0.1 % higher after four epochs (0.57343 against 0.57262 at 40M).
     return h->cfg.no_class_partition != 1;
 }
 
@@ -799,7 +794,7 @@ int apply_stats(mascot_handle* h, uint32_t epoch, uint32_t* promoted_u, uint32_t
         }
         if (*promoted_u + *promoted_i) {
             if ((rc = partition_all(h)) != MASCOT_OK) return rc;
-            if (launches && h->partitioned) (*launches) += 5;
+            if (launches && h->partitioned) (*launches) += 4;
             CU(h, cudaStreamSynchronize(h->stream));
         }
         h->timings.precision_switching_us += now_us() - t_sw;

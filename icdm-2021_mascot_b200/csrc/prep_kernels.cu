@@ -327,17 +327,14 @@ cudaError_t launch_stream_sort(const float* r, const uint32_t* u, const uint32_t
                        r2, u2, i2, src2, st);
 }
 
-// Partition by precision class.  Inside a class the ratings keep the order in which the stream was coded, whatever
-// partitions came before.  Sorting from one partition to the next instead moves each newly promoted group behind what was there, so
-// that promotions one after the other leave a stream sorted by groups: its workers all sit on the rows of a few groups at a time
-// (8M ratings, 100 + 100 groups promoted one by one: 4.1 ms per epoch, 1.32 in this order; 63M, the upper 40 of them: 9.45 and
-// 7.0, 100M, the upper 20: 9.9 and 8.6).
+// Partition by precision class.  Inside a class the ratings keep the order in which they are, so after promotions one after the
+// other a class is sorted by the groups that came into it.  Classes in the order in which the stream was coded would be faster to train (ms
+// per epoch: 8M ratings, all 100 + 100 groups promoted one by one, 4.1 and 1.32; 63M, the upper 40 of them, 9.45 and 7.0), but not
+// to the same model: runs of equal items are longer there (63M: 6.6 ratings against 1.9), an item row is written back with a plain
+// store once per run, and the test RMSE is higher (0.5193 and 0.5184 at 8M, 0.57333 and 0.57262 at 40M, four epochs).
 //
-// Tiles of kTile positions of the coded order, none of which crosses a segment: class and present place of every rating are put
-// at its coded position, the classes of each tile are counted, and one sum over (segment, class, tile) says where each
-// class of each tile begins.  A tile is then ordered in shared memory and moved with coalesced writes.  59 bytes a rating are read and
-// written (a radix sort of keys and indices with a gather after it: 88): a promotion of
-// 63M ratings takes 1.50 ms, 2.45 that way.
+// Tiles of kTile positions, none of which crosses a segment: the classes of each tile are counted, and one sum over (segment, class,
+// tile) says where each class of each tile begins.  A tile is then ordered in shared memory and moved with coalesced writes.
 constexpr int kTile = 4096, kTileWarps = 8;
 struct Tiles { const uint64_t* seg_off; const uint32_t* first; int nseg; };      // first[s]: number of tiles before segment s
 struct Tile { uint64_t begin; int count; uint32_t slot, stride; };               // its counter of class c is number slot + c * stride
@@ -348,21 +345,15 @@ __device__ __forceinline__ Tile tile_of(const Tiles& T, uint32_t t) {
     const uint64_t begin = T.seg_off[lo] + (uint64_t)in * kTile, left = T.seg_off[lo + 1] - begin;
     return Tile{begin, (int)(left < kTile ? left : kTile), 4 * T.first[lo] + in, tiles};
 }
-__global__ void class_mark_kernel(const uint32_t* u, const uint32_t* i, const uint32_t* pos, uint64_t n, uint8_t* cls, uint32_t* place) {
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t at = pos ? pos[j] : (uint32_t)j;
-        cls[at] = (uint8_t)(((u[j] & kPrecBit) ? 2u : 0u) | ((i[j] & kPrecBit) ? 1u : 0u));
-        place[at] = (uint32_t)j;
-    }
-}
-__global__ void __launch_bounds__(32 * kTileWarps) class_count_kernel(const uint8_t* cls, Tiles T, uint32_t* counts) {
+__device__ __forceinline__ int class_of(uint32_t u, uint32_t i) { return (u & kPrecBit ? 2 : 0) | (i & kPrecBit ? 1 : 0); }
+__global__ void __launch_bounds__(32 * kTileWarps) class_count_kernel(const uint32_t* u, const uint32_t* i, Tiles T, uint32_t* counts) {
     __shared__ uint32_t sum[4];
     if (threadIdx.x < 4) sum[threadIdx.x] = 0;
     __syncthreads();
     const Tile t = tile_of(T, blockIdx.x);
     uint32_t mine[4] = {0, 0, 0, 0};
     for (int e = threadIdx.x; e < t.count; e += 32 * kTileWarps) {
-        const int k = cls[t.begin + e];
+        const int k = class_of(u[t.begin + e], i[t.begin + e]);
 #pragma unroll
         for (int c = 0; c < 4; c++) mine[c] += k == c;
     }
@@ -374,9 +365,8 @@ __global__ void __launch_bounds__(32 * kTileWarps) class_count_kernel(const uint
     __syncthreads();
     if (threadIdx.x < 4) counts[t.slot + threadIdx.x * t.stride] = sum[threadIdx.x];
 }
-__global__ void __launch_bounds__(32 * kTileWarps) class_move_kernel(const uint8_t* cls, const uint32_t* place, Tiles T, const uint32_t* start, const float* r,
-                                                                     const uint32_t* u, const uint32_t* i, const uint32_t* src, float* r2, uint32_t* u2,
-                                                                     uint32_t* i2, uint32_t* src2, uint32_t* pos2) {
+__global__ void __launch_bounds__(32 * kTileWarps) class_move_kernel(Tiles T, const uint32_t* start, const float* r, const uint32_t* u, const uint32_t* i,
+                                                                     const uint32_t* src, float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2) {
     constexpr int kRounds = kTile / (32 * kTileWarps);
     __shared__ uint16_t order[kTile];                       // positions of the tile, class by class
     __shared__ uint32_t held[kTileWarps][4], begin[5];      // ratings per warp and class; where a class begins in `order`
@@ -386,7 +376,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) class_move_kernel(const uint8
     uint32_t rank[kRounds], n[4] = {0, 0, 0, 0};           // class in the upper half
 #pragma unroll
     for (int q = 0; q < kRounds; q++) {
-        const int e = e0 + 32 * q, k = e < t.count ? cls[t.begin + e] : 4;
+        const int e = e0 + 32 * q, k = e < t.count ? class_of(u[t.begin + e], i[t.begin + e]) : 4;
         rank[q] = 4u << 16;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
@@ -409,14 +399,15 @@ __global__ void __launch_bounds__(32 * kTileWarps) class_move_kernel(const uint8
 #pragma unroll
     for (int q = 0; q < kRounds; q++) if (rank[q] >> 16 < 4) order[held[warp][rank[q] >> 16] + (rank[q] & 0xffffu)] = (uint16_t)(e0 + 32 * q);
     __syncthreads();
-    // four ratings of a thread at a time, or the chain place -> rating -> store is all it does (63M ratings: 1.03 ms one at a time, 0.48 so)
+    // four ratings of a thread at a time, or the chain order -> rating -> store is all it does
     constexpr int kBatch = 4;
 #pragma unroll 1
     for (int o0 = threadIdx.x; o0 < t.count; o0 += kBatch * 32 * kTileWarps) {
-        uint32_t at[kBatch], from[kBatch], vu[kBatch], vi[kBatch], vs[kBatch];
+        uint64_t from[kBatch];
+        uint32_t vu[kBatch], vi[kBatch], vs[kBatch];
         float vr[kBatch];
 #pragma unroll
-        for (int b = 0; b < kBatch; b++) { at[b] = order[min(o0 + b * 32 * kTileWarps, t.count - 1)]; from[b] = place[t.begin + at[b]]; }
+        for (int b = 0; b < kBatch; b++) from[b] = t.begin + order[min(o0 + b * 32 * kTileWarps, t.count - 1)];
 #pragma unroll
         for (int b = 0; b < kBatch; b++) { vr[b] = r[from[b]]; vu[b] = u[from[b]]; vi[b] = i[from[b]]; vs[b] = src ? src[from[b]] : 0u; }
 #pragma unroll
@@ -427,7 +418,6 @@ __global__ void __launch_bounds__(32 * kTileWarps) class_move_kernel(const uint8
             const uint32_t to = start[t.slot + c * t.stride] + (uint32_t)(o - (int)begin[c]);
             r2[to] = vr[b]; u2[to] = vu[b]; i2[to] = vi[b];
             if (src) src2[to] = vs[b];
-            if (pos2) pos2[to] = (uint32_t)t.begin + at[b];
         }
     }
 }
@@ -452,17 +442,16 @@ size_t class_partition_temp_bytes(uint32_t tiles) {
     return bytes;
 }
 
-cudaError_t launch_class_partition(const float* r, const uint32_t* u, const uint32_t* i, const uint32_t* src, const uint32_t* pos, uint64_t n,
-                                   const uint64_t* d_seg_off, const uint32_t* d_first_tile, int nseg, uint32_t tiles, uint8_t* cls, uint32_t* place,
+cudaError_t launch_class_partition(const float* r, const uint32_t* u, const uint32_t* i, const uint32_t* src, uint64_t n,
+                                   const uint64_t* d_seg_off, const uint32_t* d_first_tile, int nseg, uint32_t tiles,
                                    uint32_t* counts, uint32_t* starts, void* temp, size_t temp_bytes, uint32_t* d_first,
-                                   float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, uint32_t* pos2, cudaStream_t st) {
+                                   float* r2, uint32_t* u2, uint32_t* i2, uint32_t* src2, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     const Tiles T{d_seg_off, d_first_tile, nseg};
-    class_mark_kernel<<<grid_for(n, 256), 256, 0, st>>>(u, i, pos, n, cls, place);
-    class_count_kernel<<<tiles, 32 * kTileWarps, 0, st>>>(cls, T, counts);
+    class_count_kernel<<<tiles, 32 * kTileWarps, 0, st>>>(u, i, T, counts);
     const cudaError_t e = cub::DeviceScan::ExclusiveSum(temp, temp_bytes, counts, starts, (uint64_t)4 * tiles, st);
     if (e != cudaSuccess) return e;
-    class_move_kernel<<<tiles, 32 * kTileWarps, 0, st>>>(cls, place, T, starts, r, u, i, src, r2, u2, i2, src2, pos2);
+    class_move_kernel<<<tiles, 32 * kTileWarps, 0, st>>>(T, starts, r, u, i, src, r2, u2, i2, src2);
     class_first_kernel<<<grid_for(4 * (uint64_t)nseg, 256), 256, 0, st>>>(starts, T, d_first);
     return cudaGetLastError();
 }

@@ -91,9 +91,9 @@ def test_reload_after_a_streamed_epoch_keeps_its_pieces(mascot):
 
 
 @pytest.mark.parametrize("seg,shuffle", [([0, 100003], 1), ([0, 5000, 5000, 40960, 60001], 1), ([0, 3001], 0), ([0, 1], 1)])
-def test_classes_keep_the_coded_order(mascot, seg, shuffle):
-    """Inside a precision class the ratings stay in the order in which the stream was coded, also after several promotions one
-    after the other, after a reload and after a streamed epoch (whose piece is a stream of its own)."""
+def test_classes_keep_the_order_before(mascot, seg, shuffle):
+    """Inside a precision class the ratings stay in the order that they had before the partition, also after several promotions one
+    after the other, after a reload (a new stream, partitioned once) and after a streamed epoch (whose piece is a stream of its own)."""
     n_users, n_items, n = 700, 301, seg[-1]
     R, P, Q = random_problem(np.random.default_rng(n), n_users, n_items, n, 64)
     cfg = mascot.default_config(version=mascot.V_MASCOT, k=64, num_workers=4096, shuffle=shuffle, sample_ratio=1.0, user_group_num=6, item_group_num=5)
@@ -108,19 +108,22 @@ def test_classes_keep_the_coded_order(mascot, seg, shuffle):
             cls = 2 * fp32[0] + fp32[1]
             return np.concatenate([order[b:e][np.argsort(cls[order[b:e]], kind="stable")] for b, e in zip(cuts, cuts[1:])])
 
-        coded = eng.stream_order()
+        coded = order = eng.stream_order()
         for side, group in ((0, len(ends[0]) - 1), (1, 0), (0, 0), (1, len(ends[1]) - 1)):
             eng.promote_group(side, min(group, len(ends[side]) - 1))
-            assert (eng.stream_order() == expected(coded, seg)).all()
+            order = expected(order, seg)
+            assert (eng.stream_order() == order).all()
         eng.reload_train(R)
-        assert (eng.stream_order() == expected(coded, seg)).all()
+        order = expected(coded, seg)
+        assert (eng.stream_order() == order).all()
         eng.promote_group(0, min(1, len(ends[0]) - 1))
-        assert (eng.stream_order() == expected(coded, seg)).all()
+        assert (eng.stream_order() == expected(order, seg)).all()
         eng.train_epoch_streamed(0, R)
         piece = eng.stream_order()
-        eng.promote_group(1, min(1, len(ends[1]) - 1))
-        eng.promote_group(0, min(2, len(ends[0]) - 1))
-        assert (eng.stream_order() == expected(piece, [0, n])).all()
+        for side, group in ((1, 1), (0, 2)):
+            eng.promote_group(side, min(group, len(ends[side]) - 1))
+            piece = expected(piece, [0, n])
+        assert (eng.stream_order() == piece).all()
 
 
 @pytest.mark.parametrize("version,parts", [("mascot", [64, 34, 17, 8.5, 8.5]), ("muppet", [8, 16, 32, 64, 12]), ("sgd", [64, 64, 4])])
