@@ -1572,6 +1572,9 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
         if constexpr (kSpread) cp_row_if<K, UM>(uring + slot * SM::kURowBytes, P, uc);
         else cp_row<K, UM>(uring + slot * SM::kURowBytes, P, uc);
     };
+    // A lane reads what it fetched itself - but of binary16 rows over K/4 lanes only one of two lanes fetches what both read, so there the lanes
+    // meet between the wait and the read (and, once a rating, between a read and the request that uses the slot again).
+    constexpr bool kMeet = UM == ROWS_HALFQ || IM == ROWS_HALFQ;
     auto request_item = [&](uint32_t ic, int slot) { cp_row_if<K, IM>(iring + slot * SM::kIRowBytes, Q, ic); };
     // Binary16 rows over K/4 lanes: copies are of 16 bytes, so the first half of the lanes fetches the user row and the second
     // half the item row, with one instruction.
@@ -1595,6 +1598,7 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
     }
     uint4 rec = recs[0];
     cp_wait<D - 1>();
+    if constexpr (kMeet) __syncwarp();
     Raw<UM> p = lds_row<K, UM>(uring, rec.z);
     bool turn = __any_sync(kAll, rec.x & (F_RS | F_UDUP));      // does the coming rating of some worker need another item row?
 
@@ -1614,6 +1618,7 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
                 if (turn) {
                     // a run of equal items ends for at least one of the warp's workers (or a row has to be read again)
                     cp_wait<DI - 1>();
+                    if constexpr (kMeet) __syncwarp();
                     const unsigned start = f & F_RS;
                     st_row_if<K, IM>(start & have_item, Q, cur_ic, q);
                     const unsigned slot = iring + (t & (NSI - 1)) * SM::kIRowBytes;
@@ -1635,6 +1640,7 @@ __global__ void __launch_bounds__(256, (kHalfRows<UM> && kHalfRows<IM> && !STATS
                         asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(req_u), "=r"(req_i) : "r"(q0 + 8 * t) : "memory");
                     } else if (part == 1) {
                         cp_wait<D - 2>();
+                        if constexpr (kMeet) __syncwarp();
                         p_next = lds_row<K, UM>(uring + ((t + 1) & (NS - 1)) * SM::kURowBytes, rec.z);
                     } else if (part == 2) {
                         if constexpr (kOneRequest) request_one(req_u, (t + D) & (NS - 1), req_i, (t + DI) & (NSI - 1));

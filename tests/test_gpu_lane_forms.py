@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from helpers import assert_bit_equal, random_problem
+from test_gpu_parity import assert_within_one_ulp
 from test_gpu_update_edges import oracle_epoch, promoted_model
 
 pytestmark = pytest.mark.gpu
@@ -104,4 +105,41 @@ def test_a_grid_of_narrow_workers(mascot, oracle, k, version):
     else:
         P, Q = oracle_epoch(oracle, version, k, R, P, Q, 0.01, 0.05)
     assert_bit_equal(Pg, P, "P")
+    assert_bit_equal(Qg, Q, "Q")
+
+
+@pytest.mark.parametrize("k", (128, 64))
+@pytest.mark.parametrize("plain_stores", (1, 0))
+@pytest.mark.parametrize("version", ["mascot_hh", "mascot_fh", "mascot_hf", "mascot_ff", "switch"])
+def test_a_grid_of_narrow_workers_of_the_precision_classes(mascot, oracle, k, plain_stores, version):
+    """Rows that one lane fetches and another one reads, over whole runs, tickets of the shared counter and both ways of
+    writing user rows back: ratings that share no row, bit for bit, or within an ulp of the user rows where these are reductions of a
+    change.  More than two runs a worker, so the grid takes K/4 lanes a worker."""
+    import torch
+    workers = 2 * (128 // k) * torch.cuda.get_device_properties(0).multi_processor_count
+    n = 2 * k * workers + 37 * k + 5
+    rng = np.random.default_rng(k)
+    R, P, Q = random_problem(rng, n, n, n, k, scale=0.2)
+    R["u"], R["i"] = rng.permutation(n), rng.permutation(n)
+    cfg = mascot.default_config(version=mascot.V_SWITCH_ONLY if version == "switch" else mascot.V_MASCOT, k=k, num_workers=workers, plain_user_stores=plain_stores,
+                                epoch=50, learning_rate=0.01, decay=0.1, lam=0.05, user_group_num=1, item_group_num=1, sample_ratio=0.0)
+    with mascot.Engine(cfg) as eng:
+        eng.set_ratings(R, R[:1], n, n)
+        eng.set_factors(P, Q)
+        if version != "switch":
+            model, u2s, i2s = promoted_model(oracle, mascot, eng, k, P, Q, version[7] == "f", version[8] == "f")
+        st = eng.train_epoch(0)
+        assert st.workers == workers and st.updates == n
+        Pg, Qg = eng.get_factors(0 if version == "switch" else 1)
+    if version == "switch":
+        P, Q = oracle_epoch(oracle, version, k, R, P, Q, 0.01, 0.05)
+    else:
+        Rs = R.copy()
+        Rs["u"], Rs["i"] = u2s[R["u"]], i2s[R["i"]]
+        model.run(Rs, None, 0.01, 0.05, oracle.rules_reference())
+        P, Q = model.factors()
+    if plain_stores:
+        assert_bit_equal(Pg, P, "P")
+    else:
+        assert_within_one_ulp(Pg, P, version in ("mascot_hh", "mascot_hf", "switch"), "P")
     assert_bit_equal(Qg, Q, "Q")
