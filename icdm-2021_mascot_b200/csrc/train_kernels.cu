@@ -1032,6 +1032,9 @@ __device__ __forceinline__ void afp_update(const Consts& c, AfpState& st, float 
     const bool estimate = st.due == 0;
     float pmax = 0.f, qmax = 0.f;
     if (__builtin_expect(estimate, 0)) {
+        // ratings without a binary16 pass have no barrier of their own, and the pass may come back with an estimate: what was read from its
+        // slot two ratings ago is kept from what is written to it next
+        __syncwarp();
         const bool new_user = active && cur == st.user.next, new_item = active && cur == st.item.next;
         pmax = worker_max<TS>(abs_max(p), kAll);
         qmax = worker_max<TS>(abs_max(q), kAll);
