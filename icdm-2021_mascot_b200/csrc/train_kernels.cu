@@ -70,6 +70,7 @@
 #include "engine.h"
 #include "launch_cache.h"
 #include "layout.cuh"
+#include "scale_bits.h"
 
 namespace mascot {
 
@@ -562,7 +563,7 @@ __device__ __forceinline__ float muppet_scale(int bits, float hi, float lo) {
     const float val = (float)(1 << (bits - 1));
     const float top = __fadd_rn(__fsub_rn(val, 1.f), 0.5f), bottom = __fsub_rn(-val, 0.5f);
     const int d = min(__float_as_int(top) - (__float_as_int(hi) & 0x7fffffff), __float_as_int(-bottom) - (__float_as_int(lo) & 0x7fffffff));
-    float s = __int_as_float((max(d, 0) & 0x7f800000) + 0x3f800000);
+    float s = __uint_as_float(scale_bits(d));
     if (((d + 256) & 0x007fffff) < 512 || d >= (120 << 23)) s = (hi == 0.f && lo == 0.f) ? 1.f : muppet_scale_exact(top, bottom, hi, lo);
     return s;
 }
@@ -577,11 +578,11 @@ __device__ __forceinline__ int2 scale_bounds(int bits) {
 __device__ __forceinline__ int scale_key(int2 bound, float hi, float lo) {
     return min(bound.x - max(__float_as_int(hi), 0), bound.y - max(__float_as_int(-lo), 0));
 }
-__device__ __forceinline__ float scale_of(int key) { return __int_as_float((max(key, 0) & 0x7f800000) + 0x3f800000); }
+__device__ __forceinline__ float scale_of(int key) { return __uint_as_float(scale_bits(key)); }
 // (From 2^60 on, the formula too: below that the reciprocal of a product of two scales is a normal number, and comes from the bits.)
 __device__ __forceinline__ bool scale_unsure(int2 bound, int key) { return ((key + 256) & 0x007fffff) < 512 + bound.y - bound.x || key >= (60 << 23); }
-__device__ __forceinline__ float near_rev(float s) { return __int_as_float(0x7f000000 - __float_as_int(s)); }
-__device__ __forceinline__ float near_rev(float s, float t) { return __int_as_float((int)0xbe800000u - __float_as_int(s) - __float_as_int(t)); }
+__device__ __forceinline__ float near_rev(float s) { return __uint_as_float(rev_bits(__float_as_uint(s))); }
+__device__ __forceinline__ float near_rev(float s, float t) { return __uint_as_float(rev_bits(__float_as_uint(s), __float_as_uint(t))); }
 // roundf (halves away from zero) in three instructions: trunc(x + copysign(largest float below one half, x)).
 // The sum is rounded to nearest-even, which is what makes it exact: x = n + f with f < 1/2 cannot reach n + 1,
 // f >= 1/2 always does.  Equal to roundf for every one of the 2^32 float patterns (checked exhaustively on the

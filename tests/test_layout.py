@@ -110,6 +110,15 @@ def test_fast_rounding_and_power_of_two_reciprocal_are_exact(tmp_path):
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout
 
 
+def test_scales_and_their_reciprocals_from_the_bits(tmp_path):
+    """MuPPET's power-of-two scales and 1 / (product of two of them): right for every pair, and without overflow of a signed number,
+    which the compiler reports where it evaluates a constant."""
+    exe = str(tmp_path / "scale_bits_check")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-I", CSRC, os.path.join(ROOT, "tests", "scale_bits_check.cpp"), "-o", exe])
+    out = subprocess.run([exe], capture_output=True, text=True)
+    assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout
+
+
 def test_integer_ceil_log2_equals_the_double_precision_formula(tmp_path):
     """The AFP trainer's kernel computes ceil((float)log2((double)x)) - the exponent of its fixed-point scale -
     from the bits of x; the host restatement of that shortcut is compared with the formula on every positive
