@@ -76,11 +76,12 @@ struct LaunchShape {
 // only one in 2^hot_user_shift is then written back.  Returns the launch shape used.
 // With `counters` == nullptr the call is dry: the instantiation the launch would use is loaded and configured
 // (so that the first real launch does not pay for it) and nothing is launched.
+// `whole`: ratings of the epoch (or segment) that this launch is a part of, for which the workers were counted.
 // MuPPET statistics use gsum_p[0..K) (sum of the sampled updates, physical order) and nsum_p[0].
 cudaError_t launch_train(int K, TrainKind kind, const Stream& s, Arena P, Arena Q, float lr, float lam,
                          const SampleStats* stats, RowClass row_class, unsigned workers,
                          WorkCounters* counters, int bits, int epoch, bool add_user_delta, unsigned hot_user_shift,
-                         cudaStream_t st, LaunchShape* shape);
+                         uint64_t whole, cudaStream_t st, LaunchShape* shape);
 
 // Folds the private statistic sets of a launch into set 0 (sets are added in index order).
 cudaError_t launch_reduce_stats(float* sets, int copies, size_t copy_stride, size_t floats_per_set, cudaStream_t st);

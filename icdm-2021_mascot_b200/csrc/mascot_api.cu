@@ -364,7 +364,7 @@ int warm_kernels(mascot_handle* h) {
     const bool sampled = h->kind == KIND_MIXED || h->kind == KIND_SWITCH || h->kind == KIND_MUPPET;
     for (int with_stats = 0; with_stats <= (sampled ? 1 : 0); with_stats++)
         CU(h, launch_train(h->K, h->kind, s, h->P, h->Q, 0.f, 0.f, with_stats ? &st : nullptr, cls, workers, nullptr, muppet_bits(h), 0,
-                           h->cfg.plain_user_stores == 0, h->hot_user_shift, h->stream, nullptr));
+                           h->cfg.plain_user_stores == 0, h->hot_user_shift, h->n_train, h->stream, nullptr));
     return MASCOT_OK;
 }
 
@@ -677,10 +677,9 @@ SampleStats stats_view(mascot_handle* h) {
 // Runs the update kernel over stream positions [begin, end), all of whose ratings are of row class
 // `cls`.  With `collect`, the last sample_ratio of the range (mf_methods.cu:102-103, 173-174) goes
 // through the statistics kernel - a second launch, so that only the sampled fraction pays for the
-// statistics.  `policy_n` (0 = the range's own length) is the stream length the automatic worker
-// count is taken from.
+// statistics.  `whole`: ratings of the epoch or segment that the range is a part of, for which the workers were counted.
 int train_span(mascot_handle* h, float lr, uint32_t epoch, uint64_t begin, uint64_t end, RowClass cls, bool collect,
-               LaunchShape* shape, uint32_t* launches, unsigned workers, cudaStream_t stream, WorkCounters* counters) {
+               LaunchShape* shape, uint32_t* launches, unsigned workers, uint64_t whole, cudaStream_t stream, WorkCounters* counters) {
     if (end <= begin) return MASCOT_OK;
     const uint64_t n = end - begin;
     // after its switch the whole-model switching trainer is the plain fp32 trainer (sgd_kernel.h:296-326)
@@ -694,7 +693,7 @@ int train_span(mascot_handle* h, float lr, uint32_t epoch, uint64_t begin, uint6
     if (head > 0) {
         Stream sa = s; sa.n = head;
         CU(h, launch_train(h->K, kind, sa, h->P, h->Q, lr, h->cfg.lambda, nullptr, cls, workers,
-                           counters, muppet_bits(h), (int)epoch, h->cfg.plain_user_stores == 0, h->hot_user_shift, stream, shape));
+                           counters, muppet_bits(h), (int)epoch, h->cfg.plain_user_stores == 0, h->hot_user_shift, whole, stream, shape));
         (*launches)++;
     }
     if (head < n) {
@@ -702,7 +701,7 @@ int train_span(mascot_handle* h, float lr, uint32_t epoch, uint64_t begin, uint6
         const SampleStats st = stats_view(h);
         LaunchShape tail_shape;            // the caller is told the shape of the plain launch when there is one
         CU(h, launch_train(h->K, kind, sb, h->P, h->Q, lr, h->cfg.lambda, &st, cls, workers,
-                           counters, muppet_bits(h), (int)epoch, h->cfg.plain_user_stores == 0, h->hot_user_shift, stream, head > 0 ? &tail_shape : shape));
+                           counters, muppet_bits(h), (int)epoch, h->cfg.plain_user_stores == 0, h->hot_user_shift, whole, stream, head > 0 ? &tail_shape : shape));
         (*launches)++;
     }
     return MASCOT_OK;
@@ -712,18 +711,19 @@ int train_span(mascot_handle* h, float lr, uint32_t epoch, uint64_t begin, uint6
 // partitioned: the launch then reads each id's precision bit), else one launch per non-empty precision
 // class, one after the other.  (Running the classes side by side on streams of their own, each with a
 // share of the workers, was measured too: 15.7 ms per promoted epoch on the 100M-rating set against 14.0 ms
-// one after the other.)  On a check epoch every launched range contributes its own sampled tail.
+// one after the other.)  On a check epoch every launched range contributes its own sampled tail.  `policy_n` (0 = the segment's
+// own length) is the stream length the automatic worker count is taken from.
 int train_range(mascot_handle* h, float lr, uint32_t epoch, size_t segment, bool collect, LaunchShape* shape, uint32_t* launches,
                 uint64_t policy_n) {
     const uint64_t begin = h->seg_off[segment], end = h->seg_off[segment + 1];
     if (!policy_n) policy_n = end - begin;
     const unsigned workers = worker_count(h, policy_n);
     if (!h->partitioned)
-        return train_span(h, lr, epoch, begin, end, any_fp32_group(h) ? ROWCLASS_ANY : ROWCLASS_HH, collect, shape, launches, workers,
+        return train_span(h, lr, epoch, begin, end, any_fp32_group(h) ? ROWCLASS_ANY : ROWCLASS_HH, collect, shape, launches, workers, policy_n,
                           h->stream, &h->counters);
     const uint64_t* off = &h->cls_off[segment * 5];
     for (int c = 0; c < 4; c++) {
-        const int rc = train_span(h, lr, epoch, off[c], off[c + 1], (RowClass)c, collect, shape, launches, workers, h->stream, &h->counters);
+        const int rc = train_span(h, lr, epoch, off[c], off[c + 1], (RowClass)c, collect, shape, launches, workers, policy_n, h->stream, &h->counters);
         if (rc != MASCOT_OK) return rc;
     }
     return MASCOT_OK;

@@ -540,6 +540,7 @@ struct KernelArgs {
                                       // worker are handed out dynamically, so the launch never depends on
                                       // every block being resident at the same time
     unsigned long long* zero_counter; // another counter, which this launch resets for a later launch
+    uint64_t whole;                   // host only: ratings of the epoch or segment that this launch is a part of
     unsigned hot_user_shift;          // one in 2^this of the updates of a marked user row is written back
 };
 
@@ -1808,11 +1809,16 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
         // again, and MPT loses by it (1.370 and 1.383).
         constexpr bool kLonger = kHalfRows<UM> && kHalfRows<IM>;
         // (a single block has exactly the workers that were asked for: they have to fit it in this form, too)
-        // Grids whose workers have less than two of their first runs each keep the wide form: such a launch is over before its steps count for
-        // much (160,000 ratings, 2,368 workers: 0.046 and 0.037 ms), and what its races leave hangs on how the steps of a single
-        // run fall together - the item factors of two forms differed four times as much as those of two passes of one.
-        const bool worth = STATS || args.s.n >= 2ull * K * workers;
-        if (2 * per_sm <= kMost && (warps > 8 ? worth : 2 * workers <= 8 * kPerWarp))
+        // Grids whose workers have few runs of K ratings each keep the wide form, in all launches of an epoch.  Workers that begin together hold
+        // the same popular items and write them back together, and whose row stays hangs on how the steps fall together: the same from pass to
+        // pass, another in the other form.  Over few runs that does not average out.  Distance of the factors after three trainings of 10
+        // to 12 epochs to those of the wide form, in multiples of what two passes of one form differ by: fp32 SGD, 300,000 ratings, two runs
+        // a worker 8.4; memory quantization, 1.45M, six runs 4.4; MPT, ten runs 3.4; from 16 runs on 1.3 to 2.4 for sets of the
+        // benchmarks' density.  It costs a set of 0.8M ratings of fp32 SGD 0.100 -> 0.132 ms per epoch.  The fixed-point updates, whose
+        // steps differ less between the forms: AFP 6 at one run, 3.4 at 2.6, 2.4 and less from 4 on.
+        constexpr unsigned kRuns = kFixedPoint ? 4 : 16;
+        const bool settled = args.whole >= (uint64_t)kRuns * K * (sms * per_sm * kPerWarp);
+        if (2 * per_sm <= kMost && (warps > 8 ? settled : 2 * workers <= 8 * kPerWarp))
             return launch_ns<K, KIND, UQ, IQ, STATS, NS, kLonger ? 8 : 4, kLonger ? 6 : D, kLonger ? 4 : DI>(args, 2 * per_sm, workers, st, shape, dry);
     }
     // With fp32 rows the deep rings leave room for fewer warps than the registers do (k=128, both sides fp32: 16 per SM
@@ -1884,9 +1890,10 @@ int sm_count() {
 
 cudaError_t launch_train(int K, TrainKind kind, const Stream& s, Arena P, Arena Q, float lr, float lam,
                          const SampleStats* stats, RowClass row_class, unsigned workers, WorkCounters* counters,
-                         int bits, int epoch, bool add_user_delta, unsigned hot_user_shift, cudaStream_t st, LaunchShape* shape) {
+                         int bits, int epoch, bool add_user_delta, unsigned hot_user_shift, uint64_t whole, cudaStream_t st, LaunchShape* shape) {
     KernelArgs a;
     a.hot_user_shift = hot_user_shift;
+    a.whole = whole;
     a.add_user_delta = add_user_delta ? 1 : 0;
     a.s = s; a.P = P; a.Q = Q; a.lr = lr; a.lam = lam; a.workers = workers; a.bits = bits; a.epoch = epoch;
     if (stats) a.st = *stats;

@@ -11,7 +11,7 @@ from test_gpu_update_edges import oracle_epoch, promoted_model
 pytestmark = pytest.mark.gpu
 
 # workers -> form: 1 to 8 (k=64: 16) of a single block are narrow; 9 to 16 (17 to 32), which fit a single block of the wide form only,
-# and grids with less than two runs a worker are wide (their statistics are not, up to 16 warps per SM)
+# and grids with few runs a worker are wide
 WORKERS = (2, 8, 12, 16, 31, 300, 60000)
 
 
@@ -74,18 +74,25 @@ def test_both_lane_forms_of_the_precision_classes(mascot, oracle, k, workers, us
         assert_bit_equal(Qg, Qo, f"n {n} Q")
 
 
+def narrow(k, runs):
+    """(workers, ratings): a single block of narrow workers, or a grid of the fewest with `runs` runs of k ratings each - and 37 ratings more."""
+    import torch
+    workers = 2 * (128 // k) * torch.cuda.get_device_properties(0).multi_processor_count if runs else 8 * (128 // k)
+    return workers, (runs or 5) * k * workers + 37
+
+
 @pytest.mark.parametrize("k", (128, 64))
 @pytest.mark.parametrize("version", ["sgd", "mpt", "memquant", "muppet8", "muppet12", "afp"])
-def test_a_grid_of_narrow_workers(mascot, oracle, k, version):
-    """Two full runs a worker on ratings that share no row, and a remainder; AFP's workers follow the oracle run by run."""
-    import torch
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    workers = 2 * (128 // k) * sms                      # one warp per SM with K/8 lanes, two with K/4
-    n = 2 * k * workers + (0 if version == "afp" else 37)
+def test_many_runs_of_narrow_workers(mascot, oracle, k, version):
+    """Ratings that share no row, in the hands of a single block - of MuPPET a grid of four runs a worker, the fewest that are narrow.
+    AFP: two full runs a worker, which follow the oracle run by run."""
+    muppet = version.startswith("muppet")
+    workers, n = narrow(k, 4 if muppet else 0)
+    if version == "afp":
+        n = 2 * k * workers
     rng = np.random.default_rng(k)
     R, P, Q = random_problem(rng, n, n, n, k, scale=0.2)
     R["u"], R["i"] = rng.permutation(n), rng.permutation(n)
-    muppet = version.startswith("muppet")
     v = dict(sgd=mascot.V_SGD, mpt=mascot.V_MPT, memquant=mascot.V_MEMQUANT, afp=mascot.V_AFP).get(version, mascot.V_MUPPET)
     width = int(version[6:]) if muppet else 0
     cfg = mascot.default_config(version=v, k=k, num_workers=workers, plain_user_stores=1, shuffle=0, epoch=50, learning_rate=0.01, decay=0.1, lam=0.05,
@@ -109,15 +116,33 @@ def test_a_grid_of_narrow_workers(mascot, oracle, k, version):
 
 
 @pytest.mark.parametrize("k", (128, 64))
-@pytest.mark.parametrize("plain_stores", (1, 0))
-@pytest.mark.parametrize("version", ["mascot_hh", "mascot_fh", "mascot_hf", "mascot_ff", "switch"])
-def test_a_grid_of_narrow_workers_of_the_precision_classes(mascot, oracle, k, plain_stores, version):
+def test_a_grid_of_narrow_afp_workers(mascot, oracle, k):
+    """Rows and ratings that are all alike are updated alike, whichever worker has them and whatever it has had before."""
+    workers, n = narrow(k, 4)
+    R, P, Q = random_problem(np.random.default_rng(k), 1, 1, 1, k, scale=0.2)
+    many = np.repeat(R, n)
+    many["u"] = many["i"] = np.arange(n)
+    cfg = mascot.default_config(version=mascot.V_AFP, k=k, num_workers=workers, plain_user_stores=1, epoch=50, learning_rate=0.01, decay=0.1, lam=0.05)
+    with mascot.Engine(cfg) as eng:
+        eng.set_ratings(many, many[:1], n, n)
+        eng.set_factors(np.repeat(P, n, 0), np.repeat(Q, n, 0))
+        assert eng.train_epoch(0).workers == workers
+        Pg, Qg = eng.get_factors(0)
+    oracle.afp_run(k, R, None, P, Q, 0.01, 0.05, 0, int(np.float32((n + workers - 1) // workers) / np.float32(10.0)), oracle.rules_reference())
+    assert_bit_equal(Pg, np.repeat(P, n, 0), "P")
+    assert_bit_equal(Qg, np.repeat(Q, n, 0), "Q")
+
+
+CLASSES = ["mascot_hh", "mascot_fh", "mascot_hf", "mascot_ff", "switch"]
+
+
+@pytest.mark.parametrize("k,runs,plain_stores,version", [(k, 0, s, v) for k in (128, 64) for s in (1, 0) for v in CLASSES]
+                         + [(64, 16, 0, "mascot_hh"), (64, 16, 1, "mascot_fh")])
+def test_many_runs_of_narrow_workers_of_the_precision_classes(mascot, oracle, k, runs, plain_stores, version):
     """Rows that one lane fetches and another one reads, over whole runs, tickets of the shared counter and both ways of
     writing user rows back: ratings that share no row, bit for bit, or within an ulp of the user rows where these are reductions of a
-    change.  More than two runs a worker, so the grid takes K/4 lanes a worker."""
-    import torch
-    workers = 2 * (128 // k) * torch.cuda.get_device_properties(0).multi_processor_count
-    n = 2 * k * workers + 37 * k + 5
+    change.  A single block, and grids of 16 runs a worker, the fewest that are narrow."""
+    workers, n = narrow(k, runs)
     rng = np.random.default_rng(k)
     R, P, Q = random_problem(rng, n, n, n, k, scale=0.2)
     R["u"], R["i"] = rng.permutation(n), rng.permutation(n)
