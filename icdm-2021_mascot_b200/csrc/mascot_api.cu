@@ -329,8 +329,8 @@ int partition_all(mascot_handle* h) {
 
 // log2 of the item-sorted run windows of the resident stream; 0 = none beyond the encode kernel's own windows.
 // The configured length (default 2^20) is shortened to the largest power of two that keeps two properties:
-//   * a window is no longer than the ratings all workers of a launch hold at one time (workers x 8 chunks of
-//     K/8 ratings): with longer windows every worker is on the same few items at once, and since item rows are
+//   * a window is no longer than the ratings all workers of a launch hold at one time (workers x K ratings, the
+//     longest run of one ticket): with longer windows every worker is on the same few items at once, and since item rows are
 //     plain stores most of their updates are lost (100M-rating set, 8,288 workers: windows of 2^20 and 2^22
 //     converge like the unsorted stream, 2^24 needs twice the epochs);
 //   * when statistics are sampled, the sampled tail of every launched range (sample_ratio of a segment) spans
@@ -338,7 +338,7 @@ int partition_all(mascot_handle* h) {
 int run_window_log2(const mascot_handle* h) {
     if (h->cfg.deterministic || !h->cfg.shuffle || h->n_train == 0 || h->n_train >= (1ull << 32) || (h->seg_off.size() - 1) * 4 > 65536) return 0;
     uint32_t w = h->cfg.run_window_log2 ? std::min<uint32_t>(h->cfg.run_window_log2, 32) : 20;
-    uint64_t limit = (uint64_t)worker_count(h, h->n_train) * 8 * (h->K / 8);
+    uint64_t limit = (uint64_t)worker_count(h, h->n_train) * h->K;
     const bool sampled = h->kind == KIND_MIXED || h->kind == KIND_SWITCH || h->kind == KIND_MUPPET;
     if (sampled && h->cfg.sample_ratio > 0.f) {
         uint64_t shortest = ~0ull;

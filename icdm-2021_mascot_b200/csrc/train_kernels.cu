@@ -25,8 +25,8 @@
 //     for an old load also waits for every younger load on the same scoreboard);
 //   * the row of an item that repeats (the stream is item-sorted inside shuffle windows) stays in
 //     registers for the whole run and is written back once;
-//   * chunks are handed out in runs of up to eight through one atomic ticket per run; the runs shrink
-//     to single chunks near the end of the stream, so that all workers finish together.
+//   * chunks are handed out in runs of up to K ratings (eight chunks, or four of K/4 lanes) through one atomic ticket per run; the
+//     runs shrink to single chunks near the end of the stream, so that all workers finish together.
 //   * user rows are written back as vector reductions of their change whenever several workers run,
 //     so racing updates of one user add up instead of overwriting each other (add_row_delta).
 // The item lead is short on purpose.  Between the request of an item row and its write-back (a plain

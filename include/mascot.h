@@ -208,8 +208,9 @@ MASCOT_API int mascot_set_factors(mascot_handle* h, const float* P, const float*
  * Per-worker state of the AFP trainer starts afresh with every launched range.
  * After a promotion, and with more than one worker, the stream is stably re-ordered inside each segment
  * by (user precision, item precision), so that every class runs a kernel instantiation without
- * per-rating precision tests (one launch per class, one after the other; models larger than the GPU's L2 keep
- * their order, see mascot_config.no_class_partition); mascot_stream_source_index / mascot_get_stream_order follow the new order.
+ * per-rating precision tests (one launch per class, one after the other; mascot_config.no_class_partition = 1 leaves
+ * the stream as it is).  Inside a class the ratings keep the order that they had before this promotion.
+ * mascot_stream_source_index / mascot_get_stream_order follow the new order.
  * The deterministic mode never re-orders. */
 MASCOT_API int mascot_train_epoch(mascot_handle* h, uint32_t epoch, mascot_epoch_stats* stats);
 
@@ -277,7 +278,8 @@ MASCOT_API int mascot_set_ratings_sharded(mascot_handle* h, const mascot_rating*
  * the array is uploaded in pieces of 8Mi ratings (beyond two of them the first or the last ones are smaller) on a copy
  * stream while the piece before it is encoded and trained, so the epoch costs max(upload, updates) instead of their sum.  The seeded
  * permutation and the item-sorted windows stay inside a piece; afterwards the pieces are the
- * segments of the resident stream, as after mascot_reload_train.  Ids must be those given to
+ * segments of the resident stream, as after mascot_reload_train - more of them than n_train / 8Mi, and how many
+ * depends on the trainer (mascot_train_segment).  Ids must be those given to
  * mascot_set_ratings (same users/items; checked on the device, MASCOT_ERR_BAD_ARG as for
  * mascot_reload_train); on a check epoch every piece contributes its own sampled tail (see
  * mascot_train_epoch).  The pieces are never re-ordered by precision class (that would need a host wait
@@ -289,7 +291,8 @@ MASCOT_API int mascot_train_epoch_streamed(mascot_handle* h, uint32_t epoch, con
 MASCOT_API int mascot_is_check_epoch(const mascot_handle* h, uint32_t epoch);
 /* Zero the statistic accumulators (start of a check epoch). */
 MASCOT_API int mascot_stats_begin(mascot_handle* h);
-/* Train one segment with lr_schedule[epoch]; with collect_stats != 0 the last sample_ratio of the
+/* Train one segment (of those that the last mascot_set_ratings_sharded or mascot_train_epoch_streamed left, in stream order;
+ * the first number beyond them is MASCOT_ERR_BAD_ARG) with lr_schedule[epoch]; with collect_stats != 0 the last sample_ratio of the
  * segment adds to the statistic accumulators.  With stats == NULL the call does not wait for the
  * kernel (use mascot_sync), so copies on other streams can overlap it. */
 MASCOT_API int mascot_train_segment(mascot_handle* h, uint32_t epoch, uint32_t segment, uint32_t collect_stats,
