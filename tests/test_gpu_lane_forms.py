@@ -1,6 +1,8 @@
 """Workers of K/4 lanes (four elements each) and of K/8 lanes (eight), on both sides of the launch rule: ratings few enough for
 the first run of one worker, in which rows come back at once, so that the sequential oracle has every bit of the result
 and of the sampled statistics."""
+import re
+
 import numpy as np
 import pytest
 
@@ -168,3 +170,37 @@ def test_many_runs_of_narrow_workers_of_the_precision_classes(mascot, oracle, k,
     else:
         assert_within_one_ulp(Pg, P, version in ("mascot_hh", "mascot_hf", "switch"), "P")
     assert_bit_equal(Qg, Q, "Q")
+
+
+def row_modes(call):
+    """How the update kernels that `call` launches spread rows over lanes: ROWS_HALFQ = 3 and ROWS_F32Q = 4 are K/4 lanes a worker."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = [re.search(r"train_kernel<([^>]*)>", e.name) for e in prof.events()]
+    modes = [re.sub(r"\([^)]*\)", "", m.group(1)).split(",")[2:4] for m in names if m]
+    if not modes:
+        pytest.skip("kernels cannot be traced here")
+    return [int(x) for both in modes for x in both]
+
+
+@pytest.mark.parametrize("k", (128, 64))
+@pytest.mark.parametrize("version,runs", [("sgd", 16), ("mpt", 16), ("memquant", 16), ("mascot", 16), ("muppet", 4), ("afp", 4)])
+def test_lines_between_the_forms(mascot, k, version, runs):
+    """Runs of k ratings a worker that make a grid narrow, sampled tails included, and the workers of a single block."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    grid = 2 * (128 // k) * sms
+    v = dict(sgd=mascot.V_SGD, mpt=mascot.V_MPT, memquant=mascot.V_MEMQUANT, mascot=mascot.V_MASCOT, muppet=mascot.V_MUPPET, afp=mascot.V_AFP)[version]
+    for workers, n, narrow_form in ((grid, runs * k * grid - 1, False), (grid, runs * k * grid, True), (8 * (128 // k), 4096, True), (8 * (128 // k) + 1, 4096, False)):
+        R, P, Q = random_problem(np.random.default_rng(n), 3000, 2000, n, k)
+        cfg = mascot.default_config(version=v, k=k, num_workers=workers, epoch=50, learning_rate=0.001, decay=0.1, lam=0.05, muppet_width=8 if version == "muppet" else 0,
+                                    user_group_num=1, item_group_num=1, sample_ratio=0.05, interval=1, error_threshold=1e30)
+        with mascot.Engine(cfg) as eng:
+            eng.set_ratings(R, R[:1], 3000, 2000)
+            eng.set_factors(P, Q)
+            modes = row_modes(lambda: eng.train_epoch(10))
+        assert len(modes) == 2 * (2 if version in ("mascot", "muppet") else 1), "plain launch and sampled tail"
+        assert [m in (3, 4) for m in modes] == [narrow_form] * len(modes)
