@@ -313,8 +313,8 @@ static int partition_by_class(mascot_handle* h) {
 bool wants_partition(const mascot_handle* h) {
     if (!(h->grouped && !h->cfg.deterministic && any_fp32_group(h) && h->n_train < (1ull << 32) && (h->seg_off.size() - 1) * 4 <= 65536)) return false;
     // Measured on one B200, ms per epoch with one launch per class and with one that reads each id's precision bit: 100M
-    // ratings, a fifth of the groups promoted 9.9 and 13.6 to 14.2; 252M, 40 % of them 34.0 and 36 to 40.  In between the one
-    // launch is faster - 63M, 40 % promoted 9.8 and 9.0; 40M 6.9 and 5.5; k=64, 100M 12.7 and 7.2 - but leaves a test RMSE
+    // ratings, a fifth of the groups promoted 10.0 and 13.6 to 14.2; 252M, 40 % of them 34.0 and 36 to 40.  In between the one
+    // launch is faster - 63M, 40 % promoted 9.2 and 9.0; 40M 7.1 and 5.5; k=64, 100M 13.0 and 7.2 - but leaves a test RMSE
     // that is 0.1 % higher after four epochs (0.57343 against 0.57262 at 40M).
     return h->cfg.no_class_partition != 1;
 }

@@ -1823,11 +1823,10 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
     }
     // With fp32 rows the deep rings leave room for fewer warps than the registers do (k=128, both sides fp32: 16 per SM
     // against 24).  Where a launch of a mixed-precision class with an fp32 side asks for more workers than the deep rings hold and
-    // rings of 4 + 2 slots hold more, it takes these, three ratings and one ahead, and has the workers.  The time is the same
-    // within a hundredth - ms per epoch, deep rings for all classes and this rule: 40 % of the groups promoted, 40M ratings 4.11 and
-    // 4.14, 63M 7.09 and 7.17, 252M 30.3 to 32.1 and 30.7 to 32.0, k=64 100M 6.56 and 6.54; 100M (a fifth) 8.60 and 8.57; all
-    // promoted, 63M 7.42 and 7.49 - as for the other trainers, which do without (SGD 7.73 and 7.74 at 63M, 10.53 and 10.58 at
-    // 100M): full GPUs are bound by what the rows' traffic allows.
+    // rings of 4 + 2 slots hold more, it takes these, three ratings and one ahead, and has the workers, which wait for rows that others have
+    // just written.  ms per epoch, deep rings for all classes and this rule: 40 % of the groups promoted, 40M ratings 7.12 and
+    // 7.11, 63M 9.37 and 9.20, k=64 100M 13.93 and 12.96; 100M (a fifth) 10.38 and 9.99; all promoted, 63M 10.97 and 10.72.  The other
+    // trainers do without (SGD 7.73 and 7.74 at 63M, 10.53 and 10.58 at 100M): they are bound by what the rows' traffic allows.
     constexpr bool kShortRings = KIND == KIND_MIXED && !STATS && UM != ROWS_DYN && (UM == ROWS_F32 || IM == ROWS_F32);
     if constexpr (kShortRings) {
         LaunchShape deep, shallow;
