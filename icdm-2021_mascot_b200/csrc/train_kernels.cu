@@ -37,13 +37,13 @@
 // took 1.39 with five and three, the k=64 one 1.97 against 1.65; user leads of six and seven gave nothing more.
 //
 // WHAT BOUNDS IT (one B200, k=128).  Sets with few workers per SM (8M ratings: two warps per scheduler, a worker each): the chain of
-// one update - dot product, its sum over the lanes, update - and the 76 instructions around it, 2.42 -> 1.18 ms per epoch (338 cycles a
+// one update - dot product, its sum over the lanes, update - and the 77 instructions around it, 2.42 -> 1.18 ms per epoch (340 cycles a
 // rating: 1.5 cycles an instruction wait for results of fixed latency, 0.6 for shared memory and shuffles, 0.5 for L2).  The
 // same with fp32 rows 1.24 ms (1.52 with K/8 lanes a worker), and with 278 instructions for 4M ratings of AFP 3.37 (5.69).  Full SMs
-// (100M ratings, 7.17 -> 5.50 ms): the traffic between SMs and L2.  The launches that fill the GPU all move 9.9 to 10.5
+// (100M ratings, 7.17 -> 5.50 ms): the traffic between SMs and L2.  The launches that fill the GPU all move 9.9 to 10.2
 // TB/s of row reads, stores and reductions (reads alone: 16 to 17.7), whatever else they do: 100M and 126M ratings with
 // binary16 rows (541 and 621 bytes an update), 63M with fp32 rows on both sides (SGD, 1,230 bytes; the fp32 class of a
-// promoted set, 1,210), with 71 down to 39 % of the issue slots busy and 16 to 28 warps per SM.  Nothing but random rows read with
+// promoted set, 1,580), with 71 down to 35 % of the issue slots busy and 16 to 28 warps per SM.  Nothing but random rows read with
 // cp.async and reduced runs at 17.4e9 binary16 or 9.0e9 fp32 rows/s (20 MB of rows; 16.8 and 8.4 with 127 MB), a reduction
 // alone at 24.5e9 and 12.0e9: the 100M-rating set, 18.1e9 updates/s, is there.
 //
