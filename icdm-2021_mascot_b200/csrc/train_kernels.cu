@@ -1797,7 +1797,7 @@ cudaError_t launch_one(const KernelArgs& args, unsigned workers, cudaStream_t st
     // epoch with K/8 and K/4 lanes, by warps of the narrow form per SM: AFP 4M ratings (4) 5.69 and 3.37, 12M (10) 8.94 and 5.17; MuPPET,
     // 8 bits, 2M (4) 2.25 and 1.13, 14M (12) 5.73 and 4.08; MPT 8M (8) 1.81 and 1.37, 18M (16) 2.38 and 2.16; SGD 8M (8) 1.52 and
     // 1.24, 16M (14) 2.08 and 1.92, k=64 0.8M (6) 0.132 and 0.100, 20M (10) 2.04 and 1.64; fp16 storage 8M 1.64 and 1.47, 16M (14) 2.13 and
-    // 2.04; MASCOT k=64 8M (4) 1.44 and 1.19, 20M (10) 1.56 and 1.41, 30M (14) 1.73 and 1.66, 40 % promoted, 16M (14) 2.25 and 2.18.  At 18 and
+    // 2.04; MASCOT k=64 8M (4) 1.44 and 1.19, 20M (10) 1.56 and 1.41, 30M (14) 1.73 and 1.66, 40 % promoted, 8M (8) 2.93 and 2.74, 16M (14) 3.80 and 3.81.  At 18 and
     // more the narrow form gives nothing more (SGD 20M 2.32 and 2.32) or loses (fp16 storage 20M 2.08 and 2.23).  Binary16 rows with
     // packed binary16 arithmetic have the shortest steps and stop gaining earlier: k=128, 2M (4) 0.637 and 0.531, 8M (8) 1.302 and
     // 1.184, 14M (12) 1.646 and 1.565, 16M (14) 1.659 and 1.671, 20M (18) 1.66 and 1.91.
